@@ -240,9 +240,6 @@ static __device__ __noinline__ bool solve_proved_x(const SceneDev& S, const ObjI
 // is in flight per CTA.
 template <bool MULTI>
 __global__ void __launch_bounds__(256, LG_SOLVE_X_BLOCKS) k_solve_x(SceneDev S, TraceBufs B, uint32_t gen) {
-  __shared__ unsigned long long blk_solves;
-  if (threadIdx.x == 0) blk_solves = 0;
-  __syncthreads();
   uint64_t off[LIST_FULL + 2];
   off[0] = 0;
   for (int l = 0; l <= LIST_FULL; ++l) {
@@ -250,8 +247,9 @@ __global__ void __launch_bounds__(256, LG_SOLVE_X_BLOCKS) k_solve_x(SceneDev S, 
     off[l + 1] = off[l] + (c < B.queue_cap ? c : B.queue_cap);
   }
   const uint64_t total = off[LIST_FULL + 1];
+  if ((uint64_t)blockIdx.x * blockDim.x >= total) return;  // no ray for this CTA
   const RayRec* q = B.queue[gen & 1];
-  unsigned long long my_solves = 0;
+  uint32_t my_solves = 0;
   // block-uniform loop (the class barrier needs every thread)
   for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x; base < total; base += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t i = base + threadIdx.x;
@@ -342,9 +340,7 @@ __global__ void __launch_bounds__(256, LG_SOLVE_X_BLOCKS) k_solve_x(SceneDev S, 
     }
     store_hit_x(B.hit[idx], best, bh, n, leaf, ev, fl);
   }
-  atomicAdd(&blk_solves, my_solves);
-  __syncthreads();
-  if (threadIdx.x == 0) atomicAdd(&B.ctr->fp64_solves, blk_solves);
+  add_block_counts<1>({my_solves}, {&B.ctr->fp64_solves});
 }
 template __global__ void k_solve_x<false>(SceneDev, TraceBufs, uint32_t);
 template __global__ void k_solve_x<true>(SceneDev, TraceBufs, uint32_t);
@@ -585,7 +581,7 @@ __device__ __forceinline__ void bounce_x(const SceneDev& S, const RayRec& r, con
 
 // appends one segment per emitting lane with one atomic per warp (all lanes call)
 __device__ __forceinline__ void emit_segments_x(const SceneDev& S, const TraceBufs& B, const BounceX& v,
-                                                const RayRec& r, unsigned long long& my_near) {
+                                                const RayRec& r, uint32_t& my_near) {
   const unsigned lane = lane_id();
   const unsigned emask = __ballot_sync(0xffffffffu, v.emit);
   if (!emask) return;
@@ -611,9 +607,6 @@ __device__ __forceinline__ void emit_segments_x(const SceneDev& S, const TraceBu
 
 template <bool MULTI, bool CULL>
 __global__ void __launch_bounds__(256, LG_BOUNCE_X_BLOCKS) k_bounce_x(SceneDev S, TraceBufs B, uint32_t gen) {
-  __shared__ unsigned long long blk_visits, blk_near;
-  if (threadIdx.x == 0) { blk_visits = 0; blk_near = 0; }
-  __syncthreads();
   // the rays with work: every work list of this generation, one after the other
   uint64_t off[N_LISTS + 1];
   off[0] = 0;
@@ -622,12 +615,13 @@ __global__ void __launch_bounds__(256, LG_BOUNCE_X_BLOCKS) k_bounce_x(SceneDev S
     off[l + 1] = off[l] + (c < B.queue_cap ? c : B.queue_cap);
   }
   const uint64_t total = off[N_LISTS];
+  if ((uint64_t)blockIdx.x * blockDim.x >= total) return;  // no ray for this CTA
   const RayRec* qin = B.queue[gen & 1];
   RayRec* qout = B.queue[(gen + 1) & 1];
   const unsigned lane = lane_id();
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
-  unsigned long long my_visits = 0, my_near = 0;
+  uint32_t my_visits = 0, my_near = 0;
   for (uint64_t base = warp * 32; base < total; base += nwarps * 32) {
     const uint64_t i = base + lane;
     BounceX v;
@@ -663,13 +657,7 @@ __global__ void __launch_bounds__(256, LG_BOUNCE_X_BLOCKS) k_bounce_x(SceneDev S
         if (first + q < B.queue_cap) qout[first + q] = v.child[q];
     }
   }
-  atomicAdd(&blk_visits, my_visits);
-  atomicAdd(&blk_near, my_near);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    atomicAdd(&B.ctr->visits, blk_visits);
-    atomicAdd(&B.ctr->near, blk_near);
-  }
+  add_block_counts<2>({my_visits, my_near}, {&B.ctr->visits, &B.ctr->near});
 }
 template __global__ void k_bounce_x<false, false>(SceneDev, TraceBufs, uint32_t);
 template __global__ void k_bounce_x<false, true>(SceneDev, TraceBufs, uint32_t);

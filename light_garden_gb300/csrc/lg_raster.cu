@@ -17,6 +17,7 @@
 #include <type_traits>
 
 #include "lg_kernels.cuh"
+#include "lg_trace_common.cuh"
 
 namespace lgd {
 
@@ -504,14 +505,13 @@ __global__ void __launch_bounds__(256, 4) k_raster(RasterArgs A) {
   Staged* stage_all = reinterpret_cast<Staged*>(smem_raw + RasterSmem<MODE>::acc_words * 4);
   uint8_t* owner_all = reinterpret_cast<uint8_t*>(stage_all + 8 * 32);
   int* pref_all = reinterpret_cast<int*>(owner_all + 8 * 1024);
-  __shared__ unsigned long long s_unit, s_pixels;
-  if (threadIdx.x == 0) s_pixels = 0;
+  __shared__ unsigned long long s_unit;
   const unsigned lane = lane_id(), warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   Staged* stage = stage_all + warp * 32;
   uint8_t* owner = owner_all + warp * 1024;
   int* pref = pref_all + warp * 33;
   const BlendDev& B = A.blend;
-  unsigned long long my_pixels = 0;
+  uint32_t my_pixels = 0;
   unsigned long long n_units = A.ctr->units;
   if (n_units > A.units_cap) n_units = A.units_cap;
   for (;;) {
@@ -697,9 +697,7 @@ __global__ void __launch_bounds__(256, 4) k_raster(RasterArgs A) {
     }
     __syncthreads();
   }
-  atomicAdd(&s_pixels, my_pixels);
-  __syncthreads();
-  if (threadIdx.x == 0) atomicAdd(&A.ctr->pixels, s_pixels);
+  add_block_counts<1>({my_pixels}, {&A.ctr->pixels});
 }
 
 // One warp per unit with a private tile: lane L owns pixel column L of the tile (x-major
@@ -721,7 +719,7 @@ __global__ void __launch_bounds__(32) k_raster_warp(RasterArgs A) {
   St* stage = reinterpret_cast<St*>(smem_raw + 4 * TILE_PX * 8);
   const unsigned lane = lane_id();
   const BlendDev& B = A.blend;
-  unsigned long long my_pixels = 0;
+  uint32_t my_pixels = 0;
   unsigned long long n_units = A.ctr->units;
   if (n_units > A.units_cap) n_units = A.units_cap;
   for (;;) {
@@ -836,7 +834,7 @@ __global__ void __launch_bounds__(32) k_raster_warp(RasterArgs A) {
     }
     __syncwarp();
   }
-  if (my_pixels) atomicAdd(&A.ctr->pixels, my_pixels);
+  add_block_counts<1>({my_pixels}, {&A.ctr->pixels});
 }
 
 template __global__ void k_raster_warp<RM_FIXED_SPLIT>(RasterArgs A);
@@ -853,7 +851,7 @@ __global__ void __launch_bounds__(256) k_raster_chords(RasterArgs A, const lg_ch
   const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   const BlendDev& B = A.blend;
   const float sc = (float)A.H * 0.5f, cx = (float)A.W * 0.5f;
-  unsigned long long my_pixels = 0;
+  uint32_t my_pixels = 0;
   for (uint64_t k = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; k < n; k += nw) {
     const lg_chord c = chords[k];
     lg_segment sg;
@@ -907,7 +905,7 @@ __global__ void __launch_bounds__(256) k_raster_chords(RasterArgs A, const lg_ch
       ++my_pixels;
     }
   }
-  if (my_pixels) atomicAdd(&A.ctr->pixels, my_pixels);
+  add_block_counts<1>({my_pixels}, {&A.ctr->pixels});
 }
 
 template __global__ void k_raster_chords<true>(RasterArgs A, const lg_chord* chords, uint64_t n);

@@ -182,7 +182,7 @@ __device__ __forceinline__ bool fast_canvas_exit(const df aspect, const RayRec& 
 // appends one segment per emitting lane with one atomic per warp (all lanes call)
 __device__ __forceinline__ void emit_segments(const SceneDev& S, const TraceBufs& B, bool emit, const RayRec& r,
                                               float x1, float y1, uint8_t flags, int hit,
-                                              unsigned long long& my_near, unsigned long long& my_ill) {
+                                              uint32_t& my_near, uint32_t& my_ill) {
   const unsigned lane = lane_id();
   const unsigned emask = __ballot_sync(0xffffffffu, emit);
   if (!emask) return;
@@ -259,15 +259,17 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, CULL ? SCAN_CULL_BLOCKS : 4)
   __shared__ __align__(8) uint64_t bar;
   ScanSmem& W = *reinterpret_cast<ScanSmem*>(smem_raw);
   ObjScan* sobj = reinterpret_cast<ObjScan*>(smem_raw + sizeof(ScanSmem));
-  __shared__ unsigned long long blk_visits, blk_near, blk_ill, blk_tests, blk_cls;
-  if (threadIdx.x == 0) { blk_visits = 0; blk_near = 0; blk_ill = 0; blk_tests = 0; blk_cls = 0; }
-  unsigned long long my_visits = 0, my_near = 0, my_ill = 0;
+  const uint64_t n_real = n_real_of(S, B, gen);
+  const uint64_t n_in = n_in_of(S, B, gen);
+  if ((uint64_t)blockIdx.x * blockDim.x >= n_in) return;  // no ray for this CTA
+  __shared__ uint32_t cls_count[SCAN_WARPS];  // classifications, one count per warp
+  if (lane_id() == 0) cls_count[threadIdx.x >> 5] = 0;
+  __syncwarp();
+  uint32_t my_visits = 0, my_near = 0, my_ill = 0;
   uint32_t my_tests = 0;
   bool failed;
   const ObjScan* objs = stage_objects(S, sobj, &bar, !MULTI && smem_fits != 0, B.ctr, failed);
   if (failed) return;
-  const uint64_t n_real = n_real_of(S, B, gen);
-  const uint64_t n_in = n_in_of(S, B, gen);
   RayRec* q = B.queue[gen & 1];
   const unsigned lane = lane_id(), w = threadIdx.x >> 5;
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
@@ -369,7 +371,7 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, CULL ? SCAN_CULL_BLOCKS : 4)
         W.off[w][lane] = incl - cnt;
         if (lane == 31) {
           W.off[w][32] = incl;
-          if (incl) atomicAdd(&blk_cls, (unsigned long long)incl);
+          cls_count[w] += (uint32_t)incl;
         }
         __syncwarp();
         const int total = W.off[w][32];
@@ -615,18 +617,13 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, CULL ? SCAN_CULL_BLOCKS : 4)
     }
     emit_segments(S, B, emit, r, x1, y1, eflags, -1, my_near, my_ill);
   }
-  atomicAdd(&blk_visits, my_visits);
-  atomicAdd(&blk_near, my_near);
-  atomicAdd(&blk_ill, my_ill);
-  atomicAdd(&blk_tests, (unsigned long long)my_tests);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    atomicAdd(&B.ctr->visits, blk_visits);
-    atomicAdd(&B.ctr->near, blk_near);
-    atomicAdd(&B.ctr->ill, blk_ill);
-    atomicAdd(&B.ctr->bound_tests, blk_tests);
-    atomicAdd(&B.ctr->object_tests, blk_cls);
-  }
+  __syncwarp();
+  const uint32_t my_cls = lane_id() == 0 ? cls_count[w] : 0u;
+  if (EXACT)  // every visit is counted by the bounce
+    add_block_counts<2>({my_tests, my_cls}, {&B.ctr->bound_tests, &B.ctr->object_tests});
+  else
+    add_block_counts<5>({my_tests, my_cls, my_visits, my_near, my_ill},
+                        {&B.ctr->bound_tests, &B.ctr->object_tests, &B.ctr->visits, &B.ctr->near, &B.ctr->ill});
 }
 
 template __global__ void k_scan<false, false, false, 8>(SceneDev, TraceBufs, uint32_t, int);
@@ -691,16 +688,15 @@ template <bool MULTI>
 __global__ void __launch_bounds__(256, 2) k_full(SceneDev S, TraceBufs B, uint32_t gen, int smem_fits) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar;
-  __shared__ unsigned long long blk_solves;
-  if (threadIdx.x == 0) blk_solves = 0;
+  unsigned long long n = B.ctr->list_count[gen][LIST_FULL];
+  if (n > B.queue_cap) n = B.queue_cap;
+  if ((uint64_t)blockIdx.x * blockDim.x >= n) return;  // no ray for this CTA
   bool failed;
   const ObjScan* objs = stage_objects(S, reinterpret_cast<ObjScan*>(smem_raw), &bar, !MULTI && smem_fits != 0, B.ctr,
                                       failed);
   if (failed) return;
-  unsigned long long n = B.ctr->list_count[gen][LIST_FULL];
-  if (n > B.queue_cap) n = B.queue_cap;
   const RayRec* q = B.queue[gen & 1];
-  unsigned long long my_solves = 0;
+  uint32_t my_solves = 0;
   // block-uniform loop: the CTA's warps solve one class at a time together (a barrier
   // between classes), so that one solver's code is in flight per CTA
   for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x; base < n; base += (uint64_t)gridDim.x * blockDim.x) {
@@ -770,9 +766,7 @@ __global__ void __launch_bounds__(256, 2) k_full(SceneDev S, TraceBufs B, uint32
       fl |= LG_PATH_NEAR_DEGENERATE;
     store_hit(B.hit[idx], best, bh, ev.ev, fl);
   }
-  atomicAdd(&blk_solves, my_solves);
-  __syncthreads();
-  if (threadIdx.x == 0) atomicAdd(&B.ctr->fp64_solves, blk_solves);
+  add_block_counts<1>({my_solves}, {&B.ctr->fp64_solves});
 }
 template __global__ void k_full<false>(SceneDev, TraceBufs, uint32_t, int);
 template __global__ void k_full<true>(SceneDev, TraceBufs, uint32_t, int);
@@ -972,12 +966,6 @@ template <bool MULTI, bool CULL>
 __global__ void __launch_bounds__(256, 3) k_bounce(SceneDev S, TraceBufs B, uint32_t gen, int smem_fits) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar;
-  __shared__ unsigned long long blk_visits, blk_near, blk_ill;
-  if (threadIdx.x == 0) { blk_visits = 0; blk_near = 0; blk_ill = 0; }
-  bool failed;
-  const ObjScan* objs = stage_objects(S, reinterpret_cast<ObjScan*>(smem_raw), &bar, !MULTI && smem_fits != 0, B.ctr,
-                                      failed);
-  if (failed) return;
   // the rays with work: every work list of this generation, one after the other
   uint64_t off[N_LISTS + 1];
   off[0] = 0;
@@ -986,12 +974,17 @@ __global__ void __launch_bounds__(256, 3) k_bounce(SceneDev S, TraceBufs B, uint
     off[l + 1] = off[l] + (c < B.queue_cap ? c : B.queue_cap);
   }
   const uint64_t total = off[N_LISTS];
+  if ((uint64_t)blockIdx.x * blockDim.x >= total) return;  // no ray for this CTA
+  bool failed;
+  const ObjScan* objs = stage_objects(S, reinterpret_cast<ObjScan*>(smem_raw), &bar, !MULTI && smem_fits != 0, B.ctr,
+                                      failed);
+  if (failed) return;
   const RayRec* qin = B.queue[gen & 1];
   RayRec* qout = B.queue[(gen + 1) & 1];
   const unsigned lane = lane_id();
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
-  unsigned long long my_visits = 0, my_near = 0, my_ill = 0;
+  uint32_t my_visits = 0, my_near = 0, my_ill = 0;
   for (uint64_t base = warp * 32; base < total; base += nwarps * 32) {
     const uint64_t i = base + lane;
     Bounce v;
@@ -1029,15 +1022,7 @@ __global__ void __launch_bounds__(256, 3) k_bounce(SceneDev S, TraceBufs B, uint
         if (first + q < B.queue_cap) qout[first + q] = v.child[q];
     }
   }
-  atomicAdd(&blk_visits, my_visits);
-  atomicAdd(&blk_near, my_near);
-  atomicAdd(&blk_ill, my_ill);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    atomicAdd(&B.ctr->visits, blk_visits);
-    atomicAdd(&B.ctr->near, blk_near);
-    atomicAdd(&B.ctr->ill, blk_ill);
-  }
+  add_block_counts<3>({my_visits, my_near, my_ill}, {&B.ctr->visits, &B.ctr->near, &B.ctr->ill});
 }
 template __global__ void k_bounce<false, false>(SceneDev, TraceBufs, uint32_t, int);
 template __global__ void k_bounce<false, true>(SceneDev, TraceBufs, uint32_t, int);
