@@ -714,7 +714,7 @@ def main():
                     help="primary stride of the CPU samples (0: the workload's default)")
     ap.add_argument("--no-extras", action="store_true", help="only the headline frame")
     ap.add_argument("--raster-variant", type=int, default=0, choices=[0, 1, 2],
-                    help="0: autotuned; 1: shared-memory tile atomics; 2: warp-private tiles")
+                    help="kept for its numbering: every value runs the one tile raster")
     ap.add_argument("--culling", default="auto", choices=sorted(CULL),
                     help="nearest-hit culling grid: auto (scenes of 96+ objects), off, on")
     ap.add_argument("--grid-density", type=float, default=0.0, help="culling grid cells per object (0: 2)")

@@ -149,7 +149,9 @@ typedef struct lg_blend_component {
 
 enum lg_accum_mode {
   LG_ACCUM_FIXED64 = 0, /* signed Q31.32 fixed point in int64: order-independent, bit-reproducible */
-  LG_ACCUM_F32 = 1      /* FP32 atomics: faster to reason about, not bit-reproducible */
+  LG_ACCUM_F32 = 1      /* FP32 values: additive sums are kept in FP64 and rounded to FP32 when
+                           the image is read (lg_accumulate_segments_noalloc: FP32 atomics, not
+                           bit-reproducible) */
 };
 
 /* ---- string-mod overlay (src/light_garden/string_mod.rs) ------------------------------- */
@@ -308,8 +310,8 @@ typedef struct lg_trace_stats {
 
 typedef struct lg_device_opts {
   int32_t device;             /* CUDA device ordinal */
-  int32_t raster_variant;     /* 0: autotune on the first accumulation; 1: shared-atomic tile
-                                 raster; 2: warp-private tile raster (results are identical) */
+  int32_t raster_variant;     /* kept for numbering: one tile raster serves every accumulation,
+                                 whatever the value */
   uint64_t segment_capacity;  /* initial segment ring size (0 = automatic); grows on overflow */
   uint64_t queue_capacity;    /* initial per-generation ray queue size (0 = automatic) */
   uint64_t stream_segments;   /* lg_render accumulates while tracing, with a ring of this many
@@ -422,8 +424,7 @@ lg_status lg_batch_upload(lg_ctx* ctx, const lg_scene_desc* scenes, uint32_t k);
 /* Traces, accumulates and resolves every scene of the batch (one captured CUDA graph).
  * dst receives the RGBA16F images one after another in scene order, each width*height*4
  * binary16 values with rows top-down and no padding; dst_bytes >= 8 * sum(width*height).
- * Each image is bit-identical to lg_render of that scene alone.  The first call of a
- * context also picks the faster tile-raster kernel for the batch (autotune). */
+ * Each image is bit-identical to lg_render of that scene alone. */
 lg_status lg_batch_render(lg_ctx* ctx, uint16_t* dst, uint64_t dst_bytes, int32_t dst_is_device,
                           lg_trace_stats* stats_or_null);
 

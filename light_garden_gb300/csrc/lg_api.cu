@@ -517,12 +517,22 @@ uint64_t sampled_rays(uint64_t num_rays, const lg_params& p) {
   return num_rays > p.ray_offset ? (num_rays - p.ray_offset + p.ray_stride - 1) / p.ray_stride : 0;
 }
 
+// What a context's accumulation image holds: int64 sums in fixed point; in F32 mode FP64 sums,
+// rounded to FP32 when the image is read (FP32 sums of a few hundred segments a pixel carry a
+// rounding each, in the order of the atomics), or FP32 values with a min / max blend, whose
+// terms are never rounded.
+int accum_kind(const lg_params& p) {
+  if (p.accum == LG_ACCUM_FIXED64) return ACC_I64;
+  return raster_mode(p) == RM_F32_ ? ACC_F64 : ACC_F32;
+}
+size_t accum_px_bytes(const lg_params& p) { return accum_kind(p) == ACC_F32 ? 16 : 32; }
+
 int raster_mode(const lg_params& p) {
-  if (p.accum == LG_ACCUM_F32) return RM_F32_;
+  const bool f32 = p.accum == LG_ACCUM_F32;
   const lg_blend_component* b[2] = {&p.color_blend, &p.alpha_blend};
   for (const lg_blend_component* x : b)
-    if (x->op == LG_BO_MIN || x->op == LG_BO_MAX) return RM_FIXED_MINMAX_;
-  return RM_FIXED_SPLIT_;
+    if (x->op == LG_BO_MIN || x->op == LG_BO_MAX) return f32 ? RM_F32_MINMAX_ : RM_FIXED_MINMAX_;
+  return f32 ? RM_F32_ : RM_FIXED_SPLIT_;
 }
 
 void to_device_leaves(const std::vector<LeafH>& in, std::vector<Leaf64>& out) {
@@ -633,7 +643,9 @@ RasterArgs raster_args(lg_ctx* c) {
   A.ntx = c->ntx;
   A.nty = c->nty;
   A.n_tiles = 2 * c->n_tiles;  // bins: x-major and y-major segments of each tile
-  A.unit_refs = c->raster_variant == 2 ? UNIT_REFS_WARP : UNIT_REFS;
+  A.unit_refs = raster_unit_refs(raster_mode(c->prm));
+  A.acc = accum_kind(c->prm);
+  A.unit_share = 3u * (uint32_t)c->raster_grid;
   for (int ch = 0; ch < 4; ++ch) {
     const lg_blend_component& b = ch < 3 ? c->prm.color_blend : c->prm.alpha_blend;
     A.blend.src[ch] = b.src_factor;
@@ -706,8 +718,7 @@ void launch_bin_count(lg_ctx* c, const RasterArgs& A, int smem_tiles, size_t bsm
 lg_status ensure_raster_buffers(lg_ctx* c) {
   lg_status st;
   const uint64_t px = (uint64_t)c->prm.width * c->prm.height;
-  const size_t elem = c->prm.accum == LG_ACCUM_F32 ? 4 : 8;
-  if ((st = ensure(c, c->d_accum, px * 4 * elem, "accumulation image"))) return st;
+  if ((st = ensure(c, c->d_accum, px * accum_px_bytes(c->prm), "accumulation image"))) return st;
   const size_t bins = 2 * (size_t)c->n_tiles;
   if ((st = ensure(c, c->d_tile_count, bins * 4, "tile counts"))) return st;
   if ((st = ensure(c, c->d_tile_off, bins * 8, "tile offsets"))) return st;
@@ -954,10 +965,11 @@ lg_status stage_event(lg_ctx* c, int i) {
 // binned_event >= 0 records that stage event between binning and the tile raster
 lg_status enqueue_accumulate(lg_ctx* c, int binned_event = -1) {
   const RasterArgs A = raster_args(c);
-  const int fixed = c->prm.accum == LG_ACCUM_FIXED64;
-  k_clear_accum<<<c->n_sm * 8, 256, 0, c->stream>>>(A, fixed);
+  const int acc = accum_kind(c->prm);
+  k_clear_accum<<<c->n_sm * 8, 256, 0, c->stream>>>(A);
   CK(cudaMemsetAsync(c->d_tile_count.p, 0, (size_t)c->n_tiles * 8, c->stream), "memset tile counts");
-  CK(cudaMemsetAsync(&((Counters*)c->d_ctr.p)->pixels, 0, sizeof(unsigned long long), c->stream), "memset pixels");
+  // pixels and, right after it, bin_refs
+  CK(cudaMemsetAsync(&((Counters*)c->d_ctr.p)->pixels, 0, 2 * sizeof(unsigned long long), c->stream), "memset pixels");
   const uint32_t bins = 2 * c->n_tiles;
   const int smem_tiles = bins <= MAX_SMEM_TILES ? 1 : 0;
   const size_t bsm = smem_tiles ? (size_t)bins * 4 : 0;
@@ -969,27 +981,15 @@ lg_status enqueue_accumulate(lg_ctx* c, int binned_event = -1) {
     lg_status st = stage_event(c, binned_event);
     if (st) return st;
   }
-  const int mode = raster_mode(c->prm);
-  const size_t rsm = (size_t)raster_smem_bytes(mode);
-  if (c->raster_variant == 2) {
-    if (mode == RM_F32_)
-      k_raster_warp<RM_F32_><<<c->raster_warp_grid, 32, raster_warp_smem_bytes(), c->stream>>>(A);
-    else
-      k_raster_warp<RM_FIXED_SPLIT_><<<c->raster_warp_grid, 32, raster_warp_smem_bytes(), c->stream>>>(A);
-  } else if (mode == RM_FIXED_SPLIT_)
-    k_raster<RM_FIXED_SPLIT_><<<c->raster_grid, 256, rsm, c->stream>>>(A);
-  else if (mode == RM_FIXED_MINMAX_)
-    k_raster<RM_FIXED_MINMAX_><<<c->raster_grid, 256, rsm, c->stream>>>(A);
-  else
-    k_raster<RM_F32_><<<c->raster_grid, 256, rsm, c->stream>>>(A);
+  launch_raster(raster_mode(c->prm), c->raster_grid, c->stream, A);
   launch_chords(c, A);
   CK(cudaGetLastError(), "accumulate launch");
   return LG_OK;
 }
 
 lg_status enqueue_resolve(lg_ctx* c, uint16_t* dst, size_t pitch) {
-  const int fixed = c->prm.accum == LG_ACCUM_FIXED64;
-  k_resolve_f16<<<c->n_sm * 8, 256, 0, c->stream>>>(c->d_accum.p, fixed, c->prm.width, c->prm.height, dst, pitch);
+  const int acc = accum_kind(c->prm);
+  k_resolve_f16<<<c->n_sm * 8, 256, 0, c->stream>>>(c->d_accum.p, acc, c->prm.width, c->prm.height, dst, pitch);
   CK(cudaGetLastError(), "resolve launch");
   return LG_OK;
 }
@@ -1065,37 +1065,7 @@ lg_status run_trace_once(lg_ctx* c, uint32_t& retries, uint64_t seg_limit) {
   return fail(c, LG_ERR_OUT_OF_MEMORY, "segment ring / ray queue kept overflowing");
 }
 
-lg_status run_accumulate_once(lg_ctx* c, uint32_t& retries);
-
-// Autotuner: the first accumulation of a context runs both tile-raster kernels (each a
-// complete, identical accumulation) and keeps the faster for every later launch and graph.
-lg_status tune_raster(lg_ctx* c, uint32_t& retries) {
-  float best = INFINITY;
-  int pick = 1;
-  for (int v = 1; v <= 2; ++v) {
-    c->raster_variant = v;
-    CK(cudaEventRecord(c->ev[4], c->stream), "event");
-    lg_status st = run_accumulate_once(c, retries);
-    if (st) return st;
-    CK(cudaEventRecord(c->ev[5], c->stream), "event");
-    CK(cudaEventSynchronize(c->ev[5]), "event");
-    const float ms = elapsed(c->ev[4], c->ev[5]);
-    if (ms < best) { best = ms; pick = v; }
-  }
-  c->graph_valid = false;
-  if (c->raster_variant != pick) {
-    c->raster_variant = pick;
-    return run_accumulate_once(c, retries);
-  }
-  return LG_OK;
-}
-
 lg_status run_accumulate(lg_ctx* c, uint32_t& retries) {
-  if (c->raster_variant == 0) return tune_raster(c, retries);
-  return run_accumulate_once(c, retries);
-}
-
-lg_status run_accumulate_once(lg_ctx* c, uint32_t& retries) {
   for (int attempt = 0; attempt < 4; ++attempt) {
     lg_status st = enqueue_accumulate(c);
     if (st) return st;
@@ -1150,7 +1120,6 @@ lg_status lg_create(lg_ctx** out, const lg_device_opts* opts) {
   if (!c) return LG_ERR_OUT_OF_MEMORY;
   c->device = opts ? opts->device : 0;
   c->seg_cap_hint = opts ? opts->segment_capacity : 0;
-  c->raster_variant = opts && (opts->raster_variant == 1 || opts->raster_variant == 2) ? opts->raster_variant : 0;
   c->queue_cap_hint = opts ? opts->queue_capacity : 0;
   if (opts && opts->stream_segments) c->stream_ring = opts->stream_segments;
   if (opts && (opts->culling < LG_CULL_AUTO || opts->culling > LG_CULL_ON || !(opts->grid_density >= 0.0f))) {
@@ -1343,22 +1312,8 @@ lg_status lg_scene_upload(lg_ctx* c, const lg_geo* geos, uint32_t n_geo, const l
   }
   if ((st = scan_grid(c, false))) return st;
   if ((st = trace_grids(c, false, tsm))) return st;
-  const int mode = raster_mode(p);
-  const int rsm = raster_smem_bytes(mode);
-  if (mode == RM_FIXED_SPLIT_) {
-    CK(cudaFuncSetAttribute(k_raster<RM_FIXED_SPLIT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, rsm), "smem attr");
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_raster<RM_FIXED_SPLIT_>, 256, rsm), "occupancy");
-  } else if (mode == RM_FIXED_MINMAX_) {
-    CK(cudaFuncSetAttribute(k_raster<RM_FIXED_MINMAX_>, cudaFuncAttributeMaxDynamicSharedMemorySize, rsm), "smem attr");
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_raster<RM_FIXED_MINMAX_>, 256, rsm), "occupancy");
-  } else {
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_raster<RM_F32_>, 256, rsm), "occupancy");
-  }
+  CK(raster_occupancy(raster_mode(p), &occ), "occupancy");
   c->raster_grid = c->n_sm * std::max(1, occ);
-  CK(cudaFuncSetAttribute(k_raster_warp<RM_FIXED_SPLIT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, raster_warp_smem_bytes()), "smem attr");
-  CK(cudaFuncSetAttribute(k_raster_warp<RM_F32_>, cudaFuncAttributeMaxDynamicSharedMemorySize, raster_warp_smem_bytes()), "smem attr");
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_raster_warp<RM_FIXED_SPLIT_>, 32, raster_warp_smem_bytes()), "occupancy");
-  c->raster_warp_grid = c->n_sm * std::max(1, occ);
   c->bin_grid = c->n_sm * 8;
   // capacities: first guesses, grown on overflow
   const uint64_t overlays = 3ull * F.cubics.size();
@@ -1454,9 +1409,9 @@ lg_status lg_resolve_rgba8(lg_ctx* c, uint8_t* dst, size_t pitch, int32_t dst_is
   if (st) return st;
   const size_t row = (size_t)c->prm.width * 4;
   if (!dst || pitch < row) return fail(c, LG_ERR_INVALID_ARGUMENT, "destination null or pitch < width * 4");
-  const int fixed = c->prm.accum == LG_ACCUM_FIXED64;
+  const int acc = accum_kind(c->prm);
   uint8_t* out = dst_is_device ? dst : (uint8_t*)c->d_stage.p;
-  k_resolve_rgba8<<<c->n_sm * 8, 256, 0, c->stream>>>(c->d_accum.p, fixed, c->prm.width, c->prm.height, out,
+  k_resolve_rgba8<<<c->n_sm * 8, 256, 0, c->stream>>>(c->d_accum.p, acc, c->prm.width, c->prm.height, out,
                                                        dst_is_device ? pitch : row);
   CK(cudaGetLastError(), "resolve launch");
   if (!dst_is_device)
@@ -1472,10 +1427,10 @@ static lg_status enqueue_stream_frame(lg_ctx* c, uint16_t* dst, size_t row, cuda
   const SceneDev S = scene_dev(c);
   const TraceBufs B = trace_bufs(c);
   const RasterArgs A = raster_args(c);
-  const int fixed = c->prm.accum == LG_ACCUM_FIXED64;
+  const int acc = accum_kind(c->prm);
   CK(cudaEventRecordWithFlags(ev[0], c->stream, cudaEventRecordExternal), "stage event");
   CK(cudaMemsetAsync(c->d_ctr.p, 0, sizeof(Counters), c->stream), "memset counters");
-  k_clear_accum<<<c->n_sm * 8, 256, 0, c->stream>>>(A, fixed);
+  k_clear_accum<<<c->n_sm * 8, 256, 0, c->stream>>>(A);
   if (c->n_lights) launch_light_setup(c, S, false, 1);
   const size_t tsm = c->smem_fits ? c->obj_smem : 0;
   const uint32_t bins = 2 * c->n_tiles;
@@ -1483,7 +1438,6 @@ static lg_status enqueue_stream_frame(lg_ctx* c, uint16_t* dst, size_t row, cuda
   const size_t bsm = smem_tiles ? (size_t)bins * 4 : 0;
   const uint32_t n_part = (bins + TILE_SCAN_CHUNK - 1) / TILE_SCAN_CHUNK;
   const int mode = raster_mode(c->prm);
-  const size_t rsm = (size_t)raster_smem_bytes(mode);
   const uint32_t G = c->prm.max_bounce;
   for (uint32_t g = 0; g < G; ++g) {
     launch_generation(c, S, B, g, false, c->trace_grid[0], (size_t)scan_smem_bytes(scan_pairs_of(c)) + tsm, tsm, c->smem_fits);
@@ -1504,22 +1458,11 @@ static lg_status enqueue_stream_frame(lg_ctx* c, uint16_t* dst, size_t row, cuda
     }
     k_build_units<<<std::max(1u, (bins + 255) / 256), 256, 0, c->stream>>>(A);
     k_bin_scatter<<<scatter_grid(c->n_sm, smem_tiles), SCATTER_THREADS, bsm, c->stream>>>(A, smem_tiles);
-    if (c->raster_variant == 2) {
-      if (mode == RM_F32_)
-        k_raster_warp<RM_F32_><<<c->raster_warp_grid, 32, raster_warp_smem_bytes(), c->stream>>>(A);
-      else
-        k_raster_warp<RM_FIXED_SPLIT_><<<c->raster_warp_grid, 32, raster_warp_smem_bytes(), c->stream>>>(A);
-    } else if (mode == RM_FIXED_SPLIT_) {
-      k_raster<RM_FIXED_SPLIT_><<<c->raster_grid, 256, rsm, c->stream>>>(A);
-    } else if (mode == RM_FIXED_MINMAX_) {
-      k_raster<RM_FIXED_MINMAX_><<<c->raster_grid, 256, rsm, c->stream>>>(A);
-    } else {
-      k_raster<RM_F32_><<<c->raster_grid, 256, rsm, c->stream>>>(A);
-    }
+    launch_raster(mode, c->raster_grid, c->stream, A);
     k_stream_rotate<<<1, 1, 0, c->stream>>>((Counters*)c->d_ctr.p, c->seg_cap);
     CK(cudaEventRecordWithFlags(ev[2 + 2 * g], c->stream, cudaEventRecordExternal), "stage event");
   }
-  k_resolve_f16<<<c->n_sm * 8, 256, 0, c->stream>>>(c->d_accum.p, fixed, c->prm.width, c->prm.height, dst, row);
+  k_resolve_f16<<<c->n_sm * 8, 256, 0, c->stream>>>(c->d_accum.p, acc, c->prm.width, c->prm.height, dst, row);
   CK(cudaEventRecordWithFlags(ev[1 + 2 * G], c->stream, cudaEventRecordExternal), "stage event");
   CK(cudaGetLastError(), "stream frame launch");
   return LG_OK;
@@ -1530,7 +1473,6 @@ static lg_status enqueue_stream_frame(lg_ctx* c, uint16_t* dst, size_t row, cuda
 static lg_status start_streaming(lg_ctx* c) {
   c->streaming = true;
   c->graph_valid = false;
-  if (c->raster_variant == 0) c->raster_variant = 1;
   const uint64_t n_ov = 3ull * c->n_cubic;
   c->seg_cap = std::max<uint64_t>(c->stream_ring, c->queue_cap + n_ov + 1024);
   c->refs_cap = std::min<uint64_t>(4 * c->seg_cap, 0xfffffff0ull);
@@ -1651,15 +1593,6 @@ static lg_status render_frame(lg_ctx* c, uint16_t* dst, size_t pitch, int32_t ds
   uint32_t retries = 0;
   if ((st = enable_kernel_events(c))) return st;
   if (c->streaming) return render_streaming(c, dst, pitch, dst_is_device, stats, retries);
-  if (c->raster_variant == 0) {  // pick the raster kernel before it is baked into the graph
-    st = run_trace(c, retries, c->stream_ring);
-    if (st == LG_ERR_TRUNCATED) {  // more segments than one pass takes: stream the frame
-      if ((st = start_streaming(c))) return st;
-      return render_streaming(c, dst, pitch, dst_is_device, stats, retries);
-    }
-    if (st) return st;
-    if ((st = tune_raster(c, retries))) return st;
-  }
   for (int attempt = 0; attempt < 8; ++attempt) {
     if (!c->graph_valid) {
       if (c->gexec) cudaGraphExecDestroy(c->gexec);
@@ -1694,6 +1627,14 @@ static lg_status render_frame(lg_ctx* c, uint16_t* dst, size_t pitch, int32_t ds
       if (ns > c->stream_ring) {
         if ((st = start_streaming(c))) return st;
         return render_streaming(c, dst, pitch, dst_is_device, stats, retries);
+      }
+      // the tile lists in proportion to what the truncated ring binned, to spare a third try
+      if (ns > c->seg_cap && c->seg_cap) {
+        const double refs = 1.125 * (double)c->h_ctr->tile_refs * (double)ns / (double)c->seg_cap + 4096.0;
+        if (refs < 4294967040.0 && (uint64_t)refs > c->refs_cap) {
+          c->refs_cap = (uint64_t)refs;
+          if ((st = ensure_raster_buffers(c))) return st;
+        }
       }
       if ((st = grow_trace(c, ns, nq))) return st;
       continue;
@@ -1766,7 +1707,14 @@ lg_status lg_accum_download(lg_ctx* c, void* out, uint64_t cap_bytes) {
   const uint64_t bytes = (uint64_t)c->prm.width * c->prm.height * 4 * (c->prm.accum == LG_ACCUM_F32 ? 4 : 8);
   if (!out) return fail(c, LG_ERR_INVALID_ARGUMENT, "null output");
   if (cap_bytes < bytes) return fail(c, LG_ERR_TRUNCATED, "output smaller than the accumulation image");
-  CK(cudaMemcpyAsync(out, c->d_accum.p, bytes, cudaMemcpyDeviceToHost, c->stream), "download accumulation image");
+  const void* src = c->d_accum.p;
+  if (accum_kind(c->prm) == ACC_F64) {
+    if ((st = ensure(c, c->d_stage, bytes, "accumulation staging"))) return st;
+    k_accum_f32<<<c->n_sm * 8, 256, 0, c->stream>>>((const double*)c->d_accum.p, (float*)c->d_stage.p, bytes / 4);
+    CK(cudaGetLastError(), "accumulation image");
+    src = c->d_stage.p;
+  }
+  CK(cudaMemcpyAsync(out, src, bytes, cudaMemcpyDeviceToHost, c->stream), "download accumulation image");
   CK(cudaStreamSynchronize(c->stream), "synchronize");
   return LG_OK;
 }

@@ -26,8 +26,7 @@ lg_status batch_buffers(lg_ctx* c) {
   lg_status st;
   if ((st = ensure_trace_buffers(c))) return st;
   if ((st = ensure(c, c->d_seg_scene, c->seg_cap * sizeof(uint16_t), "segment scenes"))) return st;
-  const size_t elem = c->prm.accum == LG_ACCUM_F32 ? 4 : 8;
-  if ((st = ensure(c, c->d_accum, c->total_px * 4 * elem, "accumulation images"))) return st;
+  if ((st = ensure(c, c->d_accum, c->total_px * accum_px_bytes(c->prm), "accumulation images"))) return st;
   if ((st = ensure(c, c->d_stage, c->total_px * 8, "resolved images"))) return st;
   const size_t bins = c->total_bins;
   if ((st = ensure(c, c->d_tile_count, bins * 4, "tile counts"))) return st;
@@ -77,18 +76,17 @@ lg_status enqueue_batch(lg_ctx* c, cudaEvent_t* ev) {
   B.seg_scene = (uint16_t*)c->d_seg_scene.p;
   B.order = (const uint32_t*)c->d_order.p;
   const RasterArgs A = batch_raster_args(c);
-  const int fixed = c->prm.accum == LG_ACCUM_FIXED64;
+  const int acc = accum_kind(c->prm);
   CK(cudaEventRecordWithFlags(ev[0], c->stream, cudaEventRecordExternal), "stage event");
   CK(cudaMemsetAsync(c->d_ctr.p, 0, sizeof(Counters), c->stream), "memset counters");
   CK(cudaMemsetAsync(c->d_scene_count.p, 0, (size_t)c->n_scenes * 4, c->stream), "memset scene counts");
-  k_clear_accum<<<c->n_sm * 8, 256, 0, c->stream>>>(A, fixed);
+  k_clear_accum<<<c->n_sm * 8, 256, 0, c->stream>>>(A);
   if (c->n_lights) launch_light_setup(c, S, true, (int)((c->n_lights + 255) / 256));
   const uint32_t bins = c->total_bins;
   const int smem_tiles = bins <= MAX_SMEM_TILES ? 1 : 0;
   const size_t bsm = smem_tiles ? (size_t)bins * 4 : 0;
   const uint32_t n_part = (bins + TILE_SCAN_CHUNK - 1) / TILE_SCAN_CHUNK;
   const int mode = raster_mode(c->prm);
-  const size_t rsm = (size_t)raster_smem_bytes(mode);
   lg_string_mod no_sm;
   std::memset(&no_sm, 0, sizeof no_sm);
   for (uint32_t g = 0; g < c->max_bounce_all; ++g) {
@@ -120,23 +118,12 @@ lg_status enqueue_batch(lg_ctx* c, cudaEvent_t* ev) {
     }
     k_build_units<<<std::max(1u, (bins + 255) / 256), 256, 0, c->stream>>>(A);
     k_bin_scatter<<<scatter_grid(c->n_sm, smem_tiles), SCATTER_THREADS, bsm, c->stream>>>(A, smem_tiles);
-    if (c->raster_variant == 2) {
-      if (mode == RM_F32_)
-        k_raster_warp<RM_F32_><<<c->raster_warp_grid, 32, raster_warp_smem_bytes(), c->stream>>>(A);
-      else
-        k_raster_warp<RM_FIXED_SPLIT_><<<c->raster_warp_grid, 32, raster_warp_smem_bytes(), c->stream>>>(A);
-    } else if (mode == RM_FIXED_SPLIT_) {
-      k_raster<RM_FIXED_SPLIT_><<<c->raster_grid, 256, rsm, c->stream>>>(A);
-    } else if (mode == RM_FIXED_MINMAX_) {
-      k_raster<RM_FIXED_MINMAX_><<<c->raster_grid, 256, rsm, c->stream>>>(A);
-    } else {
-      k_raster<RM_F32_><<<c->raster_grid, 256, rsm, c->stream>>>(A);
-    }
+    launch_raster(mode, c->raster_grid, c->stream, A);
     k_stream_rotate<<<1, 1, 0, c->stream>>>((Counters*)c->d_ctr.p, c->seg_cap);
     CK(cudaEventRecordWithFlags(ev[2 + 2 * g], c->stream, cudaEventRecordExternal), "stage event");
   }
   // all images at once: they are consecutive in both buffers
-  k_resolve_f16<<<c->n_sm * 8, 256, 0, c->stream>>>(c->d_accum.p, fixed, (uint32_t)c->total_px, 1,
+  k_resolve_f16<<<c->n_sm * 8, 256, 0, c->stream>>>(c->d_accum.p, acc, (uint32_t)c->total_px, 1,
                                                     (uint16_t*)c->d_stage.p, c->total_px * 8);
   CK(cudaEventRecordWithFlags(ev[1 + 2 * c->max_bounce_all], c->stream, cudaEventRecordExternal), "stage event");
   CK(cudaGetLastError(), "batch launch");
@@ -356,23 +343,8 @@ lg_status lg_batch_upload(lg_ctx* c, const lg_scene_desc* scenes, uint32_t k) {
   c->renders = 0;
   if ((st = scan_grid(c, true))) return st;
   if ((st = trace_grids(c, true, 0))) return st;
-  const int mode = raster_mode(c->prm);
-  const int rsm = raster_smem_bytes(mode);
-  if (mode == RM_FIXED_SPLIT_) {
-    CK(cudaFuncSetAttribute(k_raster<RM_FIXED_SPLIT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, rsm), "smem attr");
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_raster<RM_FIXED_SPLIT_>, 256, rsm), "occupancy");
-  } else if (mode == RM_FIXED_MINMAX_) {
-    CK(cudaFuncSetAttribute(k_raster<RM_FIXED_MINMAX_>, cudaFuncAttributeMaxDynamicSharedMemorySize, rsm), "smem attr");
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_raster<RM_FIXED_MINMAX_>, 256, rsm), "occupancy");
-  } else {
-    CK(cudaFuncSetAttribute(k_raster<RM_F32_>, cudaFuncAttributeMaxDynamicSharedMemorySize, rsm), "smem attr");
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_raster<RM_F32_>, 256, rsm), "occupancy");
-  }
+  CK(raster_occupancy(raster_mode(c->prm), &occ), "occupancy");
   c->raster_grid = c->n_sm * std::max(1, occ);
-  CK(cudaFuncSetAttribute(k_raster_warp<RM_FIXED_SPLIT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, raster_warp_smem_bytes()), "smem attr");
-  CK(cudaFuncSetAttribute(k_raster_warp<RM_F32_>, cudaFuncAttributeMaxDynamicSharedMemorySize, raster_warp_smem_bytes()), "smem attr");
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_raster_warp<RM_FIXED_SPLIT_>, 32, raster_warp_smem_bytes()), "occupancy");
-  c->raster_warp_grid = c->n_sm * std::max(1, occ);
   c->bin_grid = c->n_sm * 8;
   c->multi = true;  // the single-scene entry points need lg_scene_upload again
   return LG_OK;
@@ -416,26 +388,7 @@ lg_status lg_batch_render(lg_ctx* c, uint16_t* dst, uint64_t dst_bytes, int32_t 
     }
     if ((st = set_scan_pairs(c, pick, true))) return st;
   }
-  if (c->raster_variant == 0) {
-    // autotune: the whole batch with each tile-raster kernel (identical images), keep the faster
-    float best = INFINITY;
-    int pick = 1;
-    for (int v = 1; v <= 2; ++v) {
-      c->raster_variant = v;
-      c->graph_valid = false;
-      if ((st = run_batch(c, ev, retries))) { c->raster_variant = 0; return st; }
-      float ms = 0.f;
-      for (uint32_t g = 0; g < c->max_bounce_all; ++g) ms += elapsed(ev[1 + 2 * g], ev[2 + 2 * g]);
-      if (ms < best) { best = ms; pick = v; }
-    }
-    if (pick != c->raster_variant) {
-      c->raster_variant = pick;
-      c->graph_valid = false;
-      if ((st = run_batch(c, ev, retries))) return st;
-    }
-  } else if ((st = run_batch(c, ev, retries))) {
-    return st;
-  }
+  if ((st = run_batch(c, ev, retries))) return st;
   CK(cudaMemcpyAsync(dst, c->d_stage.p, bytes, dst_is_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                      c->stream), "copy images");
   CK(cudaStreamSynchronize(c->stream), "synchronize");

@@ -16,10 +16,6 @@ struct DevBuf {
   size_t bytes = 0;
 };
 
-constexpr uint32_t UNIT_REFS = SPLIT_UNIT_REFS;  // shared-atomic raster: keeps the split sums within 2^31
-constexpr uint32_t UNIT_REFS_WARP = 8192;  // warp-private raster: no bound, bigger units flush less
-// the smaller of the two: the unit table is sized for whichever raster the context runs
-constexpr uint32_t MIN_UNIT_REFS = UNIT_REFS < UNIT_REFS_WARP ? UNIT_REFS : UNIT_REFS_WARP;
 constexpr size_t OBJ_SMEM_MAX = 96 * 1024;
 
 }  // namespace lgh
@@ -64,8 +60,6 @@ struct lg_ctx {
   // launch shapes
   // scan, refine, full, bounce (fast mode), solve, bounce (exact mode)
   int trace_grid[6] = {0, 0, 0, 0, 0, 0}, raster_grid = 0, bin_grid = 0;
-  int raster_warp_grid = 0;
-  int raster_variant = 0;  // 1 shared-atomic tile raster, 2 warp-private tile raster; 0 = not tuned yet
   int scan_pairs = 0;      // pair slots per lane of the scan (8 / 16; 0: by the culling grid)
   int scan_pairs_opt = 0;  // lg_device_opts.scan_pairs (0: tune on a scene's first render)
   bool scan_tune = false;  // armed by a new scene: its second lg_render (lg_batch_render) times

@@ -150,7 +150,8 @@ struct Counters {
   unsigned long long queue_count[MAX_GEN + 1]; // entries demanded per generation
   unsigned long long list_count[MAX_GEN][N_LISTS];
   unsigned long long visits, fp64_solves, fallbacks, near, ill;
-  unsigned long long pixels, tile_refs, units;
+  unsigned long long pixels, bin_refs;  // pixel updates; (segment, tile) pairs counted by k_bin_count
+  unsigned long long tile_refs, units;
   unsigned long long unit_cursor;
   // multi-scene streaming accumulation: the ring and the tile lists are reused every
   // generation; these keep the totals and the largest per-generation demands

@@ -84,6 +84,8 @@ lg_status validate_params(std::string& err, const lg_params& p);
 lg_status validate_exact(std::string& err, const lg_params& p, const Flat& F);
 bool blend_supported(const lg_blend_component& b);
 int raster_mode(const lg_params& p);
+int accum_kind(const lg_params& p);        // ACC_* of a context's accumulation image
+size_t accum_px_bytes(const lg_params& p);  // its bytes per pixel
 void to_device_leaves(const std::vector<LeafH>& in, std::vector<Leaf64>& out);
 // Builds the culling grid of a flattened scene (culling: lg_culling; density: cells per
 // object, 0 = default).

@@ -24,6 +24,9 @@ struct SceneCanvas {
   uint64_t bin_base, px_base;
 };
 
+// values of an accumulation image: FP32, Q31.32 in int64, FP64
+enum : int { ACC_F32 = 0, ACC_I64 = 1, ACC_F64 = 2 };
+
 struct RasterArgs {
   const lg_segment* segs;
   const uint16_t* seg_scene;      // multi-scene: scene of each segment (nullptr: one scene)
@@ -32,7 +35,8 @@ struct RasterArgs {
   uint64_t seg_cap;
   uint32_t W, H, ntx, nty;
   uint32_t n_tiles;
-  uint32_t unit_refs;      // refs per work unit
+  uint32_t unit_refs;      // most refs per work unit (raster_unit_refs of the mode)
+  uint32_t unit_share;     // units to cut a small accumulation into (a few per raster CTA)
   BlendDev blend;
   uint32_t* tile_count;    // refs per tile
   uint64_t* tile_off;      // exclusive prefix of tile_count
@@ -46,7 +50,8 @@ struct RasterArgs {
   // counts here ([CTA][bin]) and k_bin_scatter reserves its ranges from them instead of
   // counting its segments again (nullptr: the scatter counts)
   uint32_t* cta_hist;
-  void* accum;             // H * W * 4 of int64 (FIXED64) or float (F32)
+  void* accum;             // H * W * 4 values of the kind acc names
+  int32_t acc;             // ACC_*
   Counters* ctr;
 };
 
@@ -98,7 +103,9 @@ __global__ void k_scene_hist(SceneDev S, TraceBufs B, uint32_t gen, unsigned* co
 __global__ void k_scene_offsets(unsigned* count, unsigned* off, uint32_t n_scenes);
 __global__ void k_scene_scatter(SceneDev S, TraceBufs B, uint32_t gen, unsigned* off, uint32_t* order);
 
-__global__ void k_clear_accum(RasterArgs A, int fixed);
+__global__ void k_clear_accum(RasterArgs A);
+// An FP64 accumulation image rounded to FP32 (n values).
+__global__ void k_accum_f32(const double* src, float* dst, uint64_t n);
 __global__ void k_bin_count(RasterArgs A, int smem_tiles);
 __global__ void k_scan_tiles(RasterArgs A);
 __global__ void k_build_units(RasterArgs A);
@@ -109,19 +116,23 @@ __global__ void k_bin_scatter(RasterArgs A, int smem_tiles);
 // reference into a DRAM read-modify-write).
 constexpr int SCATTER_THREADS = 1024;
 inline int scatter_grid(int n_sm, int smem_tiles) { return smem_tiles ? n_sm : 2 * n_sm; }
+constexpr int RM_FIXED_SPLIT_ = 0, RM_FIXED_MINMAX_ = 1, RM_F32_ = 2, RM_F32_MINMAX_ = 3;
+// Segments per work unit: bounds the split-plane sums of the mode (17 + 17 bits in fixed point,
+// 21 + 21 bits in F32).
+constexpr uint32_t SPLIT_UNIT_REFS = 16384;
+constexpr uint32_t F32_UNIT_REFS = 1024;
+constexpr uint32_t MIN_UNIT_REFS = 256;  // one round of the raster CTA's eight warps
 template <int MODE>
 __global__ void k_raster(RasterArgs A);
-int raster_smem_bytes(int mode);
-template <int MODE>
-__global__ void k_raster_warp(RasterArgs A);
+// The tile raster of a mode: its shared memory enabled and its CTAs per SM; a launch; the most
+// segments a unit may hold.
+cudaError_t raster_occupancy(int mode, int* occ);
+void launch_raster(int mode, int grid, cudaStream_t stream, const RasterArgs& A);
+uint32_t raster_unit_refs(int mode);
 // String-mod lines straight into the image (one warp per line, global atomics), colour
-// interpolated along the major axis; FIXED: int64 Q31.32, else f32.
+// interpolated along the major axis; FIXED: int64 Q31.32, else FP64 or FP32 sums.
 template <bool FIXED>
 __global__ void k_raster_chords(RasterArgs A, const lg_chord* chords, uint64_t n);
-int raster_warp_smem_bytes();
-constexpr int RM_FIXED_SPLIT_ = 0, RM_FIXED_MINMAX_ = 1, RM_F32_ = 2;
-// Segments per work unit of the shared-atomic raster: bounds the split-plane sums.
-constexpr uint32_t SPLIT_UNIT_REFS = 16384;
 constexpr uint32_t MAX_SMEM_TILES = 32768;  // tile bins (2 per tile) with 32-bit counters in 128 KB
 // multi-scene streaming accumulation
 __global__ void k_stream_rotate(Counters* ctr, uint64_t seg_cap);
@@ -131,7 +142,7 @@ constexpr int TILE_SCAN_CHUNK = 4096;  // bins per CTA of the multi-block tile s
 __global__ void k_tiles_partial(RasterArgs A, unsigned long long* part);
 __global__ void k_tiles_scan_partials(RasterArgs A, unsigned long long* part, uint32_t n_part);
 __global__ void k_tiles_apply(RasterArgs A, const unsigned long long* part);
-__global__ void k_resolve_f16(const void* accum, int fixed, uint32_t W, uint32_t H, uint16_t* dst, size_t pitch);
-__global__ void k_resolve_rgba8(const void* accum, int fixed, uint32_t W, uint32_t H, uint8_t* dst, size_t pitch);
+__global__ void k_resolve_f16(const void* accum, int acc, uint32_t W, uint32_t H, uint16_t* dst, size_t pitch);
+__global__ void k_resolve_rgba8(const void* accum, int acc, uint32_t W, uint32_t H, uint8_t* dst, size_t pitch);
 
 }  // namespace lgd

@@ -29,8 +29,7 @@ constexpr size_t NOALLOC_SCRATCH_BYTES = 32ull << 20;  // 32 MiB per device
 constexpr uint32_t NOALLOC_MAX_TILES = 4096;           // e.g. 2048 x 2048 pixels in 32 x 32 tiles
 constexpr uint32_t NOALLOC_MAX_BINS = 2 * NOALLOC_MAX_TILES;
 constexpr uint64_t NOALLOC_MAX_REFS = 8000000;         // (segment, tile) pairs per call
-constexpr uint32_t NOALLOC_UNIT_REFS = 1024;           // units well within the shared-atomic raster's bound
-constexpr uint64_t NOALLOC_MAX_UNITS = NOALLOC_MAX_BINS + NOALLOC_MAX_REFS / NOALLOC_UNIT_REFS + 1;
+constexpr uint64_t NOALLOC_MAX_UNITS = NOALLOC_MAX_BINS + NOALLOC_MAX_REFS / MIN_UNIT_REFS + 1;
 constexpr int MAX_DEVICES = 64;
 
 constexpr size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -54,7 +53,7 @@ struct DeviceSetup {
   bool ready = false;
   unsigned char* scratch = nullptr;  // device address of g_noalloc_scratch on this device
   int n_sm = 0;
-  int raster_grid = 0;
+  int raster_grid[4] = {0, 0, 0, 0};  // by raster mode
 };
 
 DeviceSetup g_setup[MAX_DEVICES];
@@ -80,23 +79,21 @@ lg_status setup_device(int dev, DeviceSetup*& out) {
     }
     int n_sm = 0;
     if (cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return LG_ERR_CUDA;
-    const int rsm[3] = {raster_smem_bytes(RM_FIXED_SPLIT_), raster_smem_bytes(RM_FIXED_MINMAX_), raster_smem_bytes(RM_F32_)};
-    cudaError_t e = cudaFuncSetAttribute(k_raster<RM_FIXED_SPLIT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, rsm[0]);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_raster<RM_FIXED_MINMAX_>, cudaFuncAttributeMaxDynamicSharedMemorySize, rsm[1]);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_raster<RM_F32_>, cudaFuncAttributeMaxDynamicSharedMemorySize, rsm[2]);
+    int occ[4] = {0, 0, 0, 0};
+    cudaError_t e = cudaSuccess;
+    for (int mode : {RM_FIXED_SPLIT_, RM_FIXED_MINMAX_, RM_F32_, RM_F32_MINMAX_})
+      if (e == cudaSuccess) e = raster_occupancy(mode, &occ[mode]);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_bin_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(MAX_SMEM_TILES * 4));
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_bin_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(MAX_SMEM_TILES * 4));
-    int occ = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_raster<RM_FIXED_SPLIT_>, 256, rsm[0]);
     if (e != cudaSuccess) {
       (void)cudaGetLastError();
       return LG_ERR_CUDA;
     }
     d.scratch = static_cast<unsigned char*>(p);
     d.n_sm = n_sm;
-    d.raster_grid = n_sm * (occ > 0 ? occ : 1);
+    for (int mode = 0; mode < 4; ++mode) d.raster_grid[mode] = n_sm * (occ[mode] > 0 ? occ[mode] : 1);
     d.ready = true;
   }
   out = &d;
@@ -134,7 +131,9 @@ extern "C" lg_status lg_accumulate_segments_noalloc(const lg_segment* segments, 
   A.ntx = ntx;
   A.nty = nty;
   A.n_tiles = 2 * n_tiles;  // bins: x-major and y-major segments of each tile
-  A.unit_refs = NOALLOC_UNIT_REFS;
+  const int mode = lgh::raster_mode(p);
+  A.unit_refs = raster_unit_refs(mode);
+  A.unit_share = 3u * (uint32_t)d->raster_grid[mode];
   for (int ch = 0; ch < 4; ++ch) {
     const lg_blend_component& b = ch < 3 ? p.color_blend : p.alpha_blend;
     A.blend.src[ch] = b.src_factor;
@@ -152,27 +151,20 @@ extern "C" lg_status lg_accumulate_segments_noalloc(const lg_segment* segments, 
   A.refs = reinterpret_cast<uint32_t*>(base + OFF_REFS);
   A.refs_cap = NOALLOC_MAX_REFS;
   A.accum = accum;
+  A.acc = p.accum == LG_ACCUM_FIXED64 ? ACC_I64 : ACC_F32;  // the caller's image
 
-  const int fixed = p.accum == LG_ACCUM_FIXED64;
   const uint32_t bins = A.n_tiles;
   const int smem_tiles = bins <= MAX_SMEM_TILES ? 1 : 0;
   const size_t bsm = smem_tiles ? (size_t)bins * 4 : 0;
-  const int mode = lgh::raster_mode(p);
-  const size_t rsm = (size_t)raster_smem_bytes(mode);
   // the previous call's contents stay in the array: counters and tile counts restart at 0
   k_noalloc_init<<<1, 256, 0, s>>>(A.ctr, (unsigned long long)n);
   if (cudaMemsetAsync(A.tile_count, 0, (size_t)bins * 4, s) != cudaSuccess) return LG_ERR_CUDA;
-  k_clear_accum<<<d->n_sm * 8, 256, 0, s>>>(A, fixed);
+  k_clear_accum<<<d->n_sm * 8, 256, 0, s>>>(A);
   k_bin_count<<<d->n_sm * 8, 256, bsm, s>>>(A, smem_tiles);
   k_scan_tiles<<<1, 1024, 0, s>>>(A);
   k_build_units<<<(bins + 255) / 256, 256, 0, s>>>(A);
   k_bin_scatter<<<scatter_grid(d->n_sm, smem_tiles), SCATTER_THREADS, bsm, s>>>(A, smem_tiles);
-  if (mode == RM_FIXED_SPLIT_)
-    k_raster<RM_FIXED_SPLIT_><<<d->raster_grid, 256, rsm, s>>>(A);
-  else if (mode == RM_FIXED_MINMAX_)
-    k_raster<RM_FIXED_MINMAX_><<<d->raster_grid, 256, rsm, s>>>(A);
-  else
-    k_raster<RM_F32_><<<d->raster_grid, 256, rsm, s>>>(A);
+  launch_raster(mode, d->raster_grid[mode], s, A);
   if (cudaGetLastError() != cudaSuccess) return LG_ERR_CUDA;
   unsigned long long counts[2] = {0, 0};
   if (cudaMemcpyAsync(&counts[0], &A.ctr->tile_refs, 8, cudaMemcpyDeviceToHost, s) != cudaSuccess ||

@@ -7,7 +7,7 @@
 //   1. k_bin_count / k_scan_tiles / k_build_units / k_bin_scatter sort (segment, tile)
 //      pairs into per-tile lists (32 x 32 px tiles) and cut each list into work units;
 //   2. k_raster: persistent CTAs take units from a device counter, accumulate the unit's
-//      segments into a shared-memory tile with shared atomics (one warp per segment, one
+//      segments into a shared-memory tile with shared atomics (a warp draws a segment, a
 //      lane per major-axis pixel), then flush the tile with one global atomic per pixel
 //      channel.  Fixed-point (int64 Q31.32) sums make the image independent of the order
 //      in which units and segments are processed, so it is bit-reproducible;
@@ -48,23 +48,34 @@ __device__ __forceinline__ float ident32(int op) {
 }
 
 // ------------------------------------------------------------------ clear
-__global__ void k_clear_accum(RasterArgs A, int fixed) {
+template <class V4, class V>
+__device__ __forceinline__ void fill_px(void* img, uint64_t n, V r, V g, V b, V a) {
+  V4 c;
+  c.x = r; c.y = g; c.z = b; c.w = a;
+  V4* p = reinterpret_cast<V4*>(img);
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    p[i] = c;
+}
+__global__ void k_clear_accum(RasterArgs A) {
   const uint64_t n = (uint64_t)A.W * A.H;
-  if (fixed) {
-    longlong4_32a c;
-    c.x = to_fixed(A.blend.clear[0]);
-    c.y = to_fixed(A.blend.clear[1]);
-    c.z = to_fixed(A.blend.clear[2]);
-    c.w = to_fixed(A.blend.clear[3]);
-    longlong4_32a* p = reinterpret_cast<longlong4_32a*>(A.accum);
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-      p[i] = c;
-  } else {
-    const float4 c = make_float4(A.blend.clear[0], A.blend.clear[1], A.blend.clear[2], A.blend.clear[3]);
-    float4* p = reinterpret_cast<float4*>(A.accum);
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-      p[i] = c;
-  }
+  const float* c = A.blend.clear;
+  if (A.acc == ACC_I64)
+    fill_px<longlong4_32a, long long>(A.accum, n, to_fixed(c[0]), to_fixed(c[1]), to_fixed(c[2]), to_fixed(c[3]));
+  else if (A.acc == ACC_F64)
+    fill_px<double4_32a, double>(A.accum, n, c[0], c[1], c[2], c[3]);
+  else
+    fill_px<float4, float>(A.accum, n, c[0], c[1], c[2], c[3]);
+}
+
+__global__ void k_accum_f32(const double* src, float* dst, uint64_t n) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+    dst[i] = __double2float_rn(src[i]);
+}
+
+// adds a term to value k of an FP64 or FP32 accumulation image
+__device__ __forceinline__ void image_add(const RasterArgs& A, uint64_t k, double v) {
+  if (A.acc == ACC_F64) atomicAdd(reinterpret_cast<double*>(A.accum) + k, v);
+  else atomicAdd(reinterpret_cast<float*>(A.accum) + k, __double2float_rn(v));
 }
 
 // ------------------------------------------------------------------ canvases
@@ -198,7 +209,9 @@ __global__ void __launch_bounds__(SCATTER_THREADS) k_bin_count(RasterArgs A, int
     for (uint32_t t = threadIdx.x; t < A.n_tiles; t += blockDim.x) hist[t] = 0;
     __syncthreads();
   }
+  uint32_t my_refs = 0;
   for_each_pair_dense(A, n, [&](uint64_t, uint32_t tile) {
+    ++my_refs;
     if (smem_tiles) {
       atomicAdd(&hist[tile], 1u);
     } else {
@@ -217,6 +230,18 @@ __global__ void __launch_bounds__(SCATTER_THREADS) k_bin_count(RasterArgs A, int
       if (c) atomicAdd(&A.tile_count[t], c);
     }
   }
+  add_block_counts<1>({my_refs}, {&A.ctr->bin_refs});
+}
+
+// Segments per raster unit of this accumulation.  A unit ends with the flush of its 32 KB tile,
+// so big accumulations take the largest units the sums allow; a small one is cut finer, down
+// to one round of the CTA's eight warps, until every CTA has about three units: a tile that
+// holds a light source has as many segments as the light has rays, and as one unit it kept a
+// single CTA busy for most of a small frame (334 us of raster in a frame of 12,000 rays).
+__device__ __forceinline__ uint32_t unit_refs_of(const RasterArgs& A) {
+  const unsigned long long share = A.ctr->bin_refs / max(A.unit_share, 1u);
+  const unsigned long long u = (share + MIN_UNIT_REFS - 1) / MIN_UNIT_REFS * MIN_UNIT_REFS;
+  return (uint32_t)(u < MIN_UNIT_REFS ? MIN_UNIT_REFS : u > A.unit_refs ? A.unit_refs : u);
 }
 
 // single-CTA exclusive scan of refs and units per tile
@@ -227,10 +252,11 @@ __global__ void __launch_bounds__(1024) k_scan_tiles(RasterArgs A) {
   if (threadIdx.x == 0) { carry_r = 0; carry_u = 0; }
   __syncthreads();
   const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
+  const uint32_t per = unit_refs_of(A);
   for (uint32_t base = 0; base < A.n_tiles; base += blockDim.x) {
     const uint32_t t = base + threadIdx.x;
-    const unsigned long long c = t < A.n_tiles ? A.tile_count[t] : 0ull;
-    const unsigned long long u = (c + A.unit_refs - 1) / A.unit_refs;
+    const uint32_t cn = t < A.n_tiles ? A.tile_count[t] : 0u;
+    const unsigned long long c = cn, u = ((unsigned long long)cn + per - 1) / per;
     unsigned long long ir = c, iu = u;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -275,10 +301,10 @@ __global__ void __launch_bounds__(1024) k_scan_tiles(RasterArgs A) {
 // Multi-block version of k_scan_tiles for the many bins of a multi-scene accumulation:
 // per-CTA sums of refs and units, one scan of the CTA sums, then each CTA scans its own
 // chunk from its offset.  part holds 2 values per CTA (refs, units).
-__device__ __forceinline__ void tile_counts(const RasterArgs& A, uint32_t t, unsigned long long& c,
+__device__ __forceinline__ void tile_counts(const RasterArgs& A, uint32_t per, uint32_t t, unsigned long long& c,
                                             unsigned long long& u) {
   c = t < A.n_tiles ? A.tile_count[t] : 0ull;
-  u = (c + A.unit_refs - 1) / A.unit_refs;
+  u = (c + per - 1) / per;
 }
 
 // inclusive block scan of (r, u) over 1024 threads; returns the block totals in tr, tu
@@ -313,11 +339,11 @@ __device__ __forceinline__ void block_scan2(unsigned long long& r, unsigned long
 
 __global__ void __launch_bounds__(1024) k_tiles_partial(RasterArgs A, unsigned long long* part) {
   if (A.ctr->skip_raster) return;
-  const uint32_t b0 = blockIdx.x * (uint32_t)TILE_SCAN_CHUNK;
+  const uint32_t b0 = blockIdx.x * (uint32_t)TILE_SCAN_CHUNK, per = unit_refs_of(A);
   unsigned long long r = 0, u = 0;
   for (uint32_t k = threadIdx.x; k < (uint32_t)TILE_SCAN_CHUNK; k += blockDim.x) {
     unsigned long long c, v;
-    tile_counts(A, b0 + k, c, v);
+    tile_counts(A, per, b0 + k, c, v);
     r += c;
     u += v;
   }
@@ -354,11 +380,11 @@ __global__ void __launch_bounds__(1024) k_tiles_apply(RasterArgs A, const unsign
   __shared__ unsigned long long carry_r, carry_u;
   if (threadIdx.x == 0) { carry_r = part[2 * blockIdx.x]; carry_u = part[2 * blockIdx.x + 1]; }
   __syncthreads();
-  const uint32_t b0 = blockIdx.x * (uint32_t)TILE_SCAN_CHUNK;
+  const uint32_t b0 = blockIdx.x * (uint32_t)TILE_SCAN_CHUNK, per = unit_refs_of(A);
   for (uint32_t k = 0; k < (uint32_t)TILE_SCAN_CHUNK; k += blockDim.x) {
     const uint32_t t = b0 + k + threadIdx.x;
     unsigned long long c, v;
-    tile_counts(A, t, c, v);
+    tile_counts(A, per, t, c, v);
     unsigned long long r = c, u = v, tr, tu;
     block_scan2(r, u, tr, tu);
     const unsigned long long cr = carry_r, cu = carry_u;
@@ -384,6 +410,7 @@ __global__ void k_stream_decide(Counters* ctr, uint32_t gen, uint64_t seg_cap, u
 
 __global__ void k_clear_counts(RasterArgs A) {
   if (A.ctr->skip_raster) return;
+  if (blockIdx.x == 0 && threadIdx.x == 0) A.ctr->bin_refs = 0;
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < A.n_tiles; t += gridDim.x * blockDim.x) A.tile_count[t] = 0u;
 }
 
@@ -401,15 +428,16 @@ __global__ void k_stream_rotate(Counters* ctr, uint64_t seg_cap) {
 
 __global__ void k_build_units(RasterArgs A) {
   if (A.ctr->skip_raster) return;
+  const uint32_t per = unit_refs_of(A);
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < A.n_tiles; t += gridDim.x * blockDim.x) {
     const uint64_t c = A.tile_count[t], off = A.tile_off[t];
     uint64_t u = A.unit_off[t];
-    for (uint64_t b = 0; b < c; b += A.unit_refs, ++u) {
+    for (uint64_t b = 0; b < c; b += per, ++u) {
       if (u >= A.units_cap) return;
       Unit U;
       U.tile = t;
       U.begin = off + b;
-      U.n = (uint32_t)(c - b < A.unit_refs ? c - b : A.unit_refs);
+      U.n = (uint32_t)(c - b < per ? c - b : per);
       A.units[u] = U;
     }
   }
@@ -456,29 +484,40 @@ __global__ void __launch_bounds__(SCATTER_THREADS) k_bin_scatter(RasterArgs A, i
 }
 
 // ------------------------------------------------------------------ tile raster
-constexpr int TILE_PX = TILE * TILE;  // cells per channel plane
+constexpr int TILE_PX = TILE * TILE;  // cells of a tile
+// Words between two sum planes: the flush reads the four channels of eight cells per warp, and
+// two planes (one channel) are 8 banks apart, so its 32 reads fall in 32 banks.
+constexpr int PLANE = TILE_PX + 4;
 
 // Layout of a unit's shared-memory tile: x-major units index cells [row][col] and their
 // 32 lanes own 32 columns; y-major units index [col][row] and their lanes own 32 rows.
 // Either way one warp's 32 accesses fall in 32 distinct banks.
 //
-// Fixed-point sums use exact split accumulation in native 32-bit shared atomics: a
-// contribution |q| < 2^34 (a colour term below 4) is split as q = b * 2^17 + c with an
-// unsigned 17-bit c and a signed b (|b| <= 2^17).  A unit holds at most SPLIT_UNIT_REFS =
-// 16384 segments and a segment adds at most once to a pixel, so both plane sums stay within
-// 2^31 and B * 2^17 + C is exact.  (Sixteen times fewer units than 1024-segment units with
-// a 21-bit split: each unit ends with a flush of its 32 KB tile by global atomics.)  A
-// segment with a larger term (up to the clamp, 2^52) skips the tile and adds its 64-bit
-// terms to the image with global atomics, which is just as exact.
-constexpr int SPLIT_BITS = 17;   // c = q mod 2^17
-constexpr int SPLIT_LIMIT = 34;  // |q| < 2^34 takes the split planes
-static_assert((1ll << (SPLIT_LIMIT - SPLIT_BITS)) * SPLIT_UNIT_REFS <= (1ll << 31) &&
-                  (1ll << SPLIT_BITS) * SPLIT_UNIT_REFS <= (1ll << 31), "split plane sums must fit 32 bits");
-enum RasterMode { RM_FIXED_SPLIT = 0, RM_FIXED_MINMAX = 1, RM_F32 = 2 };
+// Additive sums are exact split sums in native 32-bit shared atomics: a term of magnitude
+// below 2^(LIMIT - FRAC) is a whole number |q| < 2^LIMIT of units 2^-FRAC, split as
+// |q| = b * 2^SPLIT + c, and a negative term negates both.  A unit holds at most UNIT_MAX
+// segments and a segment adds at most once to a pixel, so both plane sums stay within 32
+// signed bits and B * 2^SPLIT + C is exact.
+//   FIXED: Q31.32, q rounded to nearest even (to_fixed); terms of 4 and more take 64-bit
+//     atomics on the image instead, which is just as exact.
+//   F32: units of 2^-41, in which every FP32 value in [2^-18, 2) is whole, so a unit's sum is
+//     the exact sum of its terms; the FP64 image (accum_kind) adds the units.  Terms outside
+//     that range (NaN and infinities among them) take atomics on the image.
+enum RasterMode { RM_FIXED_SPLIT = 0, RM_FIXED_MINMAX = 1, RM_F32 = 2, RM_F32_MINMAX = 3 };
+template <int MODE>
+struct Split {
+  static constexpr bool on = MODE == RM_FIXED_SPLIT || MODE == RM_F32;
+  static constexpr int frac = MODE == RM_F32 ? 41 : 32;
+  static constexpr int bits = MODE == RM_F32 ? 21 : 17;   // c = |q| mod 2^bits
+  static constexpr int limit = MODE == RM_F32 ? 42 : 34;  // |q| < 2^limit
+  static constexpr uint32_t unit_max = MODE == RM_F32 ? F32_UNIT_REFS : SPLIT_UNIT_REFS;
+  static_assert((1ll << (limit - bits)) * unit_max <= (1ll << 31) && (1ll << bits) * unit_max <= (1ll << 31),
+                "split plane sums must fit 32 bits");
+};
 
 template <int MODE>
 struct RasterSmem {
-  static constexpr int acc_words = MODE == RM_F32 ? 4 * TILE_PX : 8 * TILE_PX;
+  static constexpr int acc_words = MODE == RM_F32_MINMAX ? 4 * TILE_PX : MODE == RM_FIXED_MINMAX ? 8 * TILE_PX : 8 * PLANE;
   static constexpr int stage_words = 8 * 32 * 12;  // 8 warps x 32 staged segments x 48 B
   static constexpr int owner_words = 8 * 32 * 32 / 4;  // 8 warps x 1024 (segment, column) pairs, 1 B each
   static constexpr int pref_words = 8 * 33;
@@ -487,17 +526,67 @@ struct RasterSmem {
 
 // one staged segment: raster setup restricted to the unit's tile and the per-channel
 // source terms, 48 B
-constexpr int SPAN_BIG = 1 << 30;  // FIXED_SPLIT: terms too large for the split planes
 struct __align__(16) Staged {
   float ua, va, slope;
-  int span;             // first tile-local major-axis pixel | count << 16 | SPAN_BIG
-  unsigned q[8];        // FIXED_SPLIT: (c, b) per channel, or 4 x int64 with SPAN_BIG;
-                        // FIXED_MINMAX: 4 x int64; F32: 4 x float
+  unsigned mask;        // the tile's major-axis pixels it covers (one run of bits)
+  unsigned q[8];        // split sums: (c, b) per channel; FIXED_MINMAX: 4 x int64; F32_MINMAX: 4 x float
 };
 
+// |q| = b * 2^bits + c of a split term, signed; false when the term is out of the split's
+// range.  v * 2^(frac - bits) is exact, and so are its fraction and the fraction's scaling, so
+// rounding the fraction rounds v * 2^frac (the carry of a rounded-up fraction goes to b).  The
+// FP32 steps take the place of a 64-bit float conversion, which issues on the FP64 pipe.
+template <int MODE>
+__device__ __forceinline__ bool split_term(float v, bool neg, unsigned& c_out, unsigned& b_out) {
+  using S = Split<MODE>;
+  if (MODE == RM_FIXED_SPLIT && v != v) v = 0.0f;  // to_fixed: NaN adds nothing
+  const float m = fabsf(v);
+  if (!(m < (float)(1ll << (S::limit - S::frac)))) return false;
+  if (MODE == RM_F32 && m < 3.814697265625e-06f && m != 0.0f) return false;  // below 2^-18: not whole
+  const float t = m * (float)(1 << (S::frac - S::bits));
+  const float f = floorf(t);
+  int b = (int)f, c = __float2int_rn((t - f) * (float)(1 << S::bits));
+  if (MODE == RM_FIXED_SPLIT && c == (1 << S::bits)) {
+    c = 0;
+    ++b;
+  }
+  const bool n = (v < 0.0f) != neg;
+  c_out = (unsigned)(n ? -c : c);
+  b_out = (unsigned)(n ? -b : b);
+  return true;
+}
+
+__device__ __forceinline__ void shared_add(unsigned addr, unsigned v) {
+  asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+
+__device__ __forceinline__ void f32_minmax(float* p, float v, bool mn) {
+  float o = *p;
+  while (mn ? v < o : v > o) {
+    const float w = __int_as_float(atomicCAS(reinterpret_cast<int*>(p), __float_as_int(o), __float_as_int(v)));
+    if (w == o) break;
+    o = w;
+  }
+}
+
+// A batch of 32 segments is drawn segment by segment, a lane per column of the tile, when its
+// segments cover at least this many columns each on average; else its (segment, column) pairs
+// are spread densely over the lanes.  Drawing by segments reads its parameters from shared
+// memory once per warp (a broadcast) and its atomics hit 32 banks, at about 30 instructions a
+// segment; the dense walk takes about 75 for 32 pairs and its lanes' rows collide.
+#ifndef LG_RASTER_LANE_MIN
+#define LG_RASTER_LANE_MIN 8
+#endif
+
+// Bound: the shared-memory pipe (seven or eight 32-bit atomics and three broadcast reads per
+// segment and tile): 87 % of the L1 wavefront slots on the mid scene at 2^13 rays per light
+// (450 M pixels), 1.42 ms where spreading every pixel over the lanes took 2.78 ms (2196 M warp
+// instructions, 167 M bank conflicts; now 1030 M and 10 M).  With a branch per atomic instead
+// of masked terms the same walk took 2.42 ms.
 template <int MODE>
 __global__ void __launch_bounds__(256, 4) k_raster(RasterArgs A) {
   if (A.ctr->skip_raster) return;
+  using SP = Split<MODE>;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   unsigned* acc32 = reinterpret_cast<unsigned*>(smem_raw);
   long long* acc64 = reinterpret_cast<long long*>(smem_raw);
@@ -507,6 +596,7 @@ __global__ void __launch_bounds__(256, 4) k_raster(RasterArgs A) {
   int* pref_all = reinterpret_cast<int*>(owner_all + 8 * 1024);
   __shared__ unsigned long long s_unit;
   const unsigned lane = lane_id(), warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const unsigned acc_addr = (unsigned)__cvta_generic_to_shared(acc32);
   Staged* stage = stage_all + warp * 32;
   uint8_t* owner = owner_all + warp * 1024;
   int* pref = pref_all + warp * 33;
@@ -527,7 +617,9 @@ __global__ void __launch_bounds__(256, 4) k_raster(RasterArgs A) {
     const uint32_t tx = tile % C.ntx, ty = tile / C.ntx;
     const int tm = xmajor ? (int)tx : (int)ty, tn = xmajor ? (int)ty : (int)tx;
     const int nmin = (int)(xmajor ? C.H : C.W);
-    if (MODE == RM_FIXED_SPLIT) {
+    // minor pixels of the tile: floor(v) in [tn TILE, hi) exactly when v is
+    const float vlo = (float)(tn * TILE), vhi = (float)min(tn * TILE + TILE, nmin);
+    if (SP::on) {
       uint4* z = reinterpret_cast<uint4*>(acc32);
       for (int k = threadIdx.x; k < RasterSmem<MODE>::acc_words / 4; k += blockDim.x) z[k] = make_uint4(0, 0, 0, 0);
     } else if (MODE == RM_FIXED_MINMAX) {
@@ -536,12 +628,45 @@ __global__ void __launch_bounds__(256, 4) k_raster(RasterArgs A) {
       for (int k = threadIdx.x; k < 4 * TILE_PX; k += blockDim.x) accf[k] = ident32(B.op[k / TILE_PX]);
     }
     __syncthreads();
+    // Adds one staged segment's terms to a cell of the tile when on.  Split sums take no branch
+    // (eight predicated atomics cost a branch each): a lane that is off adds zeros to the cell
+    // of its own bank in row 0.  alpha_c: some alpha term of the batch has a low part (an alpha
+    // of 1, the usual one, has none).
+    auto deposit = [&](const uint4& q0, const uint4& q1, int cell, bool on, bool alpha_c) {
+      const unsigned qs[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
+      if (SP::on) {
+        const unsigned a = acc_addr + 4u * (unsigned)(on ? cell : (int)lane), m = on ? 0xffffffffu : 0u;
+#pragma unroll
+        for (int w = 0; w < 8; ++w)
+          if (w != 6 || alpha_c) shared_add(a + 4u * PLANE * w, qs[w] & m);
+      } else if (on) {
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch) {
+          const int op = B.op[ch];
+          if (MODE == RM_FIXED_MINMAX) {
+            const long long q = (long long)(((unsigned long long)qs[2 * ch + 1] << 32) | qs[2 * ch]);
+            long long* p = acc64 + ch * TILE_PX + cell;
+            if (op == LG_BO_MIN) atomicMin(p, q);
+            else if (op == LG_BO_MAX) atomicMax(p, q);
+            else atomicAdd(reinterpret_cast<unsigned long long*>(p), (unsigned long long)q);
+          } else {
+            const float v = __uint_as_float(qs[ch]);
+            float* pf = accf + ch * TILE_PX + cell;
+            if (op == LG_BO_MIN || op == LG_BO_MAX) f32_minmax(pf, v, op == LG_BO_MIN);
+            else atomicAdd(pf, v);
+          }
+        }
+      }
+    };
     const uint64_t end = min(U.begin + U.n, A.refs_cap);
     for (uint64_t base = U.begin + (uint64_t)warp * 32; base < end; base += (uint64_t)nwarps * 32) {
       // lane-parallel: fetch 32 segments, set them up and clip them to this tile
       const uint64_t r = base + lane;
       Staged st;
-      int cnt = 0;
+      st.mask = 0;
+      int c0 = 0, cnt = 0;
+      bool big = false;
+      float term[4];
       if (r < end) {
         const uint32_t si = A.refs[r];
         const float4* sp = reinterpret_cast<const float4*>(A.segs + si);
@@ -551,295 +676,156 @@ __global__ void __launch_bounds__(256, 4) k_raster(RasterArgs A) {
         sg.color[0] = cc.x; sg.color[1] = cc.y; sg.color[2] = cc.z; sg.color[3] = cc.w;
         RSetup R;
         if (raster_setup(sg, C.W, C.H, R)) {
-          const int c0 = max(R.lo - tm * TILE, 0), c1 = min(R.hi - tm * TILE, TILE);
-          cnt = max(c1 - c0, 0);
+          c0 = max(R.lo - tm * TILE, 0);
+          cnt = max(min(R.hi - tm * TILE, TILE) - c0, 0);
           st.ua = R.ua; st.va = R.va; st.slope = R.slope;
-          st.span = c0 | (cnt << 16);
-          long long qv[4];
-          bool big = false;
+          if (cnt > 0) st.mask = (cnt >= 32 ? 0xffffffffu : (1u << cnt) - 1u) << c0;
 #pragma unroll
           for (int ch = 0; ch < 4; ++ch) {
             const float v = contribution(B, ch, sg.color);
-            if (MODE == RM_FIXED_SPLIT) {
-              long long q = to_fixed(v);
-              if (B.op[ch] == LG_BO_REVERSE_SUBTRACT) q = -q;
-              qv[ch] = q;
-              big = big || q >= (1ll << SPLIT_LIMIT) || q < -(1ll << SPLIT_LIMIT);
+            const bool neg = B.op[ch] == LG_BO_REVERSE_SUBTRACT;
+            term[ch] = neg ? -v : v;
+            if (SP::on) {
+              if (!split_term<MODE>(v, neg, st.q[2 * ch], st.q[2 * ch + 1])) big = true;
             } else if (MODE == RM_FIXED_MINMAX) {
               long long q = to_fixed(v);
-              if (B.op[ch] == LG_BO_REVERSE_SUBTRACT) q = -q;
+              if (neg) q = -q;
               st.q[2 * ch] = (unsigned)(q & 0xffffffffll);
               st.q[2 * ch + 1] = (unsigned)(q >> 32);
             } else {
-              st.q[ch] = __float_as_uint(B.op[ch] == LG_BO_REVERSE_SUBTRACT ? -v : v);
-            }
-          }
-          if (MODE == RM_FIXED_SPLIT) {
-#pragma unroll
-            for (int ch = 0; ch < 4; ++ch) {
-              const long long q = qv[ch];
-              st.q[2 * ch] = big ? (unsigned)(q & 0xffffffffll) : (unsigned)(q & ((1ll << SPLIT_BITS) - 1));
-              st.q[2 * ch + 1] = big ? (unsigned)(q >> 32) : (unsigned)(int)(q >> SPLIT_BITS);
-            }
-            if (big) st.span |= SPAN_BIG;
-          }
-        }
-      }
-      stage[lane] = st;
-      // pack every (segment, pixel column) pair of the batch densely over the lanes
-      int incl = cnt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, incl, o);
-        if ((int)lane >= o) incl += y;
-      }
-      pref[lane] = incl - cnt;
-      for (int k = 0; k < cnt; ++k) owner[incl - cnt + k] = (uint8_t)lane;
-      const int total = __shfl_sync(0xffffffffu, incl, 31);
-      __syncwarp();
-      for (int pi = (int)lane; pi < total; pi += 32) {
-        const int k = owner[pi];
-        const Staged& sk = stage[k];
-        const int i = tm * TILE + (sk.span & 0xffff) + (pi - pref[k]);  // SPAN_BIG is above bit 16
-        RSetup R;
-        R.ua = sk.ua; R.va = sk.va; R.slope = sk.slope;
-        const int j = raster_minor(R, i);
-        const int jl = j - tn * TILE;
-        if (jl < 0 || jl >= TILE || j >= nmin) continue;
-        const int cell = jl * TILE + (i - tm * TILE);  // [row][col] for x-major, [col][row] for y-major
-        if (MODE == RM_FIXED_SPLIT) {
-          const uint4 q0 = *reinterpret_cast<const uint4*>(&sk.q[0]);
-          const uint4 q1 = *reinterpret_cast<const uint4*>(&sk.q[4]);
-          const unsigned qs[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-          if (sk.span & SPAN_BIG) {  // rare: the 64-bit terms straight into the image
-            const uint32_t x = xmajor ? (uint32_t)i : (uint32_t)j, y = xmajor ? (uint32_t)j : (uint32_t)i;
-            unsigned long long* g = reinterpret_cast<unsigned long long*>(A.accum) + (C.px_base + (uint64_t)y * C.W + x) * 4;
-#pragma unroll
-            for (int ch = 0; ch < 4; ++ch) {
-              const unsigned long long q = ((unsigned long long)qs[2 * ch + 1] << 32) | qs[2 * ch];
-              if (q) atomicAdd(g + ch, q);
-            }
-          } else {
-#pragma unroll
-            for (int w = 0; w < 8; ++w)
-              if (qs[w]) atomicAdd(acc32 + w * TILE_PX + cell, qs[w]);
-          }
-        } else if (MODE == RM_FIXED_MINMAX) {
-#pragma unroll
-          for (int ch = 0; ch < 4; ++ch) {
-            const long long q = (long long)(((unsigned long long)sk.q[2 * ch + 1] << 32) | sk.q[2 * ch]);
-            long long* p = acc64 + ch * TILE_PX + cell;
-            const int op = B.op[ch];
-            if (op == LG_BO_MIN) atomicMin(p, q);
-            else if (op == LG_BO_MAX) atomicMax(p, q);
-            else atomicAdd(reinterpret_cast<unsigned long long*>(p), (unsigned long long)q);
-          }
-        } else {
-#pragma unroll
-          for (int ch = 0; ch < 4; ++ch) {
-            const float v = __uint_as_float(sk.q[ch]);
-            float* pf = accf + ch * TILE_PX + cell;
-            const int op = B.op[ch];
-            if (op == LG_BO_ADD || op == LG_BO_REVERSE_SUBTRACT) atomicAdd(pf, v);
-            else {
-              float o = *pf;
-              while (op == LG_BO_MIN ? v < o : v > o) {
-                const float w = __int_as_float(atomicCAS(reinterpret_cast<int*>(pf), __float_as_int(o), __float_as_int(v)));
-                if (w == o) break;
-                o = w;
-              }
+              st.q[ch] = __float_as_uint(term[ch]);
             }
           }
         }
-        ++my_pixels;
       }
-      __syncwarp();
-    }
-    __syncthreads();
-    // flush: one global atomic per touched pixel channel
-    for (int k = threadIdx.x; k < TILE_PX; k += blockDim.x) {
-      const int row = k / TILE, col = k % TILE;
-      const uint32_t x = tx * TILE + col, y = ty * TILE + row;
-      if (x >= C.W || y >= C.H) continue;
-      const uint64_t px = (C.px_base + (uint64_t)y * C.W + x) * 4;
-      const int cell = xmajor ? row * TILE + col : col * TILE + row;
-#pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        const int op = B.op[ch];
-        if (MODE == RM_FIXED_SPLIT) {
-          const unsigned* base = acc32 + 2 * ch * TILE_PX + cell;
-          const long long q = (long long)(int)base[TILE_PX] * (1ll << SPLIT_BITS) + (long long)base[0];
-          if (q == 0) continue;
-          atomicAdd(reinterpret_cast<unsigned long long*>(A.accum) + px + ch, (unsigned long long)q);
-        } else if (MODE == RM_FIXED_MINMAX) {
-          const long long v = acc64[ch * TILE_PX + cell];
-          if (v == ident64(op)) continue;
-          long long* g = reinterpret_cast<long long*>(A.accum) + px + ch;
-          if (op == LG_BO_MIN) atomicMin(g, v);
-          else if (op == LG_BO_MAX) atomicMax(g, v);
-          else atomicAdd(reinterpret_cast<unsigned long long*>(g), (unsigned long long)v);
-        } else {
-          const float v = accf[ch * TILE_PX + cell];
-          if (v == ident32(op)) continue;
-          float* g = reinterpret_cast<float*>(A.accum) + px + ch;
-          if (op == LG_BO_MIN || op == LG_BO_MAX) {
-            float o = *g;
-            while (op == LG_BO_MIN ? v < o : v > o) {
-              const float w = __int_as_float(atomicCAS(reinterpret_cast<int*>(g), __float_as_int(o), __float_as_int(v)));
-              if (w == o) break;
-              o = w;
-            }
-          } else {
-            atomicAdd(g, v);
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-  add_block_counts<1>({my_pixels}, {&A.ctr->pixels});
-}
-
-// One warp per unit with a private tile: lane L owns pixel column L of the tile (x-major
-// units) or pixel row L (y-major units), and every segment of an x-major unit touches a
-// column at most once, so no two lanes or warps ever update the same accumulator and
-// plain 64-bit read-modify-write replaces atomics.  Units can therefore hold any number
-// of segments (fewer flushes); occupancy is bounded by the 32 KB tile per warp.
-template <int MODE>
-__global__ void __launch_bounds__(32) k_raster_warp(RasterArgs A) {
-  if (A.ctr->skip_raster) return;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  long long* acc64 = reinterpret_cast<long long*>(smem_raw);      // [ch][minor][lane]
-  float* accf = reinterpret_cast<float*>(smem_raw);
-  struct __align__(16) St {
-    float ua, va, slope;
-    int lohi;
-    long long q[4];
-  };
-  St* stage = reinterpret_cast<St*>(smem_raw + 4 * TILE_PX * 8);
-  const unsigned lane = lane_id();
-  const BlendDev& B = A.blend;
-  uint32_t my_pixels = 0;
-  unsigned long long n_units = A.ctr->units;
-  if (n_units > A.units_cap) n_units = A.units_cap;
-  for (;;) {
-    unsigned long long u = 0;
-    if (lane == 0) u = atomicAdd(&A.ctr->unit_cursor, 1ull);
-    u = __shfl_sync(0xffffffffu, u, 0);
-    if (u >= n_units) break;
-    const Unit U = A.units[u];
-    const CanvasLoc C = canvas_of_bin(A, U.tile);
-    const uint32_t lbin = (uint32_t)(U.tile - C.bin_base);
-    const uint32_t tile = lbin >> 1;
-    const bool xmajor = (lbin & 1u) == 0;
-    const uint32_t tx = tile % C.ntx, ty = tile / C.ntx;
-    const int tm = xmajor ? (int)tx : (int)ty, tn = xmajor ? (int)ty : (int)tx;
-    const int nmin = (int)(xmajor ? C.H : C.W);
-    const int i = tm * TILE + (int)lane;
-    for (int k = (int)lane; k < 4 * TILE_PX; k += 32) {
-      if (MODE == RM_F32) accf[k] = ident32(B.op[k / TILE_PX]);
-      else acc64[k] = ident64(B.op[k / TILE_PX]);
-    }
-    __syncwarp();
-    const uint64_t end = min(U.begin + U.n, A.refs_cap);
-    for (uint64_t base = U.begin; base < end; base += 32) {
-      const uint64_t r = base + lane;
-      St st;
-      st.lohi = -1;
-      if (r < end) {
-        const uint32_t si = A.refs[r];
-        const float4* sp = reinterpret_cast<const float4*>(A.segs + si);
-        const float4 g = __ldg(sp), cc = __ldg(sp + 1);
-        lg_segment sg;
-        sg.x0 = g.x; sg.y0 = g.y; sg.x1 = g.z; sg.y1 = g.w;
-        sg.color[0] = cc.x; sg.color[1] = cc.y; sg.color[2] = cc.z; sg.color[3] = cc.w;
-        RSetup R;
-        if (raster_setup(sg, C.W, C.H, R)) {
-          st.ua = R.ua; st.va = R.va; st.slope = R.slope;
-          st.lohi = R.lo | (R.hi << 16);
+      if (SP::on) {  // rare: terms outside the split's range go straight into the image
+        unsigned bigs = __ballot_sync(0xffffffffu, big && cnt > 0);
+        if (big) cnt = 0;
+        while (bigs) {
+          const int k = __ffs(bigs) - 1;
+          bigs &= bigs - 1;
+          const float bua = __shfl_sync(0xffffffffu, st.ua, k), bva = __shfl_sync(0xffffffffu, st.va, k);
+          const float bsl = __shfl_sync(0xffffffffu, st.slope, k);
+          const unsigned bm = __shfl_sync(0xffffffffu, st.mask, k);
+          const int i = tm * TILE + (int)lane;
+          const float v = __fmaf_rn(__fsub_rn(__fadd_rn((float)i, 0.5f), bua), bsl, bva);
+          const bool on = ((bm >> lane) & 1u) && v >= vlo && v < vhi;
+          const int j = on ? (int)v : 0;
+          const uint32_t x = xmajor ? (uint32_t)i : (uint32_t)j, y = xmajor ? (uint32_t)j : (uint32_t)i;
+          const uint64_t px = (C.px_base + (uint64_t)y * C.W + x) * 4;
 #pragma unroll
           for (int ch = 0; ch < 4; ++ch) {
-            const float v = contribution(B, ch, sg.color);
+            const float tv = __shfl_sync(0xffffffffu, term[ch], k);
+            if (!on) continue;
             if (MODE == RM_F32) {
-              st.q[ch] = (long long)__float_as_uint(B.op[ch] == LG_BO_REVERSE_SUBTRACT ? -v : v);
+              image_add(A, px + ch, (double)tv);
             } else {
-              const long long q = to_fixed(v);
-              st.q[ch] = B.op[ch] == LG_BO_REVERSE_SUBTRACT ? -q : q;
+              const long long q = to_fixed(tv);
+              if (q) atomicAdd(reinterpret_cast<unsigned long long*>(A.accum) + px + ch, (unsigned long long)q);
             }
           }
+          my_pixels += on ? 1u : 0u;
         }
       }
-      stage[lane] = st;
+      // the batch's segments with columns here, side by side in the warp's stage
+      const unsigned drawn = __ballot_sync(0xffffffffu, cnt > 0);
+      const int n_drawn = __popc(drawn), pos = __popc(drawn & lanemask_lt());
+      const int total = (int)__reduce_add_sync(0xffffffffu, (unsigned)cnt);
+      const bool alpha_c = SP::on && __any_sync(0xffffffffu, cnt > 0 && st.q[6] != 0u);
+      if (cnt > 0) stage[pos] = st;
+      if (total >= LG_RASTER_LANE_MIN * n_drawn) {
+        __syncwarp();
+        const float fi = __fadd_rn((float)(tm * TILE + (int)lane), 0.5f);
+        const int cell0 = (int)lane - tn * TILE_PX;
+        const unsigned bit = 1u << lane;
+        auto draw = [&](auto low_alpha) {
+#pragma unroll 2
+          for (int k = 0; k < n_drawn; ++k) {
+            const Staged& sk = stage[k];
+            const float4 h = *reinterpret_cast<const float4*>(&sk);
+            const uint4 q0 = *reinterpret_cast<const uint4*>(&sk.q[0]);
+            const uint4 q1 = *reinterpret_cast<const uint4*>(&sk.q[4]);
+            const float v = __fmaf_rn(__fsub_rn(fi, h.x), h.z, h.y);
+            const bool on = (__float_as_uint(h.w) & bit) && v >= vlo && v < vhi;
+            deposit(q0, q1, (int)v * TILE + cell0, on, decltype(low_alpha)::value);
+            my_pixels += on ? 1u : 0u;
+          }
+        };
+        if (alpha_c) draw(std::true_type{}); else draw(std::false_type{});
+      } else {
+        // every (segment, pixel column) pair of the batch densely over the lanes
+        int incl = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int y = __shfl_up_sync(0xffffffffu, incl, o);
+          if ((int)lane >= o) incl += y;
+        }
+        if (cnt > 0) pref[pos] = incl - cnt - c0;  // pair number less the column
+        for (int k = 0; k < cnt; ++k) owner[incl - cnt + k] = (uint8_t)pos;
+        __syncwarp();
+        for (int pi = (int)lane; pi < total; pi += 32) {
+          const int k = owner[pi];
+          const Staged& sk = stage[k];
+          const int col = pi - pref[k];
+          const float fi = __fadd_rn((float)(tm * TILE + col), 0.5f);
+          const float v = __fmaf_rn(__fsub_rn(fi, sk.ua), sk.slope, sk.va);
+          if (!(v >= vlo && v < vhi)) continue;
+          deposit(*reinterpret_cast<const uint4*>(&sk.q[0]), *reinterpret_cast<const uint4*>(&sk.q[4]),
+                  ((int)v - tn * TILE) * TILE + col, true, alpha_c);
+          ++my_pixels;
+        }
+      }
       __syncwarp();
-      const int n = (int)min((uint64_t)32, end - base);
-      for (int k = 0; k < n; ++k) {
-        const int lohi = stage[k].lohi;
-        if (lohi < 0 || i < (lohi & 0xffff) || i >= (lohi >> 16)) continue;
-        RSetup R;
-        R.ua = stage[k].ua; R.va = stage[k].va; R.slope = stage[k].slope;
-        const int j = raster_minor(R, i);
-        const int jl = j - tn * TILE;
-        if (jl < 0 || jl >= TILE || j >= nmin) continue;
-        const int cell = jl * TILE + (int)lane;
+    }
+    __syncthreads();
+    if (SP::on) {
+      // flush: four lanes per pixel, one channel each, so that a warp's atomics cover whole
+      // 32 B sectors of the image
+      for (int k = threadIdx.x; k < 4 * TILE_PX; k += blockDim.x) {
+        const int ch = k & 3, cell = k >> 2;
+        const int major = cell % TILE, minor = cell / TILE;
+        const uint32_t x = tx * TILE + (xmajor ? major : minor), y = ty * TILE + (xmajor ? minor : major);
+        const unsigned* plane = acc32 + 2 * ch * PLANE + cell;
+        const long long q = (long long)(int)plane[PLANE] * (1ll << SP::bits) + (long long)(int)plane[0];
+        if (q == 0 || x >= C.W || y >= C.H) continue;
+        const uint64_t px = (C.px_base + (uint64_t)y * C.W + x) * 4;
+        if (MODE == RM_F32)
+          image_add(A, px + ch, __dmul_rn(__ll2double_rn(q), 4.547473508864641e-13));  // 2^-41: both steps exact
+        else
+          atomicAdd(reinterpret_cast<unsigned long long*>(A.accum) + px + ch, (unsigned long long)q);
+      }
+    } else {
+      // flush: one global atomic per touched pixel channel
+      for (int k = threadIdx.x; k < TILE_PX; k += blockDim.x) {
+        const int row = k / TILE, col = k % TILE;
+        const uint32_t x = tx * TILE + col, y = ty * TILE + row;
+        if (x >= C.W || y >= C.H) continue;
+        const uint64_t px = (C.px_base + (uint64_t)y * C.W + x) * 4;
+        const int cell = xmajor ? row * TILE + col : col * TILE + row;
 #pragma unroll
         for (int ch = 0; ch < 4; ++ch) {
           const int op = B.op[ch];
-          const long long q = stage[k].q[ch];
-          if (MODE == RM_F32) {
-            float& a = accf[ch * TILE_PX + cell];
-            const float v = __uint_as_float((unsigned)q);
-            a = op == LG_BO_MIN ? fminf(a, v) : op == LG_BO_MAX ? fmaxf(a, v) : a + v;
+          if (MODE == RM_FIXED_MINMAX) {
+            const long long v = acc64[ch * TILE_PX + cell];
+            if (v == ident64(op)) continue;
+            long long* g = reinterpret_cast<long long*>(A.accum) + px + ch;
+            if (op == LG_BO_MIN) atomicMin(g, v);
+            else if (op == LG_BO_MAX) atomicMax(g, v);
+            else atomicAdd(reinterpret_cast<unsigned long long*>(g), (unsigned long long)v);
           } else {
-            long long& a = acc64[ch * TILE_PX + cell];
-            a = op == LG_BO_MIN ? min(a, q) : op == LG_BO_MAX ? max(a, q) : a + q;
+            const float v = accf[ch * TILE_PX + cell];
+            if (v == ident32(op)) continue;
+            float* g = reinterpret_cast<float*>(A.accum) + px + ch;
+            if (op == LG_BO_MIN || op == LG_BO_MAX) f32_minmax(g, v, op == LG_BO_MIN);
+            else atomicAdd(g, v);
           }
-        }
-        ++my_pixels;
-      }
-      __syncwarp();
-    }
-    // flush the private tile: one global atomic per touched pixel channel
-    for (int k = (int)lane; k < TILE_PX; k += 32) {
-      const int jl = k / TILE, c = k % TILE;  // cell k = [minor][lane]
-      const uint32_t x = xmajor ? tx * TILE + c : tx * TILE + jl;
-      const uint32_t y = xmajor ? ty * TILE + jl : ty * TILE + c;
-      if (x >= C.W || y >= C.H) continue;
-      const uint64_t px = (C.px_base + (uint64_t)y * C.W + x) * 4;
-#pragma unroll
-      for (int ch = 0; ch < 4; ++ch) {
-        const int op = B.op[ch];
-        if (MODE == RM_F32) {
-          const float v = accf[ch * TILE_PX + k];
-          if (v == ident32(op)) continue;
-          float* g = reinterpret_cast<float*>(A.accum) + px + ch;
-          if (op == LG_BO_MIN || op == LG_BO_MAX) {
-            float o = *g;
-            while (op == LG_BO_MIN ? v < o : v > o) {
-              const float w = __int_as_float(atomicCAS(reinterpret_cast<int*>(g), __float_as_int(o), __float_as_int(v)));
-              if (w == o) break;
-              o = w;
-            }
-          } else {
-            atomicAdd(g, v);
-          }
-        } else {
-          const long long v = acc64[ch * TILE_PX + k];
-          if (v == ident64(op)) continue;
-          long long* g = reinterpret_cast<long long*>(A.accum) + px + ch;
-          if (op == LG_BO_MIN) atomicMin(g, v);
-          else if (op == LG_BO_MAX) atomicMax(g, v);
-          else atomicAdd(reinterpret_cast<unsigned long long*>(g), (unsigned long long)v);
         }
       }
     }
-    __syncwarp();
+    __syncthreads();
   }
   add_block_counts<1>({my_pixels}, {&A.ctr->pixels});
 }
-
-template __global__ void k_raster_warp<RM_FIXED_SPLIT>(RasterArgs A);
-template __global__ void k_raster_warp<RM_F32>(RasterArgs A);
-int raster_warp_smem_bytes() { return 4 * TILE_PX * 8 + 32 * 48; }
 
 // ------------------------------------------------------------------ string-mod lines
 // A few thousand lines per frame: one warp per line, one lane per major-axis pixel, and
@@ -898,7 +884,7 @@ __global__ void __launch_bounds__(256) k_raster_chords(RasterArgs A, const lg_ch
               o = w;
             }
           } else {
-            atomicAdd(g, op == LG_BO_REVERSE_SUBTRACT ? -v : v);
+            image_add(A, px + ch, op == LG_BO_REVERSE_SUBTRACT ? -v : v);
           }
         }
       }
@@ -911,18 +897,43 @@ __global__ void __launch_bounds__(256) k_raster_chords(RasterArgs A, const lg_ch
 template __global__ void k_raster_chords<true>(RasterArgs A, const lg_chord* chords, uint64_t n);
 template __global__ void k_raster_chords<false>(RasterArgs A, const lg_chord* chords, uint64_t n);
 
-template __global__ void k_raster<RM_FIXED_SPLIT>(RasterArgs A);
-template __global__ void k_raster<RM_FIXED_MINMAX>(RasterArgs A);
-template __global__ void k_raster<RM_F32>(RasterArgs A);
-
-int raster_smem_bytes(int mode) {
-  return mode == RM_FIXED_SPLIT ? RasterSmem<RM_FIXED_SPLIT>::bytes
-                                : mode == RM_FIXED_MINMAX ? RasterSmem<RM_FIXED_MINMAX>::bytes : RasterSmem<RM_F32>::bytes;
+static void (*raster_kernel(int mode))(RasterArgs) {
+  switch (mode) {
+    case RM_FIXED_SPLIT_: return k_raster<RM_FIXED_SPLIT>;
+    case RM_FIXED_MINMAX_: return k_raster<RM_FIXED_MINMAX>;
+    case RM_F32_: return k_raster<RM_F32>;
+    default: return k_raster<RM_F32_MINMAX>;
+  }
+}
+static int raster_smem_bytes(int mode) {
+  switch (mode) {
+    case RM_FIXED_SPLIT_: return RasterSmem<RM_FIXED_SPLIT>::bytes;
+    case RM_FIXED_MINMAX_: return RasterSmem<RM_FIXED_MINMAX>::bytes;
+    case RM_F32_: return RasterSmem<RM_F32>::bytes;
+    default: return RasterSmem<RM_F32_MINMAX>::bytes;
+  }
 }
 
+cudaError_t raster_occupancy(int mode, int* occ) {
+  cudaError_t e = cudaFuncSetAttribute(raster_kernel(mode), cudaFuncAttributeMaxDynamicSharedMemorySize, raster_smem_bytes(mode));
+  if (e == cudaSuccess)
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(occ, raster_kernel(mode), 256, (size_t)raster_smem_bytes(mode));
+  return e;
+}
+
+void launch_raster(int mode, int grid, cudaStream_t stream, const RasterArgs& A) {
+  raster_kernel(mode)<<<grid, 256, (size_t)raster_smem_bytes(mode), stream>>>(A);
+}
+
+uint32_t raster_unit_refs(int mode) { return mode == RM_F32_ ? F32_UNIT_REFS : SPLIT_UNIT_REFS; }
+
 // ------------------------------------------------------------------ resolve
-__device__ __forceinline__ float4 load_px(const void* acc, int fixed, uint64_t i) {
-  if (fixed) {
+__device__ __forceinline__ float4 load_px(const void* acc, int kind, uint64_t i) {
+  if (kind == ACC_F64) {
+    const double4_32a v = reinterpret_cast<const double4_32a*>(acc)[i];
+    return make_float4(__double2float_rn(v.x), __double2float_rn(v.y), __double2float_rn(v.z), __double2float_rn(v.w));
+  }
+  if (kind == ACC_I64) {
     const longlong4_32a v = reinterpret_cast<const longlong4_32a*>(acc)[i];
     const float s = 2.3283064365386963e-10f;  // 2^-32
     return make_float4(__fmul_rn(__ll2float_rn(v.x), s), __fmul_rn(__ll2float_rn(v.y), s),
@@ -931,10 +942,10 @@ __device__ __forceinline__ float4 load_px(const void* acc, int fixed, uint64_t i
   return reinterpret_cast<const float4*>(acc)[i];
 }
 
-__global__ void k_resolve_f16(const void* acc, int fixed, uint32_t W, uint32_t H, uint16_t* dst, size_t pitch) {
+__global__ void k_resolve_f16(const void* acc, int kind, uint32_t W, uint32_t H, uint16_t* dst, size_t pitch) {
   const uint64_t n = (uint64_t)W * H;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const float4 f = load_px(acc, fixed, i);
+    const float4 f = load_px(acc, kind, i);
     const uint32_t y = (uint32_t)(i / W), x = (uint32_t)(i % W);
     ushort4 h;
     h.x = __half_as_ushort(__float2half_rn(f.x));
@@ -946,10 +957,10 @@ __global__ void k_resolve_f16(const void* acc, int fixed, uint32_t W, uint32_t H
 }
 
 // renderer.rs:313-328: u8 = (f16 value ^ (1 / 2.2) * 255) as u8 (saturating, truncating)
-__global__ void k_resolve_rgba8(const void* acc, int fixed, uint32_t W, uint32_t H, uint8_t* dst, size_t pitch) {
+__global__ void k_resolve_rgba8(const void* acc, int kind, uint32_t W, uint32_t H, uint8_t* dst, size_t pitch) {
   const uint64_t n = (uint64_t)W * H;
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const float4 f = load_px(acc, fixed, i);
+    const float4 f = load_px(acc, kind, i);
     const uint32_t y = (uint32_t)(i / W), x = (uint32_t)(i % W);
     const float c[4] = {f.x, f.y, f.z, f.w};
     uchar4 o;

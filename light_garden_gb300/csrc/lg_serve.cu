@@ -267,12 +267,12 @@ lg_status serve_raster_args(lg_ctx* c, ServeState& V, RasterArgs& A) {
   if ((st = ensure(c, c->d_units, c->units_cap * sizeof(Unit), "raster units"))) return st;
   const size_t parts = (bins + TILE_SCAN_CHUNK - 1) / TILE_SCAN_CHUNK;
   if ((st = ensure(c, c->d_part, std::max<size_t>(parts, 1) * 16, "tile scan partials"))) return st;
-  c->raster_variant = 1;
   A = raster_args(c);
   A.seg_scene = (const uint16_t*)c->d_seg_scene.p;
   A.canvases = (const SceneCanvas*)c->d_canvases.p;
   A.n_scenes = V.max_slots;
   A.accum = V.d_acc.p;
+  A.acc = ACC_I64;
   A.W = 0;
   A.H = 0;
   A.n_tiles = c->total_bins;
@@ -312,7 +312,7 @@ lg_status serve_raster(lg_ctx* c, ServeState& V) {
     if (bins) {
       k_build_units<<<std::max(1u, (bins + 255) / 256), 256, 0, c->stream>>>(A);
       k_bin_scatter<<<scatter_grid(c->n_sm, 0), SCATTER_THREADS, 0, c->stream>>>(A, 0);
-      k_raster<RM_FIXED_SPLIT_><<<c->raster_grid, 256, (size_t)raster_smem_bytes(RM_FIXED_SPLIT_), c->stream>>>(A);
+      launch_raster(RM_FIXED_SPLIT_, c->raster_grid, c->stream, A);
     }
     k_stream_rotate<<<1, 1, 0, c->stream>>>(dctr, c->seg_cap);
     CK(cudaGetLastError(), "raster launch");
@@ -404,9 +404,7 @@ lg_status lg_serve_begin(lg_ctx* c, const lg_serve_opts* opts) {
   c->scan_tune = false;
   if ((st = scan_grid(c, true))) { serve_free(c); return st; }
   if ((st = trace_grids(c, true, 0))) { serve_free(c); return st; }
-  const int rsm = raster_smem_bytes(RM_FIXED_SPLIT_);
-  CK(cudaFuncSetAttribute(k_raster<RM_FIXED_SPLIT_>, cudaFuncAttributeMaxDynamicSharedMemorySize, rsm), "smem attr");
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_raster<RM_FIXED_SPLIT_>, 256, rsm), "occupancy");
+  CK(raster_occupancy(RM_FIXED_SPLIT_, &occ), "occupancy");
   c->raster_grid = c->n_sm * std::max(1, occ);
   CK(cudaStreamSynchronize(c->stream), "synchronize");
   return LG_OK;
@@ -526,7 +524,8 @@ lg_status lg_serve_step(lg_ctx* c, lg_serve_step_stats* stats) {
       A.H = 1;
       A.accum = (char*)V.d_acc.p + sl.acc_off * 32;
       for (int ch = 0; ch < 4; ++ch) A.blend.clear[ch] = V.common.clear_color[ch];
-      k_clear_accum<<<c->n_sm * 4, 256, 0, c->stream>>>(A, 1);
+      A.acc = ACC_I64;
+      k_clear_accum<<<c->n_sm * 4, 256, 0, c->stream>>>(A);
     }
   } else {
     light_lo = light_hi = c->n_lights;
@@ -609,7 +608,7 @@ lg_status lg_serve_step(lg_ctx* c, lg_serve_step_stats* stats) {
   }
   for (uint32_t s : finished) {
     Slot& sl = V.slots[s];
-    k_resolve_f16<<<c->n_sm * 4, 256, 0, c->stream>>>((const char*)V.d_acc.p + sl.acc_off * 32, 1,
+    k_resolve_f16<<<c->n_sm * 4, 256, 0, c->stream>>>((const char*)V.d_acc.p + sl.acc_off * 32, ACC_I64,
                                                       (uint32_t)sl.req.px(), 1,
                                                       (uint16_t*)((char*)V.d_res.p + sl.res_off * 8), sl.req.px() * 8);
     Done d;
