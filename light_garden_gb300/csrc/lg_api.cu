@@ -801,7 +801,8 @@ lg_status trace_grids(lg_ctx* c, bool multi, size_t tsm) {
   return LG_OK;
 }
 
-void launch_light_setup(lg_ctx* c, const SceneDev& S, bool multi, int blocks) {
+void launch_light_setup(lg_ctx* c, const SceneDev& S, bool multi) {
+  const int blocks = (int)std::min<uint32_t>((S.n_lights + 7) / 8, (uint32_t)c->n_sm * 8);  // a warp per light
   if (c->prm.precision == LG_PRECISION_EXACT) {
     if (multi) k_light_setup_x<true><<<blocks, 256, 0, c->stream>>>(S);
     else k_light_setup_x<false><<<blocks, 256, 0, c->stream>>>(S);
@@ -948,7 +949,7 @@ lg_status enqueue_trace(lg_ctx* c) {
   const SceneDev S = scene_dev(c);
   const TraceBufs B = trace_bufs(c);
   CK(cudaMemsetAsync(c->d_ctr.p, 0, sizeof(Counters), c->stream), "memset counters");
-  if (c->n_lights) launch_light_setup(c, S, false, 1);
+  if (c->n_lights) launch_light_setup(c, S, false);
   const size_t tsm = c->smem_fits ? c->obj_smem : 0;
   for (uint32_t g = 0; g < c->prm.max_bounce; ++g)
     launch_generation(c, S, B, g, false, c->trace_grid[0], (size_t)scan_smem_bytes(scan_pairs_of(c)) + tsm, tsm, c->smem_fits);
@@ -1431,7 +1432,7 @@ static lg_status enqueue_stream_frame(lg_ctx* c, uint16_t* dst, size_t row, cuda
   CK(cudaEventRecordWithFlags(ev[0], c->stream, cudaEventRecordExternal), "stage event");
   CK(cudaMemsetAsync(c->d_ctr.p, 0, sizeof(Counters), c->stream), "memset counters");
   k_clear_accum<<<c->n_sm * 8, 256, 0, c->stream>>>(A);
-  if (c->n_lights) launch_light_setup(c, S, false, 1);
+  if (c->n_lights) launch_light_setup(c, S, false);
   const size_t tsm = c->smem_fits ? c->obj_smem : 0;
   const uint32_t bins = 2 * c->n_tiles;
   const int smem_tiles = bins <= MAX_SMEM_TILES ? 1 : 0;

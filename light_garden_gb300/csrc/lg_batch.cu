@@ -81,7 +81,7 @@ lg_status enqueue_batch(lg_ctx* c, cudaEvent_t* ev) {
   CK(cudaMemsetAsync(c->d_ctr.p, 0, sizeof(Counters), c->stream), "memset counters");
   CK(cudaMemsetAsync(c->d_scene_count.p, 0, (size_t)c->n_scenes * 4, c->stream), "memset scene counts");
   k_clear_accum<<<c->n_sm * 8, 256, 0, c->stream>>>(A);
-  if (c->n_lights) launch_light_setup(c, S, true, (int)((c->n_lights + 255) / 256));
+  if (c->n_lights) launch_light_setup(c, S, true);
   const uint32_t bins = c->total_bins;
   const int smem_tiles = bins <= MAX_SMEM_TILES ? 1 : 0;
   const size_t bsm = smem_tiles ? (size_t)bins * 4 : 0;

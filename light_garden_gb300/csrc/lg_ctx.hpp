@@ -136,7 +136,7 @@ TraceKernel3 bounce_x_kernel(bool multi, bool culled);
 lg_status trace_grids(lg_ctx* c, bool multi, size_t tsm);
 // The light setup and one generation's chain for the context's precision: the FP32 scan,
 // then k_refine + k_full + k_bounce (fast) or k_solve_x + k_bounce_x (exact).
-void launch_light_setup(lg_ctx* c, const SceneDev& S, bool multi, int blocks);
+void launch_light_setup(lg_ctx* c, const SceneDev& S, bool multi);
 void launch_generation(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_t g, bool multi, int scan_grid,
                        size_t scan_smem, size_t tsm, int smem_fits);
 // Uploads a flattened scene's exact-mode tables (geometry nodes, preorder trees).

@@ -64,19 +64,25 @@ __device__ __forceinline__ bool obj_contains_f(const SceneDev& S, uint32_t k, V 
 }
 
 // Light start media (tracer.rs:280-287: the last object with a material containing the
-// light's position) and spot base angles (light.rs:230-234), once per frame.
+// light's position) and spot base angles (light.rs:230-234), once per frame.  Bound: latency
+// (a chain of dependent loads and FP64 tests per object).  A warp per light tests 32 objects at
+// a time from the end of the table, each in FP32 first; one thread per light walking the table
+// took 1.2 ms on 256 CSG objects and 3.6 ms on a batch with a 1024-object scene.
 template <bool MULTI>
 __global__ void k_light_setup_x(SceneDev S) {
   const uint32_t l0 = S.serve ? S.light_lo : 0u, l1 = S.serve ? S.light_hi : S.n_lights;
-  for (uint32_t l = l0 + blockIdx.x * blockDim.x + threadIdx.x; l < l1; l += gridDim.x * blockDim.x) {
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t l = l0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); l < l1; l += warps) {
     LightDev& L = S.lights[l];
     const SceneLoc sl = scene_of<MULTI>(S, L.scene);
-    double n = 1.0;
     const V p = lgx::mk(L.ox, L.oy);
-    for (uint32_t k = sl.base; k < sl.base + sl.n; ++k)
-      if (obj_contains_x(S, k, p, nullptr) && (S.info[k].flags & INFO_MATERIAL)) n = S.info[k].n64;
-    L.n0x = n;
-    L.dir_angle = lgx::spot_base_angle(L.vx, L.vy);
+    const uint32_t k = last_object_of_warp(sl.base, sl.n, [&](uint32_t j) {
+      return (S.info[j].flags & INFO_MATERIAL) && obj_contains_f(S, j, p, nullptr);
+    });
+    if (lane_id() == 0) {
+      L.n0x = k == 0xffffffffu ? 1.0 : S.info[k].n64;
+      L.dir_angle = lgx::spot_base_angle(L.vx, L.vy);
+    }
   }
 }
 template __global__ void k_light_setup_x<false>(SceneDev);

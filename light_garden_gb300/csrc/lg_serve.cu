@@ -543,7 +543,7 @@ lg_status lg_serve_step(lg_ctx* c, lg_serve_step_stats* stats) {
     SceneDev SL = SD;
     SL.light_lo = 0;
     SL.light_hi = c->n_lights;
-    launch_light_setup(c, SL, true, (int)((c->n_lights + 255) / 256));
+    launch_light_setup(c, SL, true);
   }
   if (V.live > 0) {  // queued rays in scene order
     k_scene_hist<<<c->n_sm * 8, 256, 0, c->stream>>>(SD, B, g, (unsigned*)c->d_scene_count.p);

@@ -110,19 +110,21 @@ __device__ inline void primary_ray(const LightDev& L, uint64_t i, double& ox, do
   }
 }
 
+// Start media (tracer.rs:280-287: the last object that contains the light wins), a warp per
+// light: see k_light_setup_x.
 template <bool MULTI>
 __global__ void k_light_setup(SceneDev S) {
   const uint32_t l0 = S.serve ? S.light_lo : 0u, l1 = S.serve ? S.light_hi : S.n_lights;
-  for (uint32_t l = l0 + blockIdx.x * blockDim.x + threadIdx.x; l < l1; l += gridDim.x * blockDim.x) {
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t l = l0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); l < l1; l += warps) {
     LightDev& L = S.lights[l];
     const SceneLoc sl = scene_of<MULTI>(S, L.scene);
-    df n = DF_ONE;  // tracer.rs:280-287: the last containing object wins
     const df px = df_from_double(L.ox), py = df_from_double(L.oy);
-    for (uint32_t k = sl.base; k < sl.base + sl.n; ++k) {
+    const uint32_t k = last_object_of_warp(sl.base, sl.n, [&](uint32_t j) {
       bool near = false;
-      if ((S.info[k].flags & INFO_MATERIAL) && obj_contains64(S, k, px, py, near, 0.0f)) n = S.info[k].n;
-    }
-    L.n0 = n;
+      return (S.info[j].flags & INFO_MATERIAL) && obj_contains64(S, j, px, py, near, 0.0f);
+    });
+    if (lane_id() == 0) L.n0 = k == 0xffffffffu ? DF_ONE : S.info[k].n;
   }
 }
 template __global__ void k_light_setup<false>(SceneDev);

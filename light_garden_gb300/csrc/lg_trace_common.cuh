@@ -27,6 +27,18 @@ __device__ __forceinline__ bool bound_test(const float4& h, float ox, float oy, 
   return lb <= thr;
 }
 
+// The last object of [base, base + n) for which pred holds (0xffffffff: none): the warp's lanes
+// try 32 objects at a time, from the end.  Every lane of the warp calls it.
+template <class F>
+__device__ __forceinline__ uint32_t last_object_of_warp(uint32_t base, uint32_t n, F&& pred) {
+  for (uint32_t c = (n + 31) / 32; c-- > 0;) {
+    const uint32_t j = c * 32 + lane_id();
+    const unsigned hit = __ballot_sync(0xffffffffu, j < n && pred(base + j));
+    if (hit) return base + c * 32 + 31u - (unsigned)__clz(hit);
+  }
+  return 0xffffffffu;
+}
+
 // Queued rays a launch takes (the children of the previous generation or step) ...
 __device__ __forceinline__ uint64_t n_real_of(const SceneDev& S, const TraceBufs& B, uint32_t gen) {
   if (gen == 0 && !S.serve) return 0;
