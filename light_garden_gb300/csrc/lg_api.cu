@@ -295,9 +295,29 @@ lg_status validate_exact(std::string& err, const lg_params& p, const Flat& F) {
   return LG_OK;
 }
 
+// Constants of a geometry node that the exact solve would compute per hit, each rounded once
+// (volatile: no host compiler may fuse a product into a sum), in slots its kind leaves free:
+// CIRCLE v[1] = 1 / r; RECT v[2], v[3] = half width and height; SEGMENT v[4], v[5] = the unit left
+// normal ((0, 0) for a zero-length segment).
+static void derive_constants(lg_geo& g) {
+  if (g.kind == LG_GEO_CIRCLE) {
+    g.v[1] = 1.0 / g.v[0];
+  } else if (g.kind == LG_GEO_RECT) {
+    g.v[2] = 0.5 * g.v[0];
+    g.v[3] = 0.5 * g.v[1];
+  } else if (g.kind == LG_GEO_SEGMENT) {
+    volatile double ex = g.v[2] - g.v[0], ey = g.v[3] - g.v[1];
+    volatile double xx = ex * ex, yy = ey * ey, l2 = xx + yy;
+    volatile double l = std::sqrt(l2);
+    g.v[4] = l > 0.0 ? -ey / l : 0.0;
+    g.v[5] = l > 0.0 ? ex / l : 0.0;
+  }
+}
+
 lg_status flatten_scene(std::string& err, const lg_geo* G, uint32_t n_geo, const lg_object* O, uint32_t n_obj,
                         const lg_light* Ls, uint32_t n_lights, Flat& F) {
   F.xgeo.assign(G, G + n_geo);
+  for (lg_geo& g : F.xgeo) derive_constants(g);
   for (uint32_t k = 0; k < n_obj; ++k) {
     const lg_object& o = O[k];
     if (o.kind < 0 || o.kind > LG_OBJ_GEO) return set_err(err, LG_ERR_INVALID_ARGUMENT, "object " + std::to_string(k) + ": unknown kind");
@@ -327,6 +347,7 @@ lg_status flatten_scene(std::string& err, const lg_geo* G, uint32_t n_geo, const
                ((o.kind == LG_OBJ_STRAIGHT_MIRROR || o.kind == LG_OBJ_CURVED_MIRROR) ? INFO_NO_CONTAINS : 0u);
     oi.n = DF(o.has_material ? o.refractive_index : 1.0);
     oi.n64 = o.has_material ? o.refractive_index : 1.0;
+    oi.inv_n64 = 1.0 / oi.n64;
     oi.xnode_begin = (uint32_t)F.xnode.size();
     {
       std::vector<lgx::XNode> nodes;

@@ -76,7 +76,7 @@ struct __align__(16) ObjInfo {
   df n;               // refractive index
   double n64;         // the same in FP64 (exact mode)
   uint32_t xnode_begin, xnode_count;  // exact mode: the object's geometry tree in preorder (lgx::XNode)
-  uint64_t _pad;
+  double inv_n64;     // 1 / n64, rounded once (exact mode: the index ratio of a ray entering from air)
 };
 static_assert(sizeof(ObjInfo) == 48, "ObjInfo is 48 B");
 

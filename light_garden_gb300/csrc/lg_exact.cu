@@ -81,6 +81,7 @@ __global__ void k_light_setup_x(SceneDev S) {
     });
     if (lane_id() == 0) {
       L.n0x = k == 0xffffffffu ? 1.0 : S.info[k].n64;
+      L.n0 = k == 0xffffffffu ? DF_ONE : S.info[k].n;
       L.dir_angle = lgx::spot_base_angle(L.vx, L.vy);
     }
   }
@@ -123,8 +124,9 @@ static __device__ __noinline__ double obj_best_x(const SceneDev& S, uint32_t k, 
 // 2 axis + (outward sign > 0); s32: a cubic's curve parameter): the very operations of
 // leaf_hits for that root only.  A circle computes the quotient of its proved root (q / a or
 // c / q, told apart by their FP32 values) and not the other; a rect computes the slab quotient
-// of its proved face and not the other three; a cubic searches only the bracket that holds
-// s32.  Other leaves take leaf_hits and the root nearest t32.  False: no such hit (the caller
+// of its proved face and not the other three; a segment its ray parameter and not the place
+// along it; a cubic searches only the bracket that holds s32, and in it only near s32.  Other
+// leaves take leaf_hits and the root nearest t32.  False: no such hit (the caller
 // solves the object whole).
 __device__ __forceinline__ bool leaf_proved_hit(const lg_geo* G, const lg_geo& g, V o, V d, float t32, int face32,
                                                 float s32, double& ev, lgx::Hit& out) {
@@ -149,14 +151,24 @@ __device__ __forceinline__ bool leaf_proved_hit(const lg_geo* G, const lg_geo& g
     if (face32 < 0) return false;
     const int ax = face32 >> 1;
     const bool pos = (face32 & 1) != 0;
-    const V lo = irot(vsub(o, mk(g.origin[0], g.origin[1])), g.rot[0], g.rot[1]);
-    const V ld = irot(d, g.rot[0], g.rot[1]);
-    const double h = mul(0.5, g.v[ax]);
-    const double O = ax ? lo.y : lo.x, D = ax ? ld.y : ld.x;
+    // the face's axis of irot(o - centre) and irot(d) alone: x' = c x + s y, y' = -s x + c y
+    const V rel = vsub(o, mk(g.origin[0], g.origin[1]));
+    const double kx = ax ? -g.rot[1] : g.rot[0], ky = ax ? g.rot[0] : g.rot[1];
+    const double O = add(mul(kx, rel.x), mul(ky, rel.y)), D = add(mul(kx, d.x), mul(ky, d.y));
+    const double h = ax ? g.v[3] : g.v[2];
     if (is_zero(D)) return false;
     const double t = dvd(sub(pos ? h : -h, O), D);
     if (!gt_pos(t, T_MIN)) return false;
     out = mkhit(t, o, d, mk(0.0, 0.0), ax + (pos ? 2 : 0));
+    return true;
+  }
+  if (g.kind == LG_GEO_SEGMENT) {  // the crossing lies well inside the segment: t alone
+    const V A = mk(g.v[0], g.v[1]), e = vsub(mk(g.v[2], g.v[3]), A);
+    const double den = cross(d, e);
+    if (is_zero(den)) return false;
+    const double t = dvd(cross(vsub(A, o), e), den);
+    if (!gt_pos(t, T_MIN)) return false;
+    out = mkhit(t, o, d, mk(0.0, 0.0), 0);
     return true;
   }
   if (g.kind == LG_GEO_CUBIC && s32 > 0.0f) {
@@ -190,7 +202,16 @@ __device__ __forceinline__ bool leaf_proved_hit(const lg_geo* G, const lg_geo& g
     if (lo >= 0.0) {
       const double flo = poly3(a, lo), fhi = poly3(a, hi);
       if (!is_zero(flo) && !is_zero(fhi) && is_neg(flo) != is_neg(fhi)) {
-        const double sr = cubic_root(a, lo, hi, flo);
+        // f at s32 -+ 1e-4: where its signs are those of the bracket's ends, well above the
+        // rounding of f, f (monotone here) keeps them beyond these points
+        double wlo = sub((double)s32, 1e-4), whi = add((double)s32, 1e-4);
+        const double fa = poly3(a, wlo), fb = poly3(a, whi);
+        const float sc = 1e-9f * (fabsf((float)a[0]) + fabsf((float)a[1]) + fabsf((float)a[2]) + fabsf((float)a[3]));
+        if (is_neg(fa) != is_neg(flo) || is_neg(fb) == is_neg(flo) || !(fabsf((float)fa) > sc) || !(fabsf((float)fb) > sc)) {
+          wlo = lo;
+          whi = hi;
+        }
+        const double sr = cubic_root(a, lo, hi, flo, wlo, whi);
         const double t = dvd(dot(vsub(cubic_point(k, sr), o), d), dot(d, d));
         if (!gt_pos(t, T_MIN)) return false;
         out = mkhit(t, o, d, mk(sr, 0.0), 0);
@@ -287,13 +308,13 @@ __global__ void __launch_bounds__(256, LG_SOLVE_X_BLOCKS) k_solve_x(SceneDev S, 
         second = ob;
       }
     };
-    // proved roots (single circle and rect leaves, two-leaf CSG) first, in a phase of their own
+    // proved roots (single leaves, two-leaf CSG) first, in a phase of their own
     bool proved = false;
     uint32_t pcls = 7u;
     if (valid && i < off[LIST_FULL] && !sc.overflow && sc.nc == 1 && (sc.leaf == 0 || sc.leaf == 1))
       pcls = solve_class(__ldg(&S.scan[sl.base + sc.cand[0]].info));
     // class 3 holds single cubic leaves and deep CSG trees; only a cubic reaches a refine list
-    if (pcls == 0u || pcls == 1u || pcls == 4u || (pcls == 3u && sc.leaf == 0)) {
+    if (pcls <= 2u || pcls == 4u || (pcls == 3u && sc.leaf == 0)) {
       proved = solve_proved_x(S, S.info[sl.base + sc.cand[0]], o, d, sc.leaf, sc.face, sc.t32, sc.s32, ev, bh);
       if (proved) {
         best = sc.cand[0];
@@ -334,8 +355,8 @@ __global__ void __launch_bounds__(256, LG_SOLVE_X_BLOCKS) k_solve_x(SceneDev S, 
     }
     uint8_t fl = sc.overflow ? LG_PATH_FALLBACK : 0;
     // tracer.rs:404,417 ties within the band, and decisions in the band before the hit
-    if (best >= 0 && second < INFINITY && lgx::sub(second, best_d2) <= lgx::mul(lgx::BAND, best_d2)) fl |= lgx::NEAR;
-    if (best >= 0 ? ev <= lgx::add(lgx::mul(bh.t, 1.0 + 1e-6), 1e-12) : ev < INFINITY) fl |= lgx::NEAR;
+    if (best >= 0 && lgx::plt(second, INFINITY) && lgx::sub(second, best_d2) <= lgx::mul(lgx::BAND, best_d2)) fl |= lgx::NEAR;
+    if (lgx::plt(ev, INFINITY) && (best < 0 || ev <= lgx::add(lgx::mul(bh.t, 1.0 + 1e-6), 1e-12))) fl |= lgx::NEAR;
     V n = lgx::mk(0.0, 0.0);
     int leaf = 0;
     if (best >= 0) {  // the normal of the winning hit only
@@ -361,34 +382,73 @@ struct BounceX {
   RayRec child[2];
 };
 
+// A non-negative double as double-float (relative error 2^-48; below 2^-60 an absolute error
+// below 2^-83), on the integer pipe: a conversion each way would issue on the FP64 pipe.
+__device__ __forceinline__ df df_of(double x) {
+  const int hi = __double2hiint(x), lo = __double2loint(x);
+  const int e = ((hi >> 20) & 0x7ff) - 1023;
+  if (e < -60 || e > 60) return df{e > 60 ? INFINITY : 0.0f, 0.0f};
+  const float h = __int_as_float(((e + 127) << 23) | ((hi & 0xfffff) << 3) | (int)((unsigned)lo >> 29));
+  const float l = __fmul_rn(__uint2float_rn((unsigned)lo & 0x1fffffffu), __int_as_float((e - 52 + 127) << 23));
+  return fast_two_sum(h, l);
+}
+// a + b with an absolute error of 2^-47 (|a| + |b|) (operator+ keeps a relative one)
+__device__ __forceinline__ df add_abs(df a, df b) {
+  const df s = two_sum(a.hi, b.hi);
+  return fast_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo)));
+}
+
+// The unpolarised Fresnel reflectance rounded to FP32, which is all the colour split uses
+// (tracer.rs:454), from double-float copies of the indices and cosines: false unless the FP32
+// rounding of the FP64 formula's value is certain.  Every term n cos is within 2^-46 of itself,
+// so rs and rp are within 2^-44 and R within 2^-43 (|rs| + |rp| + R), the FP64 formula's own
+// rounding included; the bound below takes 2^-41.  It fails for about one visit in 10^4.  In FP64 the two
+// quotients, four products and their sums are half of a bounce's FP64 instructions.
+// A reflectance below 2^-26 (matched indices: a ray that leaves an object into the medium it
+// is already in) needs no exact value when dead says that the reflected colour is below the
+// cutoff whatever it is: the refracted share 1 - R is 1.
+__device__ __forceinline__ bool fresnel_f32(df n1, df n2, df ci, df ct, bool dead, float& R) {
+  const df a = n1 * ci, b = n2 * ct, c = n1 * ct, d = n2 * ci;
+  const df rs = add_abs(a, -b) / add_abs(a, b), rp = add_abs(c, -d) / add_abs(c, d);
+  const df q = add_abs(rs * rs, rp * rp);
+  const float hi = __fmul_rn(0.5f, q.hi), lo = __fmul_rn(0.5f, q.lo);
+  const int hb = __float_as_int(hi);
+  const float err = 4.5474735e-13f * (fabsf(rs.hi) + fabsf(rp.hi) + hi);  // 2^-41
+  const float half = __int_as_float((hb & 0x7f800000) - (24 << 23));     // half an ulp of hi
+  R = hi;
+  if (dead && hi + err < 1.4901161e-08f) return true;
+  return hi > 1e-20f && hi < 2.0f && (hb & 0x7fffff) != 0 && fabsf(lo) + err < half;
+}
+
 // Ray::refract restated (collision2d; called at tracer.rs:444-450): reflected direction,
-// refracted direction unless total internal reflection, unpolarised Fresnel reflectance.
-__device__ __forceinline__ bool refract_x(V d, V n, double n1, double n2, V& refl, V& refr, double& R,
-                                          uint32_t& fl) {
+// refracted direction unless total internal reflection, unpolarised Fresnel reflectance (as
+// FP32).  eta = n1 / n2; dead: see fresnel_f32.
+__device__ __forceinline__ bool refract_x(V d, V n, double n1, double n2, df n1f, df n2f, double eta, bool dead, V& refl,
+                                          V& refr, float& R, uint32_t& fl) {
   using namespace lgx;
   double ci = -dot(d, n);
-  if (ci < 0.0) {
+  if (is_neg(ci)) {
     ci = -ci;
-    n = vscl(n, -1.0);
+    n = mk(-n.x, -n.y);
   }
   refl = vadd(d, vscl(n, mul(2.0, ci)));
-  const double eta = dvd(n1, n2);
   const double k = sub(1.0, mul(mul(eta, eta), sub(1.0, mul(ci, ci))));
-  if (fabs(k) <= BAND) fl |= NEAR;
-  if (k < 0.0) {
-    R = 1.0;
+  if (bits(fabs(k)) <= bits(BAND)) fl |= NEAR;
+  if (is_neg(k)) {
+    R = 1.0f;
     return false;
   }
   const double ct = sqr(k);
   refr = vadd(vscl(d, eta), vscl(n, sub(mul(eta, ci), ct)));
+  if (fresnel_f32(n1f, n2f, df_of(ci), df_of(ct), dead, R)) return true;
   const double ds = add(mul(n1, ci), mul(n2, ct)), dp = add(mul(n1, ct), mul(n2, ci));
   if (ds == 0.0 || dp == 0.0) {
-    R = 1.0;
+    R = 1.0f;
     return true;
   }
   const double rs = dvd(sub(mul(n1, ci), mul(n2, ct)), ds);
   const double rp = dvd(sub(mul(n1, ct), mul(n2, ci)), dp);
-  R = mul(0.5, add(mul(rs, rs), mul(rp, rp)));
+  R = (float)mul(0.5, add(mul(rs, rs), mul(rp, rp)));
   return true;
 }
 
@@ -494,13 +554,29 @@ __device__ __forceinline__ void bounce_x(const SceneDev& S, const RayRec& r, con
         n2 = oi.n64;
         m2 = (uint16_t)best;
       }
-      const double n1 = r.medium == MEDIUM_AIR ? 1.0
-                        : r.medium == MEDIUM_LIGHT ? S.lights[sl.light_base + r.light].n0x : S.info[sl.base + r.medium].n64;
+      // n1 / n2 without a division where one side is air: x / 1 = x, and 1 / n is in the table
+      double n1 = 1.0, eta;
+      df n1f = DF_ONE, n2f = DF_ONE;
+      if (r.medium == MEDIUM_LIGHT) {
+        const LightDev& L = S.lights[sl.light_base + r.light];
+        n1 = L.n0x;
+        n1f = L.n0;
+      } else if (r.medium != MEDIUM_AIR) {
+        const ObjInfo& mi = S.info[sl.base + r.medium];
+        n1 = mi.n64;
+        n1f = mi.n;
+      }
+      if (m2 != MEDIUM_AIR) n2f = S.info[sl.base + m2].n;
+      if (bits(n2) == bits(1.0)) eta = n1;
+      else if (bits(n1) == bits(1.0)) eta = S.info[sl.base + m2].inv_n64;
+      else eta = dvd(n1, n2);
       V rl, rr = mk(0.0, 0.0);
-      double R;
-      const bool refr = refract_x(d, bn, n1, n2, rl, rr, R, fl);
+      float refl;
+      bool dead = true;  // c R <= c 2^-26 < cutoff in every channel
+#pragma unroll
+      for (int i = 0; i < 3; ++i) dead = dead && r.c[i] >= 0.0f && __fmul_rn(r.c[i], 1.4901161e-08f) < sl.cutoff[i];
+      const bool refr = refract_x(d, bn, n1, n2, n1f, n2f, eta, dead, rl, rr, refl, fl);
       v.flags = (uint8_t)((fl & 0xffu) | (refr ? 0u : (uint32_t)LG_PATH_TIR));
-      const float refl = (float)R;
       const float om = __fsub_rn(1.0f, refl);
       RayRec& a = v.child[0];
       a.ox = xdf(bp.x); a.oy = xdf(bp.y); a.dx = xdf(rl.x); a.dy = xdf(rl.y);
@@ -555,8 +631,8 @@ __device__ __forceinline__ void bounce_x(const SceneDev& S, const RayRec& r, con
       canvas.kind = LG_GEO_RECT;
       canvas.origin[0] = 0.0; canvas.origin[1] = 0.0;
       canvas.rot[0] = 1.0; canvas.rot[1] = 0.0;
-      canvas.v[0] = mul(2.0, aspect);
-      canvas.v[1] = 2.0;
+      canvas.v[2] = aspect;  // half width and height
+      canvas.v[3] = 1.0;
       hits_rect(canvas, o, d, cev, [&](const Hit& h) {
         if (nh == 0 || h.t < first.t) first = h;
         ++nh;

@@ -14,6 +14,8 @@
 
 #include <cstdint>
 
+#include "lg_x64.cuh"
+
 namespace {
 
 __global__ void __launch_bounds__(256, 4) k_smem_atomics(unsigned* out, int iters) {
@@ -74,9 +76,36 @@ float time_ms(L&& launch) {
   return ms;
 }
 
+__global__ void k_div_sqrt(const double* a, const double* b, double* q, double* s, uint64_t n) {
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    q[i] = lgx::dvd(a[i], b[i]);
+    s[i] = lgx::sqr(a[i]);
+  }
+}
+
 }  // namespace
 
 extern "C" {
+
+// The exact mode's quotient a / b and root of a (lg_x64.cuh) for n host values, so that a test
+// can hold them against IEEE-754: returns a cudaError_t.
+int lgp_div_sqrt(int device, const double* a, const double* b, double* q, double* s, uint64_t n) {
+  if (!a || !b || !q || !s || n == 0) return 1;
+  cudaError_t e = cudaSetDevice(device);
+  double* d = nullptr;
+  if (e == cudaSuccess) e = cudaMalloc((void**)&d, 4 * n * sizeof(double));
+  if (e != cudaSuccess) return (int)e;
+  if (e == cudaSuccess) e = cudaMemcpy(d, a, n * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(d + n, b, n * sizeof(double), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) {
+    k_div_sqrt<<<1024, 256>>>(d, d + n, d + 2 * n, d + 3 * n, n);
+    e = cudaGetLastError();
+  }
+  if (e == cudaSuccess) e = cudaMemcpy(q, d + 2 * n, n * sizeof(double), cudaMemcpyDeviceToHost);
+  if (e == cudaSuccess) e = cudaMemcpy(s, d + 3 * n, n * sizeof(double), cudaMemcpyDeviceToHost);
+  cudaFree(d);
+  return (int)e;
+}
 
 typedef struct lgp_peaks {
   double smem_atomics_per_s;

@@ -35,8 +35,84 @@ constexpr int MAX_POLY = 63;
 __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
 __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ double dvd(double a, double b) { return __ddiv_rn(a, b); }
-__device__ __forceinline__ double sqr(double a) { return __dsqrt_rn(a); }
+
+// Correctly rounded quotient and square root on the integer and FP32 pipes.  The FP64 pipe
+// issues a warp instruction in about 19 cycles on GB300 and a library quotient or root keeps it
+// for about ten of them; long division in three digits of a power-of-two base (Knuth, The Art
+// of Computer Programming 4.3.1: a quotient digit estimated from leading digits, an exact
+// remainder, one correction) takes some 80 instructions of the pipes that the exact kernels
+// leave idle.  A digit is estimated in FP32 (2^-22 relative, by an approximate reciprocal), so it is
+// off by two units at most, which the next digit takes up; the remainder is exact in 64-bit
+// integers.  The last digit leaves floor(q 2^53) after one correction, and the remainder decides
+// the rounding to nearest even.  Zeros, denormals, infinities, NaN and results outside the
+// normal range take the library's operations.
+static __device__ __noinline__ double div_x(double a, double b) {
+  const unsigned long long ab = (unsigned long long)__double_as_longlong(a), bb = (unsigned long long)__double_as_longlong(b);
+  const int ea = (int)(ab >> 52) & 0x7ff, eb = (int)(bb >> 52) & 0x7ff;
+  unsigned long long ma = (ab & 0xfffffffffffffull) | (1ull << 52);
+  const unsigned long long mb = (bb & 0xfffffffffffffull) | (1ull << 52);
+  const int lt = ma < mb ? 1 : 0;
+  ma <<= lt;  // ma / mb in [1, 2)
+  const int e = ea - eb + 1023 - lt;
+  if ((unsigned)(ea - 1) >= 0x7feu || (unsigned)(eb - 1) >= 0x7feu || (unsigned)(e - 1) >= 0x7fdu) return __ddiv_rn(a, b);
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(__uint2float_rn((unsigned)(mb >> 21))));
+  const unsigned d1 = __float2uint_rz(__fmul_rn(__uint2float_rn((unsigned)(ma >> 22)), __fmul_rn(y, 4194304.0f)));
+  long long r = (long long)((ma << 21) - (unsigned long long)d1 * mb);
+  const float y2 = __fmul_rn(y, 524288.0f);
+  const int d2 = __float2int_rn(__fmul_rn(__int2float_rn((int)(r >> 24)), y2));
+  r = (long long)(((unsigned long long)r << 16) - (unsigned long long)((long long)d2 * (long long)mb));
+  const int d3 = __float2int_rn(__fmul_rn(__int2float_rn((int)(r >> 24)), y2));
+  r = (long long)(((unsigned long long)r << 16) - (unsigned long long)((long long)d3 * (long long)mb));
+  long long q = ((long long)d1 << 32) + ((long long)d2 << 16) + d3;
+  if (r < 0) {
+    --q;
+    r += (long long)mb;
+  } else if (r >= (long long)mb) {
+    ++q;
+    r -= (long long)mb;
+  }
+  unsigned long long sig = (unsigned long long)q >> 1;
+  sig += ((unsigned)q & 1u) & ((r != 0 ? 1u : 0u) | ((unsigned)sig & 1u));
+  return __longlong_as_double((long long)((((unsigned long long)e << 52) + (sig - (1ull << 52))) | ((ab ^ bb) & (1ull << 63))));
+}
+
+// The root digit by digit: s = s1 2^32 + d2 2^16 + d3 of m 2^54, the remainder m 2^54 - s^2 kept
+// exact (scaled by the weight of the digits to come), each digit the remainder over twice the
+// root so far.
+static __device__ __noinline__ double sqrt_x(double a) {
+  const unsigned long long ab = (unsigned long long)__double_as_longlong(a);
+  const int ea = (int)(ab >> 52);
+  if ((unsigned)(ea - 1) >= 0x7feu) return __dsqrt_rn(a);  // zero, denormal, negative, infinite, NaN
+  const int e = ea - 1023;
+  const unsigned long long m = ((ab & 0xfffffffffffffull) | (1ull << 52)) << (e & 1);
+  float f, inv, inv2;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(f) : "f"(__uint2float_rn((unsigned)(m >> 22))));
+  const int s1 = __float2int_rn(__fmul_rn(f, 64.0f));
+  const float s1f = __int2float_rn(s1);
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(s1f));
+  const long long rb = (long long)(m - ((unsigned long long)((long long)s1 * s1) << 10));
+  const int d2 = __float2int_rn(__fmul_rn(__int2float_rn((int)(rb >> 8)), __fmul_rn(inv, 8192.0f)));
+  const long long rc = (rb << 22) - (((long long)s1 * d2) << 17) - (long long)d2 * d2;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv2) : "f"(__fmaf_rn(__int2float_rn(d2), 1.52587890625e-05f, s1f)));
+  const int d3 = __float2int_rn(__fmul_rn(__int2float_rn((int)(rc >> 12)), __fmul_rn(inv2, 2048.0f)));
+  const long long s2 = ((long long)s1 << 32) + ((long long)d2 << 16);
+  long long r = (long long)(((unsigned long long)rc << 32) - (unsigned long long)(2 * s2) * (unsigned long long)(long long)d3 -
+                            (unsigned long long)((long long)d3 * d3));
+  long long s = s2 + d3;
+  if (r < 0) {
+    --s;
+    r += 2 * s + 1;
+  } else if (r > 2 * s) {
+    r -= 2 * s + 1;
+    ++s;
+  }
+  unsigned long long sig = (unsigned long long)s >> 1;
+  sig += ((unsigned)s & 1u) & ((r != 0 ? 1u : 0u) | ((unsigned)sig & 1u));
+  return __longlong_as_double((long long)(((unsigned long long)((e >> 1) + 1023) << 52) + (sig - (1ull << 52))));
+}
+__device__ __forceinline__ double dvd(double a, double b) { return div_x(a, b); }
+__device__ __forceinline__ double sqr(double a) { return sqrt_x(a); }
 
 struct V {
   double x, y;
@@ -230,7 +306,7 @@ static __device__ __noinline__ bool leaf_contains(const lg_geo* G, const lg_geo&
     }
     case LG_GEO_RECT: {
       const V l = irot(vsub(p, mk(g.origin[0], g.origin[1])), g.rot[0], g.rot[1]);
-      const double hw = mul(0.5, g.v[0]), hh = mul(0.5, g.v[1]);
+      const double hw = g.v[2], hh = g.v[3];
       const double ex = sub(fabs(l.x), hw), ey = sub(fabs(l.y), hh);
       const double sd = ex > ey ? ex : ey;
       if (fl && fabs(sd) <= mul(BAND, add(hw, hh))) *fl |= NEAR;
@@ -322,7 +398,7 @@ __device__ __forceinline__ void hits_rect(const lg_geo& g, V o, V d, double& ev,
   const double c = g.rot[0], s = g.rot[1];
   const V ctr = mk(g.origin[0], g.origin[1]);
   const V lo = irot(vsub(o, ctr), c, s), ld = irot(d, c, s);
-  const double h[2] = {mul(0.5, g.v[0]), mul(0.5, g.v[1])};
+  const double h[2] = {g.v[2], g.v[3]};
   const double O[2] = {lo.x, lo.y}, D[2] = {ld.x, ld.y};
   double tn = -INFINITY, tf = INFINITY;
   int an = -1, af = -1;
@@ -382,12 +458,17 @@ __device__ __forceinline__ double cubic_t(const Cubic& k, double s, V o, V d) {
 // (a step that leaves it bisects instead) until a step moves it by 1e-15 or less (Numerical
 // Recipes 9.4, rtsafe); if twelve steps do not get there, bisection of the remaining bracket
 // to full precision.  The bracket and the points tried are non-negative, so the comparisons
-// run on the integer pipe with the FP64 comparisons' results.
-static __device__ __noinline__ double cubic_root(const double* a, double lo, double hi, double flo) {
+// run on the integer pipe with the FP64 comparisons' results.  wlo < whi: f is known to have
+// the sign of f(lo) up to wlo and the other sign from whi on, so a bisection point outside
+// (wlo, whi) needs no evaluation (lo, hi: nothing is known).
+static __device__ __noinline__ double cubic_root(const double* a, double lo, double hi, double flo, double wlo,
+                                                 double whi) {
   const bool neg_lo = is_neg(flo);
   for (int it = 0; it < 10; ++it) {
     const double mid = mul(0.5, add(lo, hi));
     if (!plt(lo, mid) || !plt(mid, hi)) return mid;
+    if (!plt(wlo, mid)) { lo = mid; continue; }
+    if (!plt(mid, whi)) { hi = mid; continue; }
     const double fm = poly3(a, mid);
     if (is_zero(fm)) return mid;
     if (is_neg(fm) == neg_lo) lo = mid; else hi = mid;
@@ -456,7 +537,7 @@ __device__ __forceinline__ void hits_cubic(const lg_geo& g, V o, V d, double& ev
       if (i + 2 == nk) roots[nr++] = hi;
       continue;
     }
-    if (is_neg(flo) != is_neg(fhi)) roots[nr++] = cubic_root(a, lo, hi, flo);
+    if (is_neg(flo) != is_neg(fhi)) roots[nr++] = cubic_root(a, lo, hi, flo, lo, hi);
   }
   if (fabs(a[0]) <= mul(BAND, scale)) event(ev, cubic_t(k, 0.0, o, d));  // end points
   if (fabs(poly3(a, 1.0)) <= mul(BAND, scale)) event(ev, cubic_t(k, 1.0, o, d));
@@ -529,17 +610,14 @@ __device__ __forceinline__ void leaf_hits(const lg_geo* G, const lg_geo& g, V o,
 static __device__ __noinline__ V leaf_normal(const lg_geo* G, const lg_geo& g, const Hit& h, V d) {
   switch (g.kind) {
     case LG_GEO_CIRCLE:
-      return vscl(vsub(h.aux, mk(g.origin[0], g.origin[1])), dvd(1.0, g.v[0]));
+      return vscl(vsub(h.aux, mk(g.origin[0], g.origin[1])), g.v[1]);
     case LG_GEO_RECT: {
       const double sg = (h.sub & 2) ? 1.0 : -1.0;
       const V nn = (h.sub & 1) == 0 ? mk(sg, 0.0) : mk(0.0, sg);
       return rot(nn, g.rot[0], g.rot[1]);
     }
-    case LG_GEO_SEGMENT: {
-      const V e = vsub(mk(g.v[2], g.v[3]), mk(g.v[0], g.v[1]));
-      const double le = sqr(dot(e, e));
-      return le > 0.0 ? mk(dvd(-e.y, le), dvd(e.x, le)) : mk(0.0, 0.0);
-    }
+    case LG_GEO_SEGMENT:
+      return mk(g.v[4], g.v[5]);
     case LG_GEO_CUBIC: {
       const V dB = cubic_tangent(cubic_of(g.v), h.aux.x);
       const double l = sqr(dot(dB, dB));
@@ -659,7 +737,8 @@ __device__ __forceinline__ V object_normal(const lg_geo* G, const XNode* nd, V d
   int chain[MAX_DEPTH + 1];
   int nc = 0;
   for (int j = nd[h.node].parent; j >= 0 && nc <= MAX_DEPTH; j = nd[j].parent) chain[nc++] = j;
-  for (int k = nc - 1; k >= 0; --k) d = irot(d, G[nd[chain[k]].geo].rot[0], G[nd[chain[k]].geo].rot[1]);
+  if (G[nd[h.node].geo].kind == LG_GEO_CUBIC)
+    for (int k = nc - 1; k >= 0; --k) d = irot(d, G[nd[chain[k]].geo].rot[0], G[nd[chain[k]].geo].rot[1]);
   V n = leaf_normal(G, G[nd[h.node].geo], h, d);
   for (int k = 0; k < nc; ++k) n = rot(n, G[nd[chain[k]].geo].rot[0], G[nd[chain[k]].geo].rot[1]);
   return n;
