@@ -477,7 +477,9 @@ void build_grid(const std::vector<ObjScan>& scan, int culling, float density, Gr
     for (size_t k = 0; k < n; ++k) {  // ascending object order within every cell
       grid_cell_range(R, scan[k].cx, scan[k].cy, scan[k].R, rx0, ry0, rx1, ry1);
       for (int iy = ry0; iy <= ry1; ++iy)
-        for (int ix = rx0; ix <= rx1; ++ix) G.cell_obj[cur[(size_t)iy * nx + ix]++] = (uint16_t)k;
+        for (int ix = rx0; ix <= rx1; ++ix)
+          G.cell_obj[cur[(size_t)iy * nx + ix]++] = (uint32_t)k | (ix > rx0 ? CELL_LEFT : 0u) | (ix < rx1 ? CELL_RIGHT : 0u) |
+                                                    (iy > ry0 ? CELL_BELOW : 0u) | (iy < ry1 ? CELL_ABOVE : 0u);
     }
     return;
   }
@@ -627,7 +629,7 @@ SceneDev scene_dev(lg_ctx* c) {
   S.light_hi = 0;
   S.grids = (const GridRec*)c->d_grids.p;
   S.cell_start = (const uint32_t*)c->d_cell_start.p;
-  S.cell_obj = (const uint16_t*)c->d_cell_obj.p;
+  S.cell_obj = (const uint32_t*)c->d_cell_obj.p;
   S.wait_polls = c->wait_polls;
   S.xgeo = (const lg_geo*)c->d_xgeo.p;
   S.xnode = (const lgx::XNode*)c->d_xnode.p;
@@ -701,7 +703,7 @@ lg_status upload_grids(lg_ctx* c, const lgh::GridTables& G) {
   lg_status st;
   if ((st = up(c->d_grids, G.recs.data(), G.recs.size() * sizeof(GridRec), "culling grids"))) return st;
   if ((st = up(c->d_cell_start, G.cell_start.data(), G.cell_start.size() * 4, "culling grids"))) return st;
-  return up(c->d_cell_obj, G.cell_obj.data(), G.cell_obj.size() * 2, "culling grids");
+  return up(c->d_cell_obj, G.cell_obj.data(), G.cell_obj.size() * 4, "culling grids");
 }
 
 lg_status ensure_trace_buffers(lg_ctx* c) {

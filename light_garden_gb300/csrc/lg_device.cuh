@@ -179,10 +179,9 @@ static_assert(sizeof(SceneRec) == 48, "SceneRec is 48 B");
 // traversal: a cell the walk reports at ray parameter t is within far less than margin of
 // the exact ray).  Cell c = iy * nx + ix lists, in ascending object order, every object
 // whose inflated box overlaps it: cell_start[cell_base + c] .. cell_start[cell_base + c + 1]
-// index cell_obj[list_base + ...] (scene-local object numbers).  An object's cell range
-// comes from grid_cell_range, the same FP32 operations on host and device, so a walk that
-// enters a cell knows whether it already met the object in the cell before.  nx == 0: no
-// grid, the scan is brute force.
+// index cell_obj[list_base + ...]: the scene-local object number and, in CELL_* bits, which of the
+// cell's neighbours list the object too, so that a walk that enters a cell knows whether it
+// already met the object in the cell before.  nx == 0: no grid, the scan is brute force.
 // Rays whose origin lies farther out than `reach` (|ox| + |oy|) carry FP32 errors above
 // the margin and test every object instead.
 struct __align__(16) GridRec {
@@ -196,6 +195,10 @@ struct __align__(16) GridRec {
   float reach;
 };
 static_assert(sizeof(GridRec) == 48, "GridRec is 48 B");
+
+// a cell list entry: object number | the neighbours that list the object
+constexpr uint32_t CELL_OBJ = 0xffffu;
+constexpr uint32_t CELL_LEFT = 1u << 16, CELL_RIGHT = 1u << 17, CELL_BELOW = 1u << 18, CELL_ABOVE = 1u << 19;
 
 struct SceneDev {
   const ObjScan* scan;
@@ -221,7 +224,7 @@ struct SceneDev {
   // culling grids: one per scene (index 0 for a single-scene trace)
   const GridRec* grids;
   const uint32_t* cell_start;
-  const uint16_t* cell_obj;
+  const uint32_t* cell_obj;
   // polls of a bounded device wait before it gives up (lg_device_opts.wait_polls; < 0: at once)
   int32_t wait_polls;
   // exact mode (LG_PRECISION_EXACT): the geometry nodes as uploaded, every object's tree in
@@ -818,6 +821,14 @@ __device__ __forceinline__ int leaf_member32(uint32_t kind, const float* L, floa
   return 0;  // segments enclose nothing
 }
 
+// Approximate root and quotients (a few ulp) serve the FP32 classification: its tolerances are a
+// hundred times wider.
+__device__ __forceinline__ float sqrt_approx(float x) {
+  float r;
+  asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // Roots of a cubic Bezier leaf in FP32: f(s) = cross(d, B(s) - o) is monotone between the
 // roots of f', so each sign change between consecutive knots is one root, found by
 // bisection.  A knot where |f| is within the FP32 error (tangency, a curve end on the ray)
@@ -840,15 +851,15 @@ __device__ __forceinline__ int cubic_roots32(const float* A, const float* Bp, fl
   if (fabsf(qa) > 1e-7f * sc) {
     const float disc = qb * qb - 4.0f * qa * qc;
     if (disc >= 0.0f) {
-      const float sq = sqrtf(disc);
+      const float sq = sqrt_approx(disc);
       const float q = -0.5f * (qb + (qb >= 0.0f ? sq : -sq));
-      float r1 = q / qa, r2 = q != 0.0f ? qc / q : r1;
+      float r1 = __fdividef(q, qa), r2 = q != 0.0f ? __fdividef(qc, q) : r1;
       if (r1 > r2) { const float x = r1; r1 = r2; r2 = x; }
       if (r1 > 0.0f && r1 < 1.0f) knots[nk++] = r1;
       if (r2 > 0.0f && r2 < 1.0f && r2 != knots[nk - 1]) knots[nk++] = r2;
     }
   } else if (fabsf(qb) > 1e-7f * sc) {
-    const float r = -qc / qb;
+    const float r = __fdividef(-qc, qb);
     if (r > 0.0f && r < 1.0f) knots[nk++] = r;
   }
   knots[nk++] = 1.0f;
@@ -863,14 +874,14 @@ __device__ __forceinline__ int cubic_roots32(const float* A, const float* Bp, fl
     if ((flo < 0.0f) == (fhi < 0.0f)) continue;
     // f is monotone between knots: Newton from the secant point, kept inside the sign
     // bracket (a step that leaves it bisects instead), until the step is below 3e-8
-    float u = (flo * hi - fhi * lo) / (flo - fhi);
+    float u = __fdividef(flo * hi - fhi * lo, flo - fhi);
     if (!(u > lo && u < hi)) u = 0.5f * (lo + hi);
     for (int it = 0; it < 40; ++it) {
       const float fu = f(u);
       if (fu == 0.0f) break;  // u is the root (the bracket update below would step off it)
       if ((fu < 0.0f) == (flo < 0.0f)) { lo = u; flo = fu; } else { hi = u; }
       const float fpu = (3.0f * a3 * u + 2.0f * a2) * u + a1;
-      float un = u - fu / fpu;
+      float un = u - __fdividef(fu, fpu);
       if (!(un > lo && un < hi)) un = 0.5f * (lo + hi);
       const bool done = fabsf(un - u) <= 3e-8f;
       u = un;
@@ -881,12 +892,12 @@ __device__ __forceinline__ int cubic_roots32(const float* A, const float* Bp, fl
     const float bx = ((c3x * u + c2x) * u + c1x) * u + c0x, by = ((c3y * u + c2y) * u + c1y) * u + c0y;
     const float dbx = (3.0f * c3x * u + 2.0f * c2x) * u + c1x, dby = (3.0f * c3y * u + 2.0f * c2y) * u + c1y;
     // constant indices only, so that t, sv and cert stay in registers (n <= 2 here)
-    const float tn = ((bx - ox) * dx + (by - oy) * dy) / dd;
+    const float tn = __fdividef((bx - ox) * dx + (by - oy) * dy, dd);
     const bool cn = u > 1e-4f && u < 1.0f - 1e-4f;
     if (n == 0) { t[0] = tn; sv[0] = u; cert[0] = cn; }
     else if (n == 1) { t[1] = tn; sv[1] = u; cert[1] = cn; }
     else { t[2] = tn; sv[2] = u; cert[2] = cn; }
-    const float tl = fabsf(dbx * dx + dby * dy) * (err / fabsf(fp) + 1e-6f) +
+    const float tl = fabsf(dbx * dx + dby * dy) * (__fdividef(err, fabsf(fp)) + 1e-6f) +
                      2e-6f * (fabsf(bx) + fabsf(by) + fabsf(ox) + fabsf(oy)) + 1e-6f;
     tol = fmaxf(tol, tl);
     ++n;
@@ -894,49 +905,67 @@ __device__ __forceinline__ int cubic_roots32(const float* A, const float* Bp, fl
   return n;
 }
 
-// roots of one FP32 leaf: t values with a certainty flag each
-__device__ __forceinline__ int leaf_roots32(uint32_t kind, const float* L, const float* L2, float ox, float oy,
-                                            float dx, float dy, float* t, bool* cert, int* face, float* sv, float& tol,
-                                            bool& unknown) {
-  unknown = false;
-  face[0] = face[1] = face[2] = -1;
-  sv[0] = sv[1] = sv[2] = 0.0f;
-  if (kind == LEAF_CUBIC) return cubic_roots32(L, L2, ox, oy, dx, dy, t, cert, sv, tol, unknown);
+// One FP32 circle, rect or segment leaf along the ray: its roots with a certainty flag each, and
+// where the ray is certainly inside (in0 < t < in1) and certainly outside (t < out0 or t > out1) of
+// the leaf.  The margins around the crossings are those of the geometry: an error of `delta` in
+// the distance to the boundary moves a crossing by delta over the sine of the crossing angle.
+struct Ival32 {
+  float t0, t1, tol;
+  float in0, in1, out0, out1;
+  int n, f0, f1;
+  bool c0, c1, unknown;
+};
+
+__device__ __forceinline__ Ival32 leaf_ival32(uint32_t kind, const float* L, float ox, float oy, float dx, float dy) {
+  Ival32 I;
+  I.n = 0;
+  I.f0 = I.f1 = -1;
+  I.t0 = I.t1 = 0.0f;
+  I.c0 = I.c1 = I.unknown = false;
+  I.tol = 1e-5f;
+  I.in0 = INFINITY; I.in1 = -INFINITY;   // inside nowhere
+  I.out0 = INFINITY; I.out1 = -INFINITY;  // outside everywhere
   if (kind == LEAF_CIRCLE) {
     const float ocx = ox - L[0], ocy = oy - L[1], r = L[2];
     const float b = ocx * dx + ocy * dy, perp = ocx * dy - ocy * dx;
     const float disc = (r - perp) * (r + perp);
     const float scale = fabsf(b) + fabsf(perp) + r;
-    tol = 4e-6f * scale + 1e-6f;
+    I.tol = 4e-6f * scale + 1e-6f;
     const float band = 2e-5f * scale * scale + 1e-3f * r * r;
-    if (disc < -band) return 0;
+    if (disc < -band) return I;
     if (disc <= band) {  // near-tangent: hit or miss is decided in FP64
-      const float w = sqrtf(band) + tol;
-      if (-b + w < -TAU32) return 0;  // the tangent point is behind the origin
-      t[0] = fmaxf(-b - w, 0.0f);
-      cert[0] = false;
-      return 1;
+      const float w = sqrt_approx(band) + I.tol;
+      I.out0 = -b - w; I.out1 = -b + w;
+      if (-b + w < -TAU32) return I;  // the tangent point is behind the origin
+      I.t0 = fmaxf(-b - w, 0.0f);
+      I.n = 1;
+      return I;
     }
-    const float sq = sqrtf(disc);
-    t[0] = -b - sq; cert[0] = true;
-    t[1] = -b + sq; cert[1] = true;
-    return 2;
+    const float sq = sqrt_approx(disc);
+    I.t0 = -b - sq; I.t1 = -b + sq;
+    I.c0 = I.c1 = true;
+    I.n = 2;
+    const float m = I.tol * __fdividef(r, sq);
+    I.in0 = I.t0 + m; I.in1 = I.t1 - m;
+    I.out0 = I.t0 - m; I.out1 = I.t1 + m;
+    return I;
   }
-  if (kind == LEAF_SEGMENT) {
+  if (kind == LEAF_SEGMENT) {  // encloses nothing
     const float ex = L[2], ey = L[3], wx = L[0] - ox, wy = L[1] - oy;
     const float den = dx * ey - dy * ex;
     const float le = fabsf(ex) + fabsf(ey);
     const float wn = fabsf(wx) + fabsf(wy);
-    if (fabsf(den) <= 1e-4f * le) { unknown = true; return 0; }
+    if (fabsf(den) <= 1e-4f * le) { I.unknown = true; return I; }
     // one approximate reciprocal (2 ulp) for both quotients: far inside the 4e-6 tolerance
     const float inv = __fdividef(1.0f, den);
     const float t0 = (wx * ey - wy * ex) * inv, u = (wx * dy - wy * dx) * inv;
-    tol = 4e-6f * (wn + le) * (1.0f + le * fabsf(inv)) + 1e-6f;
+    I.tol = 4e-6f * (wn + le) * (1.0f + le * fabsf(inv)) + 1e-6f;
     const float ub = 1e-5f * (1.0f + (wn + le) / le) * (1.0f + le * fabsf(inv));
-    if (u < -ub || u > 1.0f + ub) return 0;
-    t[0] = t0;
-    cert[0] = !(u < ub || u > 1.0f - ub);
-    return 1;
+    if (u < -ub || u > 1.0f + ub) return I;
+    I.t0 = t0;
+    I.c0 = !(u < ub || u > 1.0f - ub);
+    I.n = 1;
+    return I;
   }
   // rect: slab in the local frame
   const float rx = ox - L[0], ry = oy - L[1];
@@ -944,34 +973,47 @@ __device__ __forceinline__ int leaf_roots32(uint32_t kind, const float* L, const
   const float D[2] = {L[2] * dx + L[3] * dy, -L[3] * dx + L[2] * dy};
   const float H[2] = {L[4], L[5]};
   const float scale = fabsf(rx) + fabsf(ry) + H[0] + H[1];
+  const float band = 2e-6f * scale + 1e-6f, delta = 4e-6f * scale + 1e-6f;
   float tn = -INFINITY, tf = INFINITY, tn2 = -INFINITY, tf2 = INFINITY;
+  float in0 = -INFINITY, in1 = INFINITY, out0 = -INFINITY, out1 = INFINITY;
   int fn = -1, ff = -1;
+#pragma unroll
   for (int ax = 0; ax < 2; ++ax) {
-    const float band = 2e-6f * scale + 1e-6f;
     if (fabsf(D[ax]) < 1e-6f) {
-      if (fabsf(O[ax]) > H[ax] + band) return 0;
-      if (fabsf(O[ax]) >= H[ax] - band) { unknown = true; return 0; }
+      if (fabsf(O[ax]) > H[ax] + band) return I;
+      if (fabsf(O[ax]) >= H[ax] - band) {
+        I.unknown = true;
+        I.out0 = -INFINITY; I.out1 = INFINITY;
+        return I;
+      }
       continue;
     }
     const float inv = __fdividef(1.0f, D[ax]);  // approximate reciprocal (2 ulp): far inside tol
-    float t1 = (-H[ax] - O[ax]) * inv, t2 = (H[ax] - O[ax]) * inv;
+    const float ta = (-H[ax] - O[ax]) * inv, tb = (H[ax] - O[ax]) * inv;
     // entering through the -H face when D > 0 (outward normal -1), else the +H face
-    int f1 = 2 * ax + (D[ax] > 0.0f ? 0 : 1), f2 = 2 * ax + (D[ax] > 0.0f ? 1 : 0);
-    if (t1 > t2) { const float x = t1; t1 = t2; t2 = x; }
+    const int f1 = 2 * ax + (D[ax] > 0.0f ? 0 : 1);
+    const float t1 = fminf(ta, tb), t2 = fmaxf(ta, tb), m = delta * fabsf(inv);
+    in0 = fmaxf(in0, t1 + m); in1 = fminf(in1, t2 - m);
+    out0 = fmaxf(out0, t1 - m); out1 = fminf(out1, t2 + m);
     if (t1 > tn) { tn2 = tn; tn = t1; fn = f1; } else { tn2 = fmaxf(tn2, t1); }
-    if (t2 < tf) { tf2 = tf; tf = t2; ff = f2; } else { tf2 = fminf(tf2, t2); }
+    if (t2 < tf) { tf2 = tf; tf = t2; ff = f1 ^ 1; } else { tf2 = fminf(tf2, t2); }
   }
-  tol = 4e-6f * (scale + fabsf(tn) + fabsf(tf)) + 1e-6f;
-  if (tn > tf + tol) return 0;
+  I.in0 = in0; I.in1 = in1; I.out0 = out0; I.out1 = out1;
+  const float tol = 4e-6f * (scale + fabsf(tn) + fabsf(tf)) + 1e-6f;
+  I.tol = tol;
+  if (tn > tf + tol) return I;
+  I.t0 = tn;
+  I.f0 = fn;
   if (tn >= tf - tol) {  // corner graze
-    t[0] = tn;
-    cert[0] = false;
-    return 1;
+    I.f0 = -1;
+    I.n = 1;
+    return I;
   }
   // a root whose face is ambiguous (the ray meets a corner) stays uncertain
-  t[0] = tn; cert[0] = !(tn - tn2 <= tol); face[0] = fn;
-  t[1] = tf; cert[1] = !(tf2 - tf <= tol); face[1] = ff;
-  return 2;
+  I.c0 = !(tn - tn2 <= tol);
+  I.t1 = tf; I.c1 = !(tf2 - tf <= tol); I.f1 = ff;
+  I.n = 2;
+  return I;
 }
 
 __device__ __forceinline__ bool op_keep(uint32_t op, bool side_a, bool in_other) {
@@ -980,41 +1022,67 @@ __device__ __forceinline__ bool op_keep(uint32_t op, bool side_a, bool in_other)
   return side_a ? !in_other : in_other;
 }
 
-static // src_leaf: leaf of this object that holds the ray origin (-1: none).  On that leaf the
+// The roots of leaf `side` (interval I) into c.  A two-leaf object keeps a certain root where the
+// other leaf's interval O makes it a boundary of the combination, drops it where it does not,
+// and leaves it a candidate where the root lies within the margins of O's crossings.
+__device__ __forceinline__ void leaf_keep32(const Ival32& I, const Ival32& O, bool two, uint32_t op, int side, int src_leaf,
+                                            float lb, Class32& c) {
+  if (I.unknown) {  // near-parallel: defer the whole object to the precise solve
+    c.key = fminf(c.key, fmaxf(lb, 0.0f));
+    return;
+  }
+  // the root at the surface the ray leaves (source leaf) is skipped
+  int skip = -1;
+  if (side == src_leaf && I.n > 0) {
+    const bool second = I.n == 2 && fabsf(I.t1) < fabsf(I.t0);
+    const float near = second ? I.t1 : I.t0, far = second ? I.t0 : I.t1;
+    if (fabsf(near) < TAU32 && (second ? I.c1 : I.c0) && !(I.n == 2 && fabsf(far) < 4.0f * TAU32)) skip = second ? 1 : 0;
+  }
+  const float a = 4.0f * I.tol;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    if (k >= I.n || k == skip) continue;
+    const float t = k == 0 ? I.t0 : I.t1;
+    bool certain = k == 0 ? I.c0 : I.c1;
+    if (two && certain) {
+      if (t < -TAU32) continue;
+      const bool in = t > O.in0 + a && t < O.in1 - a, out = t < O.out0 - a || t > O.out1 + a;
+      if (!in && !out) certain = false;
+      else if (!op_keep(op, side == 0, in)) continue;
+    }
+    root32(t, I.tol, c, certain, side, k == 0 ? I.f0 : I.f1, 0.0f);
+  }
+}
+
+// src_leaf: leaf of this object that holds the ray origin (-1: none).  On that leaf the
 // root nearest t = 0 is the surface the ray leaves; it is excluded as certain unless the
 // leaf's other root is also near 0 (grazing ray or a corner), which stays uncertain.
-__device__ __noinline__ Class32 classify32(const ObjScan& r, float ox, float oy, float dx, float dy, float lb,
-                                           int src_leaf) {
+// Both leaves of a CSG object give an interval of the ray each, and a root's membership in the
+// other leaf is two comparisons with the other's interval (testing the root's point against the
+// other leaf's shape took most of a classification of about 450 instructions).
+static __device__ __noinline__ Class32 classify32(const ObjScan& r, float ox, float oy, float dx, float dy, float lb,
+                                                  int src_leaf) {
   Class32 c;
   c.key = INFINITY;
   c.ub = INFINITY;
   c.leaf = -1;
   c.face = -1;
   c.s = 0.0f;
-  const uint32_t sk = info_scan(r.info);
+  const uint32_t sk = info_scan(r.info), ka = info_leaf_a(r.info);
   if (sk == SCAN_BOUND) {
     c.key = fmaxf(lb, 0.0f);
     return c;
   }
-  const int nleaf = sk == SCAN_TWO ? 2 : 1;
-  for (int side = 0; side < nleaf; ++side) {
-    const float* L = side == 0 ? r.a : r.b;
-    const uint32_t kind = side == 0 ? info_leaf_a(r.info) : info_leaf_b(r.info);
-    float t[3] = {0.0f, 0.0f, 0.0f};
-    bool cert[3] = {false, false, false};
-    int face[3];
-    float sv[3];
-    float tol = 1e-5f;
-    bool unknown = false;
-    int n = leaf_roots32(kind, L, r.b, ox, oy, dx, dy, t, cert, face, sv, tol, unknown);
-    if (unknown) {  // near-parallel: defer the whole object to the precise solve
+  if (ka == LEAF_CUBIC) {  // a single cubic (its control points fill both slots)
+    float t[3] = {0.0f, 0.0f, 0.0f}, sv[3] = {0.0f, 0.0f, 0.0f}, tol = 1e-5f;
+    bool cert[3] = {false, false, false}, unknown = false;
+    const int n = cubic_roots32(r.a, r.b, ox, oy, dx, dy, t, cert, sv, tol, unknown);
+    if (unknown) {
       c.key = fminf(c.key, fmaxf(lb, 0.0f));
-      continue;
+      return c;
     }
-    // the root at the surface the ray leaves (source leaf) is skipped; the arrays are only
-    // read at constant indices, so they stay in registers
     int skip = -1;
-    if (side == src_leaf && n > 0) {
+    if (src_leaf == 0 && n > 0) {
       int ks = 0;
       float tks = t[0];
       bool cks = cert[0];
@@ -1027,30 +1095,22 @@ __device__ __noinline__ Class32 classify32(const ObjScan& r, float ox, float oy,
         if (k < n && k != ks && fabsf(t[k]) < 4.0f * TAU32) other_near = true;
       if (fabsf(tks) < TAU32 && cks && !other_near) skip = ks;
     }
-    // the roots move through three registers (no dynamically indexed array)
-    float ta = t[0], tb = t[1], tc = t[2], sa = sv[0], sb = sv[1], sc2 = sv[2];
-    bool ca = cert[0], cb = cert[1], cc = cert[2];
-    int fa = face[0], fb = face[1], fc = face[2];
-    for (int k = 0; k < n; ++k) {
-      const float tk = ta, svk = sa;
-      const bool ck = ca;
-      const int fk = fa;
-      ta = tb; tb = tc; sa = sb; sb = sc2; ca = cb; cb = cc; fa = fb; fb = fc;
-      if (k == skip) continue;
-      bool certain = ck;
-      if (nleaf == 2 && certain) {
-        // CSG filter at a well-located hit point; an uncertain root stays a candidate
-        if (tk < -TAU32) continue;
-        const float px = ox + dx * tk, py = oy + dy * tk;
-        const float* Lo = side == 0 ? r.b : r.a;
-        const uint32_t ko = side == 0 ? info_leaf_b(r.info) : info_leaf_a(r.info);
-        const int m = leaf_member32(ko, Lo, px, py, 4.0f * tol);
-        if (m < 0) certain = false;
-        else if (!op_keep(info_op(r.info), side == 0, m == 1)) continue;
-      }
-      root32(tk, tol, c, certain, side, fk, svk);
-    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      if (k < n && k != skip) root32(t[k], tol, c, cert[k], 0, -1, sv[k]);
+    return c;
   }
+  const bool two = sk == SCAN_TWO;
+  Ival32 A, B;
+  B.in0 = B.out0 = INFINITY;
+  B.in1 = B.out1 = -INFINITY;
+#pragma unroll 1
+  for (int side = 0; side <= (two ? 1 : 0); ++side) {  // one copy of the leaf code
+    const Ival32 I = leaf_ival32(side ? info_leaf_b(r.info) : ka, side ? r.b : r.a, ox, oy, dx, dy);
+    if (side) B = I; else A = I;
+  }
+  leaf_keep32(A, B, two, info_op(r.info), 0, src_leaf, lb, c);
+  if (two) leaf_keep32(B, A, two, info_op(r.info), 1, src_leaf, lb, c);
   return c;
 }
 

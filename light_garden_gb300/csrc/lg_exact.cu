@@ -546,9 +546,9 @@ __device__ __forceinline__ void bounce_x(const SceneDev& S, const RayRec& r, con
           const float fy = fminf(fmaxf(floorf((py32 - G.y0) * G.ih), 0.0f), (float)(G.ny - 1));
           const uint32_t c = (uint32_t)fy * G.nx + (uint32_t)fx;
           const uint32_t* cs = S.cell_start + G.cell_base;
-          const uint16_t* co = S.cell_obj + G.list_base;
+          const uint32_t* co = S.cell_obj + G.list_base;
           for (uint32_t q = __ldg(cs + c), qe = __ldg(cs + c + 1); q < qe; ++q)
-            if (far_side(__ldg(co + q))) break;
+            if (far_side(__ldg(co + q) & CELL_OBJ)) break;
         }
       } else {
         n2 = oi.n64;

@@ -26,7 +26,7 @@ struct LeafH {
 struct GridH {
   GridRec rec;
   std::vector<uint32_t> cell_start;  // nx * ny + 1 (one entry when there is no grid)
-  std::vector<uint16_t> cell_obj;
+  std::vector<uint32_t> cell_obj;
 };
 
 // One scene (or several, concatenated) in the layout of the device tables.
@@ -61,7 +61,7 @@ struct Flat {
 struct GridTables {
   std::vector<GridRec> recs;
   std::vector<uint32_t> cell_start;
-  std::vector<uint16_t> cell_obj;
+  std::vector<uint32_t> cell_obj;
   // appends a scene's cells and object lists; returns its record with the bases set
   GridRec add(const GridH& g) {
     GridRec r = g.rec;

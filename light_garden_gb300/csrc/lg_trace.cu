@@ -223,16 +223,16 @@ __device__ __forceinline__ void emit_segments(const SceneDev& S, const TraceBufs
 // the culled walk tends to do best with 8 (a smaller shared-memory buffer leaves more of the
 // SM's L1 to the grid and queue loads), the table scan with 16 (CSG frame: 8 slots 1217 ms of
 // scan, 16 slots 1469; mid frame: 16 slots 68 ms, 8 slots 73).  CTAs per SM of the culled scan
-// and its walk steps between classifications are build-time (-DLG_SCAN_CULL_BLOCKS=...,
-// -DLG_SCAN_WALK_STEPS=..., for sweeps).
+// and its cell steps between classifications are build-time (-DLG_SCAN_CULL_BLOCKS=...,
+// -DLG_SCAN_WALK_CELLS=..., for sweeps).
 #ifndef LG_SCAN_CULL_BLOCKS
 #define LG_SCAN_CULL_BLOCKS 4
 #endif
-#ifndef LG_SCAN_WALK_STEPS
-#define LG_SCAN_WALK_STEPS 32
+#ifndef LG_SCAN_WALK_CELLS
+#define LG_SCAN_WALK_CELLS 8
 #endif
 constexpr int SCAN_WARPS = 4;
-constexpr int WALK_STEPS = LG_SCAN_WALK_STEPS;  // culled scan: cell steps and object tests between classifications
+constexpr int WALK_CELLS = LG_SCAN_WALK_CELLS;  // culled scan: cell steps between classifications (2 to 16: within 2 %)
 constexpr int SCAN_CULL_BLOCKS = LG_SCAN_CULL_BLOCKS;  // culled scan: CTAs per SM the registers are sized for
 
 struct __align__(16) PairSlot {
@@ -426,12 +426,9 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, CULL ? SCAN_CULL_BLOCKS : 4)
             const float4 h = MULTI ? __ldg(&S.bounds[j]) : *reinterpret_cast<const float4*>(&objs[j]);
             float lb;
             if (mine && bound_test(h, ox, oy, dx, dy, thr, lb)) {
-              PairSlot ps;
+              PairSlot& ps = W.pairs[w][cnt++][lane];
               ps.key = lb;
-              ps.ub = 0.0f;
-              ps.s = 0.0f;
               ps.m = j - g_lo;  // scene-local object index
-              W.pairs[w][cnt++][lane] = ps;
             }
           }
           classify_fold(cnt);
@@ -446,12 +443,13 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, CULL ? SCAN_CULL_BLOCKS : 4)
         const uint32_t gny = G.ny;
         const float gx0 = G.x0, gy0 = G.y0, cw = G.cw, ch = G.ch, margin = G.margin;
         const uint32_t* cstart = S.cell_start + G.cell_base;
-        const uint16_t* cobj = S.cell_obj + G.list_base;
-        const float idx = fabsf(dx) > 1e-30f ? 1.0f / dx : 0.0f;
-        const float idy = fabsf(dy) > 1e-30f ? 1.0f / dy : 0.0f;
+        const uint32_t* cobj = S.cell_obj + G.list_base;
+        // (approximate: the grid's margin is some thousand ulp of its coordinates)
+        const float idx = fabsf(dx) > 1e-30f ? __fdividef(1.0f, dx) : 0.0f;
+        const float idy = fabsf(dy) > 1e-30f ? __fdividef(1.0f, dy) : 0.0f;
         const int sx = dx > 0.0f ? 1 : -1, sy = dy > 0.0f ? 1 : -1;
         int ix = 0, iy = 0;
-        int came = 0;  // 0: first cell; 1: entered by an x step; 2: by a y step
+        uint32_t came = 0;  // CELL_* bit of the side the walk entered the cell by (0: first cell)
         float tx = INFINITY, ty = INFINITY;
         uint32_t p = 0, pe = 0, steps = 0;
         bool act = mine, linear = false;
@@ -491,68 +489,61 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, CULL ? SCAN_CULL_BLOCKS : 4)
             }
           }
         }
-        // tests object j (scene-local) with bound h, unless met in the previous cell
-        auto test = [&](uint32_t j, const float4& h, int& cnt) {
-          if (came == 1) {
-            if (sx > 0 ? cell_lo(h.x, h.z, margin, gx0, G.iw) < (float)ix : cell_hi(h.x, h.z, margin, gx0, G.iw) > (float)ix)
-              return;
-          } else if (came == 2) {
-            if (sy > 0 ? cell_lo(h.y, h.z, margin, gy0, G.ih) < (float)iy : cell_hi(h.y, h.z, margin, gy0, G.ih) > (float)iy)
-              return;
-          }
+        // tests the object of a list entry with bound h, unless met in the previous cell
+        auto test = [&](uint32_t e, const float4& h, int& cnt) {
+          if (e & came) return;
           ++my_tests;
           float lb;
           if (bound_test(h, ox, oy, dx, dy, thr, lb)) {
-            PairSlot ps;
+            PairSlot& ps = W.pairs[w][cnt++][lane];
             ps.key = lb;
-            ps.ub = 0.0f;
-            ps.s = 0.0f;
-            ps.m = j;
-            W.pairs[w][cnt++][lane] = ps;
+            ps.m = e & CELL_OBJ;
           }
         };
         while (__any_sync(0xffffffffu, act)) {
+          // The lanes test the objects of their cells side by side, then those without pairs step
+          // to their next cells; a lane with pairs waits for the fold (a hit in its cell may end
+          // its walk there), and the warp folds after WALK_CELLS steps at the latest.
           int cnt = 0;
-          bool yield = false;  // a lane that finished a cell with pairs waits for the fold
-          for (int st = 0; st < WALK_STEPS; ++st) {
-            const bool can = act && !yield && cnt + 2 <= SCAN_CHUNK;
-            if (!__any_sync(0xffffffffu, can)) break;
-            if (!can) continue;
-            if (p < pe) {
-              // two objects of the cell per step: their loads overlap
-              const bool two = p + 1 < pe;
-              const uint32_t j0 = linear ? p : (uint32_t)__ldg(cobj + p);
-              const uint32_t j1 = two ? (linear ? p + 1 : (uint32_t)__ldg(cobj + p + 1)) : j0;
-              p += two ? 2u : 1u;
-              const float4 h0 = MULTI ? __ldg(&S.bounds[g_lo + j0]) : *reinterpret_cast<const float4*>(&objs[j0]);
-              const float4 h1 = MULTI ? __ldg(&S.bounds[g_lo + j1]) : *reinterpret_cast<const float4*>(&objs[j1]);
-              test(j0, h0, cnt);
-              if (two) test(j1, h1, cnt);
-            } else if (cnt > 0 && !linear) {
-              // fold before the next cell: a hit in this one may end the walk here
-              yield = true;
-            } else if (linear || ++steps > gnx + gny + 2) {
+          for (int st = 0;; ++st) {
+            while (__any_sync(0xffffffffu, act && p < pe && cnt + 2 <= SCAN_CHUNK)) {
+              if (act && p < pe && cnt + 2 <= SCAN_CHUNK) {
+                const bool two = p + 1 < pe;
+                const uint32_t e0 = linear ? p : __ldg(cobj + p);
+                const uint32_t e1 = two ? (linear ? p + 1 : __ldg(cobj + p + 1)) : e0;
+                p += two ? 2u : 1u;
+                const uint32_t j0 = e0 & CELL_OBJ, j1 = e1 & CELL_OBJ;
+                const float4 h0 = MULTI ? __ldg(&S.bounds[g_lo + j0]) : *reinterpret_cast<const float4*>(&objs[j0]);
+                const float4 h1 = MULTI ? __ldg(&S.bounds[g_lo + j1]) : *reinterpret_cast<const float4*>(&objs[j1]);
+                test(e0, h0, cnt);
+                if (two) test(e1, h1, cnt);
+              }
+            }
+            const bool step = act && p >= pe && (cnt == 0 || linear);
+            if (st == WALK_CELLS || !__any_sync(0xffffffffu, step)) break;
+            if (!step) continue;
+            if (linear || ++steps > gnx + gny + 2) {
               act = false;
-            } else {  // the next cell along the ray
-              float te;
-              if (tx <= ty) {
-                ix += sx;
-                te = tx;
-                tx = (gx0 + (float)(ix + (sx > 0 ? 1 : 0)) * cw - ox) * idx;
-                came = 1;
-              } else {
-                iy += sy;
-                te = ty;
-                ty = (gy0 + (float)(iy + (sy > 0 ? 1 : 0)) * ch - oy) * idy;
-                came = 2;
-              }
-              if (ix < 0 || iy < 0 || ix >= (int)gnx || iy >= (int)gny || !(te <= thr + margin) || te == INFINITY) {
-                act = false;
-              } else {
-                const uint32_t c = (uint32_t)iy * gnx + (uint32_t)ix;
-                p = __ldg(cstart + c);
-                pe = __ldg(cstart + c + 1);
-              }
+              continue;
+            }
+            float te;  // the next cell along the ray
+            if (tx <= ty) {
+              ix += sx;
+              te = tx;
+              tx = (gx0 + (float)(ix + (sx > 0 ? 1 : 0)) * cw - ox) * idx;
+              came = sx > 0 ? CELL_LEFT : CELL_RIGHT;
+            } else {
+              iy += sy;
+              te = ty;
+              ty = (gy0 + (float)(iy + (sy > 0 ? 1 : 0)) * ch - oy) * idy;
+              came = sy > 0 ? CELL_BELOW : CELL_ABOVE;
+            }
+            if (ix < 0 || iy < 0 || ix >= (int)gnx || iy >= (int)gny || !(te <= thr + margin) || te == INFINITY) {
+              act = false;
+            } else {
+              const uint32_t c = (uint32_t)iy * gnx + (uint32_t)ix;
+              p = __ldg(cstart + c);
+              pe = __ldg(cstart + c + 1);
             }
           }
           classify_fold(cnt);
@@ -848,9 +839,9 @@ __device__ __forceinline__ void bounce(const SceneDev& S, const ObjScan* objs, c
           const float fy = fminf(fmaxf(floorf((py32 - G.y0) * G.ih), 0.0f), (float)(G.ny - 1));
           const uint32_t c = (uint32_t)fy * G.nx + (uint32_t)fx;
           const uint32_t* cs = S.cell_start + G.cell_base;
-          const uint16_t* co = S.cell_obj + G.list_base;
+          const uint32_t* co = S.cell_obj + G.list_base;
           for (uint32_t q = __ldg(cs + c), qe = __ldg(cs + c + 1); q < qe; ++q)
-            if (far_side(__ldg(co + q))) break;
+            if (far_side(__ldg(co + q) & CELL_OBJ)) break;
         }
       } else {
         n2 = oi.n;
