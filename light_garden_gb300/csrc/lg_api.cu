@@ -314,6 +314,47 @@ static void derive_constants(lg_geo& g) {
   }
 }
 
+// One leaf's parameters for a SolveRec (g holds its derived constants); false for other kinds.
+static bool solve_leaf(const lg_geo& g, bool cubic, double* v, double* v2, uint32_t& kind) {
+  if (g.kind == LG_GEO_CIRCLE) {
+    kind = LEAF_CIRCLE;
+    v[0] = g.origin[0]; v[1] = g.origin[1]; v[2] = g.v[0]; v[3] = g.v[1];
+  } else if (g.kind == LG_GEO_RECT) {
+    kind = LEAF_RECT;
+    v[0] = g.origin[0]; v[1] = g.origin[1]; v[2] = g.rot[0]; v[3] = g.rot[1]; v[4] = g.v[2]; v[5] = g.v[3];
+  } else if (g.kind == LG_GEO_SEGMENT) {
+    kind = LEAF_SEGMENT;
+    for (int k = 0; k < 6; ++k) v[k] = g.v[k];
+  } else if (g.kind == LG_GEO_CUBIC && cubic) {
+    // the power basis, each operation rounded once in cubic_of's order (lg_x64.cuh)
+    kind = LEAF_CUBIC;
+    for (int ax = 0; ax < 2; ++ax) {
+      const double p0 = g.v[ax], p1 = g.v[2 + ax], p2 = g.v[4 + ax], p3 = g.v[6 + ax];
+      volatile double d10 = p1 - p0, c1 = d10 * 3.0;
+      volatile double t1 = p1 * 2.0, t2 = p2 - t1, t3 = t2 * 3.0, t4 = p0 * 3.0, c2 = t3 + t4;
+      volatile double d12 = p1 - p2, u1 = d12 * 3.0, u2 = p3 + u1, c3 = u2 - p0;
+      v[ax] = p0; v[2 + ax] = c1; v[4 + ax] = c2;
+      v2[ax] = c3;
+    }
+  } else {
+    return false;
+  }
+  return true;
+}
+static SolveRec solve_rec(const std::vector<lg_geo>& X, int32_t root) {
+  SolveRec R;
+  std::memset(&R, 0, sizeof R);
+  const lg_geo& g = X[root];
+  uint32_t ka = 0, kb = 0;
+  if (solve_leaf(g, true, R.a, R.b, ka)) {
+    R.kind = SR_ONE | (ka << 4);
+  } else if (g.kind == LG_GEO_LOGIC && solve_leaf(X[g.a], false, R.a, R.b, ka) && solve_leaf(X[g.b], false, R.b, R.b, kb)) {
+    R.kind = SR_TWO | (ka << 4) | (kb << 8);
+    R.org[0] = g.origin[0]; R.org[1] = g.origin[1]; R.rot[0] = g.rot[0]; R.rot[1] = g.rot[1];
+  }
+  return R;
+}
+
 lg_status flatten_scene(std::string& err, const lg_geo* G, uint32_t n_geo, const lg_object* O, uint32_t n_obj,
                         const lg_light* Ls, uint32_t n_lights, Flat& F) {
   F.xgeo.assign(G, G + n_geo);
@@ -359,6 +400,7 @@ lg_status flatten_scene(std::string& err, const lg_geo* G, uint32_t n_geo, const
     }
     F.prog.insert(F.prog.end(), prog.begin(), prog.end());
     F.info.push_back(oi);
+    F.solve.push_back(solve_rec(F.xgeo, o.geo));
     if (o.kind == LG_OBJ_CURVED_MIRROR) F.cubics.push_back(k);
     // FP32 scan record
     ObjScan s;
@@ -633,6 +675,7 @@ SceneDev scene_dev(lg_ctx* c) {
   S.wait_polls = c->wait_polls;
   S.xgeo = (const lg_geo*)c->d_xgeo.p;
   S.xnode = (const lgx::XNode*)c->d_xnode.p;
+  S.solve = (const SolveRec*)c->d_solve.p;
   S.aspect64 = c->aspect;
   S.ray_stride = c->prm.ray_stride > 1 ? c->prm.ray_stride : 1u;
   S.ray_offset = c->prm.ray_stride > 1 ? c->prm.ray_offset : 0u;
@@ -899,6 +942,9 @@ lg_status upload_exact(lg_ctx* c, const Flat& F) {
   lg_status st;
   if ((st = ensure(c, c->d_xgeo, F.xgeo.size() * sizeof(lg_geo) + 16, "scene"))) return st;
   if ((st = ensure(c, c->d_xnode, F.xnode.size() * sizeof(lgx::XNode) + 16, "scene"))) return st;
+  if ((st = ensure(c, c->d_solve, F.solve.size() * sizeof(SolveRec) + 16, "scene"))) return st;
+  if (!F.solve.empty())
+    CK(cudaMemcpyAsync(c->d_solve.p, F.solve.data(), F.solve.size() * sizeof(SolveRec), cudaMemcpyHostToDevice, c->stream), "upload");
   if (!F.xgeo.empty())
     CK(cudaMemcpyAsync(c->d_xgeo.p, F.xgeo.data(), F.xgeo.size() * sizeof(lg_geo), cudaMemcpyHostToDevice, c->stream), "upload");
   if (!F.xnode.empty())
@@ -1203,7 +1249,7 @@ lg_status lg_destroy(lg_ctx* c) {
                     &c->d_tile_cursor, &c->d_unit_off, &c->d_refs, &c->d_units, &c->d_accum, &c->d_stage,
                     &c->d_scenes, &c->d_canvases, &c->d_seg_scene, &c->d_cubic_scene, &c->d_part,
                     &c->d_bounds, &c->d_order, &c->d_scene_count, &c->d_scene_off,
-                    &c->d_grids, &c->d_cell_start, &c->d_cell_obj, &c->d_cta_hist};
+                    &c->d_grids, &c->d_cell_start, &c->d_cell_obj, &c->d_cta_hist, &c->d_solve};
   for (DevBuf* b : bufs) release(*b);
   if (c->h_ctr) cudaFreeHost(c->h_ctr);
   for (int i = 0; i < 6; ++i)

@@ -29,7 +29,7 @@ struct lg_ctx {
   std::string err;
   // scene
   DevBuf d_scan, d_info, d_leaves, d_prog, d_lights, d_cubics;
-  DevBuf d_xgeo, d_xnode;  // exact mode: geometry nodes and per-object preorder trees
+  DevBuf d_xgeo, d_xnode, d_solve;  // exact mode: geometry nodes, per-object preorder trees, solve records
   DevBuf d_mod_colors;     // string mod: the modulo-colour table of the mod drawn (the nested one if any)
   DevBuf d_chords;         // string mod: the frame's lines (lg_string_mod.modulo of them)
   uint64_t chords_ready = 0;  // lines the last trace left in d_chords (0: none to draw)

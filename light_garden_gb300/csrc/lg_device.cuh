@@ -80,6 +80,20 @@ struct __align__(16) ObjInfo {
 };
 static_assert(sizeof(ObjInfo) == 48, "ObjInfo is 48 B");
 
+// Exact mode: what the FP64 solve of a proved root reads of an object, in one record (a chain of
+// lookups through the scan record, the object's tree nodes and its geometry nodes took longer than
+// the arithmetic).  Objects of one circle, rect, segment or cubic leaf, or of two of the first
+// three under a Logic node; others have kind SR_TREE and take their trees.
+struct __align__(16) SolveRec {
+  double org[2], rot[2];  // the Logic node's frame (SR_TWO)
+  double a[6], b[6];      // leaves: circle cx, cy, r, 1/r | rect cx, cy, cos, sin, half width, half height |
+                          // segment ax, ay, bx, by and the unit left normal; cubic c0..c2 in a, c3 in b (power basis)
+  uint32_t kind;          // SR_* | leaf kinds: a in bits 4..7, b in bits 8..11
+  uint32_t _pad[3];
+};
+static_assert(sizeof(SolveRec) == 144, "SolveRec is 144 B");
+enum : uint32_t { SR_TREE = 0, SR_ONE = 1, SR_TWO = 2 };
+
 struct __align__(8) Leaf64 {
   uint32_t kind;
   uint32_t _pad;
@@ -231,6 +245,7 @@ struct SceneDev {
   // preorder (ObjInfo::xnode_begin / xnode_count), the canvas half width in FP64
   const lg_geo* xgeo;
   const lgx::XNode* xnode;
+  const SolveRec* solve;
   double aspect64;
   // sampled frame (one scene): queue entry v of a light is its primary ray_offset + ray_stride * v
   uint32_t ray_stride, ray_offset;
@@ -842,7 +857,9 @@ __device__ __forceinline__ int cubic_roots32(const float* A, const float* Bp, fl
   const float a0 = dx * (c0y - oy) - dy * (c0x - ox);
   const float a1 = dx * c1y - dy * c1x, a2 = dx * c2y - dy * c2x, a3 = dx * c3y - dy * c3x;
   const float sc = fabsf(a0) + fabsf(a1) + fabsf(a2) + fabsf(a3) + 1e-30f;
-  const float err = 1e-4f * sc + 2e-6f * (fabsf(c0x) + fabsf(c0y) + fabsf(ox) + fabsf(oy));
+  // |f| below this is not decided: the control points' rounding to FP32 moves f by at most
+  // 27 2^-24 |P| sqrt(2) (the power basis weighs them 1, 6, 12, 8), the evaluation by some 10 2^-24 sc
+  const float err = 1e-5f * sc + 4e-6f * (fabsf(c0x) + fabsf(c0y) + fabsf(ox) + fabsf(oy));
   auto f = [&](float u) { return ((a3 * u + a2) * u + a1) * u + a0; };
   float knots[4];
   int nk = 0;
@@ -931,7 +948,9 @@ __device__ __forceinline__ Ival32 leaf_ival32(uint32_t kind, const float* L, flo
     const float disc = (r - perp) * (r + perp);
     const float scale = fabsf(b) + fabsf(perp) + r;
     I.tol = 4e-6f * scale + 1e-6f;
-    const float band = 2e-5f * scale * scale + 1e-3f * r * r;
+    // rounding moves perp by about 3 2^-24 scale and so disc, near tangency, by 4e-7 r scale; the
+    // roots of a disc above the band then move by less than tol's order
+    const float band = 1e-5f * r * scale + 1e-3f * r * r;
     if (disc < -band) return I;
     if (disc <= band) {  // near-tangent: hit or miss is decided in FP64
       const float w = sqrt_approx(band) + I.tol;

@@ -120,63 +120,73 @@ static __device__ __noinline__ double obj_best_x(const SceneDev& S, uint32_t k, 
   return ob;
 }
 
-// The FP64 hit of one leaf at the root the FP32 scan proved (t32; face32: the rect face as
-// 2 axis + (outward sign > 0); s32: a cubic's curve parameter): the very operations of
-// leaf_hits for that root only.  A circle computes the quotient of its proved root (q / a or
-// c / q, told apart by their FP32 values) and not the other; a rect computes the slab quotient
-// of its proved face and not the other three; a segment its ray parameter and not the place
-// along it; a cubic searches only the bracket that holds s32, and in it only near s32.  Other
-// leaves take leaf_hits and the root nearest t32.  False: no such hit (the caller
-// solves the object whole).
-__device__ __forceinline__ bool leaf_proved_hit(const lg_geo* G, const lg_geo& g, V o, V d, float t32, int face32,
-                                                float s32, double& ev, lgx::Hit& out) {
+// The FP64 hit of an object whose nearest root the FP32 scan proved (a single candidate with a
+// certain root and, for a two-leaf CSG object, certain membership of that root's point in the
+// other leaf): the very operations of object_hits, leaf_hits and object_normal for that root
+// only, since the other roots, the other leaf and the membership tests cannot change which hit
+// object_hits keeps.  side: the proved leaf; t32: its root; face: the rect face as 2 axis + (outward
+// sign > 0); s32: a cubic's curve parameter.  A circle computes the quotient of its proved
+// root (q / a or c / q, told apart by their FP32 values) and not the other; a rect the slab
+// quotient of its proved face and not the other three; a segment its ray parameter and not the
+// place along it; a cubic searches only the bracket that holds s32, and in it only near s32.
+// False: no such hit (the caller solves the object whole).
+__device__ __forceinline__ bool solve_proved_x(const SolveRec& G, V o, V d, int side, int face, float t32, float s32,
+                                               double& t, V& p, V& n) {
   using namespace lgx;
-  if (g.kind == LG_GEO_CIRCLE) {
-    const V oc = vsub(o, mk(g.origin[0], g.origin[1]));
-    const double r = g.v[0];
+  const uint32_t kind = G.kind;
+  const bool two = (kind & 0xfu) == SR_TWO;
+  const V org = mk(G.org[0], G.org[1]);
+  if (two) {
+    o = irot(vsub(o, org), G.rot[0], G.rot[1]);
+    d = irot(d, G.rot[0], G.rot[1]);
+  } else if (side != 0) {
+    return false;
+  }
+  const double* L = side ? G.b : G.a;
+  const uint32_t k = (side ? kind >> 8 : kind >> 4) & 0xfu;
+  if (k == LEAF_CIRCLE) {
+    const V ctr = mk(L[0], L[1]), oc = vsub(o, ctr);
+    const double r = L[2];
     const double a = dot(d, d), b = dot(oc, d), cc = sub(dot(oc, oc), mul(r, r));
     const double disc = sub(mul(b, b), mul(a, cc));
     if (is_neg(disc)) return false;
     const double sq = sqr(disc);
-    const double q = -add(b, b >= 0.0 ? sq : -sq);
+    const double q = -add(b, is_neg(b) ? -sq : sq);
     if (is_zero(q)) return false;
     const float ra = (float)q / (float)a, rc = (float)cc / (float)q;  // selection only
-    const double t = fabsf(ra - t32) <= fabsf(rc - t32) ? dvd(q, a) : dvd(cc, q);
-    if (!gt_pos(t, T_MIN)) return false;
-    const V p = vadd(o, vscl(d, t));
-    out = Hit{t, p, p, 0, 0};
-    return true;
-  }
-  if (g.kind == LG_GEO_RECT) {
-    if (face32 < 0) return false;
-    const int ax = face32 >> 1;
-    const bool pos = (face32 & 1) != 0;
+    const bool first = fabsf(ra - t32) <= fabsf(rc - t32);
+    t = dvd(first ? q : cc, first ? a : q);
+    p = vadd(o, vscl(d, t));
+    n = vscl(vsub(p, ctr), L[3]);
+  } else if (k == LEAF_RECT) {
+    if (face < 0) return false;
+    const int ax = face >> 1;
+    const bool pos = (face & 1) != 0;
     // the face's axis of irot(o - centre) and irot(d) alone: x' = c x + s y, y' = -s x + c y
-    const V rel = vsub(o, mk(g.origin[0], g.origin[1]));
-    const double kx = ax ? -g.rot[1] : g.rot[0], ky = ax ? g.rot[0] : g.rot[1];
+    const double c = L[2], s = L[3];
+    const V rel = vsub(o, mk(L[0], L[1]));
+    const double kx = ax ? -s : c, ky = ax ? c : s;
     const double O = add(mul(kx, rel.x), mul(ky, rel.y)), D = add(mul(kx, d.x), mul(ky, d.y));
-    const double h = ax ? g.v[3] : g.v[2];
     if (is_zero(D)) return false;
-    const double t = dvd(sub(pos ? h : -h, O), D);
-    if (!gt_pos(t, T_MIN)) return false;
-    out = mkhit(t, o, d, mk(0.0, 0.0), ax + (pos ? 2 : 0));
-    return true;
-  }
-  if (g.kind == LG_GEO_SEGMENT) {  // the crossing lies well inside the segment: t alone
-    const V A = mk(g.v[0], g.v[1]), e = vsub(mk(g.v[2], g.v[3]), A);
+    const double h = L[4 + ax];
+    t = dvd(sub(pos ? h : -h, O), D);
+    p = vadd(o, vscl(d, t));
+    const double sg = pos ? 1.0 : -1.0;
+    n = rot(ax == 0 ? mk(sg, 0.0) : mk(0.0, sg), c, s);
+  } else if (k == LEAF_SEGMENT) {  // the crossing lies well inside the segment: t alone
+    const V A = mk(L[0], L[1]), e = vsub(mk(L[2], L[3]), A);
     const double den = cross(d, e);
     if (is_zero(den)) return false;
-    const double t = dvd(cross(vsub(A, o), e), den);
-    if (!gt_pos(t, T_MIN)) return false;
-    out = mkhit(t, o, d, mk(0.0, 0.0), 0);
-    return true;
-  }
-  if (g.kind == LG_GEO_CUBIC && s32 > 0.0f) {
+    t = dvd(cross(vsub(A, o), e), den);
+    p = vadd(o, vscl(d, t));
+    n = mk(L[4], L[5]);
+  } else {  // cubic
     // the bracket between the derivative's roots that holds the proved curve parameter s32:
-    // hits_cubic's operations for that bracket only (a parameter within 1e-4 of a knot, or
-    // a knot or bracket end that is itself a root, takes the whole leaf below)
-    const Cubic k = cubic_of(g.v);
-    const double a[4] = {cross(d, vsub(k.c0, o)), cross(d, k.c1), cross(d, k.c2), cross(d, k.c3)};
+    // hits_cubic's operations for that bracket only (a parameter within 1e-4 of a knot takes the
+    // whole object)
+    if (!(s32 > 0.0f)) return false;
+    const Cubic K{mk(G.a[0], G.a[1]), mk(G.a[2], G.a[3]), mk(G.a[4], G.a[5]), mk(G.b[0], G.b[1])};
+    const double a[4] = {cross(d, vsub(K.c0, o)), cross(d, K.c1), cross(d, K.c2), cross(d, K.c3)};
     double kn[4];
     int nk = 0;
     kn[nk++] = 0.0;
@@ -186,7 +196,10 @@ __device__ __forceinline__ bool leaf_proved_hit(const lg_geo* G, const lg_geo& g
       if (disc >= 0.0) {
         const double sq = sqr(disc);
         const double q = mul(-0.5, add(qb, qb >= 0 ? sq : -sq));
-        double r1 = dvd(q, qa), r2 = q != 0.0 ? dvd(qc, q) : r1;
+        // a root that FP32 puts outside [0, 1] is no knot: 2 stands for it
+        const float e1 = __fdividef((float)q, (float)qa), e2 = __fdividef((float)qc, (float)q);
+        double r1 = e1 < -0.01f || e1 > 1.01f ? 2.0 : dvd(q, qa);
+        double r2 = q != 0.0 ? (e2 < -0.01f || e2 > 1.01f ? 2.0 : dvd(qc, q)) : r1;
         if (r1 > r2) { const double x = r1; r1 = r2; r2 = x; }
         if (r1 > 0.0 && r1 < 1.0) kn[nk++] = r1;
         if (r2 > 0.0 && r2 < 1.0 && (nk == 1 || r2 != kn[1])) kn[nk++] = r2;
@@ -199,131 +212,122 @@ __device__ __forceinline__ bool leaf_proved_hit(const lg_geo* G, const lg_geo& g
     double lo = -1.0, hi = -1.0;
     for (int i = 0; i + 1 < nk; ++i)
       if ((double)s32 > kn[i] + 1e-4 && (double)s32 < kn[i + 1] - 1e-4) { lo = kn[i]; hi = kn[i + 1]; }
-    if (lo >= 0.0) {
-      const double flo = poly3(a, lo), fhi = poly3(a, hi);
-      if (!is_zero(flo) && !is_zero(fhi) && is_neg(flo) != is_neg(fhi)) {
-        // f at s32 -+ 1e-4: where its signs are those of the bracket's ends, well above the
-        // rounding of f, f (monotone here) keeps them beyond these points
-        double wlo = sub((double)s32, 1e-4), whi = add((double)s32, 1e-4);
-        const double fa = poly3(a, wlo), fb = poly3(a, whi);
-        const float sc = 1e-9f * (fabsf((float)a[0]) + fabsf((float)a[1]) + fabsf((float)a[2]) + fabsf((float)a[3]));
-        if (is_neg(fa) != is_neg(flo) || is_neg(fb) == is_neg(flo) || !(fabsf((float)fa) > sc) || !(fabsf((float)fb) > sc)) {
-          wlo = lo;
-          whi = hi;
-        }
-        const double sr = cubic_root(a, lo, hi, flo, wlo, whi);
-        const double t = dvd(dot(vsub(cubic_point(k, sr), o), d), dot(d, d));
-        if (!gt_pos(t, T_MIN)) return false;
-        out = mkhit(t, o, d, mk(sr, 0.0), 0);
-        return true;
-      }
-    }
+    if (!(lo >= 0.0)) return false;
+    // f at s32 -+ 1e-4: where both values are well above the rounding of f and their signs differ,
+    // f (monotone between the knots) keeps those signs beyond these points, to the bracket's ends
+    const double wlo = sub((double)s32, 1e-4), whi = add((double)s32, 1e-4);
+    const double fa = poly3(a, wlo), fb = poly3(a, whi);
+    const float sc = 1e-9f * (fabsf((float)a[0]) + fabsf((float)a[1]) + fabsf((float)a[2]) + fabsf((float)a[3]));
+    if (is_neg(fa) == is_neg(fb) || !(fabsf((float)fa) > sc) || !(fabsf((float)fb) > sc)) return false;
+    const double sr = cubic_root(a, lo, hi, fa, wlo, whi);
+    t = dvd(dot(vsub(cubic_point(K, sr), o), d), dot(d, d));
+    p = vadd(o, vscl(d, t));
+    const V dB = cubic_tangent(K, sr);
+    const double l = sqr(dot(dB, dB));
+    n = l > 0.0 ? mk(dvd(-dB.y, l), dvd(dB.x, l)) : unit(mk(-d.y, d.x));
   }
-  double near = INFINITY;
-  bool found = false;
-  leaf_hits(G, g, o, d, ev, [&](const Hit& h) {
-    const double e = fabs(h.t - (double)t32);  // selection only
-    if (e < near) {
-      near = e;
-      out = h;
-      found = true;
-    }
-  });
-  return found;
-}
-
-// An object whose nearest root the FP32 scan proved (a single candidate with a certain root
-// and, for a two-leaf CSG object, certain membership of that root's point in the other
-// leaf): only the proved leaf's root is computed in FP64, and a CSG hit point is lifted out
-// of the Logic frame with the operations object_hits uses.  The other roots, the other leaf
-// and the membership tests cannot change which hit object_hits keeps, so the result is the
-// same bits.
-static __device__ __noinline__ bool solve_proved_x(const SceneDev& S, const ObjInfo& oi, V o, V d, int side, int face,
-                                                   float t32, float s32, double& ev, lgx::Hit& out) {
-  const lgx::XNode* nd = S.xnode + oi.xnode_begin;
-  const lg_geo& L = S.xgeo[nd[0].geo];
-  if (oi.xnode_count == 1) {
-    if (side != 0 || !leaf_proved_hit(S.xgeo, L, o, d, t32, face, s32, ev, out)) return false;
-    out.node = 0;
-    return true;
+  if (!gt_pos(t, T_MIN)) return false;
+  if (two) {  // lifted out of the Logic frame
+    p = vadd(org, rot(p, G.rot[0], G.rot[1]));
+    n = rot(n, G.rot[0], G.rot[1]);
   }
-  if (oi.xnode_count != 3 || L.kind != LG_GEO_LOGIC) return false;
-  const V org = lgx::mk(L.origin[0], L.origin[1]);
-  const V lo = lgx::irot(lgx::vsub(o, org), L.rot[0], L.rot[1]);
-  const V ld = lgx::irot(d, L.rot[0], L.rot[1]);
-  const int li = 1 + side;
-  if (!leaf_proved_hit(S.xgeo, S.xgeo[nd[li].geo], lo, ld, t32, face, 0.0f, ev, out)) return false;
-  out.node = li;
-  out.p = lgx::vadd(org, lgx::rot(out.p, L.rot[0], L.rot[1]));
   return true;
 }
 
-// Every ray with candidates (the refine lists and the full-solve list of k_scan): the
-// nearest hit over its candidates, each object solved whole as tracer.rs:412-424 does
-// (the minimum distance_squared over the object's hits, then over objects with ties kept by
-// the lower object index), and the near-degenerate flags of tracer.rs's decisions.  The
-// CTA's warps take the candidates one solve class (circle, rect, segment, cubic / deep CSG,
-// two-leaf CSG) at a time, with a barrier between classes, so that one geometry code path
-// is in flight per CTA.
+// The nearest hit of one ray over candidate objects, each solved whole as tracer.rs:412-424
+// does: the minimum distance_squared over an object's hits, then over objects with ties kept
+// by the lower object index.
+struct Nearest {
+  double best_d2 = INFINITY, second = INFINITY, ev = INFINITY;
+  int best = -1;
+  lgx::Hit h{0.0, {0.0, 0.0}, {0.0, 0.0}, 0, 0};
+  __device__ __forceinline__ void consider(const SceneDev& S, uint32_t base, uint32_t j, V o, V d) {
+    lgx::Hit oh;
+    const double ob = obj_best_x(S, base + j, o, d, ev, oh);
+    if (!lgx::plt(ob, INFINITY)) return;
+    if (lgx::plt(ob, best_d2) || (lgx::bits(ob) == lgx::bits(best_d2) && (int)j < best)) {
+      second = best_d2;
+      best_d2 = ob;
+      best = (int)j;
+      h = oh;
+    } else if (lgx::plt(ob, second)) {
+      second = ob;
+    }
+  }
+  // the hit record with the near-degenerate flags of tracer.rs's decisions: ties within the
+  // band, decisions in the band before the hit; the normal of the winning hit only
+  __device__ __forceinline__ void store(const SceneDev& S, uint32_t base, V d, uint8_t fl, HitRec& out) const {
+    if (best >= 0 && lgx::plt(second, INFINITY) && lgx::sub(second, best_d2) <= lgx::mul(lgx::BAND, best_d2)) fl |= lgx::NEAR;
+    if (lgx::plt(ev, INFINITY) && (best < 0 || ev <= lgx::add(lgx::mul(h.t, 1.0 + 1e-6), 1e-12))) fl |= lgx::NEAR;
+    V n = lgx::mk(0.0, 0.0);
+    int leaf = 0;
+    if (best >= 0) {
+      const lgx::XNode* nd = S.xnode + S.info[base + best].xnode_begin;
+      n = lgx::object_normal(S.xgeo, nd, d, h);
+      leaf = lgx::hit_leaf(S.xgeo, nd, h);
+    }
+    store_hit_x(out, best, h, n, leaf, ev, fl);
+  }
+};
+
+// A ray of a refine list whose root is not of SolveRec's kinds or turned out not to be there:
+// its one candidate solved whole.
+static __device__ __noinline__ void solve_one_x(const SceneDev& S, uint32_t base, uint32_t j, V o, V d, HitRec& out) {
+  Nearest N;
+  N.consider(S, base, j, o, d);
+  N.store(S, base, d, 0, out);
+}
+
+// Every ray with candidates.  First the refine lists (one candidate, its root proved; a list per
+// leaf kind, so a warp's rays take one path), straight from the SolveRec; then the full-solve
+// list, where the CTA's warps take the candidates one solve class (circle, rect, segment, cubic /
+// deep CSG, two-leaf CSG) at a time, with a barrier between classes, so that one geometry code
+// path is in flight per CTA.
 template <bool MULTI>
 __global__ void __launch_bounds__(256, LG_SOLVE_X_BLOCKS) k_solve_x(SceneDev S, TraceBufs B, uint32_t gen) {
-  uint64_t off[LIST_FULL + 2];
+  uint64_t off[LIST_FULL + 1];
   off[0] = 0;
-  for (int l = 0; l <= LIST_FULL; ++l) {
+  for (int l = 0; l < LIST_FULL; ++l) {
     const unsigned long long c = B.ctr->list_count[gen][l];
     off[l + 1] = off[l] + (c < B.queue_cap ? c : B.queue_cap);
   }
-  const uint64_t total = off[LIST_FULL + 1];
-  if ((uint64_t)blockIdx.x * blockDim.x >= total) return;  // no ray for this CTA
+  const uint64_t proved = off[LIST_FULL];
+  unsigned long long full = B.ctr->list_count[gen][LIST_FULL];
+  if (full > B.queue_cap) full = B.queue_cap;
+  const uint64_t first = blockIdx.x * (uint64_t)blockDim.x;
+  if (first >= proved && (gridDim.x - 1 - blockIdx.x) * (uint64_t)blockDim.x >= full) return;  // no ray for this CTA
   const RayRec* q = B.queue[gen & 1];
   uint32_t my_solves = 0;
-  // block-uniform loop (the class barrier needs every thread)
-  for (uint64_t base = blockIdx.x * (uint64_t)blockDim.x; base < total; base += (uint64_t)gridDim.x * blockDim.x) {
+  for (uint64_t i = first + threadIdx.x; i < proved; i += (uint64_t)gridDim.x * blockDim.x) {
+    int l = 0;
+    while (i >= off[l + 1]) ++l;
+    const uint32_t idx = B.list[l][i - off[l]];
+    const RayRec& r = q[idx];
+    const ScanRec& sc = B.scan[idx];
+    const uint32_t base = MULTI ? S.scenes[r.scene].obj_base : 0u, j = sc.cand[0];
+    const V o = ray_o(r), d = ray_d(r);
+    const SolveRec& G = S.solve[base + j];
+    lgx::Hit h;
+    V n;
+    ++my_solves;
+    if ((G.kind & 0xfu) != SR_TREE && solve_proved_x(G, o, d, sc.leaf, sc.face, sc.t32, sc.s32, h.t, h.p, n))
+      store_hit_x(B.hit[idx], (int)j, h, n, sc.leaf, INFINITY, 0);
+    else
+      solve_one_x(S, base, j, o, d, B.hit[idx]);
+  }
+  // block-uniform loop (the class barrier needs every thread), from the last CTA on: in a small
+  // generation the first CTAs have the proved rays
+  for (uint64_t base = (gridDim.x - 1 - blockIdx.x) * (uint64_t)blockDim.x; base < full; base += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t i = base + threadIdx.x;
-    const bool valid = i < total;
-    uint32_t idx = 0;
-    if (valid) {
-      int l = 0;
-      while (i >= off[l + 1]) ++l;
-      idx = B.list[l][i - off[l]];
-    }
-    const RayRec r = q[idx];
+    const bool valid = i < full;
+    const uint32_t idx = valid ? B.list[LIST_FULL][i] : 0u;
+    const RayRec& r = q[idx];
     const ScanRec sc = B.scan[idx];
     const SceneLoc sl = scene_of<MULTI>(S, valid ? r.scene : 0u);
     const V o = ray_o(r), d = ray_d(r);
-    double best_d2 = INFINITY, second = INFINITY, ev = INFINITY;
-    int best = -1;
-    lgx::Hit bh{0.0, lgx::mk(0.0, 0.0), lgx::mk(0.0, 0.0), 0, 0};
-    auto consider = [&](uint32_t j) {
-      lgx::Hit oh;
-      ++my_solves;
-      const double ob = obj_best_x(S, sl.base + j, o, d, ev, oh);
-      if (!lgx::plt(ob, INFINITY)) return;
-      if (lgx::plt(ob, best_d2) || (lgx::bits(ob) == lgx::bits(best_d2) && (int)j < best)) {
-        second = best_d2;
-        best_d2 = ob;
-        best = (int)j;
-        bh = oh;
-      } else if (lgx::plt(ob, second)) {
-        second = ob;
-      }
-    };
-    // proved roots (single leaves, two-leaf CSG) first, in a phase of their own
-    bool proved = false;
-    uint32_t pcls = 7u;
-    if (valid && i < off[LIST_FULL] && !sc.overflow && sc.nc == 1 && (sc.leaf == 0 || sc.leaf == 1))
-      pcls = solve_class(__ldg(&S.scan[sl.base + sc.cand[0]].info));
-    // class 3 holds single cubic leaves and deep CSG trees; only a cubic reaches a refine list
-    if (pcls <= 2u || pcls == 4u || (pcls == 3u && sc.leaf == 0)) {
-      proved = solve_proved_x(S, S.info[sl.base + sc.cand[0]], o, d, sc.leaf, sc.face, sc.t32, sc.s32, ev, bh);
-      if (proved) {
-        best = sc.cand[0];
-        ++my_solves;
-      }
-    }
-    __syncthreads();
+    Nearest N;
     {
-      uint32_t pending = valid && !sc.overflow && !proved ? (1u << sc.nc) - 1u : 0u;
+      uint32_t pending = valid && !sc.overflow ? (1u << sc.nc) - 1u : 0u;
       uint32_t cls[CAND];
       for (int k = 0; k < CAND; ++k)
         cls[k] = (pending >> k) & 1u ? solve_class(__ldg(&S.scan[sl.base + sc.cand[k]].info)) : 7u;
@@ -335,7 +339,8 @@ __global__ void __launch_bounds__(256, LG_SOLVE_X_BLOCKS) k_solve_x(SceneDev S, 
           if (!__any_sync(0xffffffffu, k >= 0)) break;
           if (k >= 0) {
             pending &= ~(1u << k);
-            consider(sc.cand[k]);
+            ++my_solves;
+            N.consider(S, sl.base, sc.cand[k], o, d);
           }
         }
         __syncthreads();
@@ -350,22 +355,11 @@ __global__ void __launch_bounds__(256, LG_SOLVE_X_BLOCKS) k_solve_x(SceneDev S, 
         float lb;
         if (!bound_test(h, ox, oy, dx, dy, sc.thr, lb)) continue;
         if (!(classify32(sobjs[j], ox, oy, dx, dy, lb, j == r.src_obj ? (int)r.src_leaf : -1).key <= sc.thr)) continue;
-        consider(j);
+        ++my_solves;
+        N.consider(S, sl.base, j, o, d);
       }
     }
-    uint8_t fl = sc.overflow ? LG_PATH_FALLBACK : 0;
-    // tracer.rs:404,417 ties within the band, and decisions in the band before the hit
-    if (best >= 0 && lgx::plt(second, INFINITY) && lgx::sub(second, best_d2) <= lgx::mul(lgx::BAND, best_d2)) fl |= lgx::NEAR;
-    if (lgx::plt(ev, INFINITY) && (best < 0 || ev <= lgx::add(lgx::mul(bh.t, 1.0 + 1e-6), 1e-12))) fl |= lgx::NEAR;
-    V n = lgx::mk(0.0, 0.0);
-    int leaf = 0;
-    if (best >= 0) {  // the normal of the winning hit only
-      const ObjInfo& oi = S.info[sl.base + best];
-      const lgx::XNode* nd = S.xnode + oi.xnode_begin;
-      n = lgx::object_normal(S.xgeo, nd, d, bh);
-      leaf = lgx::hit_leaf(S.xgeo, nd, bh);
-    }
-    store_hit_x(B.hit[idx], best, bh, n, leaf, ev, fl);
+    N.store(S, sl.base, d, sc.overflow ? LG_PATH_FALLBACK : 0, B.hit[idx]);
   }
   add_block_counts<1>({my_solves}, {&B.ctr->fp64_solves});
 }

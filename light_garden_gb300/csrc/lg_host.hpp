@@ -42,6 +42,7 @@ struct Flat {
   // xnode_begin / xnode_count index xnode; XNode::geo indexes xgeo) and the deepest node
   std::vector<lg_geo> xgeo;
   std::vector<lgx::XNode> xnode;
+  std::vector<SolveRec> solve;  // one per object
   int xdepth = 0;
   // appends another scene's exact-mode tables, moving its node indices past this one's;
   // the caller adds the returned base to that scene's ObjInfo::xnode_begin
@@ -52,6 +53,7 @@ struct Flat {
       n.geo += (int32_t)g0;
       xnode.push_back(n);
     }
+    solve.insert(solve.end(), o.solve.begin(), o.solve.end());
     xdepth = xdepth > o.xdepth ? xdepth : o.xdepth;
     return n0;
   }

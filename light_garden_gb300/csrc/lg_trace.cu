@@ -334,7 +334,7 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, CULL ? SCAN_CULL_BLOCKS : 4)
     W.ray[w][lane] = make_float4(ox, oy, dx, dy);
     W.src[w][lane] = live ? ((uint32_t)r.src_obj << 8 | r.src_leaf) : 0xffffffffu;
     W.base[w][lane] = sl.base;
-    float thr = INFINITY;
+    float thr = 3e38f;  // finite: a certain miss (key INFINITY) is never a candidate
     int nc = 0;
     bool overflow = false;
     // The warp scans one scene at a time: a multi-scene warp (rays of several scenes, at
