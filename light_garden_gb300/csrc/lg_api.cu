@@ -878,27 +878,15 @@ void launch_light_setup(lg_ctx* c, const SceneDev& S, bool multi) {
   }
 }
 
-// Events around one generation's kernels while lg_render captures its frame graph (kev_on),
-// k = 0 before the scan, 1 after it, 2 after the precise solve, 3 after the bounce.
-static void kernel_event(lg_ctx* c, uint32_t g, int k) {
-  if (!c->kev_on || 4 * g + k >= c->kev.size()) return;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(c->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusActive) return;
-  cudaEventRecordWithFlags(c->kev[4 * g + k], c->stream, cudaEventRecordExternal);  // only inside the frame graph
-}
-
 void launch_generation(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_t g, bool multi, int scan_grid,
                        size_t scan_smem, size_t tsm, int smem_fits) {
   const bool exact = c->prm.precision == LG_PRECISION_EXACT;
-  kernel_event(c, g, 0);
   scan_kernel(multi, c->scan_walk, exact, scan_pairs_of(c))<<<scan_grid, SCAN_THREADS, scan_smem, c->stream>>>(S, B, g,
                                                                                                    smem_fits);
-  kernel_event(c, g, 1);
   if (exact) {
     if (multi) k_solve_x<true><<<c->trace_grid[4], 256, 0, c->stream>>>(S, B, g);
     else k_solve_x<false><<<c->trace_grid[4], 256, 0, c->stream>>>(S, B, g);
-    kernel_event(c, g, 2);
-    bounce_x_kernel(multi, c->culled)<<<c->trace_grid[5], 256, 0, c->stream>>>(S, B, g);
+      bounce_x_kernel(multi, c->culled)<<<c->trace_grid[5], 256, 0, c->stream>>>(S, B, g);
   } else {
     if (multi) {
       k_refine<true><<<c->trace_grid[1], 256, 0, c->stream>>>(S, B, g);
@@ -907,35 +895,23 @@ void launch_generation(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_
       k_refine<false><<<c->trace_grid[1], 256, 0, c->stream>>>(S, B, g);
       k_full<false><<<c->trace_grid[2], 256, tsm, c->stream>>>(S, B, g, smem_fits);
     }
-    kernel_event(c, g, 2);
-    bounce_kernel(multi, c->culled)<<<c->trace_grid[3], 256, tsm, c->stream>>>(S, B, g, smem_fits);
+      bounce_kernel(multi, c->culled)<<<c->trace_grid[3], 256, tsm, c->stream>>>(S, B, g, smem_fits);
   }
-  kernel_event(c, g, 3);
 }
 
-// Per-kernel trace times of the last lg_render, from the kernel events of every generation.
+// Per-kernel trace times of the last lg_render, from the kernels' own stamps.
 static void kernel_times(lg_ctx* c, lg_trace_stats* s) {
-  if (!s || !c->kev_on) return;
-  float a = 0.f, b = 0.f, d = 0.f;
-  for (uint32_t g = 0; g < c->prm.max_bounce && 4 * g + 3 < c->kev.size(); ++g) {
-    a += elapsed(c->kev[4 * g], c->kev[4 * g + 1]);
-    b += elapsed(c->kev[4 * g + 1], c->kev[4 * g + 2]);
-    d += elapsed(c->kev[4 * g + 2], c->kev[4 * g + 3]);
+  if (!s) return;
+  unsigned long long a = 0, b = 0, d = 0;
+  for (uint32_t g = 0; g < c->prm.max_bounce && g < (uint32_t)MAX_GEN; ++g) {
+    const unsigned long long* t = c->h_ctr->stamp[g];
+    a += t[1] - t[0];
+    b += t[2] - t[1];
+    d += t[3] - t[2];
   }
-  s->scan_ms = a;
-  s->solve_ms = b;
-  s->bounce_ms = d;
-}
-
-// lg_render's graphs record the kernel events (created once per context).
-static lg_status enable_kernel_events(lg_ctx* c) {
-  if (c->kev.empty()) {
-    c->kev.assign(4 * MAX_GEN, nullptr);
-    for (auto& e : c->kev) CK(cudaEventCreate(&e), "event");
-  }
-  if (!c->kev_on) c->graph_valid = false;  // the captured graph must record them
-  c->kev_on = true;
-  return LG_OK;
+  s->scan_ms = (float)((double)a * 1e-6);
+  s->solve_ms = (float)((double)b * 1e-6);
+  s->bounce_ms = (float)((double)d * 1e-6);
 }
 
 lg_status upload_exact(lg_ctx* c, const Flat& F) {
@@ -1255,8 +1231,6 @@ lg_status lg_destroy(lg_ctx* c) {
   for (int i = 0; i < 6; ++i)
     if (c->ev[i]) cudaEventDestroy(c->ev[i]);
   for (cudaEvent_t e : c->bev)
-    if (e) cudaEventDestroy(e);
-  for (cudaEvent_t e : c->kev)
     if (e) cudaEventDestroy(e);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
@@ -1661,7 +1635,6 @@ static lg_status render_frame(lg_ctx* c, uint16_t* dst, size_t pitch, int32_t ds
   const size_t row = (size_t)c->prm.width * 8;
   if (!dst || pitch < row) return fail(c, LG_ERR_INVALID_ARGUMENT, "destination null or pitch < width * 8");
   uint32_t retries = 0;
-  if ((st = enable_kernel_events(c))) return st;
   if (c->streaming) return render_streaming(c, dst, pitch, dst_is_device, stats, retries);
   for (int attempt = 0; attempt < 8; ++attempt) {
     if (!c->graph_valid) {

@@ -171,6 +171,9 @@ struct Counters {
   // generation; these keep the totals and the largest per-generation demands
   unsigned long long seg_total, seg_max, refs_total, refs_max;
   unsigned long long bound_tests, object_tests;  // nearest-hit search: bounding tests, classifications
+  // lg_render's kernel times (ns of the GPU's global timer): per generation the starts of the
+  // scan, the precise solve and the bounce, and the bounce's end
+  unsigned long long stamp[MAX_GEN][4];
   unsigned int error_flags;
   unsigned int skip_raster;  // streaming accumulation: this generation's accumulation is deferred
 };

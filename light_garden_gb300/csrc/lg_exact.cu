@@ -285,6 +285,7 @@ static __device__ __noinline__ void solve_one_x(const SceneDev& S, uint32_t base
 // path is in flight per CTA.
 template <bool MULTI>
 __global__ void __launch_bounds__(256, LG_SOLVE_X_BLOCKS) k_solve_x(SceneDev S, TraceBufs B, uint32_t gen) {
+  stamp_start(B.ctr, gen, 1);
   uint64_t off[LIST_FULL + 1];
   off[0] = 0;
   for (int l = 0; l < LIST_FULL; ++l) {
@@ -683,6 +684,7 @@ __device__ __forceinline__ void emit_segments_x(const SceneDev& S, const TraceBu
 
 template <bool MULTI, bool CULL>
 __global__ void __launch_bounds__(256, LG_BOUNCE_X_BLOCKS) k_bounce_x(SceneDev S, TraceBufs B, uint32_t gen) {
+  stamp_start(B.ctr, gen, 2);
   // the rays with work: every work list of this generation, one after the other
   uint64_t off[N_LISTS + 1];
   off[0] = 0;
@@ -733,6 +735,7 @@ __global__ void __launch_bounds__(256, LG_BOUNCE_X_BLOCKS) k_bounce_x(SceneDev S
         if (first + q < B.queue_cap) qout[first + q] = v.child[q];
     }
   }
+  stamp_end(B.ctr, gen);
   add_block_counts<2>({my_visits, my_near}, {&B.ctr->visits, &B.ctr->near});
 }
 template __global__ void k_bounce_x<false, false>(SceneDev, TraceBufs, uint32_t);

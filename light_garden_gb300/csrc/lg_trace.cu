@@ -261,6 +261,7 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, CULL ? SCAN_CULL_BLOCKS : 4)
   __shared__ __align__(8) uint64_t bar;
   ScanSmem& W = *reinterpret_cast<ScanSmem*>(smem_raw);
   ObjScan* sobj = reinterpret_cast<ObjScan*>(smem_raw + sizeof(ScanSmem));
+  stamp_start(B.ctr, gen, 0);
   const uint64_t n_real = n_real_of(S, B, gen);
   const uint64_t n_in = n_in_of(S, B, gen);
   if ((uint64_t)blockIdx.x * blockDim.x >= n_in) return;  // no ray for this CTA
@@ -649,6 +650,7 @@ __device__ __forceinline__ void store_hit(HitRec& o, int obj, const Hit64& h, fl
 // one list except at the seams, so the kinds stay apart as in four launches).
 template <bool MULTI>
 __global__ void __launch_bounds__(256) k_refine(SceneDev S, TraceBufs B, uint32_t gen) {
+  stamp_start(B.ctr, gen, 1);
   auto count = [&](int l) -> uint64_t {
     const unsigned long long c = B.ctr->list_count[gen][l];
     return c < B.queue_cap ? c : B.queue_cap;
@@ -959,6 +961,7 @@ template <bool MULTI, bool CULL>
 __global__ void __launch_bounds__(256, 3) k_bounce(SceneDev S, TraceBufs B, uint32_t gen, int smem_fits) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ __align__(8) uint64_t bar;
+  stamp_start(B.ctr, gen, 2);
   // the rays with work: every work list of this generation, one after the other
   uint64_t off[N_LISTS + 1];
   off[0] = 0;
@@ -1015,6 +1018,7 @@ __global__ void __launch_bounds__(256, 3) k_bounce(SceneDev S, TraceBufs B, uint
         if (first + q < B.queue_cap) qout[first + q] = v.child[q];
     }
   }
+  stamp_end(B.ctr, gen);
   add_block_counts<3>({my_visits, my_near, my_ill}, {&B.ctr->visits, &B.ctr->near, &B.ctr->ill});
 }
 template __global__ void k_bounce<false, false>(SceneDev, TraceBufs, uint32_t, int);

@@ -54,6 +54,25 @@ __device__ __forceinline__ uint64_t n_in_of(const SceneDev& S, const TraceBufs& 
   return n < B.queue_cap ? n : B.queue_cap;
 }
 
+// Time stamps of a generation's kernels (Counters::stamp): the first CTA's start, and for the
+// bounce the last CTA's end.  (Event nodes between the kernels of a captured frame cost more than
+// the small generations' kernels.)
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+__device__ __forceinline__ void stamp_start(Counters* ctr, uint32_t gen, int k) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const unsigned long long t = global_ns();
+    ctr->stamp[gen][k] = t;
+    if (k == 2) atomicMax(&ctr->stamp[gen][3], t);
+  }
+}
+__device__ __forceinline__ void stamp_end(Counters* ctr, uint32_t gen) {
+  if (threadIdx.x == 0) atomicMax(&ctr->stamp[gen][3], global_ns());
+}
+
 // The threads' event counts into the context's counters, at the end of a kernel: a warp
 // reduction (redux) per count, the warps' sums through shared memory, one global atomic per
 // CTA and count that is not zero.  Every thread of the CTA calls it.  (A 64-bit atomicAdd on
