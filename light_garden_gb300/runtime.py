@@ -81,20 +81,20 @@ class Context:
 
     def resolve_f16(self) -> np.ndarray:
         h, w = self._shape()
-        out = np.zeros((h, w, 4), np.uint16)
+        out = np.empty((h, w, 4), np.uint16)
         self._check(self.lib.lg_resolve_f16(self.h, out.ctypes.data_as(C.c_void_p), w * 8, 0), "lg_resolve_f16")
         return out
 
     def resolve_rgba8(self) -> np.ndarray:
         h, w = self._shape()
-        out = np.zeros((h, w, 4), np.uint8)
+        out = np.empty((h, w, 4), np.uint8)
         self._check(self.lib.lg_resolve_rgba8(self.h, out.ctypes.data_as(C.c_void_p), w * 4, 0), "lg_resolve_rgba8")
         return out
 
     def render(self, out: Optional[np.ndarray] = None) -> Tuple[np.ndarray, dict]:
         h, w = self._shape()
         if out is None:
-            out = np.zeros((h, w, 4), np.uint16)
+            out = np.empty((h, w, 4), np.uint16)
         s = abi.lg_trace_stats()
         st = self.lib.lg_render(self.h, out.ctypes.data_as(C.c_void_p), out.strides[0], 0, C.byref(s))
         self._check(st, "lg_render")
@@ -112,7 +112,7 @@ class Context:
         st = self.lib.lg_chords_download(self.h, None, 0, C.byref(n))
         if st not in (abi.LG_OK, abi.LG_ERR_TRUNCATED):
             self._check(st, "lg_chords_download")
-        out = np.zeros(int(n.value), abi.chord_dtype())
+        out = np.empty(int(n.value), abi.chord_dtype())
         self._check(self.lib.lg_chords_download(self.h, out.ctypes.data_as(C.POINTER(abi.lg_chord)), len(out),
                                                 C.byref(n)), "lg_chords_download")
         return out
@@ -123,8 +123,8 @@ class Context:
         if st not in (abi.LG_OK, abi.LG_ERR_TRUNCATED):
             self._check(st, "lg_segments_download")
         k = int(n.value)
-        segs = np.zeros(k, abi.segment_dtype())
-        recs = np.zeros(k, abi.path_dtype()) if paths else None
+        segs = np.empty(k, abi.segment_dtype())
+        recs = np.empty(k, abi.path_dtype()) if paths else None
         st = self.lib.lg_segments_download(
             self.h, segs.ctypes.data_as(C.POINTER(abi.lg_segment)),
             recs.ctypes.data_as(C.POINTER(abi.lg_path_record)) if paths else None, k, C.byref(n))
@@ -165,7 +165,7 @@ class Context:
 
     def batch_render(self):
         """All images of the batch as a list of (height, width, 4) binary16 bit patterns."""
-        flat = np.zeros(self.batch_pixels() * 4, np.uint16)
+        flat = np.empty(self.batch_pixels() * 4, np.uint16)
         stats = self.batch_render_into(flat.ctypes.data, flat.nbytes, False)
         imgs = [flat[4 * o:4 * (o + h * w)].reshape(h, w, 4) for o, (h, w) in zip(self.batch_offsets, self.batch_shapes)]
         return imgs, stats
@@ -192,7 +192,7 @@ class Context:
     def serve_poll(self, rid: int) -> Optional[np.ndarray]:
         """The finished image of request rid, or None while it is queued or in flight."""
         h, w = self.serve_shapes[rid]
-        out = np.zeros((h, w, 4), np.uint16)
+        out = np.empty((h, w, 4), np.uint16)
         st = self.lib.lg_serve_poll(self.h, rid, out.ctypes.data_as(C.c_void_p), out.nbytes, 0)
         if st == abi.LG_ERR_NOT_READY:
             return None
@@ -206,7 +206,7 @@ class Context:
     def accum(self) -> np.ndarray:
         h, w = self._shape()
         dt = np.float32 if self.params.accum == abi.LG_ACCUM_F32 else np.int64
-        out = np.zeros((h, w, 4), dt)
+        out = np.empty((h, w, 4), dt)
         self._check(self.lib.lg_accum_download(self.h, out.ctypes.data_as(C.c_void_p), out.nbytes),
                     "lg_accum_download")
         return out
