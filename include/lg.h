@@ -321,10 +321,9 @@ typedef struct lg_device_opts {
   int32_t wait_polls;         /* polls of each bounded device-side wait before it gives up with
                                  LG_ERR_TIMEOUT: 0 = default (2^22); a negative value gives up
                                  at once (exercises the timeout path in tests) */
-  int32_t scan_pairs;         /* pair slots per lane of the FP32 nearest-hit scan, 8 or 16; 0 =
-                                 autotune: the second lg_render / lg_batch_render of each scene or
-                                 batch renders with both and keeps the faster (results are
-                                 identical either way; a scene rendered once is not tuned) */
+  int32_t scan_pairs;         /* pair slots per lane of the FP32 nearest-hit scan, 8 or 16; 0 = 8
+                                 where the scan walks the culling grid, else 16 (results are
+                                 identical either way) */
 } lg_device_opts;
 
 /* Nearest-hit culling (replaces the reference's approximate tile map, tile_map.rs:18-146).
@@ -333,13 +332,12 @@ typedef struct lg_device_opts {
 typedef enum lg_culling {
   LG_CULL_AUTO = 0,  /* grid for scenes of LG_CULL_AUTO_MIN objects or more; the bounce's medium
                         test uses it, and the nearest-hit scan walks it from LG_CULL_WALK_MIN
-                        objects (batches: always) or as the scene's second lg_render measured
-                        faster (lg_device_opts.scan_pairs = 0) */
+                        objects (batches and serving: wherever a scene has one) */
   LG_CULL_OFF = 1,   /* every ray tests every object's bounding circle */
   LG_CULL_ON = 2     /* grid for every scene, walked by the scan */
 } lg_culling;
 #define LG_CULL_AUTO_MIN 16
-#define LG_CULL_WALK_MIN 96
+#define LG_CULL_WALK_MIN 48
 
 typedef struct lg_ctx lg_ctx;
 

@@ -104,7 +104,7 @@ pub const LG_CULL_AUTO: i32 = 0;
 pub const LG_CULL_OFF: i32 = 1;
 pub const LG_CULL_ON: i32 = 2;
 pub const LG_CULL_AUTO_MIN: u32 = 16;
-pub const LG_CULL_WALK_MIN: u32 = 96;
+pub const LG_CULL_WALK_MIN: u32 = 48;
 
 #[repr(C)]
 pub struct lg_ctx {

@@ -811,8 +811,10 @@ TraceKernel scan_kernel(bool multi, bool culled, bool exact, int pairs) {
   return pairs <= 8 ? scan_kernel_ch<8>(multi, culled, exact) : scan_kernel_ch<16>(multi, culled, exact);
 }
 
-// The scan's pair slots per lane: the tuned or requested value, else 8 with a culling grid
-// and 16 without.
+// The scan's pair slots per lane: as requested, else 8 for the grid walk (a smaller buffer leaves
+// more of the SM's L1 to the list and queue loads: 131072 rays, 64 objects 9.0 ms of scan against
+// 11.0 with 16, 200 objects 16.5 against 20.1, a 64-scene batch 86.1 against 89.5 ms of trace) and 16
+// for the table scan (64 CSG objects 12.2 against 12.9 ms with 8, 12 objects 0.58 against 0.62).
 int scan_pairs_of(const lg_ctx* c) { return c->scan_pairs ? c->scan_pairs : (c->scan_walk ? 8 : 16); }
 
 // Occupancy-sized grid of the scan for the context's mode and pair slots.
@@ -837,12 +839,6 @@ lg_status scan_grid(lg_ctx* c, bool multi) {
   return LG_OK;
 }
 
-// Switches the scan to `pairs` slots per lane: new grid, new graph.
-lg_status set_scan_pairs(lg_ctx* c, int pairs, bool multi) {
-  c->scan_pairs = pairs;
-  c->graph_valid = false;
-  return scan_grid(c, multi);
-}
 TraceKernel bounce_kernel(bool multi, bool culled) {
   if (multi) return culled ? k_bounce<true, true> : k_bounce<true, false>;
   return culled ? k_bounce<false, true> : k_bounce<false, false>;
@@ -967,23 +963,27 @@ lg_status upload_crossings(lg_ctx* c, const lg_string_mod& outer) {
   lg_string_mod sm = outer;
   sm.colors = nullptr;
   sm.nested = nullptr;
-  const uint64_t n_pairs = m * (m - 1);
+  const uint64_t n_pairs = m * (m - 1);  // below 2^24: m is at most LG_STRING_MOD_NESTED_MAX
   const uint32_t n_blk = (uint32_t)((n_pairs + CROSS_PAIRS_PER_BLOCK - 1) / CROSS_PAIRS_PER_BLOCK);
   lg_status st;
-  if ((st = ensure(c, c->d_sm_lines, 2 * m * sizeof(double2), "string-mod crossings"))) return st;
-  if ((st = ensure(c, c->d_cross_blk, (size_t)n_blk * 4 + 16, "string-mod crossings"))) return st;
-  double2* lines = (double2*)c->d_sm_lines.p;
-  uint32_t* blk = (uint32_t*)c->d_cross_blk.p;
-  unsigned long long* d_total = (unsigned long long*)((char*)c->d_cross_blk.p + (((size_t)n_blk * 4 + 7) & ~(size_t)7));
-  k_sm_lines<<<(int)((m + 255) / 256), 256, 0, c->stream>>>(sm, lines);
-  k_cross_count<<<n_blk, CROSS_THREADS, 0, c->stream>>>(lines, m, blk);
+  // one buffer: the masks (16-byte aligned), the block counts, the total
+  const size_t mask_bytes = (size_t)n_blk * CROSS_MASKS * 4, blk_bytes = ((size_t)n_blk * 4 + 7) & ~(size_t)7;
+  if ((st = ensure(c, c->d_sm_lines, 2 * m * (sizeof(double2) + sizeof(float2)), "string-mod crossings"))) return st;
+  if ((st = ensure(c, c->d_cross_blk, mask_bytes + blk_bytes + 16, "string-mod crossings"))) return st;
+  double2* pts = (double2*)c->d_sm_lines.p;
+  float2* pts32 = (float2*)(pts + 2 * m);  // 32 m bytes on: 16-byte aligned
+  uint32_t* masks = (uint32_t*)c->d_cross_blk.p;
+  uint32_t* blk = (uint32_t*)((char*)c->d_cross_blk.p + mask_bytes);
+  unsigned long long* d_total = (unsigned long long*)((char*)c->d_cross_blk.p + mask_bytes + blk_bytes);
+  k_sm_lines<<<(int)((2 * m + 63) / 64), 64, 0, c->stream>>>(sm, pts, pts32);
+  k_cross_count<<<n_blk, CROSS_THREADS, 0, c->stream>>>(pts, (const float4*)pts32, (uint32_t)m, blk, masks);
   k_cross_scan<<<1, 1024, 0, c->stream>>>(blk, n_blk, d_total);
   unsigned long long total = 0;
   CK(cudaMemcpyAsync(&total, d_total, sizeof total, cudaMemcpyDeviceToHost, c->stream), "string-mod crossings");
   CK(cudaStreamSynchronize(c->stream), "string-mod crossings");
   if (total) {
     if ((st = ensure(c, c->d_cross, total * sizeof(double2), "string-mod crossings"))) return st;
-    k_cross_write<<<n_blk, CROSS_THREADS, 0, c->stream>>>(lines, m, blk, (double2*)c->d_cross.p);
+    k_cross_write<<<n_blk, CROSS_THREADS, 0, c->stream>>>(pts, (uint32_t)m, blk, masks, (double2*)c->d_cross.p);
     CK(cudaGetLastError(), "string-mod crossings");
   }
   c->n_cross = total;
@@ -1179,7 +1179,7 @@ lg_status lg_create(lg_ctx** out, const lg_device_opts* opts) {
     delete c;
     return LG_ERR_INVALID_ARGUMENT;
   }
-  c->scan_pairs_opt = opts ? opts->scan_pairs : 0;
+  c->scan_pairs = opts ? opts->scan_pairs : 0;
   cudaError_t e = cudaSetDevice(c->device);
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&c->n_sm, cudaDevAttrMultiProcessorCount, c->device);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
@@ -1225,7 +1225,8 @@ lg_status lg_destroy(lg_ctx* c) {
                     &c->d_tile_cursor, &c->d_unit_off, &c->d_refs, &c->d_units, &c->d_accum, &c->d_stage,
                     &c->d_scenes, &c->d_canvases, &c->d_seg_scene, &c->d_cubic_scene, &c->d_part,
                     &c->d_bounds, &c->d_order, &c->d_scene_count, &c->d_scene_off,
-                    &c->d_grids, &c->d_cell_start, &c->d_cell_obj, &c->d_cta_hist, &c->d_solve};
+                    &c->d_grids, &c->d_cell_start, &c->d_cell_obj, &c->d_cta_hist, &c->d_solve,
+                    &c->d_mod_colors, &c->d_chords, &c->d_sm_lines, &c->d_cross_blk, &c->d_cross, &c->d_xgeo, &c->d_xnode};
   for (DevBuf* b : bufs) release(*b);
   if (c->h_ctr) cudaFreeHost(c->h_ctr);
   for (int i = 0; i < 6; ++i)
@@ -1323,11 +1324,12 @@ lg_status lg_scene_upload(lg_ctx* c, const lg_geo* geos, uint32_t n_geo, const l
     c->culled = F.grid.rec.nx > 0;
     c->graph_valid = false;
   }
-  // a new scene's scan walks the grid from LG_CULL_WALK_MIN objects until the autotuner measures
-  // it (the bounce's medium test takes the grid whenever there is one); the same scene again keeps
-  // what was tuned
+  // the scan walks the grid from LG_CULL_WALK_MIN objects (131072 rays: with 32 objects the table
+  // scan takes 3.5 / 4.4 ms for plain / CSG objects and the walk 3.6 / 5.1, with 48 6.1 / 6.7 against
+  // 5.6 / 6.6, with 64 11.9 / 12.2 against 9.0 / 9.5); the bounce's medium test takes the grid
+  // whenever there is one
   const bool walk = c->culled && (n_objects >= LG_CULL_WALK_MIN || c->culling == LG_CULL_ON);
-  if ((!same_shape || !c->culled) && c->scan_walk != walk) {
+  if (c->scan_walk != walk) {
     c->scan_walk = walk;
     c->graph_valid = false;
   }
@@ -1349,11 +1351,6 @@ lg_status lg_scene_upload(lg_ctx* c, const lg_geo* geos, uint32_t n_geo, const l
   c->smem_fits = c->obj_smem <= OBJ_SMEM_MAX ? 1 : 0;
   int occ = 0;
   const size_t tsm = c->smem_fits ? c->obj_smem : 0;
-  if (!same_shape) {  // a new scene: its second lg_render times both scan pair-buffer sizes
-    c->scan_pairs = c->scan_pairs_opt;
-    c->scan_tune = c->scan_pairs_opt == 0;
-    c->renders = 0;
-  }
   if ((st = scan_grid(c, false))) return st;
   if ((st = trace_grids(c, false, tsm))) return st;
   CK(raster_occupancy(raster_mode(p), &occ), "occupancy");
@@ -1598,40 +1595,9 @@ static lg_status render_streaming(lg_ctx* c, uint16_t* dst, size_t pitch, int32_
   return fail(c, LG_ERR_OUT_OF_MEMORY, "render buffers kept overflowing");
 }
 
-static lg_status render_frame(lg_ctx* c, uint16_t* dst, size_t pitch, int32_t dst_is_device, lg_trace_stats* stats);
-
-// The second frame of a scene (unless lg_device_opts.scan_pairs fixes the size) renders with
-// each scan pair-buffer size and keeps the one whose scan kernels ran faster; the frames are
-// identical, so the caller's image is simply the last one.  A scene rendered once keeps the
-// default (8 slots with a culling grid, 16 without) and pays no tuning.
 lg_status lg_render(lg_ctx* c, uint16_t* dst, size_t pitch, int32_t dst_is_device, lg_trace_stats* stats) {
   lg_status st = need_scene(c);
   if (st) return st;
-  if (c->renders < 0xffffffffu) ++c->renders;
-  if (c->scan_tune && c->renders >= 2) {
-    // with a culling grid: the grid walk with 8 pair slots against the table scan with 16; without
-    // one: the table scan with 8 against 16
-    c->scan_tune = false;
-    float best = INFINITY;
-    int pick = scan_pairs_of(c);
-    bool pick_walk = c->scan_walk;
-    const int opts[2][2] = {{c->culled ? 1 : 0, 8}, {0, 16}};
-    for (const auto& o : opts) {
-      c->scan_walk = o[0] != 0;
-      if ((st = set_scan_pairs(c, o[1], false))) return st;
-      lg_trace_stats s;
-      if ((st = render_frame(c, dst, pitch, dst_is_device, &s))) return st;
-      const float ms = s.trace_ms > 0.0f ? s.trace_ms : s.total_ms;  // the walk also moves work to the solve
-      if (ms < best) { best = ms; pick = o[1]; pick_walk = o[0] != 0; }
-    }
-    c->scan_walk = pick_walk;
-    if ((st = set_scan_pairs(c, pick, false))) return st;
-  }
-  return render_frame(c, dst, pitch, dst_is_device, stats);
-}
-
-static lg_status render_frame(lg_ctx* c, uint16_t* dst, size_t pitch, int32_t dst_is_device, lg_trace_stats* stats) {
-  lg_status st = LG_OK;
   const size_t row = (size_t)c->prm.width * 8;
   if (!dst || pitch < row) return fail(c, LG_ERR_INVALID_ARGUMENT, "destination null or pitch < width * 8");
   uint32_t retries = 0;

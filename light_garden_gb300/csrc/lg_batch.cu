@@ -338,9 +338,6 @@ lg_status lg_batch_upload(lg_ctx* c, const lg_scene_desc* scenes, uint32_t k) {
   if ((st = batch_buffers(c))) return st;
   // launch shapes: the multi-scene kernels read the object tables from global memory
   int occ = 0;
-  c->scan_pairs = c->scan_pairs_opt;  // a new batch: its second lg_batch_render times both scan sizes
-  c->scan_tune = c->scan_pairs_opt == 0;
-  c->renders = 0;
   if ((st = scan_grid(c, true))) return st;
   if ((st = trace_grids(c, true, 0))) return st;
   CK(raster_occupancy(raster_mode(c->prm), &occ), "occupancy");
@@ -372,22 +369,6 @@ lg_status lg_batch_render(lg_ctx* c, uint16_t* dst, uint64_t dst_bytes, int32_t 
   std::vector<cudaEvent_t>& ev = c->bev;
   uint32_t retries = 0;
   lg_status st;
-  if (c->renders < 0xffffffffu) ++c->renders;
-  if (c->scan_tune && c->renders >= 2) {
-    // autotune of the scan's pair slots per lane on the batch's second render: the whole
-    // batch with each size (identical images), keep the one whose generations trace faster
-    c->scan_tune = false;
-    float best = INFINITY;
-    int pick = scan_pairs_of(c);
-    for (int pairs : {8, 16}) {
-      if ((st = set_scan_pairs(c, pairs, true))) return st;
-      if ((st = run_batch(c, ev, retries))) return st;
-      float ms = 0.f;
-      for (uint32_t g = 0; g < c->max_bounce_all; ++g) ms += elapsed(g == 0 ? ev[0] : ev[2 * g], ev[1 + 2 * g]);
-      if (ms < best) { best = ms; pick = pairs; }
-    }
-    if ((st = set_scan_pairs(c, pick, true))) return st;
-  }
   if ((st = run_batch(c, ev, retries))) return st;
   CK(cudaMemcpyAsync(dst, c->d_stage.p, bytes, dst_is_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
                      c->stream), "copy images");

@@ -400,8 +400,6 @@ lg_status lg_serve_begin(lg_ctx* c, const lg_serve_opts* opts) {
   std::memset(c->h_ctr, 0, sizeof(Counters));
   // launch shapes of the multi-scene kernels
   int occ = 0;
-  c->scan_pairs = c->scan_pairs_opt;  // served requests keep the untuned rule (or the requested size)
-  c->scan_tune = false;
   if ((st = scan_grid(c, true))) { serve_free(c); return st; }
   if ((st = trace_grids(c, true, 0))) { serve_free(c); return st; }
   CK(raster_occupancy(RM_FIXED_SPLIT_, &occ), "occupancy");

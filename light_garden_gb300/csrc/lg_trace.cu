@@ -219,10 +219,7 @@ __device__ __forceinline__ void emit_segments(const SceneDev& S, const TraceBufs
 // either the object table in chunks of SCAN_CHUNK, or (culling grid) the objects listed
 // in the grid cells the lane's ray crosses, nearest cell first.
 // Launch shape.  The pair slots per lane between classifications (CHUNK, 8 or 16) are a
-// template parameter that each context tunes on its first frame (lg_device_opts.scan_pairs):
-// the culled walk tends to do best with 8 (a smaller shared-memory buffer leaves more of the
-// SM's L1 to the grid and queue loads), the table scan with 16 (CSG frame: 8 slots 1217 ms of
-// scan, 16 slots 1469; mid frame: 16 slots 68 ms, 8 slots 73).  CTAs per SM of the culled scan
+// template parameter (scan_pairs_of says when which).  CTAs per SM of the culled scan
 // and its cell steps between classifications are build-time (-DLG_SCAN_CULL_BLOCKS=...,
 // -DLG_SCAN_WALK_CELLS=..., for sweeps).
 #ifndef LG_SCAN_CULL_BLOCKS
@@ -1234,15 +1231,16 @@ __global__ void k_overlay(SceneDev S, TraceBufs B, const uint32_t* cubic_objs, c
 
 // ---------------------------------------------------------- nested string mods
 // StringMod::line_crossings_as_points (string_mod.rs:87-102): line k of the outer mod joins
-// point k and point ix(k) of its curve, in FP64 (lines[2k], lines[2k + 1]).
-__global__ void k_sm_lines(lg_string_mod sm, double2* lines) {
+// point k and point ix(k) of its curve, in FP64 (pts[2k], pts[2k + 1]) and rounded to FP32; a thread
+// per point.
+__global__ void k_sm_lines(lg_string_mod sm, double2* pts, float2* pts32) {
   const uint64_t m = sm.modulo;
-  for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < m; k += (uint64_t)gridDim.x * blockDim.x) {
+  for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < 2 * m; e += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t k = e >> 1;
     double x, y;
-    string_mod_point(sm, k % m, x, y);
-    lines[2 * k] = make_double2(x, y);
-    string_mod_point(sm, string_mod_target(sm, k) % m, x, y);
-    lines[2 * k + 1] = make_double2(x, y);
+    string_mod_point(sm, ((e & 1) ? string_mod_target(sm, k) : k) % m, x, y);
+    pts[e] = make_double2(x, y);
+    pts32[e] = make_float2((float)x, (float)y);
   }
 }
 
@@ -1250,7 +1248,7 @@ __global__ void k_sm_lines(lg_string_mod sm, double2* lines) {
 // is the definition include/lg.h states): the 2x2 parametric solve a + t (b - a) =
 // c + u (d - c), each FP64 operation rounded on its own, a crossing when the determinant is
 // not zero and t, u lie in [0, 1]; the point is a + t (b - a).
-__device__ __forceinline__ bool seg_cross_x(double2 a, double2 b, double2 c, double2 d, double2& p) {
+__device__ __noinline__ bool seg_cross_x(double2 a, double2 b, double2 c, double2 d, double2& p) {
   using namespace lgx;
   const double rx = sub(b.x, a.x), ry = sub(b.y, a.y), sx = sub(d.x, c.x), sy = sub(d.y, c.y);
   const double den = sub(mul(rx, sy), mul(ry, sx));
@@ -1264,50 +1262,61 @@ __device__ __forceinline__ bool seg_cross_x(double2 a, double2 b, double2 c, dou
   return true;
 }
 
+// Whether a pair crosses, in FP32 where that is certain: 1 yes, 0 no, -1 undecided.  Coordinates
+// rounded to FP32 and the products' roundings move the determinant and the numerators by at
+// most 4e-7 times the products of the sums of magnitudes (some 3 2^-24 each); with the sign of the
+// determinant taken out, t and u lie in [0, 1] where 0 <= numerator <= |determinant|.
+__device__ __forceinline__ int seg_cross32(float4 ab, float4 cd) {
+  const float rx = ab.z - ab.x, ry = ab.w - ab.y, sx = cd.z - cd.x, sy = cd.w - cd.y;
+  const float ma = fabsf(ab.x) + fabsf(ab.y) + fabsf(ab.z) + fabsf(ab.w);
+  const float mc = fabsf(cd.x) + fabsf(cd.y) + fabsf(cd.z) + fabsf(cd.w);
+  const float e = 1e-6f * (ma + mc) * (ma + mc) + 1e-30f;
+  const float den = rx * sy - ry * sx, wx = cd.x - ab.x, wy = cd.y - ab.y;
+  const float D = fabsf(den), sg = den < 0.0f ? -1.0f : 1.0f;
+  const float T = sg * (wx * sy - wy * sx), U = sg * (wx * ry - wy * rx);
+  if (!(D > e) || !(ma + mc < 1e18f)) return -1;  // (no product overflows below 1e18)
+  if (T < -e || T > D + 2.0f * e || U < -e || U > D + 2.0f * e) return 0;
+  return T > e && T < D - 2.0f * e && U > e && U < D - 2.0f * e ? 1 : -1;
+}
+
 // pair q of m (m - 1), in the reference's order: diff = q / m + 1 (outer loop), line a = q % m
-__device__ __forceinline__ bool pair_cross(const double2* lines, uint64_t m, uint64_t q, double2& p) {
-  const uint64_t diff = q / m + 1, a = q % m, b = (a + diff) % m;
-  return seg_cross_x(lines[2 * a], lines[2 * a + 1], lines[2 * b], lines[2 * b + 1], p);
+// joined with line b = (a + diff) % m
+struct CrossPair {
+  uint32_t a, b;
+};
+__device__ __forceinline__ CrossPair cross_pair(uint32_t m, uint32_t q) {
+  const uint32_t diff = q / m, a = q - diff * m, b = a + diff + 1;
+  return CrossPair{a, b >= m ? b - m : b};
 }
 
-// A thread's run of CROSS_PER_THREAD consecutive pairs: how many of them cross.
-__device__ __forceinline__ uint32_t run_crossings(const double2* lines, uint64_t m, uint64_t q0, uint64_t n_pairs) {
-  uint32_t c = 0;
-  for (int k = 0; k < CROSS_PER_THREAD; ++k) {
-    double2 p;
-    if (q0 + k < n_pairs && pair_cross(lines, m, q0 + k, p)) ++c;
+// Bound: the FP32 tests of m (m - 1) pairs.  A warp takes 32 consecutive pairs and leaves a mask of
+// those that cross; FP64 decides only pairs within the FP32 rounding.  (All in FP64, with 64-bit
+// index divisions and both quotients, 1.4 M pairs took 133 us here and 276 us again in the write.)
+__global__ void __launch_bounds__(CROSS_THREADS) k_cross_count(const double2* pts, const float4* lines32, uint32_t m,
+                                                               uint32_t* blk, uint32_t* masks) {
+  __shared__ uint32_t warp_sums[CROSS_WARPS];
+  const uint32_t n_pairs = m * (m - 1), w = threadIdx.x >> 5;
+  uint32_t count = 0;
+  for (int row = 0; row < CROSS_ROWS; ++row) {
+    const uint32_t q = blockIdx.x * CROSS_PAIRS_PER_BLOCK + row * CROSS_THREADS + threadIdx.x;
+    bool on = false;
+    if (q < n_pairs) {
+      const CrossPair P = cross_pair(m, q);
+      const int k = seg_cross32(__ldg(lines32 + P.a), __ldg(lines32 + P.b));
+      double2 p;
+      on = k > 0 || (k < 0 && seg_cross_x(pts[2 * P.a], pts[2 * P.a + 1], pts[2 * P.b], pts[2 * P.b + 1], p));
+    }
+    const uint32_t mask = __ballot_sync(0xffffffffu, on);
+    if (lane_id() == 0) masks[blockIdx.x * CROSS_MASKS + row * CROSS_WARPS + w] = mask;
+    count += __popc(mask);
   }
-  return c;
-}
-
-// exclusive sum over the CTA's threads (CROSS_THREADS of them); *total receives the sum
-__device__ __forceinline__ uint32_t cta_exclusive(uint32_t v, uint32_t* warp_sums, uint32_t* total) {
-  const unsigned lane = lane_id(), w = threadIdx.x >> 5;
-  uint32_t incl = v;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-    if ((int)lane >= o) incl += y;
-  }
-  if (lane == 31) warp_sums[w] = incl;
+  if (lane_id() == 0) warp_sums[w] = count;
   __syncthreads();
-  uint32_t before = 0, all = 0;
-  for (unsigned k = 0; k < CROSS_THREADS / 32; ++k) {
-    if (k < w) before += warp_sums[k];
-    all += warp_sums[k];
+  if (threadIdx.x == 0) {
+    uint32_t all = 0;
+    for (int k = 0; k < CROSS_WARPS; ++k) all += warp_sums[k];
+    blk[blockIdx.x] = all;
   }
-  if (total) *total = all;
-  return before + incl - v;
-}
-
-__global__ void __launch_bounds__(CROSS_THREADS) k_cross_count(const double2* lines, uint64_t m, uint32_t* blk) {
-  __shared__ uint32_t warp_sums[CROSS_THREADS / 32];
-  const uint64_t n_pairs = m * (m - 1);
-  const uint64_t q0 = blockIdx.x * CROSS_PAIRS_PER_BLOCK + (uint64_t)threadIdx.x * CROSS_PER_THREAD;
-  const uint32_t c = run_crossings(lines, m, q0, n_pairs);
-  uint32_t total = 0;
-  cta_exclusive(c, warp_sums, &total);
-  if (threadIdx.x == 0) blk[blockIdx.x] = total;
 }
 
 // one CTA of 1024 threads: exclusive scan of the per-block counts in place
@@ -1342,17 +1351,47 @@ __global__ void __launch_bounds__(1024) k_cross_scan(uint32_t* blk, uint32_t n_b
   if (threadIdx.x == 0) *total = carry;
 }
 
-// the crossing points in pair order: block offset + the thread's place in the block + its run
-__global__ void __launch_bounds__(CROSS_THREADS) k_cross_write(const double2* lines, uint64_t m,
-                                                                const uint32_t* blk_off, double2* pts) {
-  __shared__ uint32_t warp_sums[CROSS_THREADS / 32];
-  const uint64_t n_pairs = m * (m - 1);
-  const uint64_t q0 = blockIdx.x * CROSS_PAIRS_PER_BLOCK + (uint64_t)threadIdx.x * CROSS_PER_THREAD;
-  const uint32_t c = run_crossings(lines, m, q0, n_pairs);
-  uint64_t slot = (uint64_t)blk_off[blockIdx.x] + cta_exclusive(c, warp_sums, nullptr);
-  for (int k = 0; k < CROSS_PER_THREAD; ++k) {
-    double2 p;
-    if (q0 + k < n_pairs && pair_cross(lines, m, q0 + k, p)) pts[slot++] = p;
+// The crossing points in pair order: the block's offset, the masks before this one, the lane's
+// place in its mask.
+__global__ void __launch_bounds__(CROSS_THREADS) k_cross_write(const double2* pts, uint32_t m, const uint32_t* blk_off,
+                                                                const uint32_t* masks, double2* out) {
+  __shared__ uint32_t off[CROSS_MASKS + 1];
+  __shared__ uint16_t list[CROSS_PAIRS_PER_BLOCK];
+  const uint32_t w = threadIdx.x >> 5;
+  static_assert(CROSS_MASKS == 128, "four masks per lane of one warp");
+  if (threadIdx.x < 32) {  // exclusive sums of the block's 128 mask counts
+    const uint4 v = reinterpret_cast<const uint4*>(masks + blockIdx.x * CROSS_MASKS)[threadIdx.x];
+    const uint32_t c[4] = {(uint32_t)__popc(v.x), (uint32_t)__popc(v.y), (uint32_t)__popc(v.z), (uint32_t)__popc(v.w)};
+    const uint32_t own = c[0] + c[1] + c[2] + c[3];
+    uint32_t incl = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if ((int)threadIdx.x >= o) incl += y;
+    }
+    uint32_t at = incl - own;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      off[4 * threadIdx.x + k] = at;
+      at += c[k];
+    }
+    if (threadIdx.x == 31) off[CROSS_MASKS] = at;
+  }
+  __syncthreads();
+  // the block's crossing pairs side by side, so that the FP64 work fills its warps
+  for (int row = 0; row < CROSS_ROWS; ++row) {
+    const uint32_t k = row * CROSS_WARPS + w, mask = masks[blockIdx.x * CROSS_MASKS + k];
+    if ((mask >> lane_id()) & 1u) list[off[k] + __popc(mask & lanemask_lt())] = (uint16_t)(row * CROSS_THREADS + threadIdx.x);
+  }
+  __syncthreads();
+  const uint64_t base = blk_off[blockIdx.x];
+  for (uint32_t i = threadIdx.x; i < off[CROSS_MASKS]; i += CROSS_THREADS) {
+    using namespace lgx;
+    const CrossPair P = cross_pair(m, blockIdx.x * CROSS_PAIRS_PER_BLOCK + list[i]);
+    const double2 a = pts[2 * P.a], b = pts[2 * P.a + 1], c = pts[2 * P.b], d = pts[2 * P.b + 1];
+    const double rx = sub(b.x, a.x), ry = sub(b.y, a.y), sx = sub(d.x, c.x), sy = sub(d.y, c.y);
+    const double t = dvd(sub(mul(sub(c.x, a.x), sy), mul(sub(c.y, a.y), sx)), sub(mul(rx, sy), mul(ry, sx)));
+    out[base + i] = make_double2(add(a.x, mul(rx, t)), add(a.y, mul(ry, t)));
   }
 }
 
