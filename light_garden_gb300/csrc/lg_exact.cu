@@ -135,18 +135,24 @@ __device__ __forceinline__ bool solve_proved_x(const SolveRec& G, V o, V d, int 
   using namespace lgx;
   const uint32_t kind = G.kind;
   const bool two = (kind & 0xfu) == SR_TWO;
-  const V org = mk(G.org[0], G.org[1]);
+  // 16-byte loads: the record is gathered per lane, and every load is a trip of the texture pipe
+  const double2* G2 = reinterpret_cast<const double2*>(&G);
+  double2 org2 = make_double2(0.0, 0.0), rot2 = make_double2(1.0, 0.0);
   if (two) {
-    o = irot(vsub(o, org), G.rot[0], G.rot[1]);
-    d = irot(d, G.rot[0], G.rot[1]);
+    org2 = __ldg(G2);
+    rot2 = __ldg(G2 + 1);
+    o = irot(vsub(o, mk(org2.x, org2.y)), rot2.x, rot2.y);
+    d = irot(d, rot2.x, rot2.y);
   } else if (side != 0) {
     return false;
   }
-  const double* L = side ? G.b : G.a;
+  const V org = mk(org2.x, org2.y);
+  const double2* L2 = G2 + (side ? 5 : 2);
+  const double2 l0 = __ldg(L2), l1 = __ldg(L2 + 1);
   const uint32_t k = (side ? kind >> 8 : kind >> 4) & 0xfu;
   if (k == LEAF_CIRCLE) {
-    const V ctr = mk(L[0], L[1]), oc = vsub(o, ctr);
-    const double r = L[2];
+    const V ctr = mk(l0.x, l0.y), oc = vsub(o, ctr);
+    const double r = l1.x;
     const double a = dot(d, d), b = dot(oc, d), cc = sub(dot(oc, oc), mul(r, r));
     const double disc = sub(mul(b, b), mul(a, cc));
     if (is_neg(disc)) return false;
@@ -157,35 +163,38 @@ __device__ __forceinline__ bool solve_proved_x(const SolveRec& G, V o, V d, int 
     const bool first = fabsf(ra - t32) <= fabsf(rc - t32);
     t = dvd(first ? q : cc, first ? a : q);
     p = vadd(o, vscl(d, t));
-    n = vscl(vsub(p, ctr), L[3]);
+    n = vscl(vsub(p, ctr), l1.y);
   } else if (k == LEAF_RECT) {
     if (face < 0) return false;
     const int ax = face >> 1;
     const bool pos = (face & 1) != 0;
     // the face's axis of irot(o - centre) and irot(d) alone: x' = c x + s y, y' = -s x + c y
-    const double c = L[2], s = L[3];
-    const V rel = vsub(o, mk(L[0], L[1]));
+    const double2 half = __ldg(L2 + 2);
+    const double c = l1.x, s = l1.y;
+    const V rel = vsub(o, mk(l0.x, l0.y));
     const double kx = ax ? -s : c, ky = ax ? c : s;
     const double O = add(mul(kx, rel.x), mul(ky, rel.y)), D = add(mul(kx, d.x), mul(ky, d.y));
     if (is_zero(D)) return false;
-    const double h = L[4 + ax];
+    const double h = ax ? half.y : half.x;
     t = dvd(sub(pos ? h : -h, O), D);
     p = vadd(o, vscl(d, t));
     const double sg = pos ? 1.0 : -1.0;
     n = rot(ax == 0 ? mk(sg, 0.0) : mk(0.0, sg), c, s);
   } else if (k == LEAF_SEGMENT) {  // the crossing lies well inside the segment: t alone
-    const V A = mk(L[0], L[1]), e = vsub(mk(L[2], L[3]), A);
+    const double2 nl = __ldg(L2 + 2);
+    const V A = mk(l0.x, l0.y), e = vsub(mk(l1.x, l1.y), A);
     const double den = cross(d, e);
     if (is_zero(den)) return false;
     t = dvd(cross(vsub(A, o), e), den);
     p = vadd(o, vscl(d, t));
-    n = mk(L[4], L[5]);
+    n = mk(nl.x, nl.y);
   } else {  // cubic
     // the bracket between the derivative's roots that holds the proved curve parameter s32:
     // hits_cubic's operations for that bracket only (a parameter within 1e-4 of a knot takes the
     // whole object)
     if (!(s32 > 0.0f)) return false;
-    const Cubic K{mk(G.a[0], G.a[1]), mk(G.a[2], G.a[3]), mk(G.a[4], G.a[5]), mk(G.b[0], G.b[1])};
+    const double2 l2 = __ldg(L2 + 2), l3 = __ldg(L2 + 3);
+    const Cubic K{mk(l0.x, l0.y), mk(l1.x, l1.y), mk(l2.x, l2.y), mk(l3.x, l3.y)};
     const double a[4] = {cross(d, vsub(K.c0, o)), cross(d, K.c1), cross(d, K.c2), cross(d, K.c3)};
     double kn[4];
     int nk = 0;
@@ -228,8 +237,8 @@ __device__ __forceinline__ bool solve_proved_x(const SolveRec& G, V o, V d, int 
   }
   if (!gt_pos(t, T_MIN)) return false;
   if (two) {  // lifted out of the Logic frame
-    p = vadd(org, rot(p, G.rot[0], G.rot[1]));
-    n = rot(n, G.rot[0], G.rot[1]);
+    p = vadd(org, rot(p, rot2.x, rot2.y));
+    n = rot(n, rot2.x, rot2.y);
   }
   return true;
 }
@@ -303,18 +312,30 @@ __global__ void __launch_bounds__(256, LG_SOLVE_X_BLOCKS) k_solve_x(SceneDev S, 
     int l = 0;
     while (i >= off[l + 1]) ++l;
     const uint32_t idx = B.list[l][i - off[l]];
-    const RayRec& r = q[idx];
-    const ScanRec& sc = B.scan[idx];
-    const uint32_t base = MULTI ? S.scenes[r.scene].obj_base : 0u, j = sc.cand[0];
-    const V o = ray_o(r), d = ray_d(r);
+    const double2* rp = reinterpret_cast<const double2*>(q + idx);  // ox, oy, dx, dy
+    const double2 o2 = __ldcg(rp), d2 = __ldcg(rp + 1);
+    const ScanRec* sp = B.scan + idx;
+    const uint32_t j = sp->cand[0];
+    const uint4 tail = __ldcg(reinterpret_cast<const uint4*>(sp) + 1);  // nc, overflow, leaf, face | t32 | thr | s32
+    const int side = (int8_t)(tail.x >> 16), face = (int8_t)(tail.x >> 24);
+    const uint32_t base = MULTI ? S.scenes[q[idx].scene].obj_base : 0u;
+    const V o = lgx::mk(o2.x, o2.y), d = lgx::mk(d2.x, d2.y);
     const SolveRec& G = S.solve[base + j];
-    lgx::Hit h;
-    V n;
+    double t;
+    V p, n;
     ++my_solves;
-    if ((G.kind & 0xfu) != SR_TREE && solve_proved_x(G, o, d, sc.leaf, sc.face, sc.t32, sc.s32, h.t, h.p, n))
-      store_hit_x(B.hit[idx], (int)j, h, n, sc.leaf, INFINITY, 0);
-    else
+    if ((G.kind & 0xfu) != SR_TREE &&
+        solve_proved_x(G, o, d, side, face, __uint_as_float(tail.y), __uint_as_float(tail.w), t, p, n)) {
+      double2* hp = reinterpret_cast<double2*>(B.hit + idx);  // HitRec in four 16-byte stores
+      hp[0] = make_double2(t, p.x);
+      hp[1] = make_double2(p.y, n.x);
+      const uint2 ny = make_uint2((uint32_t)__double2loint(n.y), (uint32_t)__double2hiint(n.y));
+      const df ev = xdf(INFINITY);
+      reinterpret_cast<uint4*>(hp)[2] = make_uint4(ny.x, ny.y, __float_as_uint(ev.hi), __float_as_uint(ev.lo));
+      reinterpret_cast<uint4*>(hp)[3] = make_uint4(j | ((uint32_t)side << 16), 0u, 0u, 0u);
+    } else {
       solve_one_x(S, base, j, o, d, B.hit[idx]);
+    }
   }
   // block-uniform loop (the class barrier needs every thread), from the last CTA on: in a small
   // generation the first CTAs have the proved rays
