@@ -18,7 +18,7 @@
 #define LG_SOLVE_X_BLOCKS 4
 #endif
 #ifndef LG_BOUNCE_X_BLOCKS
-#define LG_BOUNCE_X_BLOCKS 4
+#define LG_BOUNCE_X_BLOCKS 3
 #endif
 
 namespace lgd {
@@ -389,14 +389,27 @@ template __global__ void k_solve_x<false>(SceneDev, TraceBufs, uint32_t);
 template __global__ void k_solve_x<true>(SceneDev, TraceBufs, uint32_t);
 
 // ------------------------------------------------------------------ bounce
+// What a ray visit leaves: its segment, and up to two rays that start at (ox, oy): the reflected
+// (or mirrored) one with direction d0 and colour scaled by f0, and the refracted one.
 struct BounceX {
-  bool emit;
+  bool emit, child0, child1;
   float x0, y0, x1, y1;
   int hit;
-  uint8_t flags;
-  int nchild;
-  RayRec child[2];
+  uint8_t flags, cflags, leaf;  // of the segment, of the children; leaf the children start on
+  uint16_t medium1;             // of the refracted ray
+  float f0, f1;
+  V o, d0, d1;
 };
+
+// the bits of two FP64 coordinates, as the queue holds them
+__device__ __forceinline__ uint4 bits2(V a) {
+  return make_uint4((uint32_t)__double2loint(a.x), (uint32_t)__double2hiint(a.x), (uint32_t)__double2loint(a.y),
+                    (uint32_t)__double2hiint(a.y));
+}
+__device__ __forceinline__ ChildRay child_x(const RayRec& r, const BounceX& v, V d, float f, uint64_t path, uint16_t medium) {
+  return ChildRay{{bits2(v.o), bits2(d)}, {__fmul_rn(r.c[0], f), __fmul_rn(r.c[1], f), __fmul_rn(r.c[2], f)},
+                  0.0f, 0.0f, path, v.cflags, v.leaf, medium, (uint16_t)v.hit};
+}
 
 // A non-negative double as double-float (relative error 2^-48; below 2^-60 an absolute error
 // below 2^-83), on the integer pipe: a conversion each way would issue on the FP64 pipe.
@@ -504,8 +517,7 @@ template <bool MULTI, bool CULL>
 __device__ __forceinline__ void bounce_x(const SceneDev& S, const RayRec& r, const ScanRec& sc, const HitRec* hrec,
                                          BounceX& v) {
   using namespace lgx;
-  v.emit = false;
-  v.nchild = 0;
+  v.emit = v.child0 = v.child1 = false;
   const SceneLoc sl = scene_of<MULTI>(S, r.scene);
   uint32_t fl = r.flags;
   if (near_cutoff(r.c, sl.cutoff)) fl |= NEAR;  // tracer.rs:378-384 in the band
@@ -593,49 +605,23 @@ __device__ __forceinline__ void bounce_x(const SceneDev& S, const RayRec& r, con
       for (int i = 0; i < 3; ++i) dead = dead && r.c[i] >= 0.0f && __fmul_rn(r.c[i], 1.4901161e-08f) < sl.cutoff[i];
       const bool refr = refract_x(d, bn, n1, n2, n1f, n2f, eta, dead, rl, rr, refl, fl);
       v.flags = (uint8_t)((fl & 0xffu) | (refr ? 0u : (uint32_t)LG_PATH_TIR));
-      const float om = __fsub_rn(1.0f, refl);
-      RayRec& a = v.child[0];
-      a.ox = xdf(bp.x); a.oy = xdf(bp.y); a.dx = xdf(rl.x); a.dy = xdf(rl.y);
-      a.medium = r.medium;
-      a.src_obj = (uint16_t)best;
-      a.src_leaf = leaf;
-      a.c[0] = __fmul_rn(r.c[0], refl); a.c[1] = __fmul_rn(r.c[1], refl); a.c[2] = __fmul_rn(r.c[2], refl);
-      a.c[3] = r.c[3];
-      a.path = r.path;
-      a.flags = (uint8_t)fl;
-      a.ex = 0.0f;
-      a.ea = 0.0f;
-      v.nchild = 1;
-      if (refr) {
-        RayRec& t = v.child[1];
-        t.ox = xdf(bp.x); t.oy = xdf(bp.y); t.dx = xdf(rr.x); t.dy = xdf(rr.y);
-        t.medium = m2;
-        t.src_obj = (uint16_t)best;
-        t.src_leaf = leaf;
-        t.c[0] = __fmul_rn(r.c[0], om); t.c[1] = __fmul_rn(r.c[1], om); t.c[2] = __fmul_rn(r.c[2], om);
-        t.c[3] = r.c[3];
-        t.path = r.path | (1ull << r.gen);
-        t.flags = (uint8_t)fl;
-        t.ex = 0.0f;
-        t.ea = 0.0f;
-        v.nchild = 2;
-      }
-    } else {  // Ray::reflect (tracer.rs:476-480)
+      v.f0 = refl;
+      v.f1 = __fsub_rn(1.0f, refl);
+      v.d0 = rl;
+      v.d1 = rr;
+      v.medium1 = m2;
+      v.child0 = true;
+      v.child1 = refr;
+    } else {  // Ray::reflect (tracer.rs:476-480): the colour as it is
       v.flags = (uint8_t)fl;
       const double dn = dot(d, bn);
-      const V rd = vsub(d, vscl(bn, mul(2.0, dn)));
-      RayRec& a = v.child[0];
-      a.ox = xdf(bp.x); a.oy = xdf(bp.y); a.dx = xdf(rd.x); a.dy = xdf(rd.y);
-      a.medium = r.medium;
-      a.src_obj = (uint16_t)best;
-      a.src_leaf = leaf;
-      a.c[0] = r.c[0]; a.c[1] = r.c[1]; a.c[2] = r.c[2]; a.c[3] = r.c[3];
-      a.path = r.path;
-      a.flags = (uint8_t)fl;
-      a.ex = 0.0f;
-      a.ea = 0.0f;
-      v.nchild = 1;
+      v.d0 = vsub(d, vscl(bn, mul(2.0, dn)));
+      v.f0 = 1.0f;
+      v.child0 = true;
     }
+    v.o = bp;
+    v.leaf = leaf;
+    v.cflags = (uint8_t)fl;
   } else {
     // canvas exit (tracer.rs:482-488): nearest hit with the canvas rectangle
     const double aspect = MULTI ? S.scenes[r.scene].aspect64 : S.aspect64;
@@ -663,32 +649,16 @@ __device__ __forceinline__ void bounce_x(const SceneDev& S, const RayRec& r, con
     }
   }
   // children: the next generation skips colours below the cutoff (tracer.rs:378-384)
-  int w = 0;
-  for (int q = 0; q < v.nchild; ++q) {
-    RayRec c = v.child[q];
-    if ((uint32_t)r.gen + 1 >= sl.max_bounce || below_cutoff(c.c, sl.cutoff)) continue;
-    c.gen = (uint8_t)(r.gen + 1);
-    c.prim = r.prim;
-    c.light = r.light;
-    c._pad = 0;
-    c.scene = r.scene;
-    v.child[w++] = c;
-  }
-  v.nchild = w;
+  const bool deeper = (uint32_t)r.gen + 1 < sl.max_bounce;
+  const float k0[4] = {__fmul_rn(r.c[0], v.f0), __fmul_rn(r.c[1], v.f0), __fmul_rn(r.c[2], v.f0), r.c[3]};
+  const float k1[4] = {__fmul_rn(r.c[0], v.f1), __fmul_rn(r.c[1], v.f1), __fmul_rn(r.c[2], v.f1), r.c[3]};
+  v.child0 = v.child0 && deeper && !below_cutoff(k0, sl.cutoff);
+  v.child1 = v.child1 && deeper && !below_cutoff(k1, sl.cutoff);
 }
 
-// appends one segment per emitting lane with one atomic per warp (all lanes call)
-__device__ __forceinline__ void emit_segments_x(const SceneDev& S, const TraceBufs& B, const BounceX& v,
-                                                const RayRec& r, uint32_t& my_near) {
-  const unsigned lane = lane_id();
-  const unsigned emask = __ballot_sync(0xffffffffu, v.emit);
-  if (!emask) return;
-  unsigned long long sbase = 0;
-  const int leader = __ffs(emask) - 1;
-  if ((int)lane == leader) sbase = atomicAdd(&B.ctr->seg_count, (unsigned long long)__popc(emask));
-  sbase = __shfl_sync(0xffffffffu, sbase, leader);
-  if (!v.emit) return;
-  const unsigned long long slot = sbase + __popc(emask & lanemask_lt());
+// the segment of an emitting lane at its place in the ring
+__device__ __forceinline__ void store_segment_x(const SceneDev& S, const TraceBufs& B, const BounceX& v, const RayRec& r,
+                                                unsigned long long slot, uint32_t& my_near) {
   if (v.flags & LG_PATH_NEAR_DEGENERATE) ++my_near;
   if (slot >= B.seg_cap) return;
   float4* dst = reinterpret_cast<float4*>(B.segs + slot);
@@ -724,10 +694,10 @@ __global__ void __launch_bounds__(256, LG_BOUNCE_X_BLOCKS) k_bounce_x(SceneDev S
   for (uint64_t base = warp * 32; base < total; base += nwarps * 32) {
     const uint64_t i = base + lane;
     BounceX v;
-    v.emit = false;
-    v.nchild = 0;
+    v.emit = v.child0 = v.child1 = false;
     v.flags = 0;
     v.hit = -1;
+    v.f0 = v.f1 = 1.0f;
     RayRec r;
     if (i < total) {
       int l = 0;
@@ -738,23 +708,12 @@ __global__ void __launch_bounds__(256, LG_BOUNCE_X_BLOCKS) k_bounce_x(SceneDev S
       ++my_visits;
       bounce_x<MULTI, CULL>(S, r, sc, &B.hit[idx], v);
     }
-    emit_segments_x(S, B, v, r, my_near);
-    // children: warp prefix sum of 0..2 per lane, one atomic per warp
-    int incl = v.nchild;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if ((int)lane >= o) incl += y;
-    }
-    const int tot = __shfl_sync(0xffffffffu, incl, 31);
-    if (tot > 0 && (MULTI || gen + 1 < S.max_bounce)) {
-      unsigned long long qbase = 0;
-      if (lane == 31) qbase = atomicAdd(&B.ctr->queue_count[gen + 1], (unsigned long long)tot);
-      qbase = __shfl_sync(0xffffffffu, qbase, 31);
-      const unsigned long long first = qbase + (unsigned long long)(incl - v.nchild);
-      for (int q = 0; q < v.nchild; ++q)
-        if (first + q < B.queue_cap) qout[first + q] = v.child[q];
-    }
+    unsigned long long seg, s0, s1;
+    reserve_out(B, gen, v.emit, v.child0, v.child1, seg, s0, s1);
+    if (v.emit) store_segment_x(S, B, v, r, seg, my_near);
+    if (v.child0 && s0 < B.queue_cap) store_child(qout + s0, r, child_x(r, v, v.d0, v.f0, r.path, r.medium));
+    if (v.child1 && s1 < B.queue_cap)
+      store_child(qout + s1, r, child_x(r, v, v.d1, v.f1, r.path | (1ull << r.gen), v.medium1));
   }
   stamp_end(B.ctr, gen);
   add_block_counts<2>({my_visits, my_near}, {&B.ctr->visits, &B.ctr->near});

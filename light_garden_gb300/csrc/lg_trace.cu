@@ -181,19 +181,10 @@ __device__ __forceinline__ bool fast_canvas_exit(const df aspect, const RayRec& 
   return true;
 }
 
-// appends one segment per emitting lane with one atomic per warp (all lanes call)
-__device__ __forceinline__ void emit_segments(const SceneDev& S, const TraceBufs& B, bool emit, const RayRec& r,
-                                              float x1, float y1, uint8_t flags, int hit,
-                                              uint32_t& my_near, uint32_t& my_ill) {
-  const unsigned lane = lane_id();
-  const unsigned emask = __ballot_sync(0xffffffffu, emit);
-  if (!emask) return;
-  unsigned long long sbase = 0;
-  const int leader = __ffs(emask) - 1;
-  if ((int)lane == leader) sbase = atomicAdd(&B.ctr->seg_count, (unsigned long long)__popc(emask));
-  sbase = __shfl_sync(0xffffffffu, sbase, leader);
-  if (!emit) return;
-  const unsigned long long slot = sbase + __popc(emask & lanemask_lt());
+// the segment of an emitting lane at its place in the ring
+__device__ __forceinline__ void store_segment(const SceneDev& S, const TraceBufs& B, const RayRec& r, float x1, float y1,
+                                              uint8_t flags, int hit, unsigned long long slot, uint32_t& my_near,
+                                              uint32_t& my_ill) {
   if (flags & LG_PATH_NEAR_DEGENERATE) ++my_near;
   if (flags & LG_PATH_ILL_CONDITIONED) ++my_ill;
   if (slot >= B.seg_cap) return;
@@ -207,6 +198,19 @@ __device__ __forceinline__ void emit_segments(const SceneDev& S, const TraceBufs
     pr.flags = flags; pr.hit = hit; pr.source = LG_SRC_TRACE;
     B.paths[slot] = pr;
   }
+}
+
+// appends one segment per emitting lane with one atomic per warp (all lanes call)
+__device__ __forceinline__ void emit_segments(const SceneDev& S, const TraceBufs& B, bool emit, const RayRec& r,
+                                              float x1, float y1, uint8_t flags, int hit,
+                                              uint32_t& my_near, uint32_t& my_ill) {
+  const unsigned emask = __ballot_sync(0xffffffffu, emit);
+  if (!emask) return;
+  unsigned long long sbase = 0;
+  const int leader = __ffs(emask) - 1;
+  if ((int)lane_id() == leader) sbase = atomicAdd(&B.ctr->seg_count, (unsigned long long)__popc(emask));
+  sbase = __shfl_sync(0xffffffffu, sbase, leader);
+  if (emit) store_segment(S, B, r, x1, y1, flags, hit, sbase + __popc(emask & lanemask_lt()), my_near, my_ill);
 }
 
 // Warp-cooperative FP32 scan.  Every lane bounding-tests its own ray against a run of
@@ -763,20 +767,22 @@ __global__ void __launch_bounds__(256, 2) k_full(SceneDev S, TraceBufs B, uint32
 template __global__ void k_full<false>(SceneDev, TraceBufs, uint32_t, int);
 template __global__ void k_full<true>(SceneDev, TraceBufs, uint32_t, int);
 
+// What a ray visit leaves: its segment, and up to two rays that start at (ox, oy): the reflected
+// (or mirrored) one with direction d0 and colour scaled by f0, and the refracted one.
 struct Bounce {
-  bool emit;
+  bool emit, child0, child1;
   float x1, y1;
   int hit;
-  uint8_t flags;
-  int nchild;
-  RayRec child[2];
+  uint8_t flags, cflags, leaf;  // of the segment, of the children; leaf the children start on
+  uint16_t medium1;             // of the refracted ray
+  float f0, f1, ex0, ea0, ex1, ea1;
+  df ox, oy, dx0, dy0, dx1, dy1;
 };
 
 template <bool MULTI, bool CULL>
 __device__ __forceinline__ void bounce(const SceneDev& S, const ObjScan* objs, const RayRec& r, const ScanRec& sc,
                                        const HitRec* hrec, Bounce& v) {
-  v.emit = false;
-  v.nchild = 0;
+  v.emit = v.child0 = v.child1 = false;
   const SceneLoc sl = scene_of<MULTI>(S, r.scene);
   uint8_t fl = r.flags;
   if (near_cutoff(r.c, sl.cutoff)) fl |= LG_PATH_NEAR_DEGENERATE;
@@ -872,51 +878,33 @@ __device__ __forceinline__ void bounce(const SceneDev& S, const ObjScan* objs, c
         }
       }
       v.flags = fl | (refr ? 0 : LG_PATH_TIR);
-      const float refl = R;
-      const float om = 1.0f - refl;
-      RayRec& a = v.child[0];
+      v.f0 = R;
+      v.f1 = 1.0f - R;
       const df ci2 = ci * 2.0f;
-      a.ox = bh.px; a.oy = bh.py; a.dx = dx + ci2 * nx; a.dy = dy + ci2 * ny;
-      a.medium = r.medium;
-      a.src_obj = (uint16_t)best;
-      a.src_leaf = bh.leaf;
-      a.c[0] = __fmul_rn(r.c[0], refl); a.c[1] = __fmul_rn(r.c[1], refl); a.c[2] = __fmul_rn(r.c[2], refl);
-      a.c[3] = r.c[3];
-      a.path = r.path;
-      a.flags = fl;
-      a.ex = L;
-      a.ea = r.ea + 2.0f * kap * ds;
-      v.nchild = 1;
-      if (refr) {
-        RayRec& t = v.child[1];
-        t.ox = bh.px; t.oy = bh.py; t.dx = tx; t.dy = ty;
-        t.medium = m2;
-        t.src_obj = (uint16_t)best;
-        t.src_leaf = bh.leaf;
-        t.c[0] = __fmul_rn(r.c[0], om); t.c[1] = __fmul_rn(r.c[1], om); t.c[2] = __fmul_rn(r.c[2], om);
-        t.c[3] = r.c[3];
-        t.path = r.path | (1ull << r.gen);
-        t.flags = fl;
-        const float gain = eta.hi * ci.hi / fmaxf(ct.hi, 1e-6f);
-        t.ex = ds * ct.hi + L;
-        t.ea = gain * (r.ea + kap * ds) + kap * ds;
-        v.nchild = 2;
-      }
+      v.dx0 = dx + ci2 * nx;
+      v.dy0 = dy + ci2 * ny;
+      v.dx1 = tx;
+      v.dy1 = ty;
+      v.medium1 = m2;
+      const float gain = eta.hi * ci.hi / fmaxf(ct.hi, 1e-6f);
+      v.ex1 = ds * ct.hi + L;
+      v.ea1 = gain * (r.ea + kap * ds) + kap * ds;
+      v.child0 = true;
+      v.child1 = refr;
     } else {
       v.flags = fl;
-      const df dn2 = ddn * 2.0f;  // Ray::reflect
-      RayRec& a = v.child[0];
-      a.ox = bh.px; a.oy = bh.py; a.dx = dx - dn2 * bh.nx; a.dy = dy - dn2 * bh.ny;
-      a.medium = r.medium;
-      a.src_obj = (uint16_t)best;
-      a.src_leaf = bh.leaf;
-      a.c[0] = r.c[0]; a.c[1] = r.c[1]; a.c[2] = r.c[2]; a.c[3] = r.c[3];
-      a.path = r.path;
-      a.flags = fl;
-      a.ex = L;
-      a.ea = r.ea + 2.0f * kap * ds;
-      v.nchild = 1;
+      const df dn2 = ddn * 2.0f;  // Ray::reflect: the colour as it is
+      v.dx0 = dx - dn2 * bh.nx;
+      v.dy0 = dy - dn2 * bh.ny;
+      v.f0 = 1.0f;
+      v.child0 = true;
     }
+    v.ox = bh.px;
+    v.oy = bh.py;
+    v.ex0 = L;
+    v.ea0 = r.ea + 2.0f * kap * ds;
+    v.leaf = bh.leaf;
+    v.cflags = fl;
   } else {
     // canvas exit: nearest hit with the canvas rectangle (tracer.rs:482-488)
     Leaf64 canvas;
@@ -938,20 +926,24 @@ __device__ __forceinline__ void bounce(const SceneDev& S, const ObjScan* objs, c
     }
   }
   // children: the next generation skips colours below the cutoff (tracer.rs:378-384)
-  int w = 0;
-  for (int q = 0; q < v.nchild; ++q) {
-    RayRec c = v.child[q];
-    if ((uint32_t)r.gen + 1 >= sl.max_bounce || below_cutoff(c.c, sl.cutoff)) continue;
-    c.gen = (uint8_t)(r.gen + 1);
-    c.prim = r.prim;
-    c.light = r.light;
-    c._pad = 0;
-    c.scene = r.scene;
-    if (near_cutoff(c.c, sl.cutoff)) c.flags |= LG_PATH_NEAR_DEGENERATE;
-    if (!(c.ex <= ILL_COND && c.ea <= ILL_COND)) c.flags |= LG_PATH_ILL_CONDITIONED;
-    v.child[w++] = c;
-  }
-  v.nchild = w;
+  const bool deeper = (uint32_t)r.gen + 1 < sl.max_bounce;
+  const float k0[4] = {__fmul_rn(r.c[0], v.f0), __fmul_rn(r.c[1], v.f0), __fmul_rn(r.c[2], v.f0), r.c[3]};
+  const float k1[4] = {__fmul_rn(r.c[0], v.f1), __fmul_rn(r.c[1], v.f1), __fmul_rn(r.c[2], v.f1), r.c[3]};
+  v.child0 = v.child0 && deeper && !below_cutoff(k0, sl.cutoff);
+  v.child1 = v.child1 && deeper && !below_cutoff(k1, sl.cutoff);
+}
+
+__device__ __forceinline__ uint4 bits2(df a, df b) {
+  return make_uint4(__float_as_uint(a.hi), __float_as_uint(a.lo), __float_as_uint(b.hi), __float_as_uint(b.lo));
+}
+__device__ __forceinline__ ChildRay child_df(const RayRec& r, const Bounce& v, df dx, df dy, float f, float ex, float ea,
+                                             const float* cutoff, uint64_t path, uint16_t medium) {
+  ChildRay c{{bits2(v.ox, v.oy), bits2(dx, dy)}, {__fmul_rn(r.c[0], f), __fmul_rn(r.c[1], f), __fmul_rn(r.c[2], f)},
+             ex, ea, path, v.cflags, v.leaf, medium, (uint16_t)v.hit};
+  const float k[4] = {c.c[0], c.c[1], c.c[2], r.c[3]};
+  if (near_cutoff(k, cutoff)) c.flags |= LG_PATH_NEAR_DEGENERATE;
+  if (!(ex <= ILL_COND && ea <= ILL_COND)) c.flags |= LG_PATH_ILL_CONDITIONED;
+  return c;
 }
 
 template <bool MULTI, bool CULL>
@@ -981,10 +973,10 @@ __global__ void __launch_bounds__(256, 3) k_bounce(SceneDev S, TraceBufs B, uint
   for (uint64_t base = warp * 32; base < total; base += nwarps * 32) {
     const uint64_t i = base + lane;
     Bounce v;
-    v.emit = false;
-    v.nchild = 0;
+    v.emit = v.child0 = v.child1 = false;
     v.flags = 0;
     v.hit = -1;
+    v.f0 = v.f1 = 1.0f;
     RayRec r;
     if (i < total) {
       int l = 0;
@@ -997,22 +989,15 @@ __global__ void __launch_bounds__(256, 3) k_bounce(SceneDev S, TraceBufs B, uint
         bounce<MULTI, CULL>(S, objs, r, sc, &B.hit[idx], v);
       }
     }
-    emit_segments(S, B, v.emit, r, v.x1, v.y1, v.flags, v.hit, my_near, my_ill);
-    // children: warp prefix sum of 0..2 per lane, one atomic per warp
-    int incl = v.nchild;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if ((int)lane >= o) incl += y;
-    }
-    const int tot = __shfl_sync(0xffffffffu, incl, 31);
-    if (tot > 0 && (MULTI || gen + 1 < S.max_bounce)) {  // multi-scene: bounce() checks each ray's scene
-      unsigned long long qbase = 0;
-      if (lane == 31) qbase = atomicAdd(&B.ctr->queue_count[gen + 1], (unsigned long long)tot);
-      qbase = __shfl_sync(0xffffffffu, qbase, 31);
-      const unsigned long long first = qbase + (unsigned long long)(incl - v.nchild);
-      for (int q = 0; q < v.nchild; ++q)
-        if (first + q < B.queue_cap) qout[first + q] = v.child[q];
+    unsigned long long seg, s0, s1;
+    reserve_out(B, gen, v.emit, v.child0, v.child1, seg, s0, s1);
+    if (v.emit) store_segment(S, B, r, v.x1, v.y1, v.flags, v.hit, seg, my_near, my_ill);
+    if (v.child0 || v.child1) {
+      const SceneLoc sl = scene_of<MULTI>(S, r.scene);
+      if (v.child0 && s0 < B.queue_cap)
+        store_child(qout + s0, r, child_df(r, v, v.dx0, v.dy0, v.f0, v.ex0, v.ea0, sl.cutoff, r.path, r.medium));
+      if (v.child1 && s1 < B.queue_cap)
+        store_child(qout + s1, r, child_df(r, v, v.dx1, v.dy1, v.f1, v.ex1, v.ea1, sl.cutoff, r.path | (1ull << r.gen), v.medium1));
     }
   }
   stamp_end(B.ctr, gen);
