@@ -35,30 +35,9 @@ __device__ __forceinline__ bool obj_contains_x(const SceneDev& S, uint32_t k, V 
   return lgx::object_contains_tree(S.xgeo, S.xnode + oi.xnode_begin, (int)oi.xnode_count, p, fl);
 }
 
-// Membership of object k at p decided in FP32 where the FP32 copy of its leaves decides it:
-// 1 inside, 0 outside, -1 undecided.  The band of leaf_member32 covers the rounding of p and
-// of the leaf parameters to FP32 (1e-6 of the coordinates against 6e-8), so a decided answer
-// is the one the FP64 tree gives; objects the scan only bounds stay undecided.
-__device__ __forceinline__ int obj_member32(const ObjScan& s, float px, float py) {
-  if (s.info & INFO_NO_CONTAINS) return 0;
-  const uint32_t sk = info_scan(s.info);
-  if (sk == SCAN_ONE) {
-    const uint32_t ka = info_leaf_a(s.info);
-    return ka == LEAF_CUBIC ? -1 : leaf_member32(ka, s.a, px, py, 1e-6f);
-  }
-  if (sk != SCAN_TWO) return -1;
-  const int a = leaf_member32(info_leaf_a(s.info), s.a, px, py, 1e-6f);
-  const int b = leaf_member32(info_leaf_b(s.info), s.b, px, py, 1e-6f);
-  switch (info_op(s.info)) {
-    case LG_OP_AND: return (a == 0 || b == 0) ? 0 : (a == 1 && b == 1 ? 1 : -1);
-    case LG_OP_OR: return (a == 1 || b == 1) ? 1 : (a == 0 && b == 0 ? 0 : -1);
-    default: return (a == 0 || b == 1) ? 0 : (a == 1 && b == 0 ? 1 : -1);  // a and not b
-  }
-}
-
 // obj_contains_x behind the FP32 pre-test (k scene-global).
 __device__ __forceinline__ bool obj_contains_f(const SceneDev& S, uint32_t k, V p, uint32_t* fl) {
-  const int m = obj_member32(S.scan[k], (float)p.x, (float)p.y);
+  const int m = obj_member32(S.scan[k], (float)p.x, (float)p.y, 1e-6f);
   if (m >= 0) return m == 1;
   return obj_contains_x(S, k, p, fl);
 }

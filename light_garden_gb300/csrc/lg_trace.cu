@@ -819,7 +819,13 @@ __device__ __forceinline__ void bounce(const SceneDev& S, const ObjScan* objs, c
       df n2 = DF_ONE;
       uint16_t m2 = MEDIUM_AIR;
       bool near = false;
-      if (obj_contains64(S, sl.base + (uint32_t)best, DF_HALF * (ox + bh.px), DF_HALF * (oy + bh.py), near, L)) {
+      // membership behind an FP32 pre-test whose band covers the ray's error bound: a decided point
+      // lies outside the precise test's near-degenerate band too
+      auto inside = [&](uint32_t k, df x, df y) -> bool {
+        const int m = obj_member32(MULTI ? S.scan[k] : objs[k], x.hi, y.hi, 1e-6f + L);
+        return m >= 0 ? m == 1 : obj_contains64(S, k, x, y, near, L);
+      };
+      if (inside(sl.base + (uint32_t)best, DF_HALF * (ox + bh.px), DF_HALF * (oy + bh.py))) {
         const float px32 = bh.px.hi, py32 = bh.py.hi;
         // the first other material object, in table order, that contains the hit point
         auto far_side = [&](uint32_t k) -> bool {
@@ -829,7 +835,7 @@ __device__ __forceinline__ void bounce(const SceneDev& S, const ObjScan* objs, c
           const float ex = px32 - h.x, ey = py32 - h.y;
           const float tol = 2e-6f * (fabsf(px32) + fabsf(py32) + fabsf(h.x) + fabsf(h.y) + h.z) + 1e-6f;
           if (ex * ex + ey * ey > (h.z + tol) * (h.z + tol)) return false;
-          if (!obj_contains64(S, sl.base + k, bh.px, bh.py, near, L)) return false;
+          if (!inside(sl.base + k, bh.px, bh.py)) return false;
           n2 = S.info[sl.base + k].n;
           m2 = (uint16_t)k;
           return true;

@@ -41,6 +41,28 @@ __device__ __forceinline__ uint32_t last_object_of_warp(uint32_t base, uint32_t 
   return 0xffffffffu;
 }
 
+// Membership of an object at a point known to within delta, decided in FP32 where the FP32 copy
+// of its leaves decides it: 1 inside, 0 outside, -1 undecided.  The band of leaf_member32 covers
+// delta and the rounding of the point and the leaf parameters to FP32 (1e-6 of the coordinates against
+// 6e-8), so a decided answer is the one the precise test gives, outside that test's own band;
+// objects the scan only bounds stay undecided.
+__device__ __forceinline__ int obj_member32(const ObjScan& s, float px, float py, float delta) {
+  if (s.info & INFO_NO_CONTAINS) return 0;
+  const uint32_t sk = info_scan(s.info);
+  if (sk == SCAN_ONE) {
+    const uint32_t ka = info_leaf_a(s.info);
+    return ka == LEAF_CUBIC ? -1 : leaf_member32(ka, s.a, px, py, delta);
+  }
+  if (sk != SCAN_TWO) return -1;
+  const int a = leaf_member32(info_leaf_a(s.info), s.a, px, py, delta);
+  const int b = leaf_member32(info_leaf_b(s.info), s.b, px, py, delta);
+  switch (info_op(s.info)) {
+    case LG_OP_AND: return (a == 0 || b == 0) ? 0 : (a == 1 && b == 1 ? 1 : -1);
+    case LG_OP_OR: return (a == 1 || b == 1) ? 1 : (a == 0 && b == 0 ? 0 : -1);
+    default: return (a == 0 || b == 1) ? 0 : (a == 1 && b == 0 ? 1 : -1);  // a and not b
+  }
+}
+
 // Queued rays a launch takes (the children of the previous generation or step) ...
 __device__ __forceinline__ uint64_t n_real_of(const SceneDev& S, const TraceBufs& B, uint32_t gen) {
   if (gen == 0 && !S.serve) return 0;
