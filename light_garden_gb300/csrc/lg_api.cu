@@ -64,6 +64,15 @@ lg_status flatten_node(std::string& err, const lg_geo* G, uint32_t n_geo, int32_
     double area = 0.0;
     for (int k = 0; k < n; ++k) area += vx[k] * vy[(k + 1) % n] - vy[k] * vx[(k + 1) % n];
     if (area == 0.0) return set_err(err, LG_ERR_INVALID_ARGUMENT, "degenerate polygon");
+    // the exact mode's orientation, a sum of cross products in vertex order with every operation
+    // rounded once, kept in the node's unused op
+    volatile double turn = 0.0;
+    for (int k = 0; k < n; ++k) {
+      const int j = (k + 1) % n;
+      volatile double xy = vx[k] * vy[j], yx = vy[k] * vx[j], cr = xy - yx;
+      turn = turn + cr;
+    }
+    F.xgeo[gi].op = turn >= 0.0 ? 1 : -1;
     const double sg = area > 0.0 ? 1.0 : -1.0;
     Xf T2;
     T.apply(g.origin[0], g.origin[1], T2.ox, T2.oy);

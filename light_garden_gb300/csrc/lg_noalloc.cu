@@ -16,6 +16,7 @@
 // time) race on it and must be serialised by the caller.  The first call on a device looks
 // the array's device address up (cudaGetSymbolAddress) and configures the kernels; make
 // that first call before any stream capture.
+#include <cstddef>
 #include <cstring>
 #include <mutex>
 
@@ -166,14 +167,15 @@ extern "C" lg_status lg_accumulate_segments_noalloc(const lg_segment* segments, 
   k_bin_scatter<<<scatter_grid(d->n_sm, smem_tiles), SCATTER_THREADS, bsm, s>>>(A, smem_tiles);
   launch_raster(mode, d->raster_grid[mode], s, A);
   if (cudaGetLastError() != cudaSuccess) return LG_ERR_CUDA;
-  unsigned long long counts[2] = {0, 0};
-  if (cudaMemcpyAsync(&counts[0], &A.ctr->tile_refs, 8, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-      cudaMemcpyAsync(&counts[1], &A.ctr->pixels, 8, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+  // pixels, bin_refs and tile_refs lie side by side
+  static_assert(offsetof(Counters, tile_refs) == offsetof(Counters, pixels) + 16, "one copy reads the three counts");
+  unsigned long long counts[3] = {0, 0, 0};
+  if (cudaMemcpyAsync(counts, &A.ctr->pixels, sizeof counts, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
       cudaStreamSynchronize(s) != cudaSuccess) {
     (void)cudaGetLastError();
     return LG_ERR_CUDA;
   }
-  if (counts[0] > NOALLOC_MAX_REFS) return LG_ERR_BUDGET;  // the image is incomplete
-  if (pixels_out) *pixels_out = counts[1];
+  if (counts[2] > NOALLOC_MAX_REFS) return LG_ERR_BUDGET;  // the image is incomplete
+  if (pixels_out) *pixels_out = counts[0];
   return LG_OK;
 }

@@ -572,17 +572,19 @@ __device__ __forceinline__ void f32_minmax(float* p, float v, bool mn) {
 // A batch of 32 segments is drawn segment by segment, a lane per column of the tile, when its
 // segments cover at least this many columns each on average; else its (segment, column) pairs
 // are spread densely over the lanes.  Drawing by segments reads its parameters from shared
-// memory once per warp (a broadcast) and its atomics hit 32 banks, at about 30 instructions a
-// segment; the dense walk takes about 75 for 32 pairs and its lanes' rows collide.
+// memory once per warp (a broadcast) and its atomics hit 32 banks; the dense walk takes about three
+// times the instructions for 32 pairs and its lanes' rows collide.  (400 k segments of 12 px: 171 us
+// a call with 12 here, 178 with 8 or 5; of 90 px: 253, 253, 257.)
 #ifndef LG_RASTER_LANE_MIN
-#define LG_RASTER_LANE_MIN 8
+#define LG_RASTER_LANE_MIN 12
 #endif
 
-// Bound: the shared-memory pipe (seven or eight 32-bit atomics and three broadcast reads per
-// segment and tile): 87 % of the L1 wavefront slots on the mid scene at 2^13 rays per light
-// (450 M pixels), 1.42 ms where spreading every pixel over the lanes took 2.78 ms (2196 M warp
-// instructions, 167 M bank conflicts; now 1030 M and 10 M).  With a branch per atomic instead
-// of masked terms the same walk took 2.42 ms.
+// Bound: the shared-memory pipe.  A segment takes seven or eight 32-bit atomics per tile and two
+// or three 16-byte broadcast reads, two wavefronts each: 94 % of the L1 wavefront slots on the mid
+// scene at 2^15 rays per light with three reads; two reads take 2.40 ms where three take 2.65 (mid
+// scene, 2^14 rays per light) and 10.6 where 11.4 (CSG frame, 2^17 rays).  Spreading every pixel over
+// the lanes, with a branch per atomic, took 2.78 ms at 2^13 rays per light; masked terms, a lane
+// per column, 1.42 ms (2196 M against 1030 M warp instructions, 167 M against 10 M bank conflicts).
 template <int MODE>
 __global__ void __launch_bounds__(256, 4) k_raster(RasterArgs A) {
   if (A.ctr->skip_raster) return;
@@ -604,6 +606,10 @@ __global__ void __launch_bounds__(256, 4) k_raster(RasterArgs A) {
   uint32_t my_pixels = 0;
   unsigned long long n_units = A.ctr->units;
   if (n_units > A.units_cap) n_units = A.units_cap;
+  if (SP::on) {  // the planes start at zero, and every flush leaves them so
+    uint4* z = reinterpret_cast<uint4*>(acc32);
+    for (int k = threadIdx.x; k < RasterSmem<MODE>::acc_words / 4; k += blockDim.x) z[k] = make_uint4(0, 0, 0, 0);
+  }
   for (;;) {
     if (threadIdx.x == 0) s_unit = atomicAdd(&A.ctr->unit_cursor, 1ull);
     __syncthreads();
@@ -619,15 +625,12 @@ __global__ void __launch_bounds__(256, 4) k_raster(RasterArgs A) {
     const int nmin = (int)(xmajor ? C.H : C.W);
     // minor pixels of the tile: floor(v) in [tn TILE, hi) exactly when v is
     const float vlo = (float)(tn * TILE), vhi = (float)min(tn * TILE + TILE, nmin);
-    if (SP::on) {
-      uint4* z = reinterpret_cast<uint4*>(acc32);
-      for (int k = threadIdx.x; k < RasterSmem<MODE>::acc_words / 4; k += blockDim.x) z[k] = make_uint4(0, 0, 0, 0);
-    } else if (MODE == RM_FIXED_MINMAX) {
+    if (MODE == RM_FIXED_MINMAX) {
       for (int k = threadIdx.x; k < 4 * TILE_PX; k += blockDim.x) acc64[k] = ident64(B.op[k / TILE_PX]);
-    } else {
+    } else if (!SP::on) {
       for (int k = threadIdx.x; k < 4 * TILE_PX; k += blockDim.x) accf[k] = ident32(B.op[k / TILE_PX]);
     }
-    __syncthreads();
+    if (!SP::on) __syncthreads();
     // Adds one staged segment's terms to a cell of the tile when on.  Split sums take no branch
     // (eight predicated atomics cost a branch each): a lane that is off adds zeros to the cell
     // of its own bank in row 0.  alpha_c: some alpha term of the batch has a low part (an alpha
@@ -659,16 +662,19 @@ __global__ void __launch_bounds__(256, 4) k_raster(RasterArgs A) {
       }
     };
     const uint64_t end = min(U.begin + U.n, A.refs_cap);
+    uint32_t next_ref = 0;  // a batch ahead: the segments' addresses do not wait for the list
+    if (U.begin + (uint64_t)warp * 32 + lane < end) next_ref = A.refs[U.begin + (uint64_t)warp * 32 + lane];
     for (uint64_t base = U.begin + (uint64_t)warp * 32; base < end; base += (uint64_t)nwarps * 32) {
       // lane-parallel: fetch 32 segments, set them up and clip them to this tile
       const uint64_t r = base + lane;
+      const uint32_t si = next_ref;
+      if (r + (uint64_t)nwarps * 32 < end) next_ref = A.refs[r + (uint64_t)nwarps * 32];
       Staged st;
       st.mask = 0;
       int c0 = 0, cnt = 0;
       bool big = false;
       float term[4];
       if (r < end) {
-        const uint32_t si = A.refs[r];
         const float4* sp = reinterpret_cast<const float4*>(A.segs + si);
         const float4 g = __ldg(sp), cc = __ldg(sp + 1);
         lg_segment sg;
@@ -732,8 +738,47 @@ __global__ void __launch_bounds__(256, 4) k_raster(RasterArgs A) {
       const int n_drawn = __popc(drawn), pos = __popc(drawn & lanemask_lt());
       const int total = (int)__reduce_add_sync(0xffffffffu, (unsigned)cnt);
       const bool alpha_c = SP::on && __any_sync(0xffffffffu, cnt > 0 && st.q[6] != 0u);
+      bool by_lane = total >= LG_RASTER_LANE_MIN * n_drawn;
+      // The usual batch: colour terms in [0, 1), whose split parts are the bits of one word each, and
+      // one alpha term for all without a low part (an alpha of 1).  Its staged rows take two
+      // 16-byte reads instead of three, and reads are a third of the shared-memory traffic.
+      if (MODE == RM_FIXED_SPLIT && by_lane && drawn) {
+        const unsigned alpha = __shfl_sync(0xffffffffu, st.q[7], __ffs(drawn) - 1);
+        const bool wide = cnt > 0 && (st.q[6] != 0u || st.q[7] != alpha || (st.q[1] | st.q[3] | st.q[5]) >> (32 - SP::bits) != 0u ||
+                                      (st.q[0] | st.q[2] | st.q[4]) >> SP::bits != 0u);
+        if (!__any_sync(0xffffffffu, wide)) {
+          uint4* rows = reinterpret_cast<uint4*>(stage);
+          if (cnt > 0) {
+            rows[2 * pos] = make_uint4(__float_as_uint(st.ua), __float_as_uint(st.va), __float_as_uint(st.slope), st.mask);
+            rows[2 * pos + 1] = make_uint4(st.q[0] | st.q[1] << SP::bits, st.q[2] | st.q[3] << SP::bits,
+                                           st.q[4] | st.q[5] << SP::bits, 0u);
+          }
+          __syncwarp();
+          const float fi = __fadd_rn((float)(tm * TILE + (int)lane), 0.5f);
+          const int cell0 = (int)lane - tn * TILE_PX;
+          const unsigned bit = 1u << lane, low = (1u << SP::bits) - 1u;
+#pragma unroll 2
+          for (int k = 0; k < n_drawn; ++k) {
+            const uint4 h = rows[2 * k], q = rows[2 * k + 1];
+            const float v = __fmaf_rn(__fsub_rn(fi, __uint_as_float(h.x)), __uint_as_float(h.z), __uint_as_float(h.y));
+            const bool on = (h.w & bit) && v >= vlo && v < vhi;
+            const unsigned a = acc_addr + 4u * (unsigned)(on ? (int)v * TILE + cell0 : (int)lane), m = on ? 0xffffffffu : 0u;
+            const unsigned qr = q.x & m, qg = q.y & m, qb = q.z & m;
+            shared_add(a, qr & low);
+            shared_add(a + 4u * PLANE, qr >> SP::bits);
+            shared_add(a + 8u * PLANE, qg & low);
+            shared_add(a + 12u * PLANE, qg >> SP::bits);
+            shared_add(a + 16u * PLANE, qb & low);
+            shared_add(a + 20u * PLANE, qb >> SP::bits);
+            shared_add(a + 28u * PLANE, alpha & m);
+            my_pixels += on ? 1u : 0u;
+          }
+          __syncwarp();
+          continue;
+        }
+      }
       if (cnt > 0) stage[pos] = st;
-      if (total >= LG_RASTER_LANE_MIN * n_drawn) {
+      if (by_lane) {
         __syncwarp();
         const float fi = __fadd_rn((float)(tm * TILE + (int)lane), 0.5f);
         const int cell0 = (int)lane - tn * TILE_PX;
@@ -785,8 +830,12 @@ __global__ void __launch_bounds__(256, 4) k_raster(RasterArgs A) {
         const int ch = k & 3, cell = k >> 2;
         const int major = cell % TILE, minor = cell / TILE;
         const uint32_t x = tx * TILE + (xmajor ? major : minor), y = ty * TILE + (xmajor ? minor : major);
-        const unsigned* plane = acc32 + 2 * ch * PLANE + cell;
-        const long long q = (long long)(int)plane[PLANE] * (1ll << SP::bits) + (long long)(int)plane[0];
+        unsigned* plane = acc32 + 2 * ch * PLANE + cell;
+        const unsigned lo = plane[0], hi = plane[PLANE];
+        if ((lo | hi) == 0u) continue;
+        plane[0] = 0u;
+        plane[PLANE] = 0u;
+        const long long q = (long long)(int)hi * (1ll << SP::bits) + (long long)(int)lo;
         if (q == 0 || x >= C.W || y >= C.H) continue;
         const uint64_t px = (C.px_base + (uint64_t)y * C.W + x) * 4;
         if (MODE == RM_F32)

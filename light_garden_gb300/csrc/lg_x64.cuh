@@ -30,7 +30,6 @@ constexpr double SPOT_EPSILON = 1e-9;  // SpotLight::set_num_rays |dir.x| < EPSI
 constexpr double PI = 3.141592653589793;
 constexpr uint32_t NEAR = LG_PATH_NEAR_DEGENERATE;
 constexpr int MAX_DEPTH = 8;    // LOGIC levels of one object's tree in this mode
-constexpr int MAX_POLY = 63;
 
 __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
 __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
@@ -277,21 +276,32 @@ __device__ __forceinline__ double spot_base_angle(double sx, double sy) {
 }
 
 // ------------------------------------------------------------------ leaves: membership
-__device__ __forceinline__ int poly_vertices(const lg_geo* G, const lg_geo& g, V* out) {
+// A polygon's vertices in order, four per node of its chain, each edge passed to f(i, from, to); no
+// local copy (63 vertices in local memory took most of a polygon's solve).
+template <class F>
+__device__ __forceinline__ void poly_edges(const lg_geo* G, const lg_geo& g, F&& f) {
   const int n = g.a;
-  int k = 0;
   const lg_geo* cur = &g;
-  while (k < n) {
-    for (int i = 0; i < 4 && k < n; ++i, ++k) out[k] = mk(cur->v[2 * i], cur->v[2 * i + 1]);
-    if (k < n) cur = &G[cur->b];
+  const V first = mk(g.v[0], g.v[1]);
+  V from = first;
+  for (int i = 0; i < n; ++i) {
+    const int k = (i + 1) & 3;
+    V to = first;
+    if (i + 1 < n) {
+      if (k == 0) cur = &G[cur->b];
+      to = mk(cur->v[2 * k], cur->v[2 * k + 1]);
+    }
+    f(i, from, to);
+    from = to;
   }
-  return n;
 }
-__device__ __forceinline__ double poly_orientation(const V* P, int n) {
-  double a = 0.0;
-  for (int i = 0; i < n; ++i) a = add(a, cross(P[i], P[(i + 1) % n]));
-  return a >= 0.0 ? 1.0 : -1.0;
+__device__ __forceinline__ V poly_vertex(const lg_geo* G, const lg_geo& g, int i) {
+  const lg_geo* cur = &g;
+  for (; i >= 4; i -= 4) cur = &G[cur->b];
+  return mk(cur->v[2 * i], cur->v[2 * i + 1]);
 }
+// +1 counter-clockwise, -1 clockwise (kept in the node by the host)
+__device__ __forceinline__ double poly_orientation(const lg_geo& g) { return g.op >= 0 ? 1.0 : -1.0; }
 
 // closed membership of one leaf, p in the leaf's frame; fl (optional) receives NEAR when the
 // point lies within the band of the boundary
@@ -313,18 +323,24 @@ static __device__ __noinline__ bool leaf_contains(const lg_geo* G, const lg_geo&
       return sd <= 0.0;
     }
     case LG_GEO_POLYGON: {
-      V P[MAX_POLY];
-      const int n = poly_vertices(G, g, P);
-      const double sgn = poly_orientation(P, n);
+      const double sgn = poly_orientation(g);
       const V l = irot(vsub(p, mk(g.origin[0], g.origin[1])), g.rot[0], g.rot[1]);
       bool in = true;
-      for (int i = 0; i < n; ++i) {
-        const V e = vsub(P[(i + 1) % n], P[i]);
+      poly_edges(G, g, [&](int, V from, V to) {
+        const V e = vsub(to, from);
+        const double cr = mul(-sgn, cross(e, vsub(l, from)));
+        // the signed distance sd = cr / |e| decides by its sign, which is cr's, and is in the band
+        // |sd| <= BAND |e| only when |cr| <= BAND |e|^2
+        const float e2 = (float)e.x * (float)e.x + (float)e.y * (float)e.y, ac = fabsf((float)cr);
+        if (ac > 2e-10f * e2 && ac > 1e-30f && e2 > 1e-30f && e2 < 1e30f) {
+          if (!is_neg(cr)) in = false;
+          return;
+        }
         const double le = sqr(dot(e, e));
-        const double sd = dvd(mul(-sgn, cross(e, vsub(l, P[i]))), le > 0.0 ? le : 1.0);
+        const double sd = dvd(cr, le > 0.0 ? le : 1.0);
         if (fl && fabs(sd) <= mul(BAND, add(le, 1e-300))) *fl |= NEAR;
         if (sd > 0.0) in = false;
-      }
+      });
       return in;
     }
     case LG_GEO_ELLIPSE: {
@@ -556,13 +572,21 @@ __device__ __forceinline__ void hits_cubic(const lg_geo& g, V o, V d, double& ev
 
 template <class F>
 __device__ __forceinline__ void hits_polygon(const lg_geo* G, const lg_geo& g, V o, V d, double& ev, F&& emit) {
-  V P[MAX_POLY];
-  const int n = poly_vertices(G, g, P);
   const double c = g.rot[0], s = g.rot[1];
   const V org = mk(g.origin[0], g.origin[1]);
   const V lo = irot(vsub(o, org), c, s), ld = irot(d, c, s);
-  for (int i = 0; i < n; ++i)
-    hits_segment(P[i], P[(i + 1) % n], lo, ld, ev, [&](const Hit& h) { emit(mkhit(h.t, o, d, mk(0.0, 0.0), i)); });
+  poly_edges(G, g, [&](int i, V from, V to) {
+    // an edge whose line the ray's line crosses well outside it, at no small angle, has neither a hit
+    // nor an event (hits_segment): its place u along the edge from the FP64 products in FP32
+    const V e = vsub(to, from), w = vsub(from, lo);
+    const float den = (float)cross(ld, e), cu = (float)cross(w, ld);
+    const float len = fabsf((float)e.x) + fabsf((float)e.y), dl = fabsf((float)ld.x) + fabsf((float)ld.y);
+    if (fabsf(den) > 1e-6f * len * dl && fabsf(den) > 1e-30f) {
+      const float u = __fdividef(cu, den);
+      if (u < -1e-3f || u > 1.001f) return;
+    }
+    hits_segment(from, to, lo, ld, ev, [&](const Hit& h) { emit(mkhit(h.t, o, d, mk(0.0, 0.0), i)); });
+  });
 }
 
 template <class F>
@@ -624,11 +648,9 @@ static __device__ __noinline__ V leaf_normal(const lg_geo* G, const lg_geo& g, c
       return l > 0.0 ? mk(dvd(-dB.y, l), dvd(dB.x, l)) : unit(mk(-d.y, d.x));
     }
     case LG_GEO_POLYGON: {
-      V P[MAX_POLY];
-      const int n = poly_vertices(G, g, P);
-      const double sgn = poly_orientation(P, n);
-      const V e = vsub(P[(h.sub + 1) % n], P[h.sub]);
-      return rot(unit(vscl(mk(e.y, -e.x), sgn)), g.rot[0], g.rot[1]);
+      const V from = poly_vertex(G, g, h.sub), to = poly_vertex(G, g, h.sub + 1 < g.a ? h.sub + 1 : 0);
+      const V e = vsub(to, from);
+      return rot(unit(vscl(mk(e.y, -e.x), poly_orientation(g))), g.rot[0], g.rot[1]);
     }
     case LG_GEO_ELLIPSE: {
       const double A = g.v[0], Bb = g.v[1];
