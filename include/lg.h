@@ -302,7 +302,8 @@ typedef struct lg_trace_stats {
      into bin (count, scan, scatter) and raster (tile accumulation) */
   float trace_ms, accumulate_ms, resolve_ms, total_ms, bin_ms, raster_ms;
   /* lg_render: the trace's kernels summed over the generations: the FP32 nearest-hit search,
-     the precise solve (k_solve_x, or k_refine + k_full), the bounce */
+     the precise solve (k_solve_x, or k_refine + k_full), the bounce; a small frame's
+     generation is one kernel, all of it in bounce_ms */
   float scan_ms, solve_ms, bounce_ms;
   float _pad2;
   uint64_t ill_conditioned; /* segments carrying LG_PATH_ILL_CONDITIONED (double-float mode) */

@@ -820,6 +820,18 @@ TraceKernel scan_kernel(bool multi, bool culled, bool exact, int pairs) {
   return pairs <= 8 ? scan_kernel_ch<8>(multi, culled, exact) : scan_kernel_ch<16>(multi, culled, exact);
 }
 
+// Whether a generation is one launch (k_small_x) or three.  One launch saves two launches' latency
+// and the records between them, and loses the three kernels' compaction: it pays while the rays
+// leave the SMs idle, less so the more geometry nodes a warp's lanes diverge over.  Trace time of
+// three launches over one, geometric mean of 6 scenes each: 24 plain objects 1.00 (256 primaries),
+// 1.20 (4096), 1.26 (16384); 8 CSG objects (24 nodes) 1.07 to 1.16, 12 (36 nodes) 0.93 to 1.11, 24
+// 0.87 to 0.98; 12 mixed objects 1.24 at 32768 primaries and 0.91 at 65536; 2 CSG objects 1.37
+// at 65536.  An explicit scan_pairs or grid walk asks for the scan kernel.
+static bool small_frame(const lg_ctx* c, const lg_params& p, uint64_t nodes) {
+  return p.precision == LG_PRECISION_EXACT && !c->scan_walk && c->scan_pairs == 0 && nodes <= 24 &&
+         c->n_primary <= 65536 && c->n_primary * nodes <= 24 * 16384;
+}
+
 // The scan's pair slots per lane: as requested, else 8 for the grid walk (a smaller buffer leaves
 // more of the SM's L1 to the list and queue loads: 131072 rays, 64 objects 9.0 ms of scan against
 // 11.0 with 16, 200 objects 16.5 against 20.1, a 64-scene batch 86.1 against 89.5 ms of trace) and 16
@@ -886,6 +898,11 @@ void launch_light_setup(lg_ctx* c, const SceneDev& S, bool multi) {
 void launch_generation(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_t g, bool multi, int scan_grid,
                        size_t scan_smem, size_t tsm, int smem_fits) {
   const bool exact = c->prm.precision == LG_PRECISION_EXACT;
+  if (!multi && c->small) {
+    if (c->culled) k_small_x<true><<<c->n_sm * 4, SMALL_THREADS, tsm, c->stream>>>(S, B, g, smem_fits);
+    else k_small_x<false><<<c->n_sm * 4, SMALL_THREADS, tsm, c->stream>>>(S, B, g, smem_fits);
+    return;
+  }
   scan_kernel(multi, c->scan_walk, exact, scan_pairs_of(c))<<<scan_grid, SCAN_THREADS, scan_smem, c->stream>>>(S, B, g,
                                                                                                    smem_fits);
   if (exact) {
@@ -1202,6 +1219,8 @@ lg_status lg_create(lg_ctx** out, const lg_device_opts* opts) {
           if (e == cudaSuccess)
             e = cudaFuncSetAttribute(scan_kernel(m != 0, cu != 0, ex != 0, pairs), cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      scan_smem_bytes(pairs) + (m ? 0 : (int)OBJ_SMEM_MAX));
+  for (TraceKernel k : {k_small_x<false>, k_small_x<true>})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OBJ_SMEM_MAX);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_full<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OBJ_SMEM_MAX);
   for (TraceKernel k : {k_bounce<false, false>, k_bounce<false, true>})
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)OBJ_SMEM_MAX);
@@ -1349,6 +1368,11 @@ lg_status lg_scene_upload(lg_ctx* c, const lg_geo* geos, uint32_t n_geo, const l
   c->n_cubic = (uint32_t)F.cubics.size();
   c->n_primary = 0;
   for (uint32_t l = 0; l < n_lights; ++l) c->n_primary += sampled_rays(lights[l].num_rays, p);
+  const bool small = small_frame(c, p, F.xnode.size());
+  if (c->small != small) {
+    c->small = small;
+    c->graph_valid = false;
+  }
   c->prm = pk;
   c->chords_ready = 0;
   c->aspect = (double)((float)p.width / (float)p.height);

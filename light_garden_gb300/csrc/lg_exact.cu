@@ -368,6 +368,32 @@ template __global__ void k_solve_x<false>(SceneDev, TraceBufs, uint32_t);
 template __global__ void k_solve_x<true>(SceneDev, TraceBufs, uint32_t);
 
 // ------------------------------------------------------------------ bounce
+// Primary number v of a frame (light.rs:103-115, 163-174, 225-249) as a queue entry.
+__device__ __forceinline__ void primary_rec(const SceneDev& S, uint64_t v, RayRec& r) {
+  uint32_t l = 0, hi = S.n_lights;
+  while (hi - l > 1) {  // the last light whose first primary is <= v
+    const uint32_t mid = (l + hi) >> 1;
+    if (S.lights[mid].first <= v) l = mid; else hi = mid;
+  }
+  const LightDev& L = S.lights[l];
+  const uint64_t i = S.ray_offset + (uint64_t)S.ray_stride * (v - L.first);
+  double ox, oy, dx, dy;
+  lgx::primary_ray_x(L.kind, L.ox, L.oy, L.vx, L.vy, L.spot_angle, L.dir_angle, (double)L.num_rays, i, ox, oy, dx, dy);
+  r.ox = xdf(ox); r.oy = xdf(oy); r.dx = xdf(dx); r.dy = xdf(dy);
+  r.medium = MEDIUM_LIGHT;
+  r.src_obj = SRC_NONE;
+  r.src_leaf = 0;
+  for (int k = 0; k < 4; ++k) r.c[k] = L.color[k];
+  r.path = 0;
+  r.prim = (uint32_t)i;
+  r.light = (uint16_t)l;
+  r.gen = 0;
+  r.flags = 0;
+  r._pad = 0;
+  r.scene = 0;
+  r.ex = r.ea = 0.0f;
+}
+
 // What a ray visit leaves: its segment, and up to two rays that start at (ox, oy): the reflected
 // (or mirrored) one with direction d0 and colour scaled by f0, and the refracted one.
 struct BounceX {
@@ -651,6 +677,122 @@ __device__ __forceinline__ void store_segment_x(const SceneDev& S, const TraceBu
     B.paths[slot] = pr;
   }
 }
+
+// One generation of a small frame in one launch: a thread takes its ray through the search, the
+// solve and the bounce.  A few thousand rays leave the GPU nearly empty whatever the order, and
+// three launches with their lists and records cost more than the lost coherence: eight
+// generations of a disc and a mirror (4096 primaries) take 127 us instead of 225, five of 12
+// objects (12,000 primaries) 212 instead of 290.  Bound by the latency of the chain from a ray's
+// record through its FP64 solve to its children, of which a warp has one and an SM few; 64
+// threads a CTA spread the warps over all SMs.  The candidates are those of k_scan (the same
+// tests in table order), so the hits are the same bits.
+template <bool CULL>
+__global__ void __launch_bounds__(SMALL_THREADS) k_small_x(SceneDev S, TraceBufs B, uint32_t gen, int smem_fits) {
+  for (int k = 0; k < 3; ++k) stamp_start(B.ctr, gen, k);
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  __shared__ __align__(8) uint64_t bar;
+  const uint64_t n_in = n_in_of(S, B, gen);
+  if ((uint64_t)blockIdx.x * blockDim.x >= n_in) return;  // no ray for this CTA
+  bool failed;
+  const ObjScan* objs = stage_objects(S, reinterpret_cast<ObjScan*>(smem_raw), &bar, smem_fits != 0, B.ctr, failed);
+  if (failed) return;
+  const RayRec* qin = B.queue[gen & 1];
+  RayRec* qout = B.queue[(gen + 1) & 1];
+  const SceneLoc sl = scene_of<false>(S, 0u);
+  uint32_t my_visits = 0, my_near = 0, my_tests = 0, my_cls = 0, my_solves = 0;
+  const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
+  for (uint64_t base = warp * 32; base < n_in; base += nwarps * 32) {
+    const uint64_t idx = base + lane_id();
+    BounceX v;
+    v.emit = v.child0 = v.child1 = false;
+    v.flags = 0;
+    v.hit = -1;
+    v.f0 = v.f1 = 1.0f;
+    RayRec r;
+    bool live = idx < n_in;
+    if (live) {
+      if (gen == 0) primary_rec(S, idx, r);
+      else r = qin[idx];
+      live = !below_cutoff(r.c, sl.cutoff);
+    }
+    if (live) {
+      ++my_visits;
+      const V o = ray_o(r), d = ray_d(r);
+      const float ox = (float)o.x, oy = (float)o.y, dx = (float)d.x, dy = (float)d.y;
+      float thr = 3e38f, key[CAND], proved_t = INFINITY, proved_s = 0.0f;
+      uint16_t cand[CAND];
+      int nc = 0, leaf = -1, face = -1;
+      ScanRec sc;
+      sc.overflow = 0;
+      for (uint32_t j = 0; j < S.n_obj; ++j) {
+        float lb;
+        ++my_tests;
+        if (!bound_test(*reinterpret_cast<const float4*>(&objs[j]), ox, oy, dx, dy, thr, lb)) continue;
+        ++my_cls;
+        const Class32 c = classify32(objs[j], ox, oy, dx, dy, lb, j == r.src_obj ? (int)r.src_leaf : -1);
+        if (c.ub < INFINITY) thr = fminf(thr, c.ub * (1.0f + 1e-4f) + 1e-4f);
+        if (!(c.key <= thr)) continue;
+        if (c.ub < proved_t) { proved_t = c.ub; leaf = c.leaf; face = c.face; proved_s = c.s; }
+        if (nc == CAND) {  // full: drop candidates the bound has since excluded
+          int w = 0;
+          for (int k = 0; k < CAND; ++k)
+            if (key[k] <= thr) { key[w] = key[k]; cand[w++] = cand[k]; }
+          nc = w;
+        }
+        if (nc < CAND) { key[nc] = c.key; cand[nc++] = (uint16_t)j; }
+        else sc.overflow = 1;
+      }
+      int m = 0;
+      float k0 = INFINITY;
+      for (int k = 0; k < nc; ++k)
+        if (key[k] <= thr) {
+          if (m == 0) k0 = key[k];
+          cand[m++] = cand[k];
+        }
+      sc.nc = (uint8_t)m;
+      HitRec hit;
+      hit.obj = HIT_NONE;
+      hit.flags = 0;
+      if (m > 0 || sc.overflow) {
+        bool done = false;
+        if (m == 1 && !sc.overflow && leaf >= 0 && k0 == proved_t) {  // the only candidate's certain root
+          const SolveRec& G = S.solve[cand[0]];
+          lgx::Hit h;
+          V n;
+          if ((G.kind & 0xfu) != SR_TREE && solve_proved_x(G, o, d, leaf, face, proved_t, proved_s, h.t, h.p, n)) {
+            store_hit_x(hit, (int)cand[0], h, n, leaf, INFINITY, 0);
+            done = true;
+            ++my_solves;
+          }
+        }
+        if (!done) {
+          Nearest N;
+          const uint32_t count = sc.overflow ? S.n_obj : (uint32_t)m;
+          for (uint32_t k = 0; k < count; ++k) {
+            const uint32_t j = sc.overflow ? k : (uint32_t)cand[k];
+            float lb;
+            if (sc.overflow && !bound_test(*reinterpret_cast<const float4*>(&objs[j]), ox, oy, dx, dy, thr, lb)) continue;
+            ++my_solves;
+            N.consider(S, 0u, j, o, d);
+          }
+          N.store(S, 0u, d, sc.overflow ? LG_PATH_FALLBACK : 0, hit);
+        }
+      }
+      bounce_x<false, CULL>(S, r, sc, &hit, v);
+    }
+    unsigned long long seg, s0, s1;
+    reserve_out(B, gen, v.emit, v.child0, v.child1, seg, s0, s1);
+    if (v.emit) store_segment_x(S, B, v, r, seg, my_near);
+    if (v.child0 && s0 < B.queue_cap) store_child(qout + s0, r, child_x(r, v, v.d0, v.f0, r.path, r.medium));
+    if (v.child1 && s1 < B.queue_cap)
+      store_child(qout + s1, r, child_x(r, v, v.d1, v.f1, r.path | (1ull << r.gen), v.medium1));
+  }
+  stamp_end(B.ctr, gen);
+  add_block_counts<5>({my_visits, my_near, my_tests, my_cls, my_solves},
+                      {&B.ctr->visits, &B.ctr->near, &B.ctr->bound_tests, &B.ctr->object_tests, &B.ctr->fp64_solves});
+}
+template __global__ void k_small_x<false>(SceneDev, TraceBufs, uint32_t, int);
+template __global__ void k_small_x<true>(SceneDev, TraceBufs, uint32_t, int);
 
 template <bool MULTI, bool CULL>
 __global__ void __launch_bounds__(256, LG_BOUNCE_X_BLOCKS) k_bounce_x(SceneDev S, TraceBufs B, uint32_t gen) {

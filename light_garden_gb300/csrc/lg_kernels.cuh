@@ -78,6 +78,10 @@ template <bool MULTI>
 __global__ void k_solve_x(SceneDev S, TraceBufs B, uint32_t gen);
 template <bool MULTI, bool CULL>
 __global__ void k_bounce_x(SceneDev S, TraceBufs B, uint32_t gen);
+// a whole generation of a small one-scene frame
+constexpr int SMALL_THREADS = 64;
+template <bool CULL>
+__global__ void k_small_x(SceneDev S, TraceBufs B, uint32_t gen, int smem_fits);
 // The string-mod lines' table and the modulo-colour table on the device (sm.colors is the
 // caller's host pointer and is never read on the device).
 struct ChordArgs {

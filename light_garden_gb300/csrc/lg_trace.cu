@@ -17,69 +17,6 @@
 
 namespace lgd {
 
-// ------------------------------------------------------------- bulk copy to shared memory
-__device__ __forceinline__ void mbar_init(uint64_t* bar, unsigned count) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(a), "r"(count) : "memory");
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, unsigned bytes) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(a), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
-  unsigned ok;
-  asm volatile(
-      "{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
-      : "=r"(ok)
-      : "r"(a), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-__device__ __forceinline__ void bulk_g2s(void* dst, const void* src, unsigned bytes, uint64_t* bar) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  const unsigned b = (unsigned)__cvta_generic_to_shared(bar);
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d),
-      "l"(src), "r"(bytes), "r"(b)
-      : "memory");
-}
-
-// Stages the ObjScan table into shared memory.  Returns the table to scan: shared memory
-// on success, the global table if it does not fit or the bounded wait expired (in which
-// case ERR_TMA_TIMEOUT is raised and the caller returns).
-__device__ const ObjScan* stage_objects(const SceneDev& S, ObjScan* sobj, uint64_t* bar, bool fits,
-                                        Counters* ctr, bool& failed) {
-  failed = false;
-  if (!fits || S.n_obj == 0) return S.scan;
-  const unsigned bytes = S.n_obj * (unsigned)sizeof(ObjScan);
-  if (threadIdx.x == 0) {
-    mbar_init(bar, 1);
-    mbar_expect_tx(bar, bytes);
-    const unsigned chunk = 32768u;
-    for (unsigned off = 0; off < bytes; off += chunk) {
-      const unsigned n = bytes - off < chunk ? bytes - off : chunk;
-      bulk_g2s(reinterpret_cast<char*>(sobj) + off, reinterpret_cast<const char*>(S.scan) + off, n, bar);
-    }
-  }
-  __syncthreads();  // barrier initialised before anyone waits on it
-  bool done = false;
-  const int polls = S.wait_polls;
-  for (int it = 0; it < polls && !done; ++it) {
-    done = mbar_try_wait(bar, 0);
-    if (!done && it > 64) __nanosleep(64);
-  }
-  if (!done) {
-    atomicOr(&ctr->error_flags, ERR_TMA_TIMEOUT);
-    // give the copy a last bounded chance to land before this CTA's shared memory is released
-    for (int it = 0; it < (1 << 20) && !mbar_try_wait(bar, 0); ++it) __nanosleep(256);
-    failed = true;
-  }
-  __syncthreads();
-  return sobj;
-}
-
 // ------------------------------------------------------------------- primary rays
 // native FP64 (only here): the reference's f64 sin_cos / atan per primary ray
 __device__ inline void primary_ray(const LightDev& L, uint64_t i, double& ox, double& oy, double& dx, double& dy) {
