@@ -79,7 +79,7 @@ lg_status enqueue_batch(lg_ctx* c, cudaEvent_t* ev) {
   const int acc = accum_kind(c->prm);
   CK(cudaEventRecordWithFlags(ev[0], c->stream, cudaEventRecordExternal), "stage event");
   CK(cudaMemsetAsync(c->d_ctr.p, 0, sizeof(Counters), c->stream), "memset counters");
-  CK(cudaMemsetAsync(c->d_scene_count.p, 0, (size_t)c->n_scenes * 4, c->stream), "memset scene counts");
+  CK(cudaMemsetAsync(c->d_scene_count.p, 0, (size_t)sort_bins(c->n_scenes) * 4, c->stream), "memset sort counts");
   k_clear_accum<<<c->n_sm * 8, 256, 0, c->stream>>>(A);
   if (c->n_lights) launch_light_setup(c, S, true);
   const uint32_t bins = c->total_bins;
@@ -90,13 +90,7 @@ lg_status enqueue_batch(lg_ctx* c, cudaEvent_t* ev) {
   lg_string_mod no_sm;
   std::memset(&no_sm, 0, sizeof no_sm);
   for (uint32_t g = 0; g < c->max_bounce_all; ++g) {
-    if (g > 0) {  // visit this generation's queue in scene order
-      k_scene_hist<<<c->n_sm * 8, 256, 0, c->stream>>>(S, B, g, (unsigned*)c->d_scene_count.p);
-      k_scene_offsets<<<1, 1024, 0, c->stream>>>((unsigned*)c->d_scene_count.p, (unsigned*)c->d_scene_off.p,
-                                                  c->n_scenes);
-      k_scene_scatter<<<c->n_sm * 8, 256, 0, c->stream>>>(S, B, g, (unsigned*)c->d_scene_off.p,
-                                                          (uint32_t*)c->d_order.p);
-    }
+    if (g > 0) launch_sort(c, S, B, g, c->n_scenes, true);
     launch_generation(c, S, B, g, true, c->batch_grid_scan, (size_t)scan_smem_bytes(scan_pairs_of(c)), 0, 0);
     if (g == 0 && c->n_cubic) {
       const int blocks = (int)std::min<uint64_t>((3ull * c->n_cubic + 255) / 256, 4096);
@@ -298,8 +292,7 @@ lg_status lg_batch_upload(lg_ctx* c, const lg_scene_desc* scenes, uint32_t k) {
   c->culled = false;
   for (const GridRec& g : grids.recs) c->culled = c->culled || g.nx > 0;
   c->scan_walk = c->culled;  // scenes without a grid take the table scan inside the walking kernel
-  if ((st = ensure(c, c->d_scene_count, (size_t)k * 4, "scene counts"))) return st;
-  if ((st = ensure(c, c->d_scene_off, (size_t)k * 4, "scene offsets"))) return st;
+  if ((st = ensure_sort_buffers(c, k))) return st;
   CK(cudaStreamSynchronize(c->stream), "upload");
   c->n_scenes = k;
   c->h_scenes = recs;

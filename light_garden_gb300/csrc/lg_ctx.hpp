@@ -84,6 +84,7 @@ struct lg_ctx {
   int32_t wait_polls = 1 << 22;  // bounded device waits (lg_device_opts.wait_polls)
   bool culled = false;  // the uploaded scene (or some scene of the batch) has a grid
   bool small = false;   // one scene, exact, few primaries: a generation is one launch (k_small_x)
+  bool sorted = false;  // one scene: generations > 0 visit their rays in place and direction order
   bool scan_walk = false;  // the nearest-hit scan walks the grid (else it scans the object table)
   uint64_t total_px = 0;
   uint32_t total_bins = 0;
@@ -129,6 +130,10 @@ lg_status trace_grids(lg_ctx* c, bool multi, size_t tsm);
 // The light setup and one generation's chain for the context's precision: the FP32 scan,
 // then k_refine + k_full + k_bounce (fast) or k_solve_x + k_bounce_x (exact).
 void launch_light_setup(lg_ctx* c, const SceneDev& S, bool multi);
+// Visiting order of queued rays (a counting sort by scene, place and direction).
+uint32_t sort_bins(uint32_t n_scenes);
+lg_status ensure_sort_buffers(lg_ctx* c, uint32_t n_scenes);
+void launch_sort(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_t g, uint32_t n_scenes, bool multi);
 void launch_generation(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_t g, bool multi, int scan_grid,
                        size_t scan_smem, size_t tsm, int smem_fits);
 // Uploads a flattened scene's exact-mode tables (geometry nodes, preorder trees).

@@ -358,7 +358,7 @@ struct TraceBufs {
   lg_segment* segs;
   lg_path_record* paths;
   uint16_t* seg_scene;      // multi-scene traces: the scene of every segment
-  const uint32_t* order;    // multi-scene traces, generations > 0: queue entries sorted by scene
+  const uint32_t* order;    // generations > 0: queue entries in visiting order (one scene: or null)
   uint64_t seg_cap;
   Counters* ctr;
 };

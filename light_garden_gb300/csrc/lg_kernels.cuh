@@ -107,8 +107,12 @@ __global__ void k_cross_write(const double2* pts, uint32_t m, const uint32_t* bl
 __global__ void k_overlay(SceneDev S, TraceBufs B, const uint32_t* cubic_objs, const uint16_t* cubic_scene,
                           uint32_t n_cubic, lg_string_mod sm, ChordArgs CA);
 __global__ void k_scene_hist(SceneDev S, TraceBufs B, uint32_t gen, unsigned* count);
-__global__ void k_scene_offsets(unsigned* count, unsigned* off, uint32_t n_scenes);
-__global__ void k_scene_scatter(SceneDev S, TraceBufs B, uint32_t gen, unsigned* off, uint32_t* order);
+template <bool MULTI, bool EXACT>
+__global__ void k_sort_keys(SceneDev S, TraceBufs B, uint32_t gen, uint32_t bits, uint32_t* keys, unsigned* count);
+template <bool MULTI>
+__global__ void k_sort_offsets(SceneDev S, TraceBufs B, uint32_t gen, unsigned* count, unsigned* off, uint32_t n_bins);
+template <bool MULTI>
+__global__ void k_sort_scatter(SceneDev S, TraceBufs B, uint32_t gen, const uint32_t* keys, unsigned* off, uint32_t* order);
 
 __global__ void k_clear_accum(RasterArgs A);
 // An FP64 accumulation image rounded to FP32 (n values).

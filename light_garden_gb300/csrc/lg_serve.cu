@@ -345,7 +345,7 @@ lg_status serve_restart(lg_ctx* c, ServeState& V) {
   V.step = 0;
   ++V.restarts;
   CK(cudaMemsetAsync(c->d_ctr.p, 0, sizeof(Counters), c->stream), "reset counters");
-  CK(cudaMemsetAsync(c->d_scene_count.p, 0, (size_t)V.max_slots * 4, c->stream), "reset scene counts");
+  CK(cudaMemsetAsync(c->d_scene_count.p, 0, (size_t)sort_bins(V.max_slots) * 4, c->stream), "reset sort counts");
   std::memset(c->h_ctr, 0, sizeof(Counters));
   return LG_OK;
 }
@@ -393,10 +393,9 @@ lg_status lg_serve_begin(lg_ctx* c, const lg_serve_opts* opts) {
   if ((st = ensure(c, V->d_acc, px * 32, "accumulation pool"))) { serve_free(c); return st; }
   if ((st = ensure(c, V->d_res, px * 8, "result pool"))) { serve_free(c); return st; }
   if ((st = ensure(c, V->d_live, (size_t)V->max_slots * 4, "live counts"))) { serve_free(c); return st; }
-  if ((st = ensure(c, c->d_scene_count, (size_t)V->max_slots * 4, "scene counts"))) { serve_free(c); return st; }
-  if ((st = ensure(c, c->d_scene_off, (size_t)V->max_slots * 4, "scene offsets"))) { serve_free(c); return st; }
+  if ((st = ensure_sort_buffers(c, V->max_slots))) { serve_free(c); return st; }
   CK(cudaMemsetAsync(c->d_ctr.p, 0, sizeof(Counters), c->stream), "reset counters");
-  CK(cudaMemsetAsync(c->d_scene_count.p, 0, (size_t)V->max_slots * 4, c->stream), "reset scene counts");
+  CK(cudaMemsetAsync(c->d_scene_count.p, 0, (size_t)sort_bins(V->max_slots) * 4, c->stream), "reset sort counts");
   std::memset(c->h_ctr, 0, sizeof(Counters));
   // launch shapes of the multi-scene kernels
   int occ = 0;
@@ -543,11 +542,7 @@ lg_status lg_serve_step(lg_ctx* c, lg_serve_step_stats* stats) {
     SL.light_hi = c->n_lights;
     launch_light_setup(c, SL, true);
   }
-  if (V.live > 0) {  // queued rays in scene order
-    k_scene_hist<<<c->n_sm * 8, 256, 0, c->stream>>>(SD, B, g, (unsigned*)c->d_scene_count.p);
-    k_scene_offsets<<<1, 1024, 0, c->stream>>>((unsigned*)c->d_scene_count.p, (unsigned*)c->d_scene_off.p, V.max_slots);
-    k_scene_scatter<<<c->n_sm * 8, 256, 0, c->stream>>>(SD, B, g, (unsigned*)c->d_scene_off.p, (uint32_t*)c->d_order.p);
-  }
+  if (V.live > 0) launch_sort(c, SD, B, g, V.max_slots, true);
   launch_generation(c, SD, B, g, true, c->batch_grid_scan, (size_t)scan_smem_bytes(scan_pairs_of(c)), 0, 0);
   if (!cubic_obj.empty()) {
     lg_string_mod no_sm;

@@ -215,12 +215,13 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, CULL ? SCAN_CULL_BLOCKS : 4)
   const unsigned lane = lane_id(), w = threadIdx.x >> 5;
   const uint64_t warp = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5;
   const uint64_t nwarps = (gridDim.x * (uint64_t)blockDim.x) >> 5;
+  const bool ordered = MULTI || (B.order && sorts<MULTI>(n_real));
   for (uint64_t base = warp * 32; base < n_in; base += nwarps * 32) {
-    // multi-scene launches visit the queued rays in scene order, so that a warp's rays (and
-    // a CTA's warps) share one scene; new primaries follow, ordered by light
+    // queued rays in visiting order (scene, place, direction), so that a warp's rays (and a
+    // CTA's warps) share one scene; new primaries follow, ordered by light
     uint64_t idx = base + lane;
     bool valid = idx < n_in;
-    if (MULTI && valid && idx < n_real) {
+    if (ordered && valid && idx < n_real) {
       idx = B.order[idx];
       valid = idx < n_real;
     }
@@ -951,9 +952,12 @@ template __global__ void k_bounce<false, true>(SceneDev, TraceBufs, uint32_t, in
 template __global__ void k_bounce<true, false>(SceneDev, TraceBufs, uint32_t, int);
 template __global__ void k_bounce<true, true>(SceneDev, TraceBufs, uint32_t, int);
 
-// ------------------------------------------------------------------- scene order
-// Multi-scene generations > 0: a counting sort of the queue entries by scene (histogram,
-// exclusive scan, scatter of entry indices), so that k_scan's warps each see one scene.
+// ------------------------------------------------------------------- visiting order
+// Generations > 0: a counting sort of the queue entries by scene, place and direction (keys and
+// histogram, exclusive scan, scatter of entry indices).  Rays that start in one cell of the canvas
+// in one octant of directions walk the same grid cells to the same few objects, so that a warp's
+// lanes stay together in the scan's walk and leaf code, and through the work lists in the solve, the
+// bounce and the segments' bins.  Bound by memory: the keys read a sector pair of each 80-byte entry.
 __device__ __forceinline__ unsigned long long warp_scene_atomic(unsigned* slot_base, uint32_t s, bool on) {
   const unsigned act = __activemask();
   const unsigned grp = __match_any_sync(act, on ? s : 0xffffffffu);
@@ -965,6 +969,7 @@ __device__ __forceinline__ unsigned long long warp_scene_atomic(unsigned* slot_b
   return base + __popc(grp & lanemask_lt());
 }
 
+// queued rays per scene
 __global__ void k_scene_hist(SceneDev S, TraceBufs B, uint32_t gen, unsigned* count) {
   const uint64_t n = n_real_of(S, B, gen);
   const RayRec* q = B.queue[gen & 1];
@@ -974,17 +979,44 @@ __global__ void k_scene_hist(SceneDev S, TraceBufs B, uint32_t gen, unsigned* co
   }
 }
 
-// single CTA: off = exclusive scan of count; count is cleared for the next generation
-__global__ void __launch_bounds__(1024) k_scene_offsets(unsigned* count, unsigned* off, uint32_t n_scenes) {
+// The lowest `bits` bits (0, or 3 + 2 k: an octant of directions and 2^k x 2^k cells of the
+// canvas; a start outside it counts to the nearest cell).  Any value serves: it only orders.
+__device__ __forceinline__ uint32_t place_key(float ox, float oy, float dx, float dy, float aspect, uint32_t bits) {
+  if (bits < 3) return 0;
+  const uint32_t k = (bits - 3) >> 1;
+  const int n = 1 << k;
+  const int cx = min(max((int)((ox / aspect + 1.0f) * (0.5f * (float)n)), 0), n - 1);
+  const int cy = min(max((int)((oy + 1.0f) * (0.5f * (float)n)), 0), n - 1);
+  const uint32_t oct = (dx > 0.0f ? 1u : 0u) | (dy > 0.0f ? 2u : 0u) | (fabsf(dx) > fabsf(dy) ? 4u : 0u);
+  return (uint32_t)((cy << k) + cx) * 8u + oct;
+}
+
+// A double's value as a float, truncated (on the integer pipe: a conversion would issue on the
+// FP64 pipe); beyond FP32's range or NaN some large value, below it zero.
+__device__ __forceinline__ float rough(uint32_t hi) {
+  const int e = (int)((hi >> 20) & 0x7ffu) - 896;
+  const uint32_t m = e <= 0 ? 0u : e >= 255 ? 0x7f000000u : ((uint32_t)e << 23) | ((hi & 0xfffffu) << 3);
+  return __uint_as_float((hi & 0x80000000u) | m);
+}
+
+// Single CTA: off = exclusive scan of count, 16 bins a thread at a time; count is cleared for the
+// next generation.  Both hold a multiple of 16 bins.  (Done by the last CTA of k_sort_keys instead,
+// the fences and the larger CTAs cost more than the launch: small frames 1 to 1.5 % slower.)
+template <bool MULTI>
+__global__ void __launch_bounds__(1024) k_sort_offsets(SceneDev S, TraceBufs B, uint32_t gen, unsigned* count, unsigned* off,
+                                                       uint32_t n_bins) {
+  if (!sorts<MULTI>(n_real_of(S, B, gen))) return;
   __shared__ unsigned wsum[32];
-  __shared__ unsigned carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
   const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
-  for (uint32_t base = 0; base < n_scenes; base += blockDim.x) {
-    const uint32_t i = base + threadIdx.x;
-    const unsigned c = i < n_scenes ? count[i] : 0u;
-    unsigned incl = c;
+  unsigned carry = 0;
+  for (uint32_t base = 0; base < n_bins; base += 16 * blockDim.x) {
+    const uint32_t i = base + 16 * threadIdx.x;
+    uint4 c[4] = {};
+    if (i < n_bins)
+      for (int k = 0; k < 4; ++k) c[k] = reinterpret_cast<const uint4*>(count + i)[k];
+    unsigned sum = 0;
+    for (int k = 0; k < 4; ++k) sum += c[k].x + c[k].y + c[k].z + c[k].w;
+    unsigned incl = sum;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
@@ -993,7 +1025,7 @@ __global__ void __launch_bounds__(1024) k_scene_offsets(unsigned* count, unsigne
     if (lane == 31) wsum[wid] = incl;
     __syncthreads();
     if (wid == 0) {
-      unsigned sw = lane < (blockDim.x >> 5) ? wsum[lane] : 0u;
+      unsigned sw = wsum[lane];
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
         const unsigned y = __shfl_up_sync(0xffffffffu, sw, o);
@@ -1002,28 +1034,62 @@ __global__ void __launch_bounds__(1024) k_scene_offsets(unsigned* count, unsigne
       wsum[lane] = sw;
     }
     __syncthreads();
-    const unsigned cr = carry;
-    const unsigned excl = cr + (wid ? wsum[wid - 1] : 0u) + incl - c;
-    if (i < n_scenes) {
-      off[i] = excl;
-      count[i] = 0u;
-    }
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry = excl + c;
-    __syncthreads();
+    unsigned at = carry + (wid ? wsum[wid - 1] : 0u) + incl - sum;
+    carry += wsum[31];
+    if (i < n_bins)
+      for (int k = 0; k < 4; ++k) {
+        uint4 v;
+        v.x = at; at += c[k].x;
+        v.y = at; at += c[k].y;
+        v.z = at; at += c[k].z;
+        v.w = at; at += c[k].w;
+        reinterpret_cast<uint4*>(off + i)[k] = v;
+        reinterpret_cast<uint4*>(count + i)[k] = make_uint4(0u, 0u, 0u, 0u);
+      }
+    __syncthreads();  // wsum is read before the next pass writes it
   }
 }
 
-__global__ void k_scene_scatter(SceneDev S, TraceBufs B, uint32_t gen, unsigned* off, uint32_t* order) {
+template <bool MULTI, bool EXACT>
+__global__ void k_sort_keys(SceneDev S, TraceBufs B, uint32_t gen, uint32_t bits, uint32_t* keys, unsigned* count) {
   const uint64_t n = n_real_of(S, B, gen);
+  if (!sorts<MULTI>(n)) return;
   const RayRec* q = B.queue[gen & 1];
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t s = q[i].scene;
+    const uint4 o = reinterpret_cast<const uint4*>(q + i)[0], d = reinterpret_cast<const uint4*>(q + i)[1];
+    const uint32_t s = MULTI ? q[i].scene : 0u;
     const bool on = s < S.n_scenes;
-    const unsigned long long pos = warp_scene_atomic(off, s, on);
+    // the leading part of a double-float, or of a double
+    auto lead = [](uint32_t lo, uint32_t hi) { return EXACT ? rough(hi) : __uint_as_float(lo); };
+    uint32_t key = 0;
+    if (on)
+      key = (s << bits) + place_key(lead(o.x, o.y), lead(o.z, o.w), lead(d.x, d.y), lead(d.z, d.w),
+                                    scene_of<MULTI>(S, s).aspect.hi, bits);
+    keys[i] = on ? key : 0xffffffffu;
+    warp_scene_atomic(count, key, on);
+  }
+}
+template __global__ void k_sort_keys<false, false>(SceneDev, TraceBufs, uint32_t, uint32_t, uint32_t*, unsigned*);
+template __global__ void k_sort_keys<false, true>(SceneDev, TraceBufs, uint32_t, uint32_t, uint32_t*, unsigned*);
+template __global__ void k_sort_keys<true, false>(SceneDev, TraceBufs, uint32_t, uint32_t, uint32_t*, unsigned*);
+template __global__ void k_sort_keys<true, true>(SceneDev, TraceBufs, uint32_t, uint32_t, uint32_t*, unsigned*);
+
+template __global__ void k_sort_offsets<false>(SceneDev, TraceBufs, uint32_t, unsigned*, unsigned*, uint32_t);
+template __global__ void k_sort_offsets<true>(SceneDev, TraceBufs, uint32_t, unsigned*, unsigned*, uint32_t);
+
+template <bool MULTI>
+__global__ void k_sort_scatter(SceneDev S, TraceBufs B, uint32_t gen, const uint32_t* keys, unsigned* off, uint32_t* order) {
+  const uint64_t n = n_real_of(S, B, gen);
+  if (!sorts<MULTI>(n)) return;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t key = keys[i];
+    const bool on = key != 0xffffffffu;
+    const unsigned long long pos = warp_scene_atomic(off, key, on);
     if (on && pos < n) order[pos] = (uint32_t)i;
   }
 }
+template __global__ void k_sort_scatter<false>(SceneDev, TraceBufs, uint32_t, const uint32_t*, unsigned*, uint32_t*);
+template __global__ void k_sort_scatter<true>(SceneDev, TraceBufs, uint32_t, const uint32_t*, unsigned*, uint32_t*);
 
 // ------------------------------------------------------------------- overlays
 // A point of the string-mod curve (string_mod.rs:33-85), the same FP64 operations as the

@@ -132,6 +132,13 @@ __device__ __forceinline__ uint64_t n_real_of(const SceneDev& S, const TraceBufs
   const unsigned long long n = B.ctr->queue_count[gen];
   return n < B.queue_cap ? n : B.queue_cap;
 }
+// Whether a generation of n queued rays visits them in sorted order: with several scenes always, for
+// one from 32768 rays (16384 and 131072 are within 1 % on large frames; the last is late for mixed
+// shapes: 64 objects, 32768 primaries 0.98 of the unsorted speed against 1.14).
+template <bool MULTI>
+__device__ __forceinline__ bool sorts(uint64_t n) {
+  return MULTI || n >= 32768;
+}
 // ... and primaries it generates (virtual queue entries after the queued ones)
 __device__ __forceinline__ uint64_t n_new_of(const SceneDev& S, uint32_t gen) {
   return S.serve ? S.n_new : (gen == 0 ? S.n_primary : 0);
