@@ -1410,8 +1410,12 @@ lg_status lg_scene_upload(lg_ctx* c, const lg_geo* geos, uint32_t n_geo, const l
   c->n_prog = (uint32_t)F.prog.size();
   c->n_lights = n_lights;
   c->n_cubic = (uint32_t)F.cubics.size();
-  c->n_primary = 0;
-  for (uint32_t l = 0; l < n_lights; ++l) c->n_primary += sampled_rays(lights[l].num_rays, p);
+  uint64_t n_primary = 0;
+  for (uint32_t l = 0; l < n_lights; ++l) n_primary += sampled_rays(lights[l].num_rays, p);
+  if (c->n_primary != n_primary) {  // the captured launches hold the count
+    c->n_primary = n_primary;
+    c->graph_valid = false;
+  }
   const bool small = small_frame(c, p, F.xnode.size());
   if (c->small != small) {
     c->small = small;
