@@ -821,14 +821,16 @@ TraceKernel scan_kernel(bool multi, bool culled, bool exact, int pairs) {
   return pairs <= 8 ? scan_kernel_ch<8>(multi, culled, exact) : scan_kernel_ch<16>(multi, culled, exact);
 }
 
-// Bits of place and direction in the sort key (see place_key).  Finer cells pay once they hold
-// several rays each: a CSG frame of 131072 primaries takes 47.6 ms with 13 bits, 46.4 with 15 and 47.3
-// with 17 (the scan of the bins), of 786432 256.9, 246.0 and 242.2; a 64-scene batch (17 bits in all)
-// 93.5 ms in scene order alone and 76.5 with 11 bits of place.  At most 2^17 bins.
-static uint32_t sort_bits(const lg_ctx* c, uint32_t n_scenes) {
-  uint32_t bits = c->n_primary < (1u << 17) ? 13 : c->n_primary < (1u << 19) ? 15 : 17;
-  if (n_scenes > 1) bits = 13;
-  while (bits >= 3 && ((uint64_t)n_scenes << bits) > (1u << 17)) bits -= 2;
+// Bits of place and direction in the sort key (see place_key), for a frame of so many primaries (or
+// a step of so many queued rays).  Finer cells pay once a generation fills them, else the scan of
+// the bins costs more: at least 2.5 rays a bin, at most 2^17 bins.  A CSG frame of 131072 primaries
+// takes 47.6 ms with 13 bits, 46.4 with 15 and 47.3 with 17, of 786432 256.9, 246.0 and 242.2; the trace
+// of a 64-scene batch of 664537 primaries 73.4 ms in scene order, 64.4 with 7, 60.1 with 9, 56.6 with
+// 11; of 83068 primaries 17.0, 15.8, 15.5 and 16.2.
+static uint32_t sort_bits(uint32_t n_scenes, uint64_t rays) {
+  const uint64_t limit = std::min<uint64_t>(1u << 17, rays * 2 / 5);
+  uint32_t bits = 17;
+  while (bits >= 3 && ((uint64_t)n_scenes << bits) > limit) bits -= 2;
   return bits >= 3 ? bits : 0;
 }
 // Room for the bins of any of these, a multiple of what k_sort_offsets takes at a time.
@@ -841,8 +843,9 @@ lg_status ensure_sort_buffers(lg_ctx* c, uint32_t n_scenes) {
 
 // The visiting order of a generation's queued rays into B.order.  The keys lie in a work list's
 // space, which the scan fills afterwards.
-void launch_sort(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_t g, uint32_t n_scenes, bool multi) {
-  const uint32_t bits = sort_bits(c, n_scenes);
+void launch_sort(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_t g, uint32_t n_scenes, uint64_t rays,
+                 bool multi) {
+  const uint32_t bits = sort_bits(n_scenes, rays);
   const bool exact = c->prm.precision == LG_PRECISION_EXACT;
   unsigned *count = (unsigned*)c->d_scene_count.p, *off = (unsigned*)c->d_scene_off.p;
   uint32_t *keys = B.list[0], *order = (uint32_t*)B.order;
@@ -946,7 +949,7 @@ void launch_generation(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_
     else k_small_x<false><<<c->n_sm * 4, SMALL_THREADS, tsm, c->stream>>>(S, B, g, smem_fits);
     return;
   }
-  if (!multi && B.order && g > 0) launch_sort(c, S, B, g, 1, false);
+  if (!multi && B.order && g > 0) launch_sort(c, S, B, g, 1, c->n_primary, false);
   scan_kernel(multi, c->scan_walk, exact, scan_pairs_of(c))<<<scan_grid, SCAN_THREADS, scan_smem, c->stream>>>(S, B, g,
                                                                                                    smem_fits);
   if (exact) {

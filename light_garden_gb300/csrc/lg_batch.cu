@@ -90,7 +90,7 @@ lg_status enqueue_batch(lg_ctx* c, cudaEvent_t* ev) {
   lg_string_mod no_sm;
   std::memset(&no_sm, 0, sizeof no_sm);
   for (uint32_t g = 0; g < c->max_bounce_all; ++g) {
-    if (g > 0) launch_sort(c, S, B, g, c->n_scenes, true);
+    if (g > 0) launch_sort(c, S, B, g, c->n_scenes, c->n_primary, true);
     launch_generation(c, S, B, g, true, c->batch_grid_scan, (size_t)scan_smem_bytes(scan_pairs_of(c)), 0, 0);
     if (g == 0 && c->n_cubic) {
       const int blocks = (int)std::min<uint64_t>((3ull * c->n_cubic + 255) / 256, 4096);

@@ -133,7 +133,7 @@ void launch_light_setup(lg_ctx* c, const SceneDev& S, bool multi);
 // Visiting order of queued rays (a counting sort by scene, place and direction).
 uint32_t sort_bins(uint32_t n_scenes);
 lg_status ensure_sort_buffers(lg_ctx* c, uint32_t n_scenes);
-void launch_sort(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_t g, uint32_t n_scenes, bool multi);
+void launch_sort(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_t g, uint32_t n_scenes, uint64_t rays, bool multi);
 void launch_generation(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_t g, bool multi, int scan_grid,
                        size_t scan_smem, size_t tsm, int smem_fits);
 // Uploads a flattened scene's exact-mode tables (geometry nodes, preorder trees).

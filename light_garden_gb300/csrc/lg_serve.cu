@@ -542,7 +542,13 @@ lg_status lg_serve_step(lg_ctx* c, lg_serve_step_stats* stats) {
     SL.light_hi = c->n_lights;
     launch_light_setup(c, SL, true);
   }
-  if (V.live > 0) launch_sort(c, SD, B, g, V.max_slots, true);
+  if (V.live > 0) {  // the queued rays' scenes hold the active slots
+    SceneDev SU = SD;
+    SU.n_scenes = 0;
+    for (uint32_t s = 0; s < V.max_slots; ++s)
+      if (V.slots[s].active) SU.n_scenes = s + 1;
+    if (SU.n_scenes) launch_sort(c, SU, B, g, SU.n_scenes, V.live, true);
+  }
   launch_generation(c, SD, B, g, true, c->batch_grid_scan, (size_t)scan_smem_bytes(scan_pairs_of(c)), 0, 0);
   if (!cubic_obj.empty()) {
     lg_string_mod no_sm;
