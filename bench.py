@@ -62,14 +62,14 @@ REF_STRIDE = {"csg": 2048, "mid": 32}
 #   bounce: FP64 thread instructions per ray visit
 #   raster: shared-memory atomic warp instructions per accumulated pixel
 INST_PER_UNIT = {
-    "csg": {"scan": 631.1, "solve": 80.2, "bounce": 71.7, "raster": 0.2805},
-    "mid": {"scan": 952.3, "solve": 67.4, "bounce": 55.9, "raster": 0.3005},
+    "csg": {"scan": 538.7, "solve": 55.3, "bounce": 28.3, "raster": 0.4011},
+    "mid": {"scan": 203.4, "solve": 36.6, "bounce": 23.2, "raster": 0.3477},
 }
 # Warp instructions issued (smsp__inst_executed.sum) per unit of the same frames: the trace
 # stages against the SM's issue ceiling (4 schedulers x 1 warp instruction per cycle per SM).
 WARP_INST_PER_UNIT = {
-    "csg": {"scan": 323.2, "solve": 52.0, "bounce": 75.2},
-    "mid": {"scan": 270.3, "solve": 66.2, "bounce": 49.8},
+    "csg": {"scan": 164.3, "solve": 20.8, "bounce": 49.7},
+    "mid": {"scan": 92.0, "solve": 30.0, "bounce": 33.9},
 }
 
 
@@ -435,7 +435,7 @@ def batch_bench(local, args, ray_scale=None):
         pk_f.params.precision = PRECISION[args.precision]
         for pk, acc in ((pk_s, "s"), (pk_f, "f")):  # same canvases: `big` holds either
             plain.upload(pk)
-            for _ in range(2):  # graph capture, then the scan autotune of the scene's second render
+            for _ in range(2):  # graph capture, then once more where a buffer grew
                 plain.render_into(big.data_ptr(), pk.params.width * 8, True)
             torch.cuda.synchronize()
             a = time.perf_counter()
@@ -547,7 +547,7 @@ def serve_bench(local, args, rate=100.0, count=256, ray_scale=1.0 / 16):
 
 def count_case(args):
     """One frame of a small case of the workload (csg: 2^18 rays at 1024^2; mid: 2^14 rays per
-    light), no autotuning, printing the frame's units of work.  Run under ncu with instruction
+    light), printing the frame's units of work.  Run under ncu with instruction
     counters, it gives the instructions per unit of INST_PER_UNIT."""
     from light_garden_gb300 import workloads as W
     from light_garden_gb300.runtime import Context
@@ -670,6 +670,8 @@ def run_ours(args, ws, rank, local):
     # light setup, 3 trace kernels per generation, overlay, accumulation clear, resolve, string-mod lines
     G = pk.params.max_bounce
     launches = 1 + 3 * G + 1 + 1 + 1 + (1 if pk.params.string_mod.modulo else 0)
+    if args.culling != "off" and pk.n_objects >= 48 and st["primary_rays"] * pk.n_objects >= 3 << 20:
+        launches += 3 * (G - 1)  # the rays' order: keys, scan, scatter
     if st["segments"] > (1 << 28):  # the frame streams: per generation decide, clear, count, scan, units, scatter, raster, rotate
         launches += 8 * G
     else:  # one accumulation: count, tile scan, units, scatter, raster
