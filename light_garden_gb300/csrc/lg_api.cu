@@ -833,7 +833,7 @@ static uint32_t sort_bits(uint32_t n_scenes, uint64_t rays) {
   while (bits >= 3 && ((uint64_t)n_scenes << bits) > limit) bits -= 2;
   return bits >= 3 ? bits : 0;
 }
-// Room for the bins of any of these, a multiple of what k_sort_offsets takes at a time.
+// Room for the bins of any of these, a multiple of what a thread of k_sort_offsets takes.
 uint32_t sort_bins(uint32_t n_scenes) { return n_scenes <= 1 ? 1u << 17 : std::max(1u << 17, (n_scenes + 15u) & ~15u); }
 
 lg_status ensure_sort_buffers(lg_ctx* c, uint32_t n_scenes) {
@@ -852,9 +852,11 @@ void launch_sort(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_t g, u
   auto k = multi ? (exact ? k_sort_keys<true, true> : k_sort_keys<true, false>)
                  : (exact ? k_sort_keys<false, true> : k_sort_keys<false, false>);
   k<<<c->n_sm * 8, 256, 0, c->stream>>>(S, B, g, bits, keys, count);
-  (multi ? k_sort_offsets<true> : k_sort_offsets<false>)<<<1, 1024, 0, c->stream>>>(S, B, g, count, off,
-                                                                                   ((n_scenes << bits) + 15u) & ~15u);
-  (multi ? k_sort_scatter<true> : k_sort_scatter<false>)<<<c->n_sm * 8, 256, 0, c->stream>>>(S, B, g, keys, off, order);
+  const uint32_t bins = ((n_scenes << bits) + 15u) & ~15u;
+  (multi ? k_sort_offsets<true> : k_sort_offsets<false>)<<<(bins + SORT_CTA_BINS - 1) / SORT_CTA_BINS, 1024, 0, c->stream>>>(
+      S, B, g, count, off, bins);
+  (multi ? k_sort_scatter<true> : k_sort_scatter<false>)<<<c->n_sm * 8, 256, 0, c->stream>>>(S, B, g, keys, off, order,
+                                                                                            count, bins);
 }
 
 // Whether one scene's generations visit their rays in sorted order.  Three launches and the keys

@@ -109,10 +109,12 @@ __global__ void k_overlay(SceneDev S, TraceBufs B, const uint32_t* cubic_objs, c
 __global__ void k_scene_hist(SceneDev S, TraceBufs B, uint32_t gen, unsigned* count);
 template <bool MULTI, bool EXACT>
 __global__ void k_sort_keys(SceneDev S, TraceBufs B, uint32_t gen, uint32_t bits, uint32_t* keys, unsigned* count);
+constexpr uint32_t SORT_CTA_BINS = 16 * 1024;  // bins of a k_sort_offsets CTA (1024 threads)
 template <bool MULTI>
-__global__ void k_sort_offsets(SceneDev S, TraceBufs B, uint32_t gen, unsigned* count, unsigned* off, uint32_t n_bins);
+__global__ void k_sort_offsets(SceneDev S, TraceBufs B, uint32_t gen, const unsigned* count, unsigned* off, uint32_t n_bins);
 template <bool MULTI>
-__global__ void k_sort_scatter(SceneDev S, TraceBufs B, uint32_t gen, const uint32_t* keys, unsigned* off, uint32_t* order);
+__global__ void k_sort_scatter(SceneDev S, TraceBufs B, uint32_t gen, const uint32_t* keys, unsigned* off, uint32_t* order,
+                               unsigned* count, uint32_t n_bins);
 
 __global__ void k_clear_accum(RasterArgs A);
 // An FP64 accumulation image rounded to FP32 (n values).

@@ -1023,57 +1023,6 @@ __device__ __forceinline__ float rough(uint32_t hi) {
   return __uint_as_float((hi & 0x80000000u) | m);
 }
 
-// Single CTA: off = exclusive scan of count, 16 bins a thread at a time; count is cleared for the
-// next generation.  Both hold a multiple of 16 bins.  (Done by the last CTA of k_sort_keys instead,
-// the fences and the larger CTAs cost more than the launch: small frames 1 to 1.5 % slower.)
-template <bool MULTI>
-__global__ void __launch_bounds__(1024) k_sort_offsets(SceneDev S, TraceBufs B, uint32_t gen, unsigned* count, unsigned* off,
-                                                       uint32_t n_bins) {
-  if (!sorts<MULTI>(n_real_of(S, B, gen))) return;
-  __shared__ unsigned wsum[32];
-  const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
-  unsigned carry = 0;
-  for (uint32_t base = 0; base < n_bins; base += 16 * blockDim.x) {
-    const uint32_t i = base + 16 * threadIdx.x;
-    uint4 c[4] = {};
-    if (i < n_bins)
-      for (int k = 0; k < 4; ++k) c[k] = reinterpret_cast<const uint4*>(count + i)[k];
-    unsigned sum = 0;
-    for (int k = 0; k < 4; ++k) sum += c[k].x + c[k].y + c[k].z + c[k].w;
-    unsigned incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
-      if ((int)lane >= o) incl += y;
-    }
-    if (lane == 31) wsum[wid] = incl;
-    __syncthreads();
-    if (wid == 0) {
-      unsigned sw = wsum[lane];
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned y = __shfl_up_sync(0xffffffffu, sw, o);
-        if ((int)lane >= o) sw += y;
-      }
-      wsum[lane] = sw;
-    }
-    __syncthreads();
-    unsigned at = carry + (wid ? wsum[wid - 1] : 0u) + incl - sum;
-    carry += wsum[31];
-    if (i < n_bins)
-      for (int k = 0; k < 4; ++k) {
-        uint4 v;
-        v.x = at; at += c[k].x;
-        v.y = at; at += c[k].y;
-        v.z = at; at += c[k].z;
-        v.w = at; at += c[k].w;
-        reinterpret_cast<uint4*>(off + i)[k] = v;
-        reinterpret_cast<uint4*>(count + i)[k] = make_uint4(0u, 0u, 0u, 0u);
-      }
-    __syncthreads();  // wsum is read before the next pass writes it
-  }
-}
-
 template <bool MULTI, bool EXACT>
 __global__ void k_sort_keys(SceneDev S, TraceBufs B, uint32_t gen, uint32_t bits, uint32_t* keys, unsigned* count) {
   const uint64_t n = n_real_of(S, B, gen);
@@ -1098,13 +1047,60 @@ template __global__ void k_sort_keys<false, true>(SceneDev, TraceBufs, uint32_t,
 template __global__ void k_sort_keys<true, false>(SceneDev, TraceBufs, uint32_t, uint32_t, uint32_t*, unsigned*);
 template __global__ void k_sort_keys<true, true>(SceneDev, TraceBufs, uint32_t, uint32_t, uint32_t*, unsigned*);
 
-template __global__ void k_sort_offsets<false>(SceneDev, TraceBufs, uint32_t, unsigned*, unsigned*, uint32_t);
-template __global__ void k_sort_offsets<true>(SceneDev, TraceBufs, uint32_t, unsigned*, unsigned*, uint32_t);
-
+// off = exclusive scan of count, 16384 bins a CTA; both hold a multiple of 16 bins.  A CTA sums the
+// bins before its own itself: eight CTAs read 1.8 MB of L2 in all, where one CTA that walked 2^17
+// bins took 47 us a generation (a 64-scene batch 73.1 -> 72.3 ms).  (Done by the last CTA of
+// k_sort_keys instead, the fences and the larger CTAs cost more than the launch.)
 template <bool MULTI>
-__global__ void k_sort_scatter(SceneDev S, TraceBufs B, uint32_t gen, const uint32_t* keys, unsigned* off, uint32_t* order) {
+__global__ void __launch_bounds__(1024) k_sort_offsets(SceneDev S, TraceBufs B, uint32_t gen, const unsigned* count,
+                                                       unsigned* off, uint32_t n_bins) {
+  if (!sorts<MULTI>(n_real_of(S, B, gen))) return;
+  __shared__ unsigned wsum[32], wbefore[32];
+  const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
+  const uint32_t first = blockIdx.x * SORT_CTA_BINS, i = first + 16 * threadIdx.x;
+  unsigned before = 0;
+  for (uint32_t j = 4 * threadIdx.x; j < first; j += 4 * blockDim.x) {
+    const uint4 v = *reinterpret_cast<const uint4*>(count + j);
+    before += v.x + v.y + v.z + v.w;
+  }
+  uint4 c[4] = {};
+  if (i < n_bins)
+    for (int k = 0; k < 4; ++k) c[k] = reinterpret_cast<const uint4*>(count + i)[k];
+  unsigned sum = 0;
+  for (int k = 0; k < 4; ++k) sum += c[k].x + c[k].y + c[k].z + c[k].w;
+  before = __reduce_add_sync(0xffffffffu, before);
+  unsigned incl = sum;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+    if ((int)lane >= o) incl += y;
+  }
+  if (lane == 31) wsum[wid] = incl;
+  if (lane == 0) wbefore[wid] = before;
+  __syncthreads();
+  const unsigned w = wsum[lane];
+  unsigned at = __reduce_add_sync(0xffffffffu, wbefore[lane] + (lane < wid ? w : 0u)) + incl - sum;
+  if (i >= n_bins) return;
+  for (int k = 0; k < 4; ++k) {
+    uint4 v;
+    v.x = at; at += c[k].x;
+    v.y = at; at += c[k].y;
+    v.z = at; at += c[k].z;
+    v.w = at; at += c[k].w;
+    reinterpret_cast<uint4*>(off + i)[k] = v;
+  }
+}
+template __global__ void k_sort_offsets<false>(SceneDev, TraceBufs, uint32_t, const unsigned*, unsigned*, uint32_t);
+template __global__ void k_sort_offsets<true>(SceneDev, TraceBufs, uint32_t, const unsigned*, unsigned*, uint32_t);
+
+// the entries' indices in sorted order; clears the histogram for the next generation
+template <bool MULTI>
+__global__ void k_sort_scatter(SceneDev S, TraceBufs B, uint32_t gen, const uint32_t* keys, unsigned* off, uint32_t* order,
+                               unsigned* count, uint32_t n_bins) {
   const uint64_t n = n_real_of(S, B, gen);
   if (!sorts<MULTI>(n)) return;
+  for (uint32_t i = 4 * (blockIdx.x * blockDim.x + threadIdx.x); i < n_bins; i += 4 * gridDim.x * blockDim.x)
+    *reinterpret_cast<uint4*>(count + i) = make_uint4(0u, 0u, 0u, 0u);
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
     const uint32_t key = keys[i];
     const bool on = key != 0xffffffffu;
@@ -1112,8 +1108,10 @@ __global__ void k_sort_scatter(SceneDev S, TraceBufs B, uint32_t gen, const uint
     if (on && pos < n) order[pos] = (uint32_t)i;
   }
 }
-template __global__ void k_sort_scatter<false>(SceneDev, TraceBufs, uint32_t, const uint32_t*, unsigned*, uint32_t*);
-template __global__ void k_sort_scatter<true>(SceneDev, TraceBufs, uint32_t, const uint32_t*, unsigned*, uint32_t*);
+template __global__ void k_sort_scatter<false>(SceneDev, TraceBufs, uint32_t, const uint32_t*, unsigned*, uint32_t*,
+                                               unsigned*, uint32_t);
+template __global__ void k_sort_scatter<true>(SceneDev, TraceBufs, uint32_t, const uint32_t*, unsigned*, uint32_t*,
+                                              unsigned*, uint32_t);
 
 // ------------------------------------------------------------------- overlays
 // A point of the string-mod curve (string_mod.rs:33-85), the same FP64 operations as the
