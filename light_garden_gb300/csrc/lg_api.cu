@@ -23,6 +23,11 @@ namespace lgh {
 struct Xf {
   double ox, oy, c, s;  // world = (ox, oy) + R(c, s) * local
   void apply(double x, double y, double& wx, double& wy) const {
+    if (ox == 0.0 && oy == 0.0 && c == 1.0 && s == 0.0) {  // as it is: a sum would lose the sign of -0.0
+      wx = x;
+      wy = y;
+      return;
+    }
     wx = ox + c * x - s * y;
     wy = oy + s * x + c * y;
   }
