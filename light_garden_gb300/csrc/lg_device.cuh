@@ -860,9 +860,17 @@ __device__ __forceinline__ int cubic_roots32(const float* A, const float* Bp, fl
   const float a0 = dx * (c0y - oy) - dy * (c0x - ox);
   const float a1 = dx * c1y - dy * c1x, a2 = dx * c2y - dy * c2x, a3 = dx * c3y - dy * c3x;
   const float sc = fabsf(a0) + fabsf(a1) + fabsf(a2) + fabsf(a3) + 1e-30f;
-  // |f| below this is not decided: the control points' rounding to FP32 moves f by at most
-  // 27 2^-24 |P| sqrt(2) (the power basis weighs them 1, 6, 12, 8), the evaluation by some 10 2^-24 sc
-  const float err = 1e-5f * sc + 4e-6f * (fabsf(c0x) + fabsf(c0y) + fabsf(ox) + fabsf(oy));
+  // |f| below this is not decided.  With M the largest control coordinate and u = 2^-24: the control
+  // points' rounding moves B(s) by at most u M a coordinate (a convex combination), the power basis
+  // (weights 1, 6, 12, 8) is formed to within 72 u M a coordinate and crossed with d to within 26 u M,
+  // 130 u M = 7.8e-6 M in all; the origin adds 4 u of its coordinates, the evaluation some 10 u sc.  A
+  // curve that starts at the canvas centre has M of its far end: with the first control point in M's
+  // place, 8 % of the rays within 3e-8 of the far end of a flat one, from beside its start, were certain
+  // misses or hits on the wrong side.
+  float M = fmaxf(fabsf(Bp[0]), fabsf(Bp[1]));
+#pragma unroll
+  for (int k = 0; k < 6; ++k) M = fmaxf(M, fabsf(A[k]));
+  const float err = 1e-5f * sc + 8e-6f * M + 4e-6f * (fabsf(ox) + fabsf(oy));
   auto f = [&](float u) { return ((a3 * u + a2) * u + a1) * u + a0; };
   float knots[4];
   int nk = 0;
@@ -933,7 +941,7 @@ __device__ __forceinline__ int cubic_roots32(const float* A, const float* Bp, fl
 // distances (`scale`), and those of the origin's and the leaf's coordinates to FP32, 2^-24 of each
 // coordinate however near the two lie (`e`, with room of a factor of six).  Without `e`, of the rays
 // within 0.3 % of tangency to a disc of radius 5e-5 near a canvas corner 1.4 % were certain on the
-// wrong side; with it the headline frame's search takes 0.7 % more time.
+// wrong side; with it the headline frame takes 0.7 % more time.
 struct Ival32 {
   float t0, t1, tol;
   float in0, in1, out0, out1;

@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from light_garden_gb300 import abi
-from light_garden_gb300.scene import Circle, Logic, Material, Object, Rect, SpotLight, pack
+from light_garden_gb300.scene import Circle, CubicBezier, Logic, Material, Object, Rect, SpotLight, pack
 from parity import exact
 
 pytestmark = pytest.mark.gpu
@@ -79,3 +79,21 @@ def test_rects_far_off_grazed(gpu, oracle, size, pairs):
         o = corner + size * rng.uniform(4.0, 40.0) * (y - x) / math.sqrt(2.0)  # across the corner's diagonal
         lights.append(_spot(o, corner, 4e-6))
     _check(oracle, objects, lights, 1600, 100, pairs, 0.2)
+
+
+@pytest.mark.parametrize("pairs", [0, 16])
+@pytest.mark.parametrize("side,bend", [(1e-4, 0.0), (1e-3, 0.0), (1e-3, 1e-7), (1e-3, 1e-5), (1e-2, 1e-7)])
+def test_flat_mirrors_from_the_centre(gpu, oracle, side, bend, pairs):
+    """Nearly straight cubic mirrors that start at the canvas centre, each seen from beside its start
+    along its length, with rays past its far end."""
+    rng = np.random.default_rng(int(1e6 * (side + 7 * bend)))
+    objects, lights = [], []
+    for k in range(10):
+        a = 2.0 * math.pi * (k + rng.uniform(0.4, 0.6)) / 10
+        t, n = np.array([math.cos(a), math.sin(a)]), np.array([-math.sin(a), math.cos(a)])
+        length = rng.uniform(0.5, 0.95)
+        pts = [t * (length * j / 3) + n * (rng.uniform(-1, 1) * bend if j else 0.0) for j in range(4)]
+        objects.append(Object.new_curved_mirror(CubicBezier(tuple(tuple(p) for p in pts))))
+        o = t * (2.0 * side) + n * (rng.choice([-1, 1]) * rng.uniform(0.2, 0.8) * side)  # on this side of its neighbours
+        lights.append(_spot(o, pts[3], 1e-7))
+    _check(oracle, objects, lights, 170, 100, pairs, 0.2)
