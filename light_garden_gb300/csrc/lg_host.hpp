@@ -44,11 +44,15 @@ struct Flat {
   std::vector<lgx::XNode> xnode;
   std::vector<SolveRec> solve;  // one per object
   int xdepth = 0;
-  // appends another scene's exact-mode tables, moving its node indices past this one's;
+  // appends another scene's exact-mode tables, moving its node indices past this one's: those of the
+  // trees, and the next node of a polygon's vertices, which the kernels follow in the joint table;
   // the caller adds the returned base to that scene's ObjInfo::xnode_begin
   uint32_t append_exact(const Flat& o) {
     const uint32_t g0 = (uint32_t)xgeo.size(), n0 = (uint32_t)xnode.size();
-    xgeo.insert(xgeo.end(), o.xgeo.begin(), o.xgeo.end());
+    for (lg_geo g : o.xgeo) {
+      if ((g.kind == LG_GEO_POLYGON || g.kind == LG_GEO_VERTICES) && g.b >= 0) g.b = (int32_t)((uint32_t)g.b + g0);
+      xgeo.push_back(g);
+    }
     for (lgx::XNode n : o.xnode) {
       n.geo += (int32_t)g0;
       xnode.push_back(n);
