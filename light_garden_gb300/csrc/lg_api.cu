@@ -726,6 +726,7 @@ RasterArgs raster_args(lg_ctx* c) {
   A.n_tiles = 2 * c->n_tiles;  // bins: x-major and y-major segments of each tile
   A.unit_refs = raster_unit_refs(raster_mode(c->prm));
   A.acc = accum_kind(c->prm);
+  A.scaled = raster_mode(c->prm) == RM_F32_ ? 1 : 0;
   A.unit_share = 3u * (uint32_t)c->raster_grid;
   for (int ch = 0; ch < 4; ++ch) {
     const lg_blend_component& b = ch < 3 ? c->prm.color_blend : c->prm.alpha_blend;
@@ -1094,8 +1095,9 @@ lg_status enqueue_accumulate(lg_ctx* c, int binned_event = -1) {
   const int acc = accum_kind(c->prm);
   k_clear_accum<<<c->n_sm * 8, 256, 0, c->stream>>>(A);
   CK(cudaMemsetAsync(c->d_tile_count.p, 0, (size_t)c->n_tiles * 8, c->stream), "memset tile counts");
-  // pixels and, right after it, bin_refs
-  CK(cudaMemsetAsync(&((Counters*)c->d_ctr.p)->pixels, 0, 2 * sizeof(unsigned long long), c->stream), "memset pixels");
+  // color_max, pixels and bin_refs lie side by side
+  static_assert(offsetof(Counters, tile_refs) == offsetof(Counters, color_max) + 32, "one memset clears the three");
+  CK(cudaMemsetAsync(((Counters*)c->d_ctr.p)->color_max, 0, 32, c->stream), "memset pixels");
   const uint32_t bins = 2 * c->n_tiles;
   const int smem_tiles = bins <= MAX_SMEM_TILES ? 1 : 0;
   const size_t bsm = smem_tiles ? (size_t)bins * 4 : 0;

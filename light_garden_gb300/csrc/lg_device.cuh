@@ -164,6 +164,9 @@ struct Counters {
   unsigned long long queue_count[MAX_GEN + 1]; // entries demanded per generation
   unsigned long long list_count[MAX_GEN][N_LISTS];
   unsigned long long visits, fp64_solves, fallbacks, near, ill;
+  // FP32 additive sums: the largest finite magnitude of the segments' colours per channel, as float
+  // bits (k_bin_count); it sets the unit of the raster's split sums
+  unsigned int color_max[4];
   unsigned long long pixels, bin_refs;  // pixel updates; (segment, tile) pairs counted by k_bin_count
   unsigned long long tile_refs, units;
   unsigned long long unit_cursor;

@@ -52,6 +52,7 @@ struct RasterArgs {
   uint32_t* cta_hist;
   void* accum;             // H * W * 4 values of the kind acc names
   int32_t acc;             // ACC_*
+  int32_t scaled;          // FP32 additive sums: k_bin_count finds Counters::color_max
   Counters* ctr;
 };
 

@@ -134,6 +134,7 @@ extern "C" lg_status lg_accumulate_segments_noalloc(const lg_segment* segments, 
   A.n_tiles = 2 * n_tiles;  // bins: x-major and y-major segments of each tile
   const int mode = lgh::raster_mode(p);
   A.unit_refs = raster_unit_refs(mode);
+  A.scaled = mode == RM_F32_ ? 1 : 0;
   A.unit_share = 3u * (uint32_t)d->raster_grid[mode];
   for (int ch = 0; ch < 4; ++ch) {
     const lg_blend_component& b = ch < 3 ? p.color_blend : p.alpha_blend;

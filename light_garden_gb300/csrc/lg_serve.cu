@@ -273,6 +273,7 @@ lg_status serve_raster_args(lg_ctx* c, ServeState& V, RasterArgs& A) {
   A.n_scenes = V.max_slots;
   A.accum = V.d_acc.p;
   A.acc = ACC_I64;
+  A.scaled = 0;
   A.W = 0;
   A.H = 0;
   A.n_tiles = c->total_bins;
