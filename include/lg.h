@@ -149,9 +149,9 @@ typedef struct lg_blend_component {
 
 enum lg_accum_mode {
   LG_ACCUM_FIXED64 = 0, /* signed Q31.32 fixed point in int64: order-independent, bit-reproducible */
-  LG_ACCUM_F32 = 1      /* FP32 values: additive sums are kept in FP64 and rounded to FP32 when
-                           the image is read (lg_accumulate_segments_noalloc: FP32 atomics, not
-                           bit-reproducible) */
+  LG_ACCUM_F32 = 1      /* FP32 values: additive sums are kept in FP64 (32 B a pixel, as much as
+                           FIXED64 takes) and rounded to FP32 when the image is read
+                           (lg_accumulate_segments_noalloc: FP32 atomics, not bit-reproducible) */
 };
 
 /* ---- string-mod overlay (src/light_garden/string_mod.rs) ------------------------------- */

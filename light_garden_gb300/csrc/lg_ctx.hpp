@@ -54,6 +54,7 @@ struct lg_ctx {
   uint64_t seg_cap_hint = 0, queue_cap_hint = 0;
   // raster
   DevBuf d_tile_count, d_tile_off, d_tile_cursor, d_unit_off, d_refs, d_units, d_accum, d_stage;
+  DevBuf d_acc32;     // pieces of an FP32 accumulation on their way to the host
   DevBuf d_cta_hist;  // per-CTA bin counts of the shared-memory binning (scatter launch shape)
   uint64_t refs_cap = 0, units_cap = 0;
   uint32_t n_tiles = 0, ntx = 0, nty = 0;
