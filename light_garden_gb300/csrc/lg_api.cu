@@ -656,6 +656,17 @@ lg_status ensure(lg_ctx* c, DevBuf& b, size_t bytes, const char* what) {
   return LG_OK;
 }
 
+// After a growth of the capacities: a failed one leaves buffers missing, or smaller than the
+// capacities that the launches go by, so there is no scene left to trace, and the next upload
+// starts from its first guesses.
+lg_status grown(lg_ctx* c, lg_status st) {
+  if (st) {
+    c->has_scene = c->multi = c->graph_valid = false;
+    c->seg_cap = c->queue_cap = c->refs_cap = 0;
+  }
+  return st;
+}
+
 void release(DevBuf& b) {
   if (b.p) cudaFree(b.p);
   b.p = nullptr;
@@ -1146,8 +1157,8 @@ lg_status grow_trace(lg_ctx* c, uint64_t need_seg, uint64_t need_q) {
   const double want = (double)c->seg_cap * (sizeof(lg_segment) + (c->prm.record_paths ? sizeof(lg_path_record) : 0)) +
                       (double)c->queue_cap * (2 * sizeof(RayRec) + sizeof(ScanRec) + sizeof(HitRec) + 4 * N_LISTS);
   if (want > (double)total_b * 0.9)
-    return fail(c, LG_ERR_OUT_OF_MEMORY, "trace needs " + std::to_string(want / 1e9) + " GB of segment ring and ray queues");
-  return ensure_trace_buffers(c);
+    return grown(c, fail(c, LG_ERR_OUT_OF_MEMORY, "trace needs " + std::to_string(want / 1e9) + " GB of segment ring and ray queues"));
+  return grown(c, ensure_trace_buffers(c));
 }
 
 float elapsed(cudaEvent_t a, cudaEvent_t b) {
@@ -1201,9 +1212,10 @@ lg_status run_accumulate(lg_ctx* c, uint32_t& retries) {
     if (c->h_ctr->tile_refs <= c->refs_cap) return LG_OK;
     ++retries;
     c->refs_cap = c->h_ctr->tile_refs + c->h_ctr->tile_refs / 8 + 4096;
-    if (c->refs_cap >= 0xffffffffull) return fail(c, LG_ERR_UNSUPPORTED, "more than 2^32 (segment, tile) pairs in one frame");
+    if (c->refs_cap >= 0xffffffffull)
+      return grown(c, fail(c, LG_ERR_UNSUPPORTED, "more than 2^32 (segment, tile) pairs in one frame"));
     c->graph_valid = false;
-    if ((st = ensure_raster_buffers(c))) return st;
+    if ((st = grown(c, ensure_raster_buffers(c)))) return st;
   }
   return fail(c, LG_ERR_OUT_OF_MEMORY, "tile reference list kept overflowing");
 }
@@ -1465,9 +1477,9 @@ lg_status lg_scene_upload(lg_ctx* c, const lg_geo* geos, uint32_t n_geo, const l
   const uint64_t want_q = c->queue_cap_hint ? c->queue_cap_hint : 2 * c->n_primary + 1024;
   c->seg_cap = std::max(c->seg_cap, want_seg);
   c->queue_cap = std::max(c->queue_cap, std::max<uint64_t>(want_q, c->n_primary));  // gen 0 stores every primary
-  if ((st = ensure_trace_buffers(c))) return st;
+  if ((st = grown(c, ensure_trace_buffers(c)))) return st;
   c->refs_cap = std::max<uint64_t>(c->refs_cap, 1u << 20);
-  if ((st = ensure_raster_buffers(c))) return st;
+  if ((st = grown(c, ensure_raster_buffers(c)))) return st;
   if ((st = ensure(c, c->d_stage, (size_t)p.width * p.height * 8, "resolve staging"))) return st;
   if (!same_shape) {
     c->graph_valid = false;
@@ -1519,7 +1531,7 @@ lg_status lg_accumulate_segments(lg_ctx* c, const lg_segment* segs, uint64_t n, 
   if (n && !segs) return fail(c, LG_ERR_INVALID_ARGUMENT, "null segments");
   if (n > c->seg_cap) {
     c->seg_cap = n;
-    if ((st = ensure_trace_buffers(c))) return st;
+    if ((st = grown(c, ensure_trace_buffers(c)))) return st;
   }
   if (n) CK(cudaMemcpyAsync(c->d_segs.p, segs, n * sizeof(lg_segment), cudaMemcpyHostToDevice, c->stream), "upload segments");
   Counters* d = (Counters*)c->d_ctr.p;
@@ -1623,11 +1635,11 @@ static lg_status start_streaming(lg_ctx* c) {
     c->bev.assign(2 * MAX_GEN + 2, nullptr);
     for (auto& e : c->bev) CK(cudaEventCreate(&e), "event");
   }
-  lg_status st = ensure_trace_buffers(c);
+  lg_status st = grown(c, ensure_trace_buffers(c));
   if (st) return st;
-  if ((st = ensure_raster_buffers(c))) return st;
+  if ((st = grown(c, ensure_raster_buffers(c)))) return st;
   const size_t parts = (2 * (size_t)c->n_tiles + TILE_SCAN_CHUNK - 1) / TILE_SCAN_CHUNK;
-  return ensure(c, c->d_part, std::max<size_t>(parts, 1) * 16, "tile scan partials");
+  return grown(c, ensure(c, c->d_part, std::max<size_t>(parts, 1) * 16, "tile scan partials"));
 }
 
 static lg_status render_streaming(lg_ctx* c, uint16_t* dst, size_t pitch, int32_t dst_is_device, lg_trace_stats* stats,
@@ -1665,10 +1677,11 @@ static lg_status render_streaming(lg_ctx* c, uint16_t* dst, size_t pitch, int32_
       if (nq > c->queue_cap) c->queue_cap = nq + nq / 2 + 1024;
       c->seg_cap = std::max<uint64_t>(c->seg_cap, c->queue_cap + 3ull * c->n_cubic + 1024);
       if (k.refs_max > c->refs_cap) c->refs_cap = k.refs_max + k.refs_max / 4 + 4096;
-      if (c->refs_cap >= 0xffffffffull) return fail(c, LG_ERR_UNSUPPORTED, "more than 2^32 (segment, tile) pairs in one pass");
-      lg_status st = ensure_trace_buffers(c);
+      if (c->refs_cap >= 0xffffffffull)
+        return grown(c, fail(c, LG_ERR_UNSUPPORTED, "more than 2^32 (segment, tile) pairs in one pass"));
+      lg_status st = grown(c, ensure_trace_buffers(c));
       if (st) return st;
-      if ((st = ensure_raster_buffers(c))) return st;
+      if ((st = grown(c, ensure_raster_buffers(c)))) return st;
       continue;
     }
     CK(cudaMemcpy2DAsync(dst, pitch, c->d_stage.p, row, row, c->prm.height,
@@ -1744,7 +1757,7 @@ lg_status lg_render(lg_ctx* c, uint16_t* dst, size_t pitch, int32_t dst_is_devic
         const double refs = 1.125 * (double)c->h_ctr->tile_refs * (double)ns / (double)c->seg_cap + 4096.0;
         if (refs < 4294967040.0 && (uint64_t)refs > c->refs_cap) {
           c->refs_cap = (uint64_t)refs;
-          if ((st = ensure_raster_buffers(c))) return st;
+          if ((st = grown(c, ensure_raster_buffers(c)))) return st;
         }
       }
       if ((st = grow_trace(c, ns, nq))) return st;
@@ -1757,7 +1770,7 @@ lg_status lg_render(lg_ctx* c, uint16_t* dst, size_t pitch, int32_t dst_is_devic
         if ((st = start_streaming(c))) return st;
         return render_streaming(c, dst, pitch, dst_is_device, stats, retries);
       }
-      if ((st = ensure_raster_buffers(c))) return st;
+      if ((st = grown(c, ensure_raster_buffers(c)))) return st;
       c->graph_valid = false;
       continue;
     }

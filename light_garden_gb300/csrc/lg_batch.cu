@@ -163,8 +163,9 @@ lg_status run_batch(lg_ctx* c, std::vector<cudaEvent_t>& ev, uint32_t& retries) 
     if (nq > c->queue_cap) c->queue_cap = nq + nq / 2 + 1024;
     c->seg_cap = std::max(c->seg_cap, std::max(ns, c->queue_cap + c->n_overlay));
     if (nr > c->refs_cap) c->refs_cap = nr + nr / 4 + 4096;
-    if (c->refs_cap >= 0xffffffffull) return fail(c, LG_ERR_UNSUPPORTED, "more than 2^32 (segment, tile) pairs in one generation");
-    lg_status st = batch_buffers(c);
+    if (c->refs_cap >= 0xffffffffull)
+      return grown(c, fail(c, LG_ERR_UNSUPPORTED, "more than 2^32 (segment, tile) pairs in one generation"));
+    lg_status st = grown(c, batch_buffers(c));
     if (st) return st;
   }
   return fail(c, LG_ERR_OUT_OF_MEMORY, "batch buffers kept overflowing");
@@ -328,7 +329,7 @@ lg_status lg_batch_upload(lg_ctx* c, const lg_scene_desc* scenes, uint32_t k) {
   const uint64_t ring = std::min<uint64_t>(RING_SEGMENTS, free_b / 8 / (sizeof(lg_segment) + 2));
   c->seg_cap = std::max(c->seg_cap, std::max(c->queue_cap + c->n_overlay, std::max<uint64_t>(ring, c->seg_cap_hint)));
   c->refs_cap = std::max<uint64_t>(c->refs_cap, std::min<uint64_t>(4 * c->seg_cap + 4096, 0xfffffff0ull));
-  if ((st = batch_buffers(c))) return st;
+  if ((st = grown(c, batch_buffers(c)))) return st;
   // launch shapes: the multi-scene kernels read the object tables from global memory
   int occ = 0;
   if ((st = scan_grid(c, true))) return st;

@@ -102,6 +102,8 @@ namespace lgh {
 lg_status fail(lg_ctx* c, lg_status st, const std::string& msg);
 lg_status cuda_fail(lg_ctx* c, cudaError_t e, const char* what);
 lg_status ensure(lg_ctx* c, DevBuf& b, size_t bytes, const char* what);
+// Passes the status of a growth of the capacities on; after a failed one the context holds no scene.
+lg_status grown(lg_ctx* c, lg_status st);
 void release(DevBuf& b);
 lg_status sync_counters(lg_ctx* c);
 float elapsed(cudaEvent_t a, cudaEvent_t b);

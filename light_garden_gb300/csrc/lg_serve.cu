@@ -390,7 +390,7 @@ lg_status lg_serve_begin(lg_ctx* c, const lg_serve_opts* opts) {
   V->acc_pool.reset(px);
   V->res_pool.reset(px);
   lg_status st;
-  if ((st = serve_buffers(c))) { serve_free(c); return st; }
+  if ((st = grown(c, serve_buffers(c)))) { serve_free(c); return st; }
   if ((st = ensure(c, V->d_acc, px * 32, "accumulation pool"))) { serve_free(c); return st; }
   if ((st = ensure(c, V->d_res, px * 8, "result pool"))) { serve_free(c); return st; }
   if ((st = ensure(c, V->d_live, (size_t)V->max_slots * 4, "live counts"))) { serve_free(c); return st; }
@@ -580,7 +580,10 @@ lg_status lg_serve_step(lg_ctx* c, lg_serve_step_stats* stats) {
       return fail(c, LG_ERR_BUDGET, "a step needs more ray queue than the HBM budget allows");
     c->queue_cap = want;
     c->seg_cap = std::max(c->seg_cap, c->queue_cap + c->queue_cap / 4 + 4096);
-    if ((st = serve_buffers(c))) return st;
+    if ((st = grown(c, serve_buffers(c)))) {  // the rays in flight are lost with the buffers
+      serve_free(c);
+      return st;
+    }
     if ((st = serve_restart(c, V))) return st;
     S0.restarted = 1;
     if (stats) *stats = S0;
