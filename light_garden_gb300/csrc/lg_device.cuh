@@ -812,6 +812,14 @@ struct Class32 {
   float s;         // cubic: curve parameter of the root at ub
 };
 
+// What the FP32 errors, with room, may move a root by at most; beyond it the leaf is "unknown" (precise
+// solve).  A certain root bounds the search with a slack of 1e-4 (1 + t) for its own error and that of
+// the roots it is compared with, and the margins are five to thirteen times the error.  At a steep
+// crossing they are some 1e-5; a ray along a face crosses it where the distance to the face, over the
+// sine of the angle, puts it: without the limit, of the rays that met a rect's face at 1e-5 rad beside
+// discs that touch it one in eight found the wrong one of the two.
+constexpr float SHARP32 = 3e-4f;
+
 __device__ __forceinline__ void root32(float t, float tol, Class32& c, bool certain, int leaf, int face, float sv) {
   if (t < -TAU32) return;                     // certainly behind the origin
   if (certain && t > TAU32) {
@@ -922,14 +930,15 @@ __device__ __forceinline__ int cubic_roots32(const float* A, const float* Bp, fl
     if (fabsf(fp) < 1e-3f * sc) { unknown = true; return 0; }
     const float bx = ((c3x * u + c2x) * u + c1x) * u + c0x, by = ((c3y * u + c2y) * u + c1y) * u + c0y;
     const float dbx = (3.0f * c3x * u + 2.0f * c2x) * u + c1x, dby = (3.0f * c3y * u + 2.0f * c2y) * u + c1y;
+    const float tl = fabsf(dbx * dx + dby * dy) * (__fdividef(err, fabsf(fp)) + 1e-6f) +
+                     2e-6f * (fabsf(bx) + fabsf(by) + fabsf(ox) + fabsf(oy)) + 1e-6f;
+    if (!(tl < 2.0f * SHARP32)) { unknown = true; return 0; }  // (margins a dozen times the error here)
     // constant indices only, so that t, sv and cert stay in registers (n <= 2 here)
     const float tn = __fdividef((bx - ox) * dx + (by - oy) * dy, dd);
     const bool cn = u > 1e-4f && u < 1.0f - 1e-4f;
     if (n == 0) { t[0] = tn; sv[0] = u; cert[0] = cn; }
     else if (n == 1) { t[1] = tn; sv[1] = u; cert[1] = cn; }
     else { t[2] = tn; sv[2] = u; cert[2] = cn; }
-    const float tl = fabsf(dbx * dx + dby * dy) * (__fdividef(err, fabsf(fp)) + 1e-6f) +
-                     2e-6f * (fabsf(bx) + fabsf(by) + fabsf(ox) + fabsf(oy)) + 1e-6f;
     tol = fmaxf(tol, tl);
     ++n;
   }
@@ -1002,6 +1011,7 @@ __device__ __forceinline__ Ival32 leaf_ival32(uint32_t kind, const float* L, flo
     I.tol = (4e-6f * (wn + le) + e) * (1.0f + le * fabsf(inv)) + 1e-6f;
     const float ub = (1e-5f * (1.0f + (wn + le) / le) + e / le) * (1.0f + le * fabsf(inv));
     if (u < -ub || u > 1.0f + ub) return I;
+    if (I.tol > SHARP32) { I.unknown = true; return I; }
     I.t0 = t0;
     I.c0 = !(u < ub || u > 1.0f - ub);
     I.n = 1;
@@ -1014,8 +1024,9 @@ __device__ __forceinline__ Ival32 leaf_ival32(uint32_t kind, const float* L, flo
   const float H[2] = {L[4], L[5]};
   const float scale = fabsf(rx) + fabsf(ry) + H[0] + H[1];
   const float band = 2e-6f * scale + e + 1e-6f, delta = 4e-6f * scale + e + 1e-6f;
-  float tn = -INFINITY, tf = INFINITY, tn2 = -INFINITY, tf2 = INFINITY;
+  float tn = -INFINITY, tf = INFINITY;
   float in0 = -INFINITY, in1 = INFINITY, out0 = -INFINITY, out1 = INFINITY;
+  float en1 = INFINITY, ex0 = -INFINITY;  // where the first axis is certainly entered, the last one still certainly not left
   int fn = -1, ff = -1;
 #pragma unroll
   for (int ax = 0; ax < 2; ++ax) {
@@ -1026,32 +1037,31 @@ __device__ __forceinline__ Ival32 leaf_ival32(uint32_t kind, const float* L, flo
         I.out0 = -INFINITY; I.out1 = INFINITY;
         return I;
       }
+      en1 = -INFINITY; ex0 = INFINITY;
       continue;
     }
-    const float inv = __fdividef(1.0f, D[ax]);  // approximate reciprocal (2 ulp): far inside tol
+    const float inv = __fdividef(1.0f, D[ax]);  // approximate reciprocal (2 ulp): far inside the margin m
     const float ta = (-H[ax] - O[ax]) * inv, tb = (H[ax] - O[ax]) * inv;
     // entering through the -H face when D > 0 (outward normal -1), else the +H face
     const int f1 = 2 * ax + (D[ax] > 0.0f ? 0 : 1);
     const float t1 = fminf(ta, tb), t2 = fmaxf(ta, tb), m = delta * fabsf(inv);
     in0 = fmaxf(in0, t1 + m); in1 = fminf(in1, t2 - m);
     out0 = fmaxf(out0, t1 - m); out1 = fminf(out1, t2 + m);
-    if (t1 > tn) { tn2 = tn; tn = t1; fn = f1; } else { tn2 = fmaxf(tn2, t1); }
-    if (t2 < tf) { tf2 = tf; tf = t2; ff = f1 ^ 1; } else { tf2 = fminf(tf2, t2); }
+    en1 = fminf(en1, t1 + m); ex0 = fmaxf(ex0, t2 - m);
+    if (t1 > tn) { tn = t1; fn = f1; }
+    if (t2 < tf) { tf = t2; ff = f1 ^ 1; }
   }
   I.in0 = in0; I.in1 = in1; I.out0 = out0; I.out1 = out1;
-  const float tol = 4e-6f * (scale + fabsf(tn) + fabsf(tf)) + e + 1e-6f;
-  I.tol = tol;
-  if (tn > tf + tol) return I;
-  I.t0 = tn;
-  I.f0 = fn;
-  if (tn >= tf - tol) {  // corner graze
-    I.f0 = -1;
-    I.n = 1;
+  if (out0 > out1) return I;
+  // a corner met or grazed, or a face run along: hit, faces or places are decided in FP64
+  if (!(out0 > en1 && out1 < ex0 && in0 < in1 && fmaxf(in0 - out0, out1 - in1) < 2.0f * SHARP32)) {
+    I.unknown = true;
     return I;
   }
-  // a root whose face is ambiguous (the ray meets a corner) stays uncertain
-  I.c0 = !(tn - tn2 <= tol);
-  I.t1 = tf; I.c1 = !(tf2 - tf <= tol); I.f1 = ff;
+  I.tol = 4e-6f * (scale + fabsf(tn) + fabsf(tf)) + e + 1e-6f;
+  I.t0 = tn; I.f0 = fn;
+  I.t1 = tf; I.f1 = ff;
+  I.c0 = I.c1 = true;
   I.n = 2;
   return I;
 }
