@@ -416,8 +416,8 @@ __device__ __forceinline__ ChildRay child_x(const RayRec& r, const BounceX& v, V
                   0.0f, 0.0f, path, v.cflags, v.leaf, medium, (uint16_t)v.hit};
 }
 
-// A non-negative double as double-float (relative error 2^-48; below 2^-60 an absolute error
-// below 2^-83), on the integer pipe: a conversion each way would issue on the FP64 pipe.
+// A non-negative double as double-float (relative error 2^-48; below 2^-60 it is 0, above 2^60
+// infinite), on the integer pipe: a conversion each way would issue on the FP64 pipe.
 __device__ __forceinline__ df df_of(double x) {
   const int hi = __double2hiint(x), lo = __double2loint(x);
   const int e = ((hi >> 20) & 0x7ff) - 1023;
@@ -436,8 +436,13 @@ __device__ __forceinline__ df add_abs(df a, df b) {
 // (tracer.rs:454), from double-float copies of the indices and cosines: false unless the FP32
 // rounding of the FP64 formula's value is certain.  Every term n cos is within 2^-46 of itself,
 // so rs and rp are within 2^-44 and R within 2^-43 (|rs| + |rp| + R), the FP64 formula's own
-// rounding included; the bound below takes 2^-41.  It fails for about one visit in 10^4.  In FP64 the two
-// quotients, four products and their sums are half of a bounce's FP64 instructions.
+// rounding included; the bound below takes 2^-41.  A copy that df_of gave as 0 makes one term of either
+// quotient 0 (a and d, b and c, a and c or b and d), so that both are 1 or -1 and the sum's high part is
+// 1, whose zero mantissa is never certain; two such copies may give 0 / 0, and an infinite one NaN or
+// the same, and NaN compares false.  So FP64 decides all of these.  (The refracted cosine is 0 or at least
+// 2^-27, the root of a difference from 1: its conversion loses nothing.)  The test fails for about one
+// visit in 10^4.  In FP64 the two quotients, four products and their sums are half of a bounce's FP64
+// instructions.
 // A reflectance below 2^-26 (matched indices: a ray that leaves an object into the medium it
 // is already in) needs no exact value when dead says that the reflected colour is below the
 // cutoff whatever it is: the refracted share 1 - R is 1.
