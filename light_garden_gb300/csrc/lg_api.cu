@@ -877,10 +877,13 @@ void launch_sort(lg_ctx* c, const SceneDev& S, const TraceBufs& B, uint32_t g, u
 }
 
 // Whether one scene's generations visit their rays in sorted order.  Three launches and the keys
-// cost 10 us a generation and 4 % of a large one.  Frame time in queue order over sorted order at
-// 3 * 2^20 primaries x objects: 48 objects, CSG 0.99, plain 1.04, mixed 1.31; 128 objects 1.02, 1.03,
-// 1.29; 300 (10480 primaries) 0.99 to 1.01.  At four times that 64 CSG objects 1.06, mixed 1.35.
-// 30 CSG objects (no grid walk to keep together) never gain: 0.93 to 0.99.
+// cost 10 us a generation and 4 % of a large one.  The line lies where no kind of scene loses; mixed
+// shapes (ellipses, polygons) gain well below it.  Trace and accumulation in queue order over sorted
+// order, CSG / plain / mixed, geometric means of 6 scenes each: 48 objects 0.95 / 0.98 / 1.04 at
+// 0.75 * 2^20 primaries x objects, 0.98 / 1.02 / 1.13 at 1.5, 1.02 / 1.04 / 1.20 at 3; 128 objects 1.02 /
+// 1.02 / 1.18 at 2 and 1.06 / 1.06 / 1.28 at 3; 300 objects (8192 primaries) 1.02 / 1.02 / 1.07 at 2.3.  At 12
+// 64 CSG objects 1.06, mixed 1.35.  30 CSG objects (no grid walk to keep together) never gain: 0.93 to
+// 0.99.
 static bool sorted_frame(const lg_ctx* c) {
   return c->scan_walk && c->n_primary >= 16384 && c->n_primary * c->n_obj >= (3u << 20);
 }
