@@ -718,7 +718,7 @@ def main():
     ap.add_argument("--raster-variant", type=int, default=0, choices=[0, 1, 2],
                     help="kept for its numbering: every value runs the one tile raster")
     ap.add_argument("--culling", default="auto", choices=sorted(CULL),
-                    help="nearest-hit culling grid: auto (scenes of 96+ objects), off, on")
+                    help="nearest-hit culling grid: auto (scenes of 16 and more objects), off, on")
     ap.add_argument("--grid-density", type=float, default=0.0, help="culling grid cells per object (0: 2)")
     ap.add_argument("--count-case", action="store_true",
                     help="render one small frame of the workload and print its units of work (for ncu counts)")

@@ -470,11 +470,12 @@ lg_status lg_serve_end(lg_ctx* ctx);
  * (plug-ins whose host owns every allocation, real-time loops that must not take the
  * allocator's locks or risk the implicit synchronisation of cudaMalloc / cudaFree, code
  * under a fixed memory budget): clears `accum` to params->clear_color and rasterises the
- * n segments into it exactly like lg_accumulate_segments, on the calling thread's current
- * device and the given stream (NULL = default stream), without a context and without
- * allocating.  `segments` and `accum` must be device-accessible (accum: width*height*4
- * int64 for LG_ACCUM_FIXED64, float for LG_ACCUM_F32).  Canvas sides, accumulation mode
- * and blend state follow lg_params' rules (LG_ERR_INVALID_ARGUMENT / LG_ERR_UNSUPPORTED).
+ * n segments into it like lg_accumulate_segments (FIXED64: the same bits; F32: its tiles' sums
+ * are added in FP32, see lg_accum_mode), on the calling thread's current device and the given
+ * stream (NULL = default stream), without a context and without allocating.  `segments` and
+ * `accum` must be device-accessible (accum: width*height*4 int64 for LG_ACCUM_FIXED64, float
+ * for LG_ACCUM_F32).  Canvas sides, accumulation mode and blend state follow lg_params' rules
+ * (LG_ERR_INVALID_ARGUMENT / LG_ERR_UNSUPPORTED).
  * Binning scratch lives in one 32 MiB array per device, resident until the process exits;
  * limits per call: at most 4096 tiles of 32x32 pixels (e.g. 2048x2048) and 8,000,000
  * (segment, tile) pairs, else LG_ERR_BUDGET (and the image is not valid; the next call

@@ -5,10 +5,11 @@
 // loops that must not take the allocator's locks or trigger the implicit device
 // synchronisation cudaMalloc / cudaFree can cause, and code that runs against a fixed
 // device-memory budget.  lg_accumulate_segments_noalloc serves them: it rasterises the
-// caller's segments into the caller's accumulation image exactly like
-// lg_accumulate_segments, without a context, and keeps all of its binning scratch (tile
-// counts, offsets, cursors, work units and (segment, tile) references) in one file-scope
-// device array of fixed size, g_noalloc_scratch, instead of allocating.
+// caller's segments into the caller's accumulation image like lg_accumulate_segments (bit for
+// bit in fixed point; in F32 the caller's image is FP32, so the tiles' sums are added to it
+// there, where a context adds them in FP64), without a context, and keeps all of its binning
+// scratch (tile counts, offsets, cursors, work units and (segment, tile) references) in one
+// file-scope device array of fixed size, g_noalloc_scratch, instead of allocating.
 //
 // The array exists once per device that loads the library and stays resident until the
 // process exits.  Every call shares it: each call clears the parts that must start at

@@ -402,8 +402,9 @@ __global__ void __launch_bounds__(SCAN_WARPS * 32, CULL ? SCAN_CULL_BLOCKS : 4)
         // at the first cell entered beyond its bound thr.  The walk moves one cell in x or
         // in y at a time, so the cells of an object's range that it visits are consecutive:
         // an object whose range holds the previous cell was tested there and is skipped,
-        // and each object is tested at most once per ray.  Only the range's edge on the
-        // side the walk came from needs checking (step in +x: does it start left of ix?).
+        // and each object is tested at most once per ray.  A list entry carries a bit for each
+        // side on which the object's range goes on (CELL_*); the one of the side the walk came
+        // from says that the previous cell held the object.
         const uint32_t gny = G.ny;
         const float gx0 = G.x0, gy0 = G.y0, cw = G.cw, ch = G.ch, margin = G.margin;
         const uint32_t* cstart = S.cell_start + G.cell_base;
