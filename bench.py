@@ -62,14 +62,14 @@ REF_STRIDE = {"csg": 2048, "mid": 32}
 #   bounce: FP64 thread instructions per ray visit
 #   raster: shared-memory atomic warp instructions per accumulated pixel
 INST_PER_UNIT = {
-    "csg": {"scan": 538.7, "solve": 55.3, "bounce": 28.3, "raster": 0.4011},
-    "mid": {"scan": 203.4, "solve": 36.6, "bounce": 23.2, "raster": 0.3477},
+    "csg": {"scan": 595.0, "solve": 55.4, "bounce": 28.3, "raster": 0.4009},
+    "mid": {"scan": 215.9, "solve": 36.7, "bounce": 23.2, "raster": 0.3476},
 }
 # Warp instructions issued (smsp__inst_executed.sum) per unit of the same frames: the trace
 # stages against the SM's issue ceiling (4 schedulers x 1 warp instruction per cycle per SM).
 WARP_INST_PER_UNIT = {
-    "csg": {"scan": 164.3, "solve": 20.8, "bounce": 49.7},
-    "mid": {"scan": 92.0, "solve": 30.0, "bounce": 33.9},
+    "csg": {"scan": 165.9, "solve": 21.0, "bounce": 49.8},
+    "mid": {"scan": 92.8, "solve": 30.2, "bounce": 33.8},
 }
 
 
